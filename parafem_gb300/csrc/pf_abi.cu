@@ -6,7 +6,7 @@
 // p121.f90:86-104.  All device work is issued on the context's stream; every
 // entry point synchronises before it returns, as xx3's layer does
 // (src/programs/dev/xx3/cuda_helpers.cu:355-365).
-#include "pf_internal.h"
+#include "pf_fix.cuh"
 #include "pfgpu.h"
 
 #include <cmath>
@@ -104,6 +104,36 @@ static void drop_graph(Ctx &c)
     c.it_launches = 0;
 }
 
+int ctx_malloc(Ctx &c, void **p, size_t bytes)
+{
+    *p = nullptr;
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess && c.kmfix) {
+        cudaGetLastError();
+        drop_graph(c);
+        cudaStreamSynchronize(c.stream);
+        dfree(c.kmfix);
+        e = cudaMalloc(p, bytes);
+    }
+    if (e == cudaSuccess) return 0;
+    cudaGetLastError();
+    *p = nullptr;
+    return 1;
+}
+
+int ensure_km32(Ctx &c)
+{
+    if (c.km32_ok) return 0;
+    const size_t bytes = (size_t)c.nels * 3600 * sizeof(float);
+    if (!c.km32 && ctx_malloc(c, (void **)&c.km32, bytes)) {
+        set_error("cannot allocate FP32 storkm (%zu bytes)", bytes);
+        return 1;
+    }
+    if (launch_cast_km32(c)) return 1;
+    c.km32_ok = true;
+    return 0;
+}
+
 static void free_mesh(Ctx &c)
 {
     drop_graph(c);
@@ -111,8 +141,9 @@ static void free_mesh(Ctx &c)
     dfree(c.conn); dfree(c.node_ptr); dfree(c.node_list); dfree(c.slot_eq); dfree(c.eq_slot);
     dfree(c.freemask); dfree(c.coord); dfree(c.mat_e); dfree(c.mat_v); dfree(c.km64); dfree(c.km32);
     dfree(c.km32p); dfree(c.skm64); dfree(c.skm32); dfree(c.fstore); dfree(c.fscale); dfree(c.psplit);
-    dfree(c.km16p);
+    dfree(c.km16p); dfree(c.kmfix); dfree(c.skmfix);
     c.km16_ok = false;
+    c.km32_ok = false;
     c.mr_ok = false;
     c.shared = false;
     c.kind = KIND_SOLID20;
@@ -379,8 +410,8 @@ try {
     if (c->nsm < 1) c->nsm = 1;
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaMalloc((void **)&c->st, sizeof(PcgState)) != cudaSuccess ||
-        cudaMalloc((void **)&c->kerr, sizeof(int)) != cudaSuccess ||
-        cudaMemset(c->kerr, 0, sizeof(int)) != cudaSuccess ||
+        cudaMalloc((void **)&c->kerr, 2 * sizeof(int)) != cudaSuccess ||
+        cudaMemset(c->kerr, 0, 2 * sizeof(int)) != cudaSuccess ||
         cudaMalloc((void **)&c->gbar, sizeof(unsigned long long) * kPersistSlots * kBarWords) != cudaSuccess ||
         cudaMemset(c->gbar, 0, sizeof(unsigned long long) * kPersistSlots * kBarWords) != cudaSuccess ||
         cudaMallocHost((void **)&c->hst, sizeof(PcgState)) != cudaSuccess) {
@@ -671,9 +702,9 @@ try {
     return pf::host_exception("pf_set_material");
 }
 
-// The per-element storkm arrays (FP64, FP32, packed FP32), allocated on the
-// first pf_form_storkm / pf_set_storkm: a context that only ever uses a
-// shared element matrix never holds them.
+// The per-element storkm arrays (FP64, packed FP32, fixed-point records),
+// allocated on the first pf_form_storkm / pf_set_storkm: a context that only
+// ever uses a shared element matrix never holds them.
 static int ensure_storkm(Ctx &c)
 {
     const size_t ne = (size_t)c.nels;
@@ -683,12 +714,30 @@ static int ensure_storkm(Ctx &c)
         return 0;
     }
     if (!c.km64 && dalloc(&c.km64, ne * 3600, "FP64 storkm")) return 1;
-    if (!c.km32 && dalloc(&c.km32, ne * 3600, "FP32 storkm")) return 1;
     if (!c.km32p && dalloc(&c.km32p, ne * 1832, "packed FP32 storkm")) return 1;
+    if (!c.kmfix && cudaMalloc((void **)&c.kmfix, ne * fx::kRecBytes) != cudaSuccess) {
+        cudaGetLastError();   // FP64 products by FP64 FMA instead
+        c.kmfix = nullptr;
+    }
+    c.km32_ok = false;   // cast again on the next full-FP32 use
     c.km16_ok = false;   // repacked on the next FP16 use
     c.mr_ok = false;     // and the tensor-core block records on the next block product
     c.shared = false;
     drop_graph(c);
+    return 0;
+}
+
+// The packed forms of the FP64 storkm, in one pass over it.  Matrices that
+// do not fit the fixed-point records (not symmetric to the last bit, above
+// all) leave the context without them.
+static int pack_storkm(Ctx &c)
+{
+    CK(cudaMemsetAsync(c.kerr + 1, 0, sizeof(int), c.stream));
+    TRY(launch_pack_storkm(c, c.nels, c.km64, c.km32p, c.kmfix, c.kerr + 1));
+    int bad = 0;
+    CK(cudaMemcpyAsync(&bad, c.kerr + 1, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    TRY(sync(c));
+    if (bad) dfree(c.kmfix);
     return 0;
 }
 
@@ -712,15 +761,15 @@ try {
     const bool exact = (*flags & PF_FORM_EXACT_WEIGHTS) != 0;
     TRY(ensure_storkm(c));
     if (c.kind == KIND_SOLID8) {   // FP64 storkm, the diagonal; fixed freedoms cleared
-        TRY(launch_form_storkm(c, *nip, exact, false));
+        TRY(launch_form_storkm(c, *nip, exact));
         TRY(launch_assemble_diag(c));
         CK(cudaMemsetAsync(c.fstore, 0, (size_t)c.nslots * sizeof(double), c.stream));
         TRY(sync(c));
         c.have_km = true;
         return PF_SUCCESS;
     }
-    TRY(launch_form_storkm(c, *nip, exact, true));
-    TRY(launch_pack_sym32(c));
+    TRY(launch_form_storkm(c, *nip, exact));
+    TRY(pack_storkm(c));
     TRY(launch_assemble_diag(c));
     TRY(autotune_sym32(c, c.x));
     TRY(sync(c));
@@ -743,8 +792,8 @@ try {
     TRY(ensure_storkm(c));
     CK(cudaMemcpyAsync(c.km64, storkm, (size_t)c.nels * 3600 * sizeof(double), cudaMemcpyHostToDevice,
                        c.stream));
-    TRY(launch_cast_km32(c));
-    TRY(launch_pack_sym32(c));
+    TRY(launch_extract_ediag(c));
+    TRY(pack_storkm(c));
     TRY(launch_assemble_diag(c));
     TRY(autotune_sym32(c, c.x));
     TRY(sync(c));
@@ -778,7 +827,7 @@ try {
     int bad = launch_sample(c.stream, *nip, (*flags & PF_FORM_EXACT_WEIGHTS) != 0, buf);
     if (!bad)
         bad = launch_form_storkm_raw(c.stream, c.nsm, 1, *nip, buf, c.coord + e * 60, c.mat_e + m, c.mat_v + m, 1,
-                                     buf + 108, nullptr, buf + 108 + 3600);
+                                     buf + 108, buf + 108 + 3600);
     if (!bad) c.launches += 2;
     cudaError_t ec = bad ? cudaSuccess : cudaMemcpyAsync(km, buf + 108, 3600 * sizeof(double), cudaMemcpyDeviceToHost,
                                                          c.stream);
@@ -828,8 +877,15 @@ try {
         }
     CK(cudaMemcpyAsync(c.skm64, km, 3600 * sizeof(double), cudaMemcpyHostToDevice, c.stream));
     CK(cudaMemcpyAsync(c.skm32, k32.data(), (3600 + 192) * sizeof(float), cudaMemcpyHostToDevice, c.stream));
-    c.shared = true;
+    if (!c.skmfix && dalloc(&c.skmfix, fx::kRecBytes, "shared km")) return PF_FAILURE;
+    CK(cudaMemsetAsync(c.kerr + 1, 0, sizeof(int), c.stream));
+    TRY(launch_pack_storkm(c, 1, c.skm64, nullptr, c.skmfix, c.kerr + 1));
+    int bad = 0;
+    CK(cudaMemcpyAsync(&bad, c.kerr + 1, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    TRY(sync(c));
     drop_graph(c);
+    if (bad) dfree(c.skmfix);
+    c.shared = true;
     TRY(launch_shared_ediag(c));
     TRY(launch_assemble_diag(c));
     TRY(sync(c));
@@ -891,6 +947,7 @@ try {
         return PF_FAILURE;
     }
     if (*prec == 16) TRY(ensure_km16(c));
+    if (*prec == 31 && !c.shared) TRY(ensure_km32(c));
     CK(cudaMemcpyAsync(c.eqbuf, p, (size_t)c.neq * sizeof(double), cudaMemcpyHostToDevice, c.stream));
     TRY(launch_eq_to_slot(c, c.eqbuf, c.rres));
     TRY(launch_matvec(c, *prec, c.rres, c.u));
@@ -1066,6 +1123,7 @@ try {
         return PF_FAILURE;
     }
     if (*prec == 16) TRY(ensure_km16(c));
+    if (*prec == 31 && !c.shared) TRY(ensure_km32(c));
     const int n = *steps;
     // never-converging run on the resident load vector (tol 0, no limit hit)
     TRY(launch_pcg_init(c, c.f, c.c, STOP_RELRES, 0.0, n + 1));

@@ -1040,7 +1040,7 @@ try {
         B.gp_nip = nip;
     }
     if (launch_form_storkm_raw(B.stream, B.nsm, nels, nip, B.gp, B.coord + (size_t)el0 * 60, B.mat_e + el0,
-                               B.mat_v + el0, nmat, B.km64 + (size_t)el0 * 3600, nullptr,
+                               B.mat_v + el0, nmat, B.km64 + (size_t)el0 * 3600,
                                B.ediag + (size_t)el0 * 60))
         return PF_FAILURE;
     B.launches++;

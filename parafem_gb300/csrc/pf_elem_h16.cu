@@ -299,8 +299,7 @@ int ensure_km16(Ctx &c)
         return 1;
     }
     if (!c.km16p) {
-        if (cudaMalloc((void **)&c.km16p, (size_t)c.nels * kH16Bytes) != cudaSuccess) {
-            cudaGetLastError();
+        if (ctx_malloc(c, (void **)&c.km16p, (size_t)c.nels * kH16Bytes)) {
             set_error("FP16 products: cannot allocate %zu bytes of packed storkm", (size_t)c.nels * kH16Bytes);
             return 1;
         }

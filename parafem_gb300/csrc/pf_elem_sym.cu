@@ -328,18 +328,6 @@ int launch_pack_sym32_raw(cudaStream_t stream, int nsm, int nels, const double *
     return 0;
 }
 
-int launch_pack_sym32(Ctx &c)
-{
-    k_pack_sym32<<<c.nsm * 8, 256, 0, c.stream>>>(c.nels, c.km64, c.km32p);
-    c.launches++;
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) {
-        set_error("k_pack_sym32: launch failed: %s", cudaGetErrorString(e));
-        return 1;
-    }
-    return 0;
-}
-
 int launch_elem_sym32(Ctx &c, const double *p, const PcgState *st)
 {
     return launch_sym_index(c, c.sym_cfg, p, st);

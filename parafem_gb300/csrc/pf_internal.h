@@ -74,9 +74,14 @@ struct Ctx {
     double *mat_e = nullptr, *mat_v = nullptr;
 
     double *km64 = nullptr;     // [nels*3600] storkm(60,60,e)
-    float *km32 = nullptr;      // [nels*3600] full FP32 copy
+    float *km32 = nullptr;      // [nels*3600] full FP32 copy, cast on first use (ensure_km32)
+    bool km32_ok = false;       // km32 holds the current storkm
+    unsigned char *kmfix = nullptr;   // [nels] fixed-point records (pf_fix.cuh) for the FP64 products, or null:
+                                      //   storkm not symmetric, or no device memory for them
     float *km32p = nullptr;     // [nels*1832] packed symmetric storkm (packed_off), FP32
-    int *kerr = nullptr;        // device error word: 2 = a bulk-copy wait timed out, 3 = a grid barrier did
+    int *kerr = nullptr;        // device error word: 2 = a bulk-copy wait timed out, 3 = a grid barrier did;
+                                //   kerr[1]: set by k_pack_storkm when a matrix does not fit its record
+    bool fix_attr = false;      // shared-memory attribute of the fixed-point kernel set
     bool have_km = false;
 
     double *ediag = nullptr;    // [nels*60] element diagonals
@@ -103,6 +108,7 @@ struct Ctx {
     bool shared = false;
     double *skm64 = nullptr;    // [3600] column-major
     float *skm32 = nullptr;     // [3600 + 192]: km, then the direction sums of its rows ([3][64])
+    unsigned char *skmfix = nullptr;   // km's fixed-point record, or null (km not symmetric)
     bool shared_attr = false;   // shared-memory attribute of the tensor-core kernel set
     float2 *psplit = nullptr;   // [nslots] FP32 high and low parts of p (shared km): written with p
     uint32_t *km16p = nullptr;  // [nels*916] packed FP16 storkm (pf_elem_h16.cu), packed on first use
@@ -137,12 +143,21 @@ struct Ctx {
 };
 
 // Kernel launchers (pf_kernels.cu).  All run on ctx.stream and count launches.
-int launch_form_storkm(Ctx &c, int nip, bool exact_weights, bool keep32);
+int launch_form_storkm(Ctx &c, int nip, bool exact_weights);
 int launch_sample(cudaStream_t stream, int nip, bool exact_weights, double *gp);
 int launch_form_storkm_raw(cudaStream_t stream, int nsm, int nels, int nip, const double *gp,
                            const double *coord, const double *me, const double *mv, int nmat, double *km64,
-                           float *km32, double *ediag);
+                           double *ediag);
 int launch_cast_km32(Ctx &c);
+int launch_extract_ediag(Ctx &c);
+// cudaMalloc for a context; when it fails, the fixed-point records (which
+// the FP64 products can do without) are given back and it is tried again
+int ctx_malloc(Ctx &c, void **p, size_t bytes);
+int ensure_km32(Ctx &c);   // the full FP32 storkm, if storkm changed; outside stream capture
+// pf_fix.cu: the packed forms of nels FP64 element matrices (kp or rec may be null), FP64 products from the records
+int launch_pack_storkm(Ctx &c, int nels, const double *km, float *kp, unsigned char *rec, int *bad);
+int launch_elem_fix(Ctx &c, const double *p, const PcgState *st);
+int launch_elem_shared_fix(Ctx &c, const double *p, const PcgState *st);
 int launch_assemble_diag(Ctx &c);
 int launch_eq_to_slot(Ctx &c, const double *eq, double *slot);
 int launch_slot_to_eq(Ctx &c, const double *slot, double *eq);
@@ -183,7 +198,6 @@ int sym16_prepare();   // shared-memory attribute of the mapped FP16 launch (onc
 int launch_elem_sym16_mapped(cudaStream_t stream, int nsm, int n, const uint32_t *kh, const int *conn,
                              const double *p, float *ut, int *err, const int *emap);
 int launch_pack_sym16_raw(cudaStream_t stream, int nsm, int nels, const double *km, uint32_t *kh);
-int launch_pack_sym32(Ctx &c);
 void multi_release(Ctx &c);   // frees the context's block-solve buffers (pf_multi.cu)
 int launch_elem_sym32(Ctx &c, const double *p, const PcgState *st);
 int sym32_prepare();   // shared-memory attribute of the mapped launch (once per device, outside capture)

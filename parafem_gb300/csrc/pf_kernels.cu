@@ -8,7 +8,7 @@
 //   storkm(60,60,e) keeps p121's column-major element blocks.
 // Reductions are deterministic: fixed per-thread assignment, xor-shuffle
 // trees, per-block partials summed in a fixed order by the consumer kernel.
-#include "pf_device.cuh"
+#include "pf_fix.cuh"
 #include "pf_tc.cuh"
 
 #include <cmath>
@@ -92,7 +92,7 @@ template <int NOD>
 __global__ void __launch_bounds__(kFormThreads)
 k_form_storkm(int nels, int nip, const double *__restrict__ gp, const double *__restrict__ coord,
               const double *__restrict__ me, const double *__restrict__ mv, int nmat,
-              double *__restrict__ km64, float *__restrict__ km32, double *__restrict__ ediag)
+              double *__restrict__ km64, double *__restrict__ ediag)
 {
     constexpr int NE = 3 * NOD, NP = NOD * (NOD + 1) / 2;
     __shared__ double s_der[27][NE];   // der(3,NOD) at each point
@@ -164,22 +164,20 @@ k_form_storkm(int nels, int nip, const double *__restrict__ gp, const double *__
                         K[i + 3 * j] = D12 * M[i + 3 * j] + D44 * M[j + 3 * i];
                     }
                 }
-            double *ke = km64 ? km64 + (size_t)e * NE * NE : nullptr;
-            float *kf = km32 ? km32 + (size_t)e * NE * NE : nullptr;
+            if (pa == pb) {   // M_aa is symmetric up to the rounding of its sums: storkm is so to the last bit
+                K[1] = K[3];
+                K[2] = K[6];
+                K[5] = K[7];
+            }
+            double *ke = km64 + (size_t)e * NE * NE;
 #pragma unroll
             for (int j = 0; j < 3; ++j)
 #pragma unroll
                 for (int i = 0; i < 3; ++i) {
                     const double v = K[i + 3 * j];
                     const int ab = (3 * pb + j) * NE + 3 * pa + i, ba = (3 * pa + i) * NE + 3 * pb + j;
-                    if (ke) {
-                        ke[ab] = v;
-                        if (pa != pb) ke[ba] = v;
-                    }
-                    if (kf) {
-                        kf[ab] = (float)v;
-                        if (pa != pb) kf[ba] = (float)v;
-                    }
+                    ke[ab] = v;
+                    if (pa != pb) ke[ba] = v;
                     if (pa == pb && i == j) ediag[(size_t)e * NE + 3 * pa + i] = v;
                 }
         }
@@ -569,6 +567,7 @@ k_pcg_finish(PcgState *__restrict__ st, const double *__restrict__ part, int G)
 struct PersistArgs {
     int nels, nn, ns, G, Gs, niters;
     const double *km64;   // FP64 storkm (ELEM64)
+    const unsigned char *rec;   // its fixed-point records, or null
     const int *conn;
     void *ut;             // element results
     const int *node_ptr, *node_list;
@@ -596,8 +595,13 @@ __global__ void __launch_bounds__(256, MINB) k_pcg_persistent(PersistArgs a)
         if (ELEM64) {
             const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
             const int nw = (gridDim.x * blockDim.x) >> 5;
-            for (int e = warp; e < a.nels; e += nw)
-                elem_warp<double, true>(e, lane, a.km64, a.conn, a.p, (double *)a.ut);
+            __shared__ int4 pq[8][60];
+            for (int e = warp; e < a.nels; e += nw) {
+                if (a.rec)
+                    fx::elem_warp<false>((size_t)e, lane, a.rec, a.conn, a.p, (double *)a.ut, pq[threadIdx.x >> 5]);
+                else
+                    elem_warp<double, true>(e, lane, a.km64, a.conn, a.p, (double *)a.ut);
+            }
             if (!grid_barrier(a.bar, a.kerr, a.st)) return;
         }
         for (int vb = blockIdx.x; vb < a.Gs; vb += gridDim.x)
@@ -799,7 +803,7 @@ static int grid_for(const Ctx &c, long long work, int per_block, int max_per_sm)
     return (int)g;
 }
 
-int launch_form_storkm(Ctx &c, int nip, bool exact_weights, bool keep32)
+int launch_form_storkm(Ctx &c, int nip, bool exact_weights)
 {
     double *gp = nullptr;
     if (cudaMallocAsync(&gp, sizeof(double) * 4 * 27, c.stream) != cudaSuccess) {
@@ -811,10 +815,10 @@ int launch_form_storkm(Ctx &c, int nip, bool exact_weights, bool keep32)
     const int grid = c.nels < c.nsm * 16 ? c.nels : c.nsm * 16;
     if (c.kind == KIND_SOLID8)
         k_form_storkm<8><<<grid, kFormThreads, 0, c.stream>>>(c.nels, nip, gp, c.coord, c.mat_e, c.mat_v, c.nmat,
-                                                              c.km64, nullptr, c.ediag);
+                                                              c.km64, c.ediag);
     else
         k_form_storkm<20><<<grid, kFormThreads, 0, c.stream>>>(c.nels, nip, gp, c.coord, c.mat_e, c.mat_v, c.nmat,
-                                                               c.km64, keep32 ? c.km32 : nullptr, c.ediag);
+                                                               c.km64, c.ediag);
     if (check_launch(c, "k_form_storkm")) return 1;
     cudaFreeAsync(gp, c.stream);
     return 0;
@@ -833,10 +837,10 @@ int launch_sample(cudaStream_t stream, int nip, bool exact_weights, double *gp)
 
 int launch_form_storkm_raw(cudaStream_t stream, int nsm, int nels, int nip, const double *gp,
                            const double *coord, const double *me, const double *mv, int nmat, double *km64,
-                           float *km32, double *ediag)
+                           double *ediag)
 {
     const int grid = nels < nsm * 16 ? nels : nsm * 16;
-    k_form_storkm<20><<<grid, kFormThreads, 0, stream>>>(nels, nip, gp, coord, me, mv, nmat, km64, km32, ediag);
+    k_form_storkm<20><<<grid, kFormThreads, 0, stream>>>(nels, nip, gp, coord, me, mv, nmat, km64, ediag);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_error("k_form_storkm: launch failed: %s", cudaGetErrorString(e));
@@ -849,7 +853,11 @@ int launch_cast_km32(Ctx &c)
 {
     const size_t n = (size_t)c.nels * 3600;
     k_cast_km32<<<c.nsm * 8, 256, 0, c.stream>>>(n, c.km64, c.km32);
-    if (check_launch(c, "k_cast_km32")) return 1;
+    return check_launch(c, "k_cast_km32");
+}
+
+int launch_extract_ediag(Ctx &c)
+{
     k_extract_ediag<<<c.nsm * 8, 256, 0, c.stream>>>(c.nels, c.km64, c.ediag);
     return check_launch(c, "k_extract_ediag");
 }
@@ -874,21 +882,28 @@ int launch_slot_to_eq(Ctx &c, const double *slot, double *eq)
     return check_launch(c, "k_slot_to_eq");
 }
 
-int launch_elem(Ctx &c, int prec, const double *p)
+// Element products into c.utemp; st: PCG state whose stop flag turns the
+// launch into a no-op (nullptr outside a PCG run).  The FP64 products of
+// 20-node elements are formed in fixed point where the mesh has records
+// (c.kmfix), and by FP64 FMA where storkm is not symmetric or the records
+// found no memory.
+static int launch_products(Ctx &c, int prec, const double *p, const PcgState *st)
 {
-    if (c.kind == KIND_SCALAR8) return launch_elem8(c, p, c.st);
-    if (c.kind == KIND_SOLID8) return launch_elem24(c, p, c.st);
-    if (c.shared) return launch_elem_shared(c, prec, p, c.st);
-    if (prec == PREC_FP32_SYM) return launch_elem_sym32(c, p, c.st);
-    if (prec == PREC_FP16_SYM) return launch_elem_sym16(c, p, c.st);
+    if (c.kind == KIND_SCALAR8) return launch_elem8(c, p, st);
+    if (c.kind == KIND_SOLID8) return launch_elem24(c, p, st);
+    if (c.shared) return launch_elem_shared(c, prec, p, st);
+    if (prec == PREC_FP32_SYM) return launch_elem_sym32(c, p, st);
+    if (prec == PREC_FP16_SYM) return launch_elem_sym16(c, p, st);
+    if (prec == PREC_FP64 && c.kmfix) return launch_elem_fix(c, p, st);
     const int grid = grid_for(c, c.nels, 8, 8);
-    if (prec == PREC_FP32_FULL) {
-        k_elem<float, true><<<grid, 256, 0, c.stream>>>(c.nels, c.km32, c.conn, p, (float *)c.utemp, c.st);
-    } else {
-        k_elem<double, true><<<grid, 256, 0, c.stream>>>(c.nels, c.km64, c.conn, p, (double *)c.utemp, c.st);
-    }
+    if (prec == PREC_FP32_FULL)
+        k_elem<float, true><<<grid, 256, 0, c.stream>>>(c.nels, c.km32, c.conn, p, (float *)c.utemp, st);
+    else
+        k_elem<double, true><<<grid, 256, 0, c.stream>>>(c.nels, c.km64, c.conn, p, (double *)c.utemp, st);
     return check_launch(c, "k_elem");
 }
+
+int launch_elem(Ctx &c, int prec, const double *p) { return launch_products(c, prec, p, c.st); }
 
 int launch_scatter(Ctx &c, int prec, int mode, const double *pf, double *out)
 {
@@ -916,28 +931,9 @@ int launch_scatter(Ctx &c, int prec, int mode, const double *pf, double *out)
 // u = K p outside a PCG run (state-independent).
 int launch_matvec(Ctx &c, int prec, const double *p, double *u)
 {
-    if (c.kind == KIND_SCALAR8) {
-        if (launch_elem8(c, p, nullptr)) return 1;
-        return launch_scatter1(c, 0, p, p, u, nullptr);
-    }
-    if (c.kind == KIND_SOLID8) {
-        if (launch_elem24(c, p, nullptr)) return 1;
-        return launch_scatter3_fixed(c, p, u, nullptr);
-    }
-    const int grid = grid_for(c, c.nels, 8, 8);
-    if (c.shared) {
-        if (launch_elem_shared(c, prec, p, nullptr)) return 1;
-    } else if (prec == PREC_FP32_SYM) {
-        if (launch_elem_sym32(c, p, nullptr)) return 1;
-    } else if (prec == PREC_FP16_SYM) {
-        if (launch_elem_sym16(c, p, nullptr)) return 1;
-    } else {
-        if (prec == PREC_FP32_FULL)
-            k_elem<float, true><<<grid, 256, 0, c.stream>>>(c.nels, c.km32, c.conn, p, (float *)c.utemp, nullptr);
-        else
-            k_elem<double, true><<<grid, 256, 0, c.stream>>>(c.nels, c.km64, c.conn, p, (double *)c.utemp, nullptr);
-        if (check_launch(c, "k_elem")) return 1;
-    }
+    if (launch_products(c, prec, p, nullptr)) return 1;
+    if (c.kind == KIND_SCALAR8) return launch_scatter1(c, 0, p, p, u, nullptr);
+    if (c.kind == KIND_SOLID8) return launch_scatter3_fixed(c, p, u, nullptr);
     if (prec != PREC_FP64)
         k_scatter<float, 0><<<c.Gs, 256, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, (const float *)c.utemp,
                                                         c.freemask, p, u, c.part_s, nullptr);
@@ -957,20 +953,9 @@ int launch_scatter_add64(Ctx &c, double *out)
 
 int launch_residual(Ctx &c, const double *f, const double *x, double *rres)
 {
-    if (c.kind == KIND_SCALAR8) {
-        if (launch_elem8(c, x, nullptr)) return 1;
-        return launch_scatter1(c, 1, x, f, rres, nullptr);
-    }
-    const int grid = grid_for(c, c.nels, 8, 8);
-    if (c.kind == KIND_SOLID8) {
-        // f - K x with the plain K, as p122 forms r = loads - K x (p122.f90:142-146)
-        if (launch_elem24(c, x, nullptr)) return 1;
-    } else if (c.shared) {
-        if (launch_elem_shared(c, PREC_FP64, x, nullptr)) return 1;
-    } else {
-        k_elem<double, true><<<grid, 256, 0, c.stream>>>(c.nels, c.km64, c.conn, x, (double *)c.utemp, nullptr);
-        if (check_launch(c, "k_elem")) return 1;
-    }
+    // f - K x with the plain K (p122.f90:142-146 forms r = loads - K x so)
+    if (launch_products(c, PREC_FP64, x, nullptr)) return 1;
+    if (c.kind == KIND_SCALAR8) return launch_scatter1(c, 1, x, f, rres, nullptr);
     k_scatter<double, 1><<<c.Gs, 256, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, (const double *)c.utemp,
                                                      c.freemask, f, rres, c.part_s, nullptr);
     return check_launch(c, "k_scatter");
@@ -1032,7 +1017,7 @@ static int persist_grid(const Ctx &c)
 template <typename UT, bool ELEM64, bool CHECON>
 static int launch_persist_t(Ctx &c, double *xsol, int niters)
 {
-    constexpr int MINB = 4, PF = sizeof(UT) == 8 ? 4 : 8;
+    constexpr int MINB = ELEM64 ? 2 : 4, PF = sizeof(UT) == 8 ? 4 : 8;   // the products hold 100-odd registers
     const int idx = (ELEM64 ? 4 : 0) + (sizeof(UT) == 4 ? 2 : 0) + (CHECON ? 1 : 0);
     if (c.pk_grid[idx] == 0) c.pk_grid[idx] = persist_grid<UT, ELEM64, CHECON, MINB, PF>(c);
     const int grid = c.pk_grid[idx];
@@ -1042,7 +1027,7 @@ static int launch_persist_t(Ctx &c, double *xsol, int niters)
     }
     PersistArgs a;
     a.nels = c.nels; a.nn = c.nn; a.ns = c.nslots; a.G = c.G; a.Gs = c.Gs; a.niters = niters;
-    a.km64 = c.km64; a.conn = c.conn; a.ut = c.utemp; a.node_ptr = c.node_ptr; a.node_list = c.node_list;
+    a.km64 = c.km64; a.rec = c.kmfix; a.conn = c.conn; a.ut = c.utemp; a.node_ptr = c.node_ptr; a.node_list = c.node_list;
     a.fm = c.freemask; a.x = xsol; a.r = c.r; a.d = c.d; a.p = c.p; a.u = c.u; a.dinv = c.dinv;
     a.part_s = c.part_s; a.part_u = c.part_u; a.psplit = c.shared ? c.psplit : nullptr; a.st = c.st;
     a.bar = c.gbar + (size_t)idx * kBarWords; a.kerr = c.kerr;

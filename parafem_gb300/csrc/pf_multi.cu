@@ -1236,7 +1236,7 @@ static int mr_alloc(Ctx &c, int k)
         mb_free(m);
         c.mr_ok = false;
     }
-    if (!m.rec && cudaMalloc((void **)&m.rec, (size_t)c.nels * kRecBytes) != cudaSuccess) {
+    if (!m.rec && ctx_malloc(c, (void **)&m.rec, (size_t)c.nels * kRecBytes)) {
         set_error("pf_solve_multi: cannot allocate the tensor-core element records (%zu bytes)",
                   (size_t)c.nels * kRecBytes);
         return 1;
@@ -1248,14 +1248,14 @@ static int mr_alloc(Ctx &c, int k)
     const size_t parts = (size_t)(c.Gs > c.G ? c.Gs : c.G) * k * 4 + 64;
     double **v[] = {&m.F, &m.X, &m.R, &m.D, &m.P, &m.U, &m.RR};
     for (double **q : v)
-        if (cudaMalloc((void **)q, n * 8) != cudaSuccess) goto fail;
-    if (cudaMalloc((void **)&m.eq, (size_t)(c.neq > 0 ? c.neq : 1) * k * 8) != cudaSuccess) goto fail;
-    if (cudaMalloc((void **)&m.ut32, (size_t)c.nels * 60 * k * 4) != cudaSuccess) goto fail;
-    if (cudaMalloc((void **)&m.Ps, n * 8) != cudaSuccess) goto fail;
-    if (cudaMalloc((void **)&m.ut64, (size_t)c.nels * 60 * k * 8) != cudaSuccess) goto fail;
-    if (cudaMalloc((void **)&m.part, parts * 8) != cudaSuccess) goto fail;
-    if (cudaMalloc((void **)&m.sums, kMaxK * 8) != cudaSuccess) goto fail;
-    if (cudaMalloc((void **)&m.st, sizeof(MState)) != cudaSuccess) goto fail;
+        if (ctx_malloc(c, (void **)q, n * 8)) goto fail;
+    if (ctx_malloc(c, (void **)&m.eq, (size_t)(c.neq > 0 ? c.neq : 1) * k * 8)) goto fail;
+    if (ctx_malloc(c, (void **)&m.ut32, (size_t)c.nels * 60 * k * 4)) goto fail;
+    if (ctx_malloc(c, (void **)&m.Ps, n * 8)) goto fail;
+    if (ctx_malloc(c, (void **)&m.ut64, (size_t)c.nels * 60 * k * 8)) goto fail;
+    if (ctx_malloc(c, (void **)&m.part, parts * 8)) goto fail;
+    if (ctx_malloc(c, (void **)&m.sums, kMaxK * 8)) goto fail;
+    if (ctx_malloc(c, (void **)&m.st, sizeof(MState))) goto fail;
     if (cudaMallocHost((void **)&m.hst, sizeof(MState)) != cudaSuccess) goto fail;
     m.ns = c.nslots;
     m.k = k;
@@ -1377,6 +1377,7 @@ try {
     MCK(cudaMemcpyAsync(m.eq, r, (size_t)c.neq * k * 8, cudaMemcpyHostToDevice, c.stream));
     k_mr_eq_to_slot<<<c.nsm * 8, 256, 0, c.stream>>>(c.nslots, k, c.slot_eq, c.neq, m.eq, m.F);
     if (mr_launched(c, "k_mr_eq_to_slot")) return PF_FAILURE;
+    if (*prec == 32 && ensure_km32(c)) return PF_FAILURE;
     if (*prec == 16) {
         // the autotuner times products of the initial search directions
         k_mr_init<<<G, T, 0, c.stream>>>(c.nslots, k, m.F, c.dinv, m.X, m.R, m.D, m.P, m.Ps, m.part, G);
@@ -1509,6 +1510,7 @@ try {
     MCK(cudaMemcpyAsync(m.eq, p, (size_t)c.neq * k * 8, cudaMemcpyHostToDevice, c.stream));
     k_mr_eq_to_slot<<<c.nsm * 8, 256, 0, c.stream>>>(c.nslots, k, c.slot_eq, c.neq, m.eq, m.P);
     if (mr_launched(c, "k_mr_eq_to_slot")) return PF_FAILURE;
+    if (*prec == 32 && ensure_km32(c)) return PF_FAILURE;
     if (*prec == 16) {
         k_mr_psplit<<<c.nsm * 8, 256, 0, c.stream>>>((size_t)c.nslots * k, m.P, m.Ps);
         if (mr_launched(c, "k_mr_psplit")) return PF_FAILURE;

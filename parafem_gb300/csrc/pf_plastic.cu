@@ -325,6 +325,7 @@ using namespace pf;
             return PF_FAILURE;                                                           \
         }                                                                                \
     } while (0)
+#define PMALLOC(ptr, bytes) PCK(ctx_malloc(c, (void **)(ptr), bytes) ? cudaErrorMemoryAllocation : cudaSuccess)
 #define PTRY(call)              \
     do {                        \
         if (call) {             \
@@ -381,19 +382,19 @@ try {
     P122 q;
     q.nip = *nip;
     const size_t ns = c.nslots, ngp = (size_t)c.nels * q.nip;
-    PCK(cudaMalloc(&q.bee, ngp * 6 * ne * sizeof(double)));
-    PCK(cudaMalloc(&q.detw, ngp * 2 * sizeof(double)));
-    PCK(cudaMalloc(&q.evpt, ngp * 6 * sizeof(double)));
-    PCK(cudaMalloc(&q.tensor, ngp * 6 * sizeof(double)));
+    PMALLOC(&q.bee, ngp * 6 * ne * sizeof(double));
+    PMALLOC(&q.detw, ngp * 2 * sizeof(double));
+    PMALLOC(&q.evpt, ngp * 6 * sizeof(double));
+    PMALLOC(&q.tensor, ngp * 6 * sizeof(double));
     double **vecs[] = {&q.loads, &q.bdylds, &q.oldis, &q.totd};
-    for (double **v : vecs) PCK(cudaMalloc(v, ns * sizeof(double)));
-    PCK(cudaMalloc(&q.red, (2 * (size_t)c.G + 8) * sizeof(double)));
+    for (double **v : vecs) PMALLOC(v, ns * sizeof(double));
+    PMALLOC(&q.red, (2 * (size_t)c.G + 8) * sizeof(double));
     PCK(cudaMemsetAsync(q.tensor, 0, ngp * 6 * sizeof(double), c.stream));
     PCK(cudaMemsetAsync(q.oldis, 0, ns * sizeof(double), c.stream));
     PCK(cudaMemsetAsync(q.totd, 0, ns * sizeof(double), c.stream));
     PCK(cudaMemsetAsync(c.x, 0, ns * sizeof(double), c.stream));
     if (ld0) {   // ld0 to slots
-        PCK(cudaMalloc(&q.ld0, ns * sizeof(double)));
+        PMALLOC(&q.ld0, ns * sizeof(double));
         PCK(cudaMemcpyAsync(c.eqbuf, ld0, (size_t)c.neq * sizeof(double), cudaMemcpyHostToDevice, c.stream));
         PTRY(launch_eq_to_slot(c, c.eqbuf, q.ld0));
     }
@@ -410,15 +411,15 @@ try {
             }
             slots[i] = eq_slot[fix_eqs[i] - 1];
         }
-        PCK(cudaMalloc(&q.fslot, nfix * sizeof(int)));
-        PCK(cudaMalloc(&q.fval, nfix * sizeof(double)));
+        PMALLOC(&q.fslot, nfix * sizeof(int));
+        PMALLOC(&q.fval, nfix * sizeof(double));
         PCK(cudaMemcpyAsync(q.fslot, slots.data(), nfix * sizeof(int), cudaMemcpyHostToDevice, c.stream));
         PCK(cudaMemcpyAsync(q.fval, fix_vals, nfix * sizeof(double), cudaMemcpyHostToDevice, c.stream));
         PTRY(launch_set_fixed(c, nfix, q.fslot, 1.e20));
     }
     // B, det, w at every Gauss point
     double *gp = nullptr;
-    PCK(cudaMalloc(&gp, sizeof(double) * 4 * 27));
+    PMALLOC(&gp, sizeof(double) * 4 * 27);
     if (launch_sample(c.stream, q.nip, false, gp)) {
         cudaFree(gp);
         p122_free(q);
