@@ -412,6 +412,8 @@ try {
         cudaMalloc((void **)&c->st, sizeof(PcgState)) != cudaSuccess ||
         cudaMalloc((void **)&c->kerr, 2 * sizeof(int)) != cudaSuccess ||
         cudaMemset(c->kerr, 0, 2 * sizeof(int)) != cudaSuccess ||
+        cudaMalloc((void **)&c->count, 2 * sizeof(unsigned)) != cudaSuccess ||
+        cudaMemset(c->count, 0, 2 * sizeof(unsigned)) != cudaSuccess ||
         cudaMalloc((void **)&c->gbar, sizeof(unsigned long long) * kPersistSlots * kBarWords) != cudaSuccess ||
         cudaMemset(c->gbar, 0, sizeof(unsigned long long) * kPersistSlots * kBarWords) != cudaSuccess ||
         cudaMallocHost((void **)&c->hst, sizeof(PcgState)) != cudaSuccess) {
@@ -437,6 +439,7 @@ try {
     free_mesh(*c);   // also drops the iteration graph
     if (c->st) cudaFree(c->st);
     if (c->kerr) cudaFree(c->kerr);
+    if (c->count) cudaFree(c->count);
     if (c->gbar) cudaFree(c->gbar);
     if (c->hst) cudaFreeHost(c->hst);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -526,10 +529,10 @@ static int setup_mesh(void **ctx, const int *nels_p, const int *nn_p, const int 
     c.nels = nels; c.nn = nn; c.neq = neq; c.nslots = ns;
     c.kind = nod == 8 ? (nodof == 1 ? KIND_SCALAR8 : KIND_SOLID8) : KIND_SOLID20;
     long long g = ((long long)ns + 255) / 256;
-    if (g > (long long)c.nsm * 8) g = (long long)c.nsm * 8;
+    if (g > (long long)c.nsm * kVecBlocks) g = (long long)c.nsm * kVecBlocks;
     c.G = (int)(g < 1 ? 1 : g);
     long long gs = ((long long)nn + 255) / 256;
-    if (gs > (long long)c.nsm * 16) gs = (long long)c.nsm * 16;
+    if (gs > (long long)c.nsm * kScatterBlocks) gs = (long long)c.nsm * kScatterBlocks;
     c.Gs = (int)(gs < 1 ? 1 : gs);
     const size_t ne = (size_t)nels;
     if (dalloc(&c.conn, ne * nod, "connectivity") || dalloc(&c.node_ptr, nn + 1, "node table") ||

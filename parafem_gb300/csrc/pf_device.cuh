@@ -53,6 +53,113 @@ static __device__ __forceinline__ void block_reduce(double (&v)[NV], unsigned ki
     __syncthreads();
 }
 
+// The reductions of the PCG vector kernels (256 threads).  GB300 issues one
+// FP64 warp instruction per SM in 16 clocks, so a tree in every warp (eight
+// warps x five levels per value) costs more than the sums over a block's
+// slots; here one warp per value adds the 256 partial sums from shared
+// memory, eight per lane in a fixed order, and runs the one tree.  The sums
+// are valid in every thread.
+constexpr int kRedThreads = 256;
+template <int NV>
+static __device__ __forceinline__ void block_sum(double (&v)[NV])
+{
+    __shared__ double sh[NV][kRedThreads];
+    __shared__ double res[NV];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) sh[k][t] = v[k];
+    __syncthreads();
+    if (w < NV) {
+        double s = sh[w][lane];
+#pragma unroll
+        for (int j = 1; j < kRedThreads / 32; ++j) s += sh[w][lane + 32 * j];
+        s = warp_sum(s);
+        if (lane == 0) res[w] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] = res[k];
+}
+
+// Maxima of magnitudes, as the bits of their absolute values: those order as
+// the values do, so no FP64 compare is needed (a NaN counts as the largest).
+static __device__ __forceinline__ long long abs_bits(double x) { return __double_as_longlong(x) & 0x7fffffffffffffffLL; }
+static __device__ __forceinline__ void block_max2(long long &a, long long &b)
+{
+    __shared__ long long sh[2][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a = max(a, __shfl_xor_sync(FULLMASK, a, o));
+        b = max(b, __shfl_xor_sync(FULLMASK, b, o));
+    }
+    __syncthreads();
+    if (lane == 0) {
+        sh[0][w] = a;
+        sh[1][w] = b;
+    }
+    __syncthreads();
+    for (int i = 0; i < nw; ++i) {
+        a = max(a, sh[0][i]);
+        b = max(b, sh[1][i]);
+    }
+}
+
+// Sums of G block partials (value k at part[k * stride + block]) in a fixed
+// order, by one block of 256 threads; valid in every thread.
+template <int NV>
+static __device__ __forceinline__ void sum_partials(const double *part, size_t stride, int G, double (&v)[NV])
+{
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] = 0.0;
+    for (int i = threadIdx.x; i < G; i += kRedThreads)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) v[k] += __ldcg(part + k * stride + i);
+    block_sum<NV>(v);
+}
+
+// Maxima of the same two rows of partials (abs_bits held as doubles)
+static __device__ __forceinline__ void max_partials2(const double *part, size_t stride, int G, double &ma, double &mb)
+{
+    long long a = 0, b = 0;
+    for (int i = threadIdx.x; i < G; i += blockDim.x) {
+        a = max(a, __double_as_longlong(__ldcg(part + i)));
+        b = max(b, __double_as_longlong(__ldcg(part + stride + i)));
+    }
+    block_max2(a, b);
+    ma = __longlong_as_double(a);
+    mb = __longlong_as_double(b);
+}
+
+// True in the block that arrives last of the grid (in all its threads): the
+// others' writes before their arrival are visible to it.  The counter wraps
+// to zero by itself.  Thread 0 must have made the block's writes.
+static __device__ __forceinline__ bool last_block(unsigned *count)
+{
+    __shared__ int s_last;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicInc(count, gridDim.x - 1) == gridDim.x - 1;
+    }
+    __syncthreads();
+    const bool last = s_last != 0;
+    if (last) __threadfence();
+    return last;
+}
+
+// The end of a PCG scatter: the block's share of p.u, and in the last block
+// the step length alpha = r.d / p.u.  One thread divides: the vector kernels
+// only read the result.
+static __device__ __forceinline__ void scatter_tail(double loc, double *part, PcgState *st, unsigned *count)
+{
+    double v[1] = {loc};
+    block_sum<1>(v);
+    if (threadIdx.x == 0) part[blockIdx.x] = v[0];
+    if (!st || !last_block(count)) return;
+    sum_partials<1>(part, 0, gridDim.x, v);
+    if (threadIdx.x == 0) st->alpha = st->up / v[0];
+}
+
 // Block-uniform read of the stop flag: thread 0 reads it once for the whole
 // block, so a block never splits at a barrier when another block of the same
 // kernel sets the flag meanwhile.

@@ -29,9 +29,10 @@ void set_error(const char *fmt, ...);
 int host_exception(const char *name);
 
 // Scalars of one PCG run, resident on the device (pinned host mirror).
-// Only the single-block finish kernel of an iteration (or block 0 of a
-// persistent kernel, after its last barrier of the iteration) writes them,
-// so no kernel writes a value that another block of the same kernel reads.
+// They are written by one block of an iteration's kernels: the last to
+// arrive of the scatter (alpha) and of update1 (the rest), when every block
+// has read what it needs, or block 0 of a persistent kernel after its last
+// barrier of the iteration.
 // The one exception is the error path of a grid-wide barrier, which sets
 // `stop` so that the run's later launches return at once.
 struct PcgState {
@@ -39,10 +40,12 @@ struct PcgState {
     double ff;         // f.f (relative-residual denominator)
     double metric;     // last stopping metric
     double rr;         // last r.r
-    double alpha;      // batched solves: the iteration's step length, formed once per mesh
+    double alpha;      // the iteration's step length, formed once (by the scatter's last block)
+    double beta;       // and its direction factor (by update1's last block)
     double tol;        // stopping tolerance
     int iters;         // iterations completed
-    int stop;          // 1 once converged or at the limit: later kernels return
+    int stop;          // 1 once converged or at the limit: later kernels return,
+    int stop2;         //   update2 one iteration later (it completes p in the last one)
     int converged;
     int limit;
     int stop_mode;     // 0 checon_par, 1 relative residual
@@ -50,6 +53,11 @@ struct PcgState {
 };
 
 enum { STOP_CHECON = 0, STOP_RELRES = 1 };
+// Most blocks per SM of the vector kernels and of the node scatter: few
+// enough that the block reductions stay small beside the sums over slots
+// (4 to 8 measured alike for the vector kernels, 8 to 16 for the scatter;
+// 40 scatter blocks cost 20 % at 80^3).
+constexpr int kVecBlocks = 6, kScatterBlocks = 12;
 constexpr int kPersistSlots = 8;   // persistent-kernel instantiations, one barrier counter and grid each
 constexpr int kBarWords = 16;      // u64 words per counter (one 128-byte line each)
 // 20-node elasticity (p121), 8-node scalar (p123), 8-node elasticity (p122's demo)
@@ -81,6 +89,7 @@ struct Ctx {
     float *km32p = nullptr;     // [nels*1832] packed symmetric storkm (packed_off), FP32
     int *kerr = nullptr;        // device error word: 2 = a bulk-copy wait timed out, 3 = a grid barrier did;
                                 //   kerr[1]: set by k_pack_storkm when a matrix does not fit its record
+    unsigned *count = nullptr;  // [2] arrivals of the blocks of the scatter and of update1 (last_block)
     bool fix_attr = false;      // shared-memory attribute of the fixed-point kernel set
     bool have_km = false;
 
@@ -132,7 +141,7 @@ struct Ctx {
     int Gs = 0;                 // blocks of the node scatter
     double *part = nullptr;     // [Gs + 6*G + 16] block partials, split as:
     double *part_s = nullptr;   //   [Gs]  scatter partials (p.u or rres.rres)
-    double *part_u = nullptr;   //   [4G]  update partials (r.d, r.r, max|x|, max|dx|)
+    double *part_u = nullptr;   //   [4G]  update partials (r.d, r.r, and the bits of max|x|, max|dx|)
     double *part_r = nullptr;   //   [2G]  residual-replacement partials
     double *scr = nullptr;      //   [16]  scalars read back by the host
     PcgState *st = nullptr;     // device
@@ -173,7 +182,7 @@ int launch_scatter_add64(Ctx &c, double *out);   // out += scatter of the FP64 e
 int launch_pcg_init(Ctx &c, const double *rhs, double *xsol, int stop_mode, double tol, int limit,
                     bool keep_x = false);
 int launch_update1(Ctx &c, double *xsol);
-int launch_update2(Ctx &c);   // update2 + the one-block finish kernel
+int launch_update2(Ctx &c);
 int launch_pcg_iteration(Ctx &c, int prec, double *xsol);
 // Persistent forms: the scatter + updates + finish of one iteration in one
 // cooperative launch (after the element products), and whole FP64
@@ -209,12 +218,12 @@ int launch_elem_shared(Ctx &c, int prec, const double *p, const PcgState *st);  
 // 8-node scalar (p123) kernels; km64 holds storkc(8,8,e) in such a context
 int launch_form_storkc(Ctx &c, int nip, double kx, double ky, double kz);
 int launch_elem8(Ctx &c, const double *p, const PcgState *st);
-int launch_scatter1(Ctx &c, int mode, const double *xin, const double *pf, double *out, const PcgState *st);
+int launch_scatter1(Ctx &c, int mode, const double *xin, const double *pf, double *out, PcgState *st);
 int launch_assemble_diag1(Ctx &c);
 int launch_set_fixed(Ctx &c, int nfix, const int *slots_dev, double penalty);
 // pf_solid8.cu: 8-node elasticity bricks (24 freedoms per element), FP64
 int launch_elem24(Ctx &c, const double *p, const PcgState *st);
-int launch_scatter3_fixed(Ctx &c, const double *p, double *out, const PcgState *st);
+int launch_scatter3_fixed(Ctx &c, const double *p, double *out, PcgState *st);
 int launch_shared_ediag(Ctx &c);
 void set_sym_config(Ctx &c, int idx);           // 0: 14 warps x 2 stages, 1: 12 x 2, 2: 8 x 3
 int launch_matvec_generic(int n_mat, int n_row, int n_col, const double *lhs,

@@ -297,22 +297,24 @@ k_elem(int nels, const KT *__restrict__ km, const int *__restrict__ conn,
 // indices e*20+a.  FP64 results are read as three doubles at (e*20+a)*3;
 // FP32 results are node-padded, so one 16-byte load fetches a contribution,
 // and they are summed in FP32 (the precision of the products themselves).
-// Contributions are fetched eight at a time so that a node's loads are in
-// flight together.
+// Contributions are fetched two at a time: eight at a time (80 registers,
+// three blocks per SM) took 143 us in FP64 and 85 us in FP32 on an 80^3 cube,
+// two at a time 115 and 72 us.
 //   MODE 0: out = u (restrained 0), partial p.u       (pf = p)
 //   MODE 1: out = f - u (restrained 0), partial out.out (pf = f)
 //   MODE 2: out += u at free dofs, no partials          (pf unused)
+// In a PCG run the last block also forms the step length (scatter_tail).
 // One (virtual) block vb of nvb of the scatter: the body of k_scatter,
 // shared with the persistent iteration kernels, which run the same blocks
 // so that every partial sum is formed in the same order.  NC: the element
 // results may be read through the non-coherent path (they were written by an
-// earlier launch).  PF contributions are fetched at a time; the sums are
+// earlier launch).  Returns the thread's share of the partial sum.  PF contributions are fetched at a time; the sums are
 // formed in ascending order whatever PF is.
-template <typename UT, int MODE, bool NC, int PF = 8>
-__device__ __forceinline__ void scatter_block(int vb, int nvb, int nn, const int *__restrict__ ptr,
+template <typename UT, int MODE, bool NC, int PF = 2>
+__device__ __forceinline__ double scatter_block(int vb, int nvb, int nn, const int *__restrict__ ptr,
                                               const int *__restrict__ list, const UT *__restrict__ ut,
                                               const uint8_t *__restrict__ fm, const double *__restrict__ pf,
-                                              double *__restrict__ out, double *__restrict__ part)
+                                              double *__restrict__ out)
 {
     double loc = 0.0;
     for (int n = vb * blockDim.x + threadIdx.x; n < nn; n += nvb * blockDim.x) {
@@ -374,20 +376,18 @@ __device__ __forceinline__ void scatter_block(int vb, int nvb, int nn, const int
             }
         }
     }
-    if (MODE == 2) return;   // no partial sums (the kernel has no block barrier after this point)
-    double v[1] = {loc};
-    block_reduce<1>(v, 0u);
-    if (threadIdx.x == 0) part[vb] = v[0];
+    return loc;
 }
 
 template <typename UT, int MODE>
 __global__ void __launch_bounds__(256)
 k_scatter(int nn, const int *__restrict__ ptr, const int *__restrict__ list,
           const UT *__restrict__ ut, const uint8_t *__restrict__ fm, const double *__restrict__ pf,
-          double *__restrict__ out, double *__restrict__ part, const PcgState *__restrict__ st)
+          double *__restrict__ out, double *__restrict__ part, PcgState *st, unsigned *__restrict__ count)
 {
-    if (block_stopped(st)) return;
-    scatter_block<UT, MODE, true>(blockIdx.x, gridDim.x, nn, ptr, list, ut, fm, pf, out, part);
+    if (st && st->stop) return;   // not written by this kernel
+    const double loc = scatter_block<UT, MODE, true>(blockIdx.x, gridDim.x, nn, ptr, list, ut, fm, pf, out);
+    if (MODE != 2) scatter_tail(loc, part, MODE == 0 ? st : nullptr, count);
 }
 
 // ---------------------------------------------------------------------------
@@ -417,7 +417,7 @@ k_pcg_init(int ns, const double *__restrict__ rhs, const double *__restrict__ di
         rr = fma(rv, rv, rr);
     }
     double v[2] = {rd, rr};
-    block_reduce<2>(v, 0u);
+    block_sum<2>(v);
     if (threadIdx.x == 0) {
         part[blockIdx.x] = v[0];
         part[G + blockIdx.x] = v[1];
@@ -427,8 +427,9 @@ k_pcg_init(int ns, const double *__restrict__ rhs, const double *__restrict__ di
 __global__ void k_pcg_init2(PcgState *st, const double *__restrict__ part, int G, int stop_mode,
                             double tol, int limit)
 {
-    const double rd = reduce_partials(part, G, false);
-    const double rr = reduce_partials(part + G, G, false);
+    double v[2];
+    sum_partials<2>(part, G, G, v);
+    const double rd = v[0], rr = v[1];
     if (threadIdx.x == 0) {
         st->up = rd;
         st->ff = rr;
@@ -441,64 +442,123 @@ __global__ void k_pcg_init2(PcgState *st, const double *__restrict__ part, int G
         st->stop_mode = stop_mode;
         st->err = 0;
         // a zero load vector is already solved by x = 0
-        st->stop = (rr == 0.0) ? 1 : 0;
+        st->stop = st->stop2 = (rr == 0.0) ? 1 : 0;
         if (rr == 0.0) st->converged = 1;
     }
 }
 
-// update1: alpha = up/(p.u); xnew = x + p*alpha (in place, checon_par's
-// x = xnew, maths.f90:1062); r = r - u*alpha; d = diag*r; block partials of
-// r.d, r.r and, for checon_par only (CHECON), max|xnew| and max|xnew-x|,
-// into pu[0..4G).  p.u comes from the scatter's Gs partials ps.  Reads
-// st->up only.  The max terms cost four FP64 operations per dof, a slow pipe
-// on GB300, so the residual-stopped runs skip them.
+// update1: xnew = x + p*alpha (in place, checon_par's x = xnew,
+// maths.f90:1062); r = r - u*alpha; d = diag*r; block partials of r.d, r.r
+// and, for checon_par only (CHECON), max|xnew| and max|xnew-x|, into
+// pu[0..4G).  Bound by HBM (64 B per slot) and by the FP64 pipe (two
+// operations per SM and clock): five operations per slot, six with CHECON,
+// whose maxima are integer compares of the magnitudes' bits; checon_par does
+// not use r.r, so CHECON leaves it out.
 template <bool CHECON>
 __device__ __forceinline__ void update1_block(int vb, int nvb, int ns, double alpha, double *__restrict__ pu_out,
                                               int G, double *__restrict__ x, double *__restrict__ r,
                                               double *__restrict__ d, const double *__restrict__ p,
                                               const double *__restrict__ u, const double *__restrict__ dinv)
 {
-    double rd = 0.0, rr = 0.0, mx = 0.0, md = 0.0;
+    double rd = 0.0, rr = 0.0;
+    long long mx = 0, md = 0;
     for (int s = vb * blockDim.x + threadIdx.x; s < ns; s += nvb * blockDim.x) {
         const double xo = x[s];
         const double xn = fma(p[s], alpha, xo);
         x[s] = xn;
         if (CHECON) {
-            mx = fmax(mx, fabs(xn));
-            md = fmax(md, fabs(xn - xo));
+            mx = max(mx, abs_bits(xn));
+            md = max(md, abs_bits(xn - xo));
         }
         const double rn = fma(-u[s], alpha, r[s]);
         r[s] = rn;
         const double dn = dinv[s] * rn;
         d[s] = dn;
         rd = fma(rn, dn, rd);
-        rr = fma(rn, rn, rr);
+        if (!CHECON) rr = fma(rn, rn, rr);
     }
-    double v[4] = {rd, rr, mx, md};
-    block_reduce<4>(v, 0xCu);
+    if (CHECON) {
+        double v[1] = {rd};
+        block_sum<1>(v);
+        rd = v[0];
+        block_max2(mx, md);
+    } else {
+        double v[2] = {rd, rr};
+        block_sum<2>(v);
+        rd = v[0];
+        rr = v[1];
+    }
     if (threadIdx.x == 0) {
-        pu_out[0 * G + vb] = v[0];
-        pu_out[1 * G + vb] = v[1];
-        pu_out[2 * G + vb] = v[2];
-        pu_out[3 * G + vb] = v[3];
+        pu_out[0 * G + vb] = rd;
+        pu_out[1 * G + vb] = rr;
+        pu_out[2 * G + vb] = __longlong_as_double(mx);
+        pu_out[3 * G + vb] = __longlong_as_double(md);
     }
 }
 
+// The finish of an iteration, by one block: r.d, the stopping metric
+// (checon_par, maths.f90:1052-1062, or the relative residual) and what
+// follows from them.  Valid in every thread.
+struct Finish {
+    double rd, rr, metric;
+    bool conv, bad;
+};
+template <bool CHECON>
+__device__ __forceinline__ Finish finish_sums(const double *part, int G, double ff, double tol)
+{
+    Finish f;
+    f.rr = 0.0;
+    double mx = 1.0;
+    if (CHECON) {
+        double v[1], md;
+        sum_partials<1>(part, 0, G, v);
+        f.rd = v[0];
+        max_partials2(part + 2 * (size_t)G, G, G, mx, md);
+        f.metric = md / mx;
+    } else {
+        double v[2];
+        sum_partials<2>(part, G, G, v);
+        f.rd = v[0];
+        f.rr = v[1];
+        f.metric = sqrt(f.rr) / sqrt(ff);
+    }
+    f.conv = f.metric <= tol;
+    f.bad = !isfinite(f.rd) || !isfinite(mx);
+    return f;
+}
+
+// The last block to arrive runs the iteration's bookkeeping: every other
+// block has read the state by then.  (As a launch of its own it took 4 to 6
+// us of a 25 us iteration on 10^3 elements, and each of the next kernel's
+// blocks summed the partials again.)
 template <bool CHECON>
 __global__ void __launch_bounds__(256)
-k_pcg_update1(int ns, const PcgState *__restrict__ st, const double *__restrict__ ps, int Gs,
-              double *__restrict__ pu_out, int G, double *__restrict__ x, double *__restrict__ r,
-              double *__restrict__ d, const double *__restrict__ p, const double *__restrict__ u,
-              const double *__restrict__ dinv)
+k_pcg_update1(int ns, PcgState *st, unsigned *__restrict__ count, double *__restrict__ pu_out, int G,
+              double *__restrict__ x, double *__restrict__ r, double *__restrict__ d, const double *__restrict__ p,
+              const double *__restrict__ u, const double *__restrict__ dinv)
 {
-    if (block_stopped(st)) return;
-    const double pu = reduce_partials(ps, Gs, false);
-    const double alpha = st->up / pu;
-    update1_block<CHECON>(blockIdx.x, gridDim.x, ns, alpha, pu_out, G, x, r, d, p, u, dinv);
+    if (st->stop) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) st->stop2 = 1;   // read by update2 only
+        return;
+    }
+    update1_block<CHECON>(blockIdx.x, gridDim.x, ns, st->alpha, pu_out, G, x, r, d, p, u, dinv);
+    if (!last_block(count)) return;
+    const Finish f = finish_sums<CHECON>(pu_out, G, st->ff, st->tol);
+    if (threadIdx.x == 0) {
+        const int k = st->iters + 1;
+        st->beta = f.rd / st->up;
+        st->up = f.rd;
+        st->iters = k;
+        st->rr = f.rr;
+        st->metric = f.metric;
+        st->converged = f.conv ? 1 : 0;
+        if (f.bad) st->err = 1;
+        if (f.conv || k >= st->limit || f.bad) st->stop = 1;
+    }
 }
 
-// update2: beta = (r.d)/up; p = d + p*beta (and its FP32 high and low
-// parts into ps, shared-km contexts).  Reads st->up only.
+// update2: p = d + p*beta (and its FP32 high and low parts into ps,
+// shared-km contexts).
 __device__ __forceinline__ void update2_block(int vb, int nvb, int ns, double beta, const double *__restrict__ d,
                                               double *__restrict__ p, float2 *__restrict__ ps)
 {
@@ -514,40 +574,11 @@ __device__ __forceinline__ void update2_block(int vb, int nvb, int ns, double be
 }
 
 __global__ void __launch_bounds__(256)
-k_pcg_update2(int ns, const PcgState *__restrict__ st, const double *__restrict__ part, int G,
-              const double *__restrict__ d, double *__restrict__ p, float2 *__restrict__ ps)
+k_pcg_update2(int ns, const PcgState *__restrict__ st, const double *__restrict__ d, double *__restrict__ p,
+              float2 *__restrict__ ps)
 {
-    if (block_stopped(st)) return;
-    const double rd = reduce_partials(part, G, false);
-    const double beta = rd / st->up;
-    update2_block(blockIdx.x, gridDim.x, ns, beta, d, p, ps);
-}
-
-// finish (one block): the iteration's bookkeeping -- up for the next
-// iteration, the iteration count and the stopping test (checon_par,
-// maths.f90:1052-1062, or the relative residual).  It is the only kernel
-// of an iteration that writes the state.
-__global__ void __launch_bounds__(256)
-k_pcg_finish(PcgState *__restrict__ st, const double *__restrict__ part, int G)
-{
-    if (block_stopped(st)) return;
-    const double rd = reduce_partials(part, G, false);
-    const double rr = reduce_partials(part + 1 * G, G, false);
-    const bool checon = st->stop_mode == STOP_CHECON;   // uniform: written only by init kernels
-    const double mx = checon ? reduce_partials(part + 2 * G, G, true) : 1.0;
-    const double md = checon ? reduce_partials(part + 3 * G, G, true) : 0.0;
-    if (threadIdx.x == 0) {
-        const int k = st->iters + 1;
-        const double metric = checon ? md / mx : sqrt(rr) / sqrt(st->ff);
-        const bool conv = metric <= st->tol;
-        st->up = rd;
-        st->iters = k;
-        st->rr = rr;
-        st->metric = metric;
-        st->converged = conv ? 1 : 0;
-        if (!isfinite(rd) || !isfinite(mx)) st->err = 1;
-        if (conv || k >= st->limit || st->err) st->stop = 1;
-    }
+    if (st->stop2) return;
+    update2_block(blockIdx.x, gridDim.x, ns, st->beta, d, p, ps);
 }
 
 // ---------------------------------------------------------------------------
@@ -581,6 +612,16 @@ struct PersistArgs {
     int *kerr;
 };
 
+// a / b by one thread of the block (a division holds the FP64 pipe)
+__device__ __forceinline__ double divide(double a, double b)
+{
+    __shared__ double q;
+    __syncthreads();
+    if (threadIdx.x == 0) q = a / b;
+    __syncthreads();
+    return q;
+}
+
 template <typename UT, bool ELEM64, bool CHECON, int MINB, int PF>
 __global__ void __launch_bounds__(256, MINB) k_pcg_persistent(PersistArgs a)
 {
@@ -604,36 +645,35 @@ __global__ void __launch_bounds__(256, MINB) k_pcg_persistent(PersistArgs a)
             }
             if (!grid_barrier(a.bar, a.kerr, a.st)) return;
         }
-        for (int vb = blockIdx.x; vb < a.Gs; vb += gridDim.x)
-            scatter_block<UT, 0, !ELEM64, PF>(vb, a.Gs, a.nn, a.node_ptr, a.node_list, (const UT *)a.ut, a.fm, a.p,
-                                          a.u, a.part_s);
+        for (int vb = blockIdx.x; vb < a.Gs; vb += gridDim.x) {
+            double v[1] = {scatter_block<UT, 0, !ELEM64, PF>(vb, a.Gs, a.nn, a.node_ptr, a.node_list, (const UT *)a.ut,
+                                                             a.fm, a.p, a.u)};
+            block_sum<1>(v);
+            if (threadIdx.x == 0) a.part_s[vb] = v[0];
+        }
         if (!grid_barrier(a.bar, a.kerr, a.st)) return;
-        const double alpha = up / reduce_partials(a.part_s, a.Gs, false);
+        double v[1];
+        sum_partials<1>(a.part_s, 0, a.Gs, v);
+        const double alpha = divide(up, v[0]);
         for (int vb = blockIdx.x; vb < a.G; vb += gridDim.x)
             update1_block<CHECON>(vb, a.G, a.ns, alpha, a.part_u, a.G, a.x, a.r, a.d, a.p, a.u, a.dinv);
         if (!grid_barrier(a.bar, a.kerr, a.st)) return;
-        const double rd = reduce_partials(a.part_u, a.G, false);
-        const double beta = rd / up;
+        // the finish of k_pcg_update1, formed by every block
+        const Finish f = finish_sums<CHECON>(a.part_u, a.G, ff, tol);
+        const double beta = divide(f.rd, up);
         for (int vb = blockIdx.x; vb < a.G; vb += gridDim.x) update2_block(vb, a.G, a.ns, beta, a.d, a.p, a.psplit);
-        // the finish of k_pcg_finish, formed by every block
-        const double rr = reduce_partials(a.part_u + a.G, a.G, false);
-        const double mx = CHECON ? reduce_partials(a.part_u + 2 * a.G, a.G, true) : 1.0;
-        const double md = CHECON ? reduce_partials(a.part_u + 3 * a.G, a.G, true) : 0.0;
         ++iters;
-        const double metric = CHECON ? md / mx : sqrt(rr) / sqrt(ff);
-        const bool conv = metric <= tol;
-        const bool bad = !isfinite(rd) || !isfinite(mx);
-        const bool stop = conv || iters >= limit || bad;
+        const bool stop = f.conv || iters >= limit || f.bad;
         if (blockIdx.x == 0 && threadIdx.x == 0) {
-            vs->up = rd;
+            vs->up = f.rd;
             vs->iters = iters;
-            vs->rr = rr;
-            vs->metric = metric;
-            vs->converged = conv ? 1 : 0;
-            if (bad) vs->err = 1;
+            vs->rr = f.rr;
+            vs->metric = f.metric;
+            vs->converged = f.conv ? 1 : 0;
+            if (f.bad) vs->err = 1;
             if (stop) vs->stop = 1;
         }
-        up = rd;
+        up = f.rd;
         if (stop) return;
         if (it + 1 < a.niters && !grid_barrier(a.bar, a.kerr, a.st)) return;
     }
@@ -656,7 +696,7 @@ k_pcg_replace(int ns, const double *__restrict__ rres, const double *__restrict_
         rr = fma(rv, rv, rr);
     }
     double v[2] = {rd, rr};
-    block_reduce<2>(v, 0u);
+    block_sum<2>(v);
     if (threadIdx.x == 0) {
         part[blockIdx.x] = v[0];
         part[G + blockIdx.x] = v[1];
@@ -665,15 +705,16 @@ k_pcg_replace(int ns, const double *__restrict__ rres, const double *__restrict_
 
 __global__ void k_pcg_replace2(PcgState *st, const double *__restrict__ part, int G, double tol)
 {
-    const double rd = reduce_partials(part, G, false);
-    const double rr = reduce_partials(part + G, G, false);
+    double v[2];
+    sum_partials<2>(part, G, G, v);
+    const double rd = v[0], rr = v[1];
     if (threadIdx.x == 0) {
         st->up = rd;
         st->rr = rr;
         st->metric = sqrt(rr) / sqrt(st->ff);
         st->tol = tol;
         st->converged = 0;
-        st->stop = (rr == 0.0) ? 1 : 0;
+        st->stop = st->stop2 = (rr == 0.0) ? 1 : 0;
     }
 }
 
@@ -681,8 +722,9 @@ __global__ void k_sum_partials(const double *__restrict__ part, int G, int nvals
                                double *__restrict__ out)
 {
     for (int k = 0; k < nvals; ++k) {
-        const double v = reduce_partials(part + (size_t)k * G, G, false);
-        if (threadIdx.x == 0) out[k] = v;
+        double v[1];
+        sum_partials<1>(part + (size_t)k * G, 0, G, v);
+        if (threadIdx.x == 0) out[k] = v[0];
     }
 }
 
@@ -909,21 +951,21 @@ int launch_scatter(Ctx &c, int prec, int mode, const double *pf, double *out)
 {
     if (c.kind == KIND_SCALAR8) return launch_scatter1(c, mode, pf, pf, out, mode == 0 ? c.st : nullptr);
     if (c.kind == KIND_SOLID8 && mode == 0) return launch_scatter3_fixed(c, pf, out, c.st);
-    const PcgState *st = mode == 0 ? c.st : nullptr;
+    PcgState *st = mode == 0 ? c.st : nullptr;
     if (prec != PREC_FP64) {
         if (mode == 0)
             k_scatter<float, 0><<<c.Gs, 256, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, (const float *)c.utemp,
-                                                            c.freemask, pf, out, c.part_s, st);
+                                                            c.freemask, pf, out, c.part_s, st, c.count);
         else
             k_scatter<float, 1><<<c.Gs, 256, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, (const float *)c.utemp,
-                                                            c.freemask, pf, out, c.part_s, st);
+                                                            c.freemask, pf, out, c.part_s, st, c.count);
     } else {
         if (mode == 0)
             k_scatter<double, 0><<<c.Gs, 256, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, (const double *)c.utemp,
-                                                             c.freemask, pf, out, c.part_s, st);
+                                                             c.freemask, pf, out, c.part_s, st, c.count);
         else
             k_scatter<double, 1><<<c.Gs, 256, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, (const double *)c.utemp,
-                                                             c.freemask, pf, out, c.part_s, st);
+                                                             c.freemask, pf, out, c.part_s, st, c.count);
     }
     return check_launch(c, "k_scatter");
 }
@@ -936,10 +978,10 @@ int launch_matvec(Ctx &c, int prec, const double *p, double *u)
     if (c.kind == KIND_SOLID8) return launch_scatter3_fixed(c, p, u, nullptr);
     if (prec != PREC_FP64)
         k_scatter<float, 0><<<c.Gs, 256, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, (const float *)c.utemp,
-                                                        c.freemask, p, u, c.part_s, nullptr);
+                                                        c.freemask, p, u, c.part_s, nullptr, c.count);
     else
         k_scatter<double, 0><<<c.Gs, 256, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, (const double *)c.utemp,
-                                                         c.freemask, p, u, c.part_s, nullptr);
+                                                         c.freemask, p, u, c.part_s, nullptr, c.count);
     return check_launch(c, "k_scatter");
 }
 
@@ -947,7 +989,7 @@ int launch_matvec(Ctx &c, int prec, const double *p, double *u)
 int launch_scatter_add64(Ctx &c, double *out)
 {
     k_scatter<double, 2><<<c.Gs, 256, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, (const double *)c.utemp,
-                                                     c.freemask, nullptr, out, c.part_s, nullptr);
+                                                     c.freemask, nullptr, out, c.part_s, nullptr, c.count);
     return check_launch(c, "k_scatter");
 }
 
@@ -957,7 +999,7 @@ int launch_residual(Ctx &c, const double *f, const double *x, double *rres)
     if (launch_products(c, PREC_FP64, x, nullptr)) return 1;
     if (c.kind == KIND_SCALAR8) return launch_scatter1(c, 1, x, f, rres, nullptr);
     k_scatter<double, 1><<<c.Gs, 256, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, (const double *)c.utemp,
-                                                     c.freemask, f, rres, c.part_s, nullptr);
+                                                     c.freemask, f, rres, c.part_s, nullptr, c.count);
     return check_launch(c, "k_scatter");
 }
 
@@ -978,20 +1020,18 @@ int launch_pcg_init(Ctx &c, const double *rhs, double *xsol, int stop_mode, doub
 int launch_update1(Ctx &c, double *xsol)
 {
     if (c.stop_mode == STOP_CHECON)
-        k_pcg_update1<true><<<c.G, 256, 0, c.stream>>>(c.nslots, c.st, c.part_s, c.Gs, c.part_u, c.G, xsol, c.r, c.d,
-                                                       c.p, c.u, c.dinv);
+        k_pcg_update1<true><<<c.G, 256, 0, c.stream>>>(c.nslots, c.st, c.count + 1, c.part_u, c.G, xsol, c.r, c.d, c.p,
+                                                       c.u, c.dinv);
     else
-        k_pcg_update1<false><<<c.G, 256, 0, c.stream>>>(c.nslots, c.st, c.part_s, c.Gs, c.part_u, c.G, xsol, c.r, c.d,
-                                                        c.p, c.u, c.dinv);
+        k_pcg_update1<false><<<c.G, 256, 0, c.stream>>>(c.nslots, c.st, c.count + 1, c.part_u, c.G, xsol, c.r, c.d, c.p,
+                                                        c.u, c.dinv);
     return check_launch(c, "k_pcg_update1");
 }
 
 int launch_update2(Ctx &c)
 {
-    k_pcg_update2<<<c.G, 256, 0, c.stream>>>(c.nslots, c.st, c.part_u, c.G, c.d, c.p, c.shared ? c.psplit : nullptr);
-    if (check_launch(c, "k_pcg_update2")) return 1;
-    k_pcg_finish<<<1, 256, 0, c.stream>>>(c.st, c.part_u, c.G);
-    return check_launch(c, "k_pcg_finish");
+    k_pcg_update2<<<c.G, 256, 0, c.stream>>>(c.nslots, c.st, c.d, c.p, c.shared ? c.psplit : nullptr);
+    return check_launch(c, "k_pcg_update2");
 }
 
 // Blocks of the cooperative launch of one persistent-kernel instantiation:
@@ -1017,7 +1057,7 @@ static int persist_grid(const Ctx &c)
 template <typename UT, bool ELEM64, bool CHECON>
 static int launch_persist_t(Ctx &c, double *xsol, int niters)
 {
-    constexpr int MINB = ELEM64 ? 2 : 4, PF = sizeof(UT) == 8 ? 4 : 8;   // the products hold 100-odd registers
+    constexpr int MINB = ELEM64 ? 2 : 4, PF = 2;   // the products hold 100-odd registers
     const int idx = (ELEM64 ? 4 : 0) + (sizeof(UT) == 4 ? 2 : 0) + (CHECON ? 1 : 0);
     if (c.pk_grid[idx] == 0) c.pk_grid[idx] = persist_grid<UT, ELEM64, CHECON, MINB, PF>(c);
     const int grid = c.pk_grid[idx];

@@ -282,25 +282,24 @@ __global__ void k_p122_fixed_loads(int nfix, const int *__restrict__ slot, const
 __global__ void __launch_bounds__(256)
 k_p122_checon(int ns, const double *__restrict__ x, double *__restrict__ oldis, double *__restrict__ part, int G)
 {
-    double ml = 0.0, md = 0.0;
+    long long ml = 0, md = 0;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < ns; s += gridDim.x * blockDim.x) {
         const double xv = x[s];
-        ml = fmax(ml, fabs(xv));
-        md = fmax(md, fabs(xv - oldis[s]));
+        ml = max(ml, abs_bits(xv));
+        md = max(md, abs_bits(xv - oldis[s]));
         oldis[s] = xv;
     }
-    double v[2] = {ml, md};
-    block_reduce<2>(v, 3u);
+    block_max2(ml, md);
     if (threadIdx.x == 0) {
-        part[blockIdx.x] = v[0];
-        part[G + blockIdx.x] = v[1];
+        part[blockIdx.x] = __longlong_as_double(ml);
+        part[G + blockIdx.x] = __longlong_as_double(md);
     }
 }
 
 __global__ void k_p122_checon2(const double *__restrict__ part, int G, double *__restrict__ out)
 {
-    const double ml = reduce_partials(part, G, true);
-    const double md = reduce_partials(part + G, G, true);
+    double ml, md;
+    max_partials2(part, G, G, ml, md);
     if (threadIdx.x == 0) {
         out[0] = ml;
         out[1] = md;

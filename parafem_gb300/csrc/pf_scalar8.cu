@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(256)
 k_elem8(int nels, const double *__restrict__ kc, const int *__restrict__ conn, const double *__restrict__ p,
         double *__restrict__ ut, const PcgState *__restrict__ st)
 {
-    if (block_stopped(st)) return;
+    if (st && st->stop) return;
     const int i = threadIdx.x & 7;
     const unsigned gmask = 0xFFu << (threadIdx.x & 24);   // the 8 lanes of this element
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < (long long)nels * 8;
@@ -88,9 +88,9 @@ __global__ void __launch_bounds__(256)
 k_scatter1(int nn, const int *__restrict__ ptr, const int *__restrict__ list, const double *__restrict__ ut,
            const uint8_t *__restrict__ fm, const double *__restrict__ fstore, const double *__restrict__ xin,
            const double *__restrict__ pf, double *__restrict__ out, double *__restrict__ part,
-           const PcgState *__restrict__ st)
+           PcgState *st, unsigned *__restrict__ count)
 {
-    if (block_stopped(st)) return;
+    if (st && st->stop) return;
     double loc = 0.0;
     for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < nn; n += gridDim.x * blockDim.x) {
         double a = 0.0;
@@ -108,9 +108,7 @@ k_scatter1(int nn, const int *__restrict__ ptr, const int *__restrict__ list, co
             loc = fma(rv, rv, loc);
         }
     }
-    double v[1] = {loc};
-    block_reduce<1>(v, 0u);
-    if (threadIdx.x == 0) part[blockIdx.x] = v[0];
+    scatter_tail(loc, part, MODE == 0 ? st : nullptr, count);
 }
 
 __global__ void k_assemble_diag1(int nn, const int *__restrict__ ptr, const int *__restrict__ list,
@@ -181,14 +179,14 @@ int launch_elem8(Ctx &c, const double *p, const PcgState *st)
     return launched8(c, "k_elem8");
 }
 
-int launch_scatter1(Ctx &c, int mode, const double *xin, const double *pf, double *out, const PcgState *st)
+int launch_scatter1(Ctx &c, int mode, const double *xin, const double *pf, double *out, PcgState *st)
 {
     if (mode == 0)
         k_scatter1<0><<<c.Gs, 256, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, (const double *)c.utemp, c.freemask,
-                                                  c.fstore, xin, pf, out, c.part_s, st);
+                                                  c.fstore, xin, pf, out, c.part_s, st, c.count);
     else
         k_scatter1<1><<<c.Gs, 256, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, (const double *)c.utemp, c.freemask,
-                                                  c.fstore, xin, pf, out, c.part_s, st);
+                                                  c.fstore, xin, pf, out, c.part_s, st, c.count);
     return launched8(c, "k_scatter1");
 }
 

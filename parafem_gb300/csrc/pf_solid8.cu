@@ -44,9 +44,9 @@ __global__ void __launch_bounds__(256)
 k_scatter3_fix(int nn, const int *__restrict__ ptr, const int *__restrict__ list, const double *__restrict__ ut,
                const uint8_t *__restrict__ fm, const double *__restrict__ fstore, const double *__restrict__ fscale,
                const double *__restrict__ p, double *__restrict__ out, double *__restrict__ part,
-               const PcgState *__restrict__ st)
+               PcgState *st, unsigned *__restrict__ count)
 {
-    if (block_stopped(st)) return;
+    if (st && st->stop) return;
     const double fsc = *fscale;
     double loc = 0.0;
     for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < nn; n += gridDim.x * blockDim.x) {
@@ -68,9 +68,7 @@ k_scatter3_fix(int nn, const int *__restrict__ ptr, const int *__restrict__ list
             loc = fma(p[s], uv, loc);
         }
     }
-    double v[1] = {loc};
-    block_reduce<1>(v, 0u);
-    if (threadIdx.x == 0) part[blockIdx.x] = v[0];
+    scatter_tail(loc, part, st, count);
 }
 
 static int launched24(Ctx &c, const char *name)
@@ -92,10 +90,10 @@ int launch_elem24(Ctx &c, const double *p, const PcgState *st)
     return launched24(c, "k_elem24");
 }
 
-int launch_scatter3_fixed(Ctx &c, const double *p, double *out, const PcgState *st)
+int launch_scatter3_fixed(Ctx &c, const double *p, double *out, PcgState *st)
 {
     k_scatter3_fix<<<c.Gs, 256, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, (const double *)c.utemp, c.freemask,
-                                               c.fstore, c.fscale, p, out, c.part_s, st);
+                                               c.fstore, c.fscale, p, out, c.part_s, st, c.count);
     return launched24(c, "k_scatter3_fix");
 }
 
