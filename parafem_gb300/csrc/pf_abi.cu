@@ -527,6 +527,7 @@ static int setup_mesh(void **ctx, const int *nels_p, const int *nn_p, const int 
         }
 
     c.nels = nels; c.nn = nn; c.neq = neq; c.nslots = ns;
+    c.dependent = ns <= kDependentSlots;
     c.kind = nod == 8 ? (nodof == 1 ? KIND_SCALAR8 : KIND_SOLID8) : KIND_SOLID20;
     long long g = ((long long)ns + 255) / 256;
     if (g > (long long)c.nsm * kVecBlocks) g = (long long)c.nsm * kVecBlocks;

@@ -19,7 +19,7 @@
 // lane: forward distance d needs (D[d][l], D[d][l+30]) = word 30d + l, and
 // backward distance t = 30 - d needs D[t][l+d] and D[t][(l+d+30) mod 60],
 // the two halves of word 30t + (l+d) mod 30 (swapped when l+d >= 30).
-#include "pf_internal.h"
+#include "pf_device.cuh"
 #include "pf_tc.cuh"
 
 #include <cstdint>
@@ -87,6 +87,7 @@ k_elem_sym16(int nels, const uint32_t *__restrict__ kh, const int *__restrict__ 
                                                  kWarps * kPSlot * 4) + w * kStages;
     static_assert((kWarps * kStages * kH16Bytes + kWarps * kPSlot * 4) % 8 == 0, "mbarrier alignment");
 
+    pdl_enter();
     int stopped = 0;
     if (lane == 0 && st) stopped = st->stop;
     stopped = __shfl_sync(kFull, stopped, 0);
@@ -259,9 +260,9 @@ static int launch_h16_cfg(Ctx &c, const double *p, const PcgState *st, int bit)
         }
         c.h16_attr |= 1u << bit;
     }
-    const int grid = c.nels < c.nsm * W ? (c.nels + W - 1) / W : c.nsm;
-    k_elem_sym16<W, S, A, false><<<grid, W * 32, smem, c.stream>>>(c.nels, c.km16p, c.conn, p, (float *)c.utemp,
-                                                                   st, c.kerr, nullptr);
+    const int grid = c.nels < c.nsm ? c.nels : c.nsm;   // a small mesh spreads its warps over the SMs
+    launch_dependent(c.dependent && st, c.stream, grid, W * 32, smem, k_elem_sym16<W, S, A, false>, c.nels, c.km16p, c.conn, p,
+                     (float *)c.utemp, st, c.kerr, nullptr);
     c.launches++;
     e = cudaGetLastError();
     if (e != cudaSuccess) {

@@ -29,7 +29,7 @@
 // Every wait on an mbarrier is bounded; a wait that runs out writes 2 to
 // the context's device error word and the warp drains its in-flight copies
 // (again with a bound) before it returns.
-#include "pf_internal.h"
+#include "pf_device.cuh"
 #include "pf_tc.cuh"
 
 #include <cstdint>
@@ -85,6 +85,7 @@ k_elem_sym32(int nels, const float *__restrict__ kp, const int *__restrict__ con
                                                  kWarps * kPSlot * 4) + w * kStages;
     static_assert((kWarps * kStages * kPackedBytes + kWarps * kPSlot * 4) % 8 == 0, "mbarrier alignment");
 
+    pdl_enter();
     // stop flag: uniform per warp (no block barrier after this point)
     int stopped = 0;
     if (lane == 0 && st) stopped = st->stop;
@@ -261,9 +262,9 @@ static int launch_sym_cfg(Ctx &c, const double *p, const PcgState *st)
         }
         c.sym_attr |= bit;
     }
-    const int grid = c.nels < c.nsm * W ? (c.nels + W - 1) / W : c.nsm;
-    k_elem_sym32<W, S, false><<<grid, W * 32, smem, c.stream>>>(c.nels, c.km32p, c.conn, p, (float *)c.utemp, st,
-                                                                c.kerr, nullptr);
+    const int grid = c.nels < c.nsm ? c.nels : c.nsm;   // a small mesh spreads its warps over the SMs
+    launch_dependent(c.dependent && st, c.stream, grid, W * 32, smem, k_elem_sym32<W, S, false>, c.nels, c.km32p, c.conn, p,
+                     (float *)c.utemp, st, c.kerr, nullptr);
     c.launches++;
     e = cudaGetLastError();
     if (e != cudaSuccess) {

@@ -124,6 +124,7 @@ k_elem_fix(int nels, const unsigned char *__restrict__ rec, const int *__restric
     unsigned char *stage = smem + (size_t)w * 3 * fx::kChunk0;
     int4 *pq = reinterpret_cast<int4 *>(smem + (size_t)kFixWarps * 3 * fx::kChunk0) + w * 60;
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem + (size_t)kFixWarps * (3 * fx::kChunk0 + 960)) + 3 * w;
+    pdl_enter();
     int stopped = 0;
     if (lane == 0 && st) stopped = st->stop;
     if (__shfl_sync(FULLMASK, stopped, 0)) return;
@@ -193,6 +194,7 @@ k_elem_shared_fix(int nels, const unsigned char *__restrict__ rec, const int *__
 {
     __shared__ int4 pq[kSharedFixWarps][60];
     __shared__ __align__(16) unsigned char r[fx::kRecBytes];
+    pdl_enter();
     if (st && st->stop) return;
     for (int i = threadIdx.x; i < fx::kRecBytes / 16; i += blockDim.x)
         reinterpret_cast<int4 *>(r)[i] = reinterpret_cast<const int4 *>(rec)[i];
@@ -246,7 +248,8 @@ int launch_elem_fix(Ctx &c, const double *p, const PcgState *st)
     }
     // one CTA per SM, and on small meshes as few warps per SM as the mesh has
     const int grid = c.nels < c.nsm ? c.nels : c.nsm;
-    k_elem_fix<<<grid, kFixWarps * 32, kFixSmem, c.stream>>>(c.nels, c.kmfix, c.conn, p, (double *)c.utemp, st, c.kerr);
+    launch_dependent(c.dependent && st, c.stream, grid, kFixWarps * 32, kFixSmem, k_elem_fix, c.nels, c.kmfix, c.conn, p,
+                     (double *)c.utemp, st, c.kerr);
     return fix_launched(c, "k_elem_fix");
 }
 
@@ -254,7 +257,8 @@ int launch_elem_shared_fix(Ctx &c, const double *p, const PcgState *st)
 {
     const int nb = (c.nels + kSharedFixWarps - 1) / kSharedFixWarps;
     const int grid = nb < c.nsm * 2 ? nb : c.nsm * 2;
-    k_elem_shared_fix<<<grid, kSharedFixWarps * 32, 0, c.stream>>>(c.nels, c.skmfix, c.conn, p, (double *)c.utemp, st);
+    launch_dependent(c.dependent && st, c.stream, grid, kSharedFixWarps * 32, 0, k_elem_shared_fix, c.nels, c.skmfix, c.conn, p,
+                     (double *)c.utemp, st);
     return fix_launched(c, "k_elem_shared_fix");
 }
 

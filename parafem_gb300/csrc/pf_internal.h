@@ -58,6 +58,11 @@ enum { STOP_CHECON = 0, STOP_RELRES = 1 };
 // (4 to 8 measured alike for the vector kernels, 8 to 16 for the scatter;
 // 40 scatter blocks cost 20 % at 80^3).
 constexpr int kVecBlocks = 6, kScatterBlocks = 12;
+// Most slots of a mesh whose iterations use programmatic dependent launches:
+// they save 1.5 to 3 us of an iteration (10^3 elements: 24.0 -> 22.0 us FP64,
+// 26.5 -> 23.6 mixed; 20^3: 47 -> 45, 34 -> 31), nothing measurable of the
+// 113 us at 40^3, and lose 0.5 % at 80^3.
+constexpr int kDependentSlots = 500000;
 constexpr int kPersistSlots = 8;   // persistent-kernel instantiations, one barrier counter and grid each
 constexpr int kBarWords = 16;      // u64 words per counter (one 128-byte line each)
 // 20-node elasticity (p121), 8-node scalar (p123), 8-node elasticity (p122's demo)
@@ -137,6 +142,7 @@ struct Ctx {
     unsigned long long *gbar = nullptr;   // [kPersistSlots] grid-barrier arrival counters, zeroed per run
     int pk_grid[kPersistSlots] = {};      // blocks of each persistent instantiation (0 = not sized)
 
+    bool dependent = false;     // programmatic dependent launches in the iteration (small meshes)
     int G = 0;                  // blocks of the vector kernels
     int Gs = 0;                 // blocks of the node scatter
     double *part = nullptr;     // [Gs + 6*G + 16] block partials, split as:

@@ -283,6 +283,7 @@ __global__ void __launch_bounds__(256)
 k_elem(int nels, const KT *__restrict__ km, const int *__restrict__ conn,
        const double *__restrict__ p, KT *__restrict__ ut, const PcgState *__restrict__ st)
 {
+    pdl_enter();
     if (st && st->stop) return;
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -387,6 +388,7 @@ k_scatter(int nn, const int *__restrict__ ptr, const int *__restrict__ list,
 {
     if (st && st->stop) return;   // not written by this kernel
     const double loc = scatter_block<UT, MODE, true>(blockIdx.x, gridDim.x, nn, ptr, list, ut, fm, pf, out);
+    pdl_exit();
     if (MODE != 2) scatter_tail(loc, part, MODE == 0 ? st : nullptr, count);
 }
 
@@ -537,11 +539,13 @@ k_pcg_update1(int ns, PcgState *st, unsigned *__restrict__ count, double *__rest
               double *__restrict__ x, double *__restrict__ r, double *__restrict__ d, const double *__restrict__ p,
               const double *__restrict__ u, const double *__restrict__ dinv)
 {
+    pdl_enter();
     if (st->stop) {
         if (blockIdx.x == 0 && threadIdx.x == 0) st->stop2 = 1;   // read by update2 only
         return;
     }
     update1_block<CHECON>(blockIdx.x, gridDim.x, ns, st->alpha, pu_out, G, x, r, d, p, u, dinv);
+    pdl_exit();
     if (!last_block(count)) return;
     const Finish f = finish_sums<CHECON>(pu_out, G, st->ff, st->tol);
     if (threadIdx.x == 0) {
@@ -577,8 +581,10 @@ __global__ void __launch_bounds__(256)
 k_pcg_update2(int ns, const PcgState *__restrict__ st, const double *__restrict__ d, double *__restrict__ p,
               float2 *__restrict__ ps)
 {
+    pdl_enter();
     if (st->stop2) return;
     update2_block(blockIdx.x, gridDim.x, ns, st->beta, d, p, ps);
+    pdl_exit();
 }
 
 // ---------------------------------------------------------------------------
@@ -939,9 +945,11 @@ static int launch_products(Ctx &c, int prec, const double *p, const PcgState *st
     if (prec == PREC_FP64 && c.kmfix) return launch_elem_fix(c, p, st);
     const int grid = grid_for(c, c.nels, 8, 8);
     if (prec == PREC_FP32_FULL)
-        k_elem<float, true><<<grid, 256, 0, c.stream>>>(c.nels, c.km32, c.conn, p, (float *)c.utemp, st);
+        launch_dependent(c.dependent && st, c.stream, grid, 256, 0, k_elem<float, true>, c.nels, c.km32, c.conn, p, (float *)c.utemp,
+                         st);
     else
-        k_elem<double, true><<<grid, 256, 0, c.stream>>>(c.nels, c.km64, c.conn, p, (double *)c.utemp, st);
+        launch_dependent(c.dependent && st, c.stream, grid, 256, 0, k_elem<double, true>, c.nels, c.km64, c.conn, p,
+                         (double *)c.utemp, st);
     return check_launch(c, "k_elem");
 }
 
@@ -1019,18 +1027,15 @@ int launch_pcg_init(Ctx &c, const double *rhs, double *xsol, int stop_mode, doub
 
 int launch_update1(Ctx &c, double *xsol)
 {
-    if (c.stop_mode == STOP_CHECON)
-        k_pcg_update1<true><<<c.G, 256, 0, c.stream>>>(c.nslots, c.st, c.count + 1, c.part_u, c.G, xsol, c.r, c.d, c.p,
-                                                       c.u, c.dinv);
-    else
-        k_pcg_update1<false><<<c.G, 256, 0, c.stream>>>(c.nslots, c.st, c.count + 1, c.part_u, c.G, xsol, c.r, c.d, c.p,
-                                                        c.u, c.dinv);
+    launch_dependent(c.dependent, c.stream, c.G, 256, 0, c.stop_mode == STOP_CHECON ? k_pcg_update1<true> : k_pcg_update1<false>,
+                     c.nslots, c.st, c.count + 1, c.part_u, c.G, xsol, c.r, c.d, c.p, c.u, c.dinv);
     return check_launch(c, "k_pcg_update1");
 }
 
 int launch_update2(Ctx &c)
 {
-    k_pcg_update2<<<c.G, 256, 0, c.stream>>>(c.nslots, c.st, c.d, c.p, c.shared ? c.psplit : nullptr);
+    launch_dependent(c.dependent, c.stream, c.G, 256, 0, k_pcg_update2, c.nslots, c.st, c.d, c.p,
+                     c.shared ? c.psplit : nullptr);
     return check_launch(c, "k_pcg_update2");
 }
 

@@ -63,6 +63,7 @@ __global__ void __launch_bounds__(256)
 k_elem8(int nels, const double *__restrict__ kc, const int *__restrict__ conn, const double *__restrict__ p,
         double *__restrict__ ut, const PcgState *__restrict__ st)
 {
+    pdl_enter();
     if (st && st->stop) return;
     const int i = threadIdx.x & 7;
     const unsigned gmask = 0xFFu << (threadIdx.x & 24);   // the 8 lanes of this element
@@ -108,6 +109,7 @@ k_scatter1(int nn, const int *__restrict__ ptr, const int *__restrict__ list, co
             loc = fma(rv, rv, loc);
         }
     }
+    pdl_exit();
     scatter_tail(loc, part, MODE == 0 ? st : nullptr, count);
 }
 
@@ -174,8 +176,8 @@ int launch_form_storkc(Ctx &c, int nip, double kx, double ky, double kz)
 
 int launch_elem8(Ctx &c, const double *p, const PcgState *st)
 {
-    k_elem8<<<grid8(c, (long long)c.nels * 8, 256, 8), 256, 0, c.stream>>>(c.nels, c.km64, c.conn, p,
-                                                                           (double *)c.utemp, st);
+    launch_dependent(c.dependent && st, c.stream, grid8(c, (long long)c.nels * 8, 256, 8), 256, 0, k_elem8, c.nels, c.km64, c.conn, p,
+                     (double *)c.utemp, st);
     return launched8(c, "k_elem8");
 }
 

@@ -69,7 +69,8 @@ k_elem_shared64(int nels, const double *__restrict__ km, const int *__restrict__
                 const double *__restrict__ p, double *__restrict__ ut, const PcgState *__restrict__ st)
 {
     __shared__ __align__(16) double ks[3600];
-    if (block_stopped(st)) return;
+    pdl_enter();
+    if (st && st->stop) return;
     for (int i = threadIdx.x; i < 3600; i += blockDim.x) ks[i] = km[i];
     __syncthreads();
     const int lane = threadIdx.x & 31;
@@ -132,6 +133,7 @@ k_elem_shared_tc(int nels, const float *__restrict__ km32, const int *__restrict
     int *s_count = reinterpret_cast<int *>(tslot + 2);   // [0] copies issued, [1] MMA groups committed
     int *s_stop = s_count + 2;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    pdl_enter();
     if (tid == 0) *s_stop = st ? st->stop : 0;
     __syncthreads();
     if (*s_stop) return;   // uniform: read once per block
@@ -397,7 +399,7 @@ int launch_elem_shared(Ctx &c, int prec, const double *p, const PcgState *st)
         long long g = ((long long)c.nels + 7) / 8;
         if (g > (long long)c.nsm * 8) g = (long long)c.nsm * 8;
         if (g < 1) g = 1;
-        k_elem_shared64<<<(int)g, 256, 0, c.stream>>>(c.nels, c.skm64, c.conn, p, (double *)c.utemp, st);
+        launch_dependent(c.dependent && st, c.stream, (int)g, 256, 0, k_elem_shared64, c.nels, c.skm64, c.conn, p, (double *)c.utemp, st);
     } else {
         if (!c.shared_attr) {   // set once, before any stream capture
             e = cudaFuncSetAttribute(k_elem_shared_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kSSmem);
@@ -416,8 +418,8 @@ int launch_elem_shared(Ctx &c, int prec, const double *p, const PcgState *st)
         }
         const int ntiles = (c.nels + kNT - 1) / kNT;
         const int grid = ntiles < c.nsm ? ntiles : c.nsm;
-        k_elem_shared_tc<<<grid, kSThreads, kSSmem, c.stream>>>(c.nels, c.skm32, c.conn, c.psplit, (float *)c.utemp,
-                                                                 st, c.kerr);
+        launch_dependent(c.dependent && st, c.stream, grid, kSThreads, kSSmem, k_elem_shared_tc, c.nels, c.skm32, c.conn, c.psplit,
+                         (float *)c.utemp, st, c.kerr);
     }
     c.launches++;
     e = cudaGetLastError();

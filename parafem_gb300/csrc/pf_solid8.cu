@@ -22,6 +22,7 @@ __global__ void __launch_bounds__(256)
 k_elem24(int nels, const double *__restrict__ km, const int *__restrict__ conn, const double *__restrict__ p,
          double *__restrict__ ut, const PcgState *__restrict__ st)
 {
+    pdl_enter();
     if (st && st->stop) return;
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -68,6 +69,7 @@ k_scatter3_fix(int nn, const int *__restrict__ ptr, const int *__restrict__ list
             loc = fma(p[s], uv, loc);
         }
     }
+    pdl_exit();
     scatter_tail(loc, part, st, count);
 }
 
@@ -86,7 +88,8 @@ int launch_elem24(Ctx &c, const double *p, const PcgState *st)
 {
     long long g = ((long long)c.nels + 7) / 8;
     if (g > (long long)c.nsm * 8) g = (long long)c.nsm * 8;
-    k_elem24<<<(int)(g < 1 ? 1 : g), 256, 0, c.stream>>>(c.nels, c.km64, c.conn, p, (double *)c.utemp, st);
+    launch_dependent(c.dependent && st, c.stream, (int)(g < 1 ? 1 : g), 256, 0, k_elem24, c.nels, c.km64, c.conn, p,
+                     (double *)c.utemp, st);
     return launched24(c, "k_elem24");
 }
 
