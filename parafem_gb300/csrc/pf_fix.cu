@@ -184,6 +184,82 @@ k_elem_fix(int nels, const unsigned char *__restrict__ rec, const int *__restric
     }
 }
 
+// K_e P_e for the k load cases of P (slot-major, P[slot * k + j]) into
+// ut[(60 e + i) * k + j]: k_elem_fix with the cases inside the element, so
+// that a record is read once for all of them and the products are bitwise
+// those of the single-case kernel.  Bound by instruction issue (1.8 ns per
+// element and case over the chip, against 6.3 ns by FP64 FMA).
+__global__ void __launch_bounds__(kFixWarps * 32, 1)
+k_mr_elem_fix(int nels, int nk, const unsigned char *__restrict__ rec, const int *__restrict__ conn,
+              const double *__restrict__ P, double *__restrict__ ut, int *__restrict__ err)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned char *stage = smem + (size_t)w * 3 * fx::kChunk0;
+    int4 *pq = reinterpret_cast<int4 *>(smem + (size_t)kFixWarps * 3 * fx::kChunk0) + w * 60;
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + (size_t)kFixWarps * (3 * fx::kChunk0 + 960)) + 3 * w;
+    const int per_cta = (nels + gridDim.x - 1) / gridDim.x;
+    const int first = blockIdx.x * per_cta + w, e1 = min(nels, (int)(blockIdx.x + 1) * per_cta);
+    if (first >= e1) return;
+    if (lane == 0) {
+        for (int c = 0; c < 3; ++c) tc::mbar_init(&bar[c], 1);
+        tc::mbar_fence_init();
+    }
+    __syncwarp();
+    const uint64_t pol = tc::l2_evict_first_policy();
+    auto issue = [&](int c, int e) {
+        tc::mbar_expect_tx(&bar[c], fx::chunk_bytes(c));
+        tc::bulk_g2s_hint(stage + c * fx::kChunk0, rec + (size_t)e * fx::kRecBytes + fx::chunk_off(c), fx::chunk_bytes(c),
+                          &bar[c], pol);
+    };
+    if (lane == 0)
+        for (int c = 0; c < 3; ++c) issue(c, first);
+    const int l = lane < 30 ? lane : 29;
+    bool ok = true;
+    uint32_t parity = 0;
+    int e = first, chunk = 0, j = 0;
+    for (; e < e1 && ok; e += kFixWarps, parity ^= 1) {
+        const int nd = lane < 20 ? conn[(size_t)e * 20 + lane] : 0;
+        const int n0 = __shfl_sync(FULLMASK, nd, 2 * l / 3), n1 = __shfl_sync(FULLMASK, nd, (2 * l + 1) / 3);
+        const double *qa = P + ((size_t)3 * n0 + 2 * l % 3) * nk, *qb = P + ((size_t)3 * n1 + (2 * l + 1) % 3) * nk;
+        double pa = qa[0], pb = qb[0];
+        double *o = ut + ((size_t)e * 60 + 2 * l) * nk;
+        for (j = 0; j < nk; ++j) {
+            const int jn = j + 1 < nk ? j + 1 : j;
+            const double na = qa[jn], nb = qb[jn];   // of the next case
+            double u0, u1;
+            ok = fx::product(
+                lane, pa, pb, pq,
+                [&](int c) -> const unsigned char * {
+                    if (j > 0) return stage + c * fx::kChunk0;
+                    chunk = c;
+                    return __all_sync(FULLMASK, tc::mbar_wait(&bar[c], parity)) ? stage + c * fx::kChunk0 : nullptr;
+                },
+                [&](int c) {
+                    if (j + 1 < nk) return;
+                    __syncwarp();   // every lane is done with the stage
+                    if (lane == 0 && e + kFixWarps < e1) {
+                        tc::fence_proxy_async();
+                        issue(c, e + kFixWarps);
+                    }
+                },
+                u0, u1);
+            if (!ok) break;
+            if (lane < 30) {
+                o[j] = u0;
+                o[nk + j] = u1;
+            }
+            pa = na;
+            pb = nb;
+        }
+        if (!ok) break;
+    }
+    if (!ok) {   // in the first case of element e: chunks from `chunk` on are in flight
+        if (lane == 0) atomicExch(err, 2);
+        for (int c = chunk; c < 3; ++c) tc::mbar_wait(&bar[c], parity);
+    }
+}
+
 // The same with one record for every element (PCG_KM), held in shared
 // memory; bitwise the products of k_elem_fix on copies of it.  Bound by
 // instruction issue: 0.93 ms on an 80^3 cube, k_elem_shared64 3.29 ms.
@@ -236,21 +312,38 @@ int launch_pack_storkm(Ctx &c, int nels, const double *km, float *kp, unsigned c
     return fix_launched(c, "k_pack_storkm");
 }
 
+// Shared-memory attributes of the bulk-copy kernels, set once per context by
+// their first products, which are outside any stream capture.
+static int fix_attributes(Ctx &c)
+{
+    if (c.fix_attr) return 0;
+    cudaError_t e = cudaFuncSetAttribute(k_elem_fix, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFixSmem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_mr_elem_fix, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFixSmem);
+    if (e != cudaSuccess) {
+        set_error("fixed-point products: cannot reserve %zu bytes of shared memory: %s", kFixSmem, cudaGetErrorString(e));
+        return 1;
+    }
+    c.fix_attr = true;
+    return 0;
+}
+
 int launch_elem_fix(Ctx &c, const double *p, const PcgState *st)
 {
-    if (!c.fix_attr) {   // set once, by the first product, which is outside any stream capture
-        const cudaError_t e = cudaFuncSetAttribute(k_elem_fix, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFixSmem);
-        if (e != cudaSuccess) {
-            set_error("k_elem_fix: cannot reserve %zu bytes of shared memory: %s", kFixSmem, cudaGetErrorString(e));
-            return 1;
-        }
-        c.fix_attr = true;
-    }
+    if (fix_attributes(c)) return 1;
     // one CTA per SM, and on small meshes as few warps per SM as the mesh has
     const int grid = c.nels < c.nsm ? c.nels : c.nsm;
     launch_dependent(c.dependent && st, c.stream, grid, kFixWarps * 32, kFixSmem, k_elem_fix, c.nels, c.kmfix, c.conn, p,
                      (double *)c.utemp, st, c.kerr);
     return fix_launched(c, "k_elem_fix");
+}
+
+int launch_mr_elem_fix(Ctx &c, int k, const double *P, double *ut)
+{
+    if (fix_attributes(c)) return 1;
+    const int grid = c.nels < c.nsm ? c.nels : c.nsm;
+    k_mr_elem_fix<<<grid, kFixWarps * 32, kFixSmem, c.stream>>>(c.nels, k, c.kmfix, c.conn, P, ut, c.kerr);
+    return fix_launched(c, "k_mr_elem_fix");
 }
 
 int launch_elem_shared_fix(Ctx &c, const double *p, const PcgState *st)

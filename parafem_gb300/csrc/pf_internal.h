@@ -173,6 +173,7 @@ int ensure_km32(Ctx &c);   // the full FP32 storkm, if storkm changed; outside s
 int launch_pack_storkm(Ctx &c, int nels, const double *km, float *kp, unsigned char *rec, int *bad);
 int launch_elem_fix(Ctx &c, const double *p, const PcgState *st);
 int launch_elem_shared_fix(Ctx &c, const double *p, const PcgState *st);
+int launch_mr_elem_fix(Ctx &c, int k, const double *P, double *ut);   // k cases, P[slot * k + j] -> ut[(60 e + i) * k + j]
 int launch_assemble_diag(Ctx &c);
 int launch_eq_to_slot(Ctx &c, const double *eq, double *slot);
 int launch_slot_to_eq(Ctx &c, const double *slot, double *eq);

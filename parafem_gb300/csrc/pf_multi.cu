@@ -682,10 +682,23 @@ k_mr_elem_cc(int nels, int k, const KT *__restrict__ km, const int *__restrict__
 // grid-stride loop.
 __host__ __device__ inline int case_threads(int k) { return k * (256 / k); }
 
+// Per-case state.  Written by the last block of the scatter (alpha) and of
+// update1 (the rest), when every block has read what it needs.
+struct MState {
+    double up[kMaxK], ff[kMaxK], rr[kMaxK], thr[kMaxK];
+    double alpha[kMaxK], beta[kMaxK];   // this iteration's step lengths (0 for inactive cases)
+    int active[kMaxK];   // 1 until the case's true residual reaches tol
+    int flag[kMaxK];     // recursive residual reached thr (replacement wanted)
+    int iters[kMaxK];
+    int any_flag;        // stop iterating: some active case wants a replacement
+    int any_flag2;       // the same one iteration later, for update2 (it completes P in the last one)
+    int err;
+};
+
 // Sums NV per-thread values over the threads of each case in thread order
-// (kinds bit = max) and writes part[v * stride + blockIdx.x * k + j].
+// and writes part[v * stride + blockIdx.x * k + j].
 template <int NV>
-__device__ __forceinline__ void case_block_reduce(double (&v)[NV], unsigned kinds, double *out, size_t stride, int k)
+__device__ __forceinline__ void case_block_reduce(double (&v)[NV], double *out, size_t stride, int k)
 {
     __shared__ double sh[NV][256];
 #pragma unroll
@@ -696,14 +709,42 @@ __device__ __forceinline__ void case_block_reduce(double (&v)[NV], unsigned kind
 #pragma unroll
         for (int q = 0; q < NV; ++q) {
             double s = 0.0;
-            for (int g = 0; g < ng; ++g) {
-                const double x = sh[q][g * k + threadIdx.x];
-                s = ((kinds >> q) & 1) ? fmax(s, x) : s + x;
-            }
+            for (int g = 0; g < ng; ++g) s += sh[q][g * k + threadIdx.x];
             out[q * stride + (size_t)blockIdx.x * k + threadIdx.x] = s;
         }
     }
     __syncthreads();
+}
+
+// Per-case sums of the partials of G blocks (value q of case j and block b at
+// part[q * stride + b * k + j]), by one block of case_threads(k) threads:
+// thread (g, j) adds the partials g, g + ng, ... of case j in four running
+// sums, which keeps the loads and the slow FP64 adds of a long list in
+// flight, then thread j adds the ng groups.  Fixed order.  Valid in threads
+// 0..k-1.
+template <int NV>
+__device__ __forceinline__ void case_sums(const double *part, size_t stride, int G, int k, double (&v)[NV])
+{
+    __shared__ double sh[NV][256];
+    const int ng = blockDim.x / k, j = threadIdx.x % k, g = threadIdx.x / k;
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+        const double *p = part + q * stride + j;
+        double s[4] = {0.0, 0.0, 0.0, 0.0};
+        int b = g;
+        for (; b + 3 * ng < G; b += 4 * ng)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s[i] += __ldcg(p + (size_t)(b + i * ng) * k);
+        for (; b < G; b += ng) s[0] += __ldcg(p + (size_t)b * k);
+        sh[q][threadIdx.x] = (s[0] + s[1]) + (s[2] + s[3]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+        v[q] = 0.0;
+        if ((int)threadIdx.x < k)
+            for (int i = 0; i < ng; ++i) v[q] += sh[q][i * k + threadIdx.x];
+    }
 }
 
 // Node scatter for k load cases: thread (node, j), ascending element order.
@@ -712,9 +753,9 @@ template <typename UT, int MODE>
 __global__ void __launch_bounds__(256)
 k_mr_scatter(int nn, int k, const int *__restrict__ ptr, const int *__restrict__ list, const UT *__restrict__ ut,
              const uint8_t *__restrict__ fm, const double *__restrict__ pf, double *__restrict__ out,
-             double *__restrict__ part, const int *__restrict__ skip)
+             double *__restrict__ part, MState *st, unsigned *__restrict__ count)
 {
-    if (skip && *skip) return;   // uniform: the flag does not change during the kernel
+    if (st && st->any_flag) return;   // uniform: the flag does not change during the kernel
     const int j = threadIdx.x % k;
     double loc = 0.0;
     // the block size is a multiple of k: a thread's case stays j and its
@@ -724,11 +765,20 @@ k_mr_scatter(int nn, int k, const int *__restrict__ ptr, const int *__restrict__
     int n = (int)(t0 / k);
     for (size_t t = t0; t < (size_t)nn * k; t += stride, n += dn) {
         UT a0 = 0, a1 = 0, a2 = 0;   // FP32 products are summed in FP32, FP64 ones in FP64
-        for (int q = ptr[n]; q < ptr[n + 1]; ++q) {
-            const size_t base = (size_t)list[q] * 3 * k + j;   // list holds e*20+a
-            a0 += ut[base];
-            a1 += ut[base + k];
-            a2 += ut[base + 2 * k];
+        const int q1 = ptr[n + 1];
+        for (int q = ptr[n]; q < q1; q += 2) {   // two contributions in flight, added in order
+            const bool two = q + 1 < q1;
+            const UT *u0 = ut + (size_t)list[q] * 3 * k + j;   // list holds e*20+a
+            const UT *u1 = two ? ut + (size_t)list[q + 1] * 3 * k + j : u0;
+            const UT x0 = u0[0], y0 = u0[k], z0 = u0[2 * k], x1 = u1[0], y1 = u1[k], z1 = u1[2 * k];
+            a0 += x0;
+            a1 += y0;
+            a2 += z0;
+            if (two) {
+                a0 += x1;
+                a1 += y1;
+                a2 += z1;
+            }
         }
         const int m = fm[n];
         const double a[3] = {(double)a0, (double)a1, (double)a2};
@@ -748,47 +798,11 @@ k_mr_scatter(int nn, int k, const int *__restrict__ ptr, const int *__restrict__
         }
     }
     double v[1] = {loc};
-    case_block_reduce<1>(v, 0u, part, 0, k);
-}
-
-// per-case state
-struct MState {
-    double up[kMaxK], ff[kMaxK], rr[kMaxK], thr[kMaxK];
-    double alpha[kMaxK], beta[kMaxK];   // this iteration's step lengths (0 for inactive cases)
-    int active[kMaxK];   // 1 until the case's true residual reaches tol
-    int flag[kMaxK];     // recursive residual reached thr (replacement wanted)
-    int iters[kMaxK];
-    int any_flag;        // stop iterating: some active case wants a replacement
-    int pending;         // set by this iteration's k_mr_beta, moved to any_flag by k_mr_finish
-    int err;
-};
-
-// per-case sums of block partials (fixed order)
-__device__ __forceinline__ double case_sum(const double *part, int G, int j, int k)
-{
-    double s = 0.0;
-    for (int b = 0; b < G; ++b) s += part[(size_t)b * k + j];
-    return s;
-}
-
-// The same sums by one 256-thread block: thread (g, j) adds partials g, g+ng,
-// ... of case j (ng = 256 / k groups), then thread j adds the ng group sums
-// in order.  Fixed order, so the result is the same in every run.  Valid in
-// threads 0..k-1.
-__device__ __forceinline__ double case_sum_block(const double *part, int G, double *sh, int k)
-{
-    const int ng = 256 / k;
-    const int j = threadIdx.x % k, g = threadIdx.x / k;
-    double s = 0.0;
-    if (g < ng)
-        for (int b = g; b < G; b += ng) s += part[(size_t)b * k + j];
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    double t = 0.0;
-    if ((int)threadIdx.x < k)
-        for (int i = 0; i < ng; ++i) t += sh[i * k + threadIdx.x];
-    __syncthreads();
-    return t;
+    case_block_reduce<1>(v, part, 0, k);
+    // in a solve the last block forms alpha = up / (p.u) per case
+    if (!st || !last_block(count)) return;
+    case_sums<1>(part, 0, gridDim.x, k, v);
+    if ((int)threadIdx.x < k) st->alpha[threadIdx.x] = st->active[threadIdx.x] ? st->up[threadIdx.x] / v[0] : 0.0;
 }
 
 __global__ void __launch_bounds__(256)
@@ -813,13 +827,16 @@ k_mr_init(int ns, int k, const double *__restrict__ F, const double *__restrict_
         rr = fma(rv, rv, rr);
     }
     double v[2] = {rd, rr};
-    case_block_reduce<2>(v, 0u, part, (size_t)G * k, k);
+    case_block_reduce<2>(v, part, (size_t)G * k, k);
 }
 
 __global__ void k_mr_init2(MState *st, const double *__restrict__ part, int G, int k, double tol)
 {
-    for (int j = threadIdx.x; j < k; j += blockDim.x) {
-        const double rd = case_sum(part, G, j, k), rr = case_sum(part + (size_t)G * k, G, j, k);
+    double v[2];
+    case_sums<2>(part, (size_t)G * k, G, k, v);
+    const int j = threadIdx.x;
+    if (j < k) {
+        const double rd = v[0], rr = v[1];
         st->up[j] = rd;
         st->ff[j] = rr;
         st->rr[j] = rr;
@@ -829,34 +846,27 @@ __global__ void k_mr_init2(MState *st, const double *__restrict__ part, int G, i
         st->iters[j] = 0;
     }
     if (threadIdx.x == 0) {
-        st->any_flag = 0;
-        st->pending = 0;
+        st->any_flag = st->any_flag2 = 0;
         st->err = 0;
     }
 }
 
-// alpha = up / (p.u) per case, from the scatter's partials (one block)
-__global__ void __launch_bounds__(256) k_mr_alpha(MState *st, const double *__restrict__ ps, int Gs, int k)
-{
-    __shared__ double sh[256];
-    if (st->any_flag) return;
-    const double pu = case_sum_block(ps, Gs, sh, k);
-    const int j = threadIdx.x;
-    if (j < k) st->alpha[j] = st->active[j] ? st->up[j] / pu : 0.0;
-}
-
 __global__ void __launch_bounds__(256)
-k_mr_update1(int ns, int k, const MState *__restrict__ st, double *__restrict__ pu_out, int G, double *__restrict__ X,
-             double *__restrict__ R, double *__restrict__ D, const double *__restrict__ P,
+k_mr_update1(int ns, int k, MState *st, unsigned *__restrict__ count, int limit, double *__restrict__ pu_out, int G,
+             double *__restrict__ X, double *__restrict__ R, double *__restrict__ D, const double *__restrict__ P,
              const double *__restrict__ U, const double *__restrict__ dinv)
 {
-    if (st->any_flag) return;
+    if (st->any_flag) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) st->any_flag2 = 1;   // read by update2 only
+        return;
+    }
     const int j = threadIdx.x % k;
     const double alpha = st->alpha[j];
     double rd = 0.0, rr = 0.0;
     const size_t stride = (size_t)gridDim.x * blockDim.x, t0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     const size_t ds = stride / k;   // the block size is a multiple of k
     size_t s = t0 / k;
+#pragma unroll 2
     for (size_t t = t0; t < (size_t)ns * k; t += stride, s += ds) {
         X[t] = fma(P[t], alpha, X[t]);
         const double rn = fma(-U[t], alpha, R[t]);
@@ -867,37 +877,32 @@ k_mr_update1(int ns, int k, const MState *__restrict__ st, double *__restrict__ 
         rr = fma(rn, rn, rr);
     }
     double v[2] = {rd, rr};
-    case_block_reduce<2>(v, 0u, pu_out, (size_t)G * k, k);
-}
-
-// r.d and r.r per case; beta = (r.d)_new / up; the new up, rr and iteration
-// count; the stopping test (one block).  The flag raised here reaches
-// any_flag only in k_mr_finish, after this iteration's k_mr_update2.
-__global__ void __launch_bounds__(256) k_mr_beta(MState *st, const double *__restrict__ part, int G, int k, int limit)
-{
-    __shared__ double sh[256];
+    case_block_reduce<2>(v, pu_out, (size_t)G * k, k);
+    // The last block: r.d and r.r per case; beta = (r.d)_new / up; the new up,
+    // rr and iteration count; the stopping test.  (As one-block kernels of
+    // their own these and alpha took 28 us of a 180 us iteration at 28^3 x 16.)
+    if (!last_block(count)) return;
     __shared__ int s_any;
-    if (st->any_flag) return;
     if (threadIdx.x == 0) s_any = 0;
-    const double rd = case_sum_block(part, G, sh, k);
-    const double rr = case_sum_block(part + (size_t)G * k, G, sh, k);
-    const int j = threadIdx.x;
-    if (j < k) {
-        if (st->active[j]) {
-            st->beta[j] = rd / st->up[j];
-            st->up[j] = rd;
-            st->rr[j] = rr;
-            st->iters[j] += 1;
-            const bool f = sqrt(rr) / sqrt(st->ff[j]) <= st->thr[j] || st->iters[j] >= limit || !isfinite(rd);
-            st->flag[j] = f ? 1 : 0;
-            if (!isfinite(rd)) st->err = 1;
+    case_sums<2>(pu_out, (size_t)G * k, G, k, v);
+    if ((int)threadIdx.x < k) {
+        const int c = threadIdx.x;
+        if (st->active[c]) {
+            const double rdn = v[0], rrn = v[1];
+            st->beta[c] = rdn / st->up[c];
+            st->up[c] = rdn;
+            st->rr[c] = rrn;
+            st->iters[c] += 1;
+            const bool f = sqrt(rrn) / sqrt(st->ff[c]) <= st->thr[c] || st->iters[c] >= limit || !isfinite(rdn);
+            st->flag[c] = f ? 1 : 0;
+            if (!isfinite(rdn)) st->err = 1;
             if (f) atomicOr(&s_any, 1);
         } else {
-            st->beta[j] = 0.0;
+            st->beta[c] = 0.0;
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0 && s_any) st->pending = 1;
+    if (threadIdx.x == 0 && s_any) st->any_flag = 1;
 }
 
 // p = d + beta p for the active cases, with p's FP32 high and low parts
@@ -906,10 +911,11 @@ __global__ void __launch_bounds__(256)
 k_mr_update2(int ns, int k, const MState *__restrict__ st, const double *__restrict__ D, double *__restrict__ P,
              float2 *__restrict__ Ps)
 {
-    if (st->any_flag) return;
+    if (st->any_flag2) return;
     const int j = threadIdx.x % k;
     const double beta = st->beta[j];
     if (!st->active[j]) return;   // this thread's case is fixed
+#pragma unroll 4
     for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < (size_t)ns * k;
          t += (size_t)gridDim.x * blockDim.x) {
         const double pn = fma(P[t], beta, D[t]);
@@ -927,14 +933,6 @@ __global__ void k_mr_psplit(size_t n, const double *__restrict__ P, float2 *__re
         float h, l;
         split_f64(P[t], h, l);
         Ps[t] = make_float2(h, l);
-    }
-}
-
-__global__ void k_mr_finish(MState *st)
-{
-    if (threadIdx.x == 0 && !st->any_flag && st->pending) {
-        st->any_flag = 1;
-        st->pending = 0;
     }
 }
 
@@ -959,26 +957,29 @@ k_mr_replace(int ns, int k, const MState *__restrict__ st, const double *__restr
         rr = fma(rv, rv, rr);
     }
     double v[2] = {rd, rr};
-    case_block_reduce<2>(v, 0u, part, (size_t)G * k, k);
+    case_block_reduce<2>(v, part, (size_t)G * k, k);
 }
 
 __global__ void k_mr_replace2(MState *st, const double *__restrict__ part, int G, int k)
 {
-    for (int j = threadIdx.x; j < k; j += blockDim.x)
-        if (st->active[j]) {
-            st->up[j] = case_sum(part, G, j, k);
-            st->rr[j] = case_sum(part + (size_t)G * k, G, j, k);
-            st->flag[j] = 0;
-        }
+    double v[2];
+    case_sums<2>(part, (size_t)G * k, G, k, v);
+    const int j = threadIdx.x;
+    if (j < k && st->active[j]) {
+        st->up[j] = v[0];
+        st->rr[j] = v[1];
+        st->flag[j] = 0;
+    }
     if (threadIdx.x == 0) {
-        st->any_flag = 0;
-        st->pending = 0;
+        st->any_flag = st->any_flag2 = 0;
     }
 }
 
 __global__ void k_mr_sums(const double *__restrict__ part, int G, int k, double *__restrict__ out)
 {
-    for (int j = threadIdx.x; j < k; j += blockDim.x) out[j] = case_sum(part, G, j, k);
+    double v[1];
+    case_sums<1>(part, 0, G, k, v);
+    if ((int)threadIdx.x < k) out[threadIdx.x] = v[0];
 }
 
 __global__ void k_mr_eq_to_slot(int ns, int k, const int *__restrict__ slot_eq, int neq, const double *__restrict__ Req,
@@ -1005,6 +1006,7 @@ __global__ void k_mr_slot_to_eq(int neq, int k, const int *__restrict__ eq_slot,
 // ---------------------------------------------------------------------------
 // Block-solve buffers of one context (Ctx::multi), allocated on the first
 // block solve or product and kept while the mesh and k are unchanged.
+constexpr int kMrVecBlocks = 6, kMrScatterBlocks = 4;   // most blocks per SM (8, 16, 32 scatter blocks: 4, 12, 37 us more)
 struct MultiBufs {
     int ns = 0, ne = 0, k = 0;
     double *F = nullptr, *X = nullptr, *R = nullptr, *D = nullptr, *P = nullptr, *U = nullptr, *RR = nullptr,
@@ -1015,6 +1017,8 @@ struct MultiBufs {
     double *ut64 = nullptr, *part = nullptr, *sums = nullptr;
     MState *st = nullptr;
     MState *hst = nullptr;
+    unsigned *count = nullptr;      // [2] arrivals of the blocks of the scatter and of update1 (last_block)
+    int G = 0, Gs = 0;              // blocks of the vector kernels and of the scatter
     // TMA maps of Ps for the tensor-core product's gathers: rows of one node
     // (box 3k x 1, passes over all k cases) and rows of one slot (box kb x 1
     // for kb = 8, 16, 32, 64); bit 0 / bit 1 + i set once encoded for Ps
@@ -1030,7 +1034,7 @@ struct MultiBufs {
 namespace {
 void mb_free_vectors(MultiBufs &m)
 {
-    void *p[] = {m.F, m.X, m.R, m.D, m.P, m.U, m.RR, m.eq, m.ut32, m.Ps, m.ut64, m.part, m.sums, m.st};
+    void *p[] = {m.F, m.X, m.R, m.D, m.P, m.U, m.RR, m.eq, m.ut32, m.Ps, m.ut64, m.part, m.sums, m.st, m.count};
     for (void *q : p)
         if (q) cudaFree(q);
     if (m.hst) cudaFreeHost(m.hst);
@@ -1039,6 +1043,7 @@ void mb_free_vectors(MultiBufs &m)
     m.Ps = nullptr;
     m.st = nullptr;
     m.hst = nullptr;
+    m.count = nullptr;
     m.ns = 0;
     m.k = 0;
     m.kb = 0;
@@ -1202,28 +1207,26 @@ static int mr_elem(Ctx &c, int prec, const double *P, const int *skip)
         k_mr_elem_cc<float, float><<<grid, 256, 0, c.stream>>>(c.nels, m.k, c.km32, c.conn, P, m.ut32, skip);
         return mr_launched(c, "k_mr_elem_cc<float>");
     }
+    if (c.kmfix) return launch_mr_elem_fix(c, m.k, P, m.ut64);   // outside the iterations: no flag
     k_mr_elem_cc<double, double><<<grid, 256, 0, c.stream>>>(c.nels, m.k, c.km64, c.conn, P, m.ut64, skip);
     return mr_launched(c, "k_mr_elem_cc<double>");
 }
 
-static int mr_scatter(Ctx &c, int prec, int mode, const double *pf, double *out, const int *skip)
+// st: the solve's state (null for a product of its own and for residuals)
+static int mr_scatter(Ctx &c, int prec, int mode, const double *pf, double *out, MState *st)
 {
     MultiBufs &m = *c.multi;
-    const int G = c.Gs, T = case_threads(m.k);
+    const int G = m.Gs, T = case_threads(m.k);
     if (prec == 64) {
         if (mode == 0)
             k_mr_scatter<double, 0><<<G, T, 0, c.stream>>>(c.nn, m.k, c.node_ptr, c.node_list, m.ut64, c.freemask, pf,
-                                                          out, m.part, skip);
+                                                          out, m.part, st, m.count);
         else
             k_mr_scatter<double, 1><<<G, T, 0, c.stream>>>(c.nn, m.k, c.node_ptr, c.node_list, m.ut64, c.freemask, pf,
-                                                          out, m.part, skip);
+                                                          out, m.part, st, m.count);
     } else {
-        if (mode == 0)
-            k_mr_scatter<float, 0><<<G, T, 0, c.stream>>>(c.nn, m.k, c.node_ptr, c.node_list, m.ut32, c.freemask, pf,
-                                                         out, m.part, skip);
-        else
-            k_mr_scatter<float, 1><<<G, T, 0, c.stream>>>(c.nn, m.k, c.node_ptr, c.node_list, m.ut32, c.freemask, pf,
-                                                         out, m.part, skip);
+        k_mr_scatter<float, 0><<<G, T, 0, c.stream>>>(c.nn, m.k, c.node_ptr, c.node_list, m.ut32, c.freemask, pf, out,
+                                                     m.part, st, m.count);
     }
     return mr_launched(c, "k_mr_scatter");
 }
@@ -1245,7 +1248,16 @@ static int mr_alloc(Ctx &c, int k)
     if (m.ns == c.nslots && m.k == k && m.F) return 0;
     mb_free_vectors(m);
     const size_t n = (size_t)c.nslots * k;
-    const size_t parts = (size_t)(c.Gs > c.G ? c.Gs : c.G) * k * 4 + 64;
+    // blocks over (slot, case) and (node, case): enough to fill the SMs, few
+    // enough that the last block's sums over them stay short
+    const int T = case_threads(k);
+    auto blocks = [&](size_t n, int per_sm) {
+        const size_t g = (n * k + T - 1) / T, cap = (size_t)c.nsm * per_sm;
+        return (int)(g < 1 ? 1 : g < cap ? g : cap);
+    };
+    m.G = blocks(c.nslots, kMrVecBlocks);
+    m.Gs = blocks(c.nn, kMrScatterBlocks);
+    const size_t parts = (size_t)(m.Gs > m.G ? m.Gs : m.G) * k * 4 + 64;
     double **v[] = {&m.F, &m.X, &m.R, &m.D, &m.P, &m.U, &m.RR};
     for (double **q : v)
         if (ctx_malloc(c, (void **)q, n * 8)) goto fail;
@@ -1256,6 +1268,8 @@ static int mr_alloc(Ctx &c, int k)
     if (ctx_malloc(c, (void **)&m.part, parts * 8)) goto fail;
     if (ctx_malloc(c, (void **)&m.sums, kMaxK * 8)) goto fail;
     if (ctx_malloc(c, (void **)&m.st, sizeof(MState))) goto fail;
+    if (ctx_malloc(c, (void **)&m.count, 2 * sizeof(unsigned))) goto fail;
+    if (cudaMemset(m.count, 0, 2 * sizeof(unsigned)) != cudaSuccess) goto fail;
     if (cudaMallocHost((void **)&m.hst, sizeof(MState)) != cudaSuccess) goto fail;
     m.ns = c.nslots;
     m.k = k;
@@ -1323,7 +1337,7 @@ static int mr_true_residual(Ctx &c, double *rr_out)
     MultiBufs &m = *c.multi;
     if (mr_elem(c, 64, m.X, nullptr)) return 1;
     if (mr_scatter(c, 64, 1, m.F, m.RR, nullptr)) return 1;
-    k_mr_sums<<<1, 128, 0, c.stream>>>(m.part, c.Gs, m.k, m.sums);
+    k_mr_sums<<<1, case_threads(m.k), 0, c.stream>>>(m.part, m.Gs, m.k, m.sums);
     if (mr_launched(c, "k_mr_sums")) return 1;
     MCK(cudaMemcpyAsync(rr_out, m.sums, m.k * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
     MCK(cudaStreamSynchronize(c.stream));
@@ -1372,7 +1386,7 @@ try {
     }
     if (mr_alloc(c, k)) return PF_FAILURE;
     MultiBufs &m = *c.multi;
-    const int G = c.G, Gs = c.Gs, T = case_threads(k);
+    const int G = m.G, Gs = m.Gs, T = case_threads(k);
     // load cases: r(neq, k) column-major
     MCK(cudaMemcpyAsync(m.eq, r, (size_t)c.neq * k * 8, cudaMemcpyHostToDevice, c.stream));
     k_mr_eq_to_slot<<<c.nsm * 8, 256, 0, c.stream>>>(c.nslots, k, c.slot_eq, c.neq, m.eq, m.F);
@@ -1390,7 +1404,7 @@ try {
     MCK(cudaEventRecord(e0, c.stream));
     k_mr_init<<<G, T, 0, c.stream>>>(c.nslots, k, m.F, c.dinv, m.X, m.R, m.D, m.P, m.Ps, m.part, G);
     if (mr_launched(c, "k_mr_init")) return PF_FAILURE;
-    k_mr_init2<<<1, 128, 0, c.stream>>>(m.st, m.part, G, k, *tol);
+    k_mr_init2<<<1, T, 0, c.stream>>>(m.st, m.part, G, k, *tol);
     if (mr_launched(c, "k_mr_init2")) return PF_FAILURE;
     double *pu = m.part + (size_t)Gs * k;   // update partials after the scatter partials
     int total = 0, chunk = 4, corrections = 0;
@@ -1407,18 +1421,13 @@ try {
             MCK(cudaEventRecord(tev[3 * i], c.stream));
             if (mr_elem(c, *prec, m.P, skip)) return PF_FAILURE;
             MCK(cudaEventRecord(tev[3 * i + 1], c.stream));
-            if (mr_scatter(c, *prec, 0, m.P, m.U, skip)) return PF_FAILURE;
+            if (mr_scatter(c, *prec, 0, m.P, m.U, m.st)) return PF_FAILURE;
             MCK(cudaEventRecord(tev[3 * i + 2], c.stream));
-            k_mr_alpha<<<1, 256, 0, c.stream>>>(m.st, m.part, Gs, k);
-            if (mr_launched(c, "k_mr_alpha")) return PF_FAILURE;
-            k_mr_update1<<<G, T, 0, c.stream>>>(c.nslots, k, m.st, pu, G, m.X, m.R, m.D, m.P, m.U, c.dinv);
+            k_mr_update1<<<G, T, 0, c.stream>>>(c.nslots, k, m.st, m.count + 1, *limit, pu, G, m.X, m.R, m.D, m.P, m.U,
+                                                c.dinv);
             if (mr_launched(c, "k_mr_update1")) return PF_FAILURE;
-            k_mr_beta<<<1, 256, 0, c.stream>>>(m.st, pu, G, k, *limit);
-            if (mr_launched(c, "k_mr_beta")) return PF_FAILURE;
             k_mr_update2<<<G, T, 0, c.stream>>>(c.nslots, k, m.st, m.D, m.P, m.Ps);
             if (mr_launched(c, "k_mr_update2")) return PF_FAILURE;
-            k_mr_finish<<<1, 32, 0, c.stream>>>(m.st);
-            if (mr_launched(c, "k_mr_finish")) return PF_FAILURE;
         }
         total += chunk;
         MCK(cudaMemcpyAsync(m.hst, m.st, sizeof(MState), cudaMemcpyDeviceToHost, c.stream));
@@ -1457,7 +1466,7 @@ try {
         MCK(cudaMemcpyAsync(m.st, m.hst, sizeof(MState), cudaMemcpyHostToDevice, c.stream));
         k_mr_replace<<<G, T, 0, c.stream>>>(c.nslots, k, m.st, m.RR, c.dinv, m.R, m.D, m.part, G);
         if (mr_launched(c, "k_mr_replace")) return PF_FAILURE;
-        k_mr_replace2<<<1, 128, 0, c.stream>>>(m.st, m.part, G, k);
+        k_mr_replace2<<<1, T, 0, c.stream>>>(m.st, m.part, G, k);
         if (mr_launched(c, "k_mr_replace2")) return PF_FAILURE;
         ++corrections;
         chunk = 4;
