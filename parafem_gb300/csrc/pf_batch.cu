@@ -9,8 +9,9 @@
 //     every reduction (p.u, r.d, r.r, max|x|, max|dx|) is summed over the
 //     blocks of ONE mesh in a fixed order.  A mesh's partition depends on its
 //     own size only, so its result is bitwise the same alone and in any mix;
-//   * a one-block-per-mesh finish kernel does each mesh's bookkeeping and
-//     sets its stop flag; the next iterations skip stopped meshes.
+//   * the block of a mesh that arrives last in the scatter and in update1
+//     does the mesh's bookkeeping and sets its stop flag; the next iterations
+//     skip stopped meshes.
 // Requests are admitted while others iterate: their arrays are copied into
 // free arena ranges and their storkm is formed on the same stream, between
 // iterations of the running solves.  Converged solves retire at the next
@@ -52,7 +53,7 @@ struct BSeg {
 };
 
 constexpr int kScatterNodes = 256;   // nodes per scatter block
-constexpr int kVectorSlots = 2048;   // slots per vector block (8 per thread)
+constexpr int kVectorSlots = 1024;   // slots per vector block (4 per thread)
 
 __device__ __forceinline__ void elem_product(size_t e, int lane, const double *__restrict__ km,
                                              const int *__restrict__ conn, const double *__restrict__ p,
@@ -83,11 +84,12 @@ __device__ __forceinline__ void elem_product(size_t e, int lane, const double *_
     }
 }
 
-// element products of every active mesh
+// FP64 element products of every active mesh whose stop flag equals `stopped`
+// (0: the running ones' K p; 1: the paused ones' K x, for their residuals)
 __global__ void __launch_bounds__(256)
 k_bt_elem(int nseg, const BSeg *__restrict__ segs, long long total, const double *__restrict__ km,
           const int *__restrict__ conn, const double *__restrict__ p, double *__restrict__ ut,
-          const PcgState *__restrict__ st)
+          const PcgState *__restrict__ st, int stopped)
 {
     const int lane = threadIdx.x & 31;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -100,7 +102,7 @@ k_bt_elem(int nseg, const BSeg *__restrict__ segs, long long total, const double
             else hi = mid - 1;
         }
         const int sid = segs[lo].sid;
-        if (st[sid].stop) continue;
+        if (st[sid].stop != stopped) continue;
         const size_t e = (size_t)segs[lo].el0 + (size_t)(g - segs[lo].el_cum);
         elem_product(e, lane, km, conn, p, ut);
     }
@@ -122,55 +124,6 @@ __global__ void k_bt_emap(int nseg, const BSeg *__restrict__ segs, long long tot
     }
 }
 
-// residual replacement of one mesh: r = rres, d = dinv*r; partials r.d, r.r
-__global__ void __launch_bounds__(256)
-k_bt_replace1(BSeg S, const double *__restrict__ rres, const double *__restrict__ dinv, double *__restrict__ r,
-              double *__restrict__ d, double *__restrict__ part, int cap)
-{
-    const size_t s0 = (size_t)3 * S.node0 + (size_t)blockIdx.x * kVectorSlots;
-    const size_t s1 = min(s0 + kVectorSlots, (size_t)3 * (S.node0 + S.nn));
-    double rd = 0.0, rr = 0.0;
-    for (size_t s = s0 + threadIdx.x; s < s1; s += blockDim.x) {
-        const double rv = rres[s], dv = dinv[s] * rv;
-        r[s] = rv;
-        d[s] = dv;
-        rd = fma(rv, dv, rd);
-        rr = fma(rv, rv, rr);
-    }
-    double v[2] = {rd, rr};
-    block_reduce<2>(v, 0u);
-    if (threadIdx.x == 0) {
-        part[blockIdx.x] = v[0];
-        part[cap + blockIdx.x] = v[1];
-    }
-}
-
-__global__ void k_bt_replace2(BSeg S, const double *__restrict__ part, int cap, double thr,
-                              PcgState *__restrict__ st)
-{
-    const double rd = reduce_partials(part, S.nbv, false);
-    const double rr = reduce_partials(part + cap, S.nbv, false);
-    if (threadIdx.x == 0) {
-        PcgState &T = st[S.sid];
-        T.up = rd;
-        T.rr = rr;
-        T.tol = thr;
-        T.converged = 0;
-        T.stop = rr == 0.0 ? 1 : 0;
-    }
-}
-
-// element products of one mesh (residual at retirement)
-__global__ void __launch_bounds__(256)
-k_bt_elem1(BSeg S, const double *__restrict__ km, const int *__restrict__ conn, const double *__restrict__ p,
-           double *__restrict__ ut)
-{
-    const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int g = warp; g < S.nels; g += nwarps) elem_product((size_t)S.el0 + g, lane, km, conn, p, ut);
-}
-
 // node-centric scatter of one node (ascending element order).  list[]
 // holds contribution indices e*20+a: FP64 results sit at ci*3, FP32 results
 // are node-padded float4s at ci and are summed in FP32.
@@ -181,39 +134,31 @@ __device__ __forceinline__ double scatter_node(int n, const int2 *__restrict__ n
 {
     const int2 pr = nptr[n];
     UT a0 = 0, a1 = 0, a2 = 0;
-    for (int k = pr.x; k < pr.y; k += 8) {
-        int ci[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) ci[i] = (k + i < pr.y) ? __ldg(list + k + i) : -1;
+    for (int k = pr.x; k < pr.y; k += 2) {   // two contributions in flight
+        const bool two = k + 1 < pr.y;
+        const int c0 = __ldg(list + k), c1 = two ? __ldg(list + k + 1) : c0;
         if constexpr (sizeof(UT) == 4) {
-            float4 v[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (ci[i] >= 0) v[i] = __ldg(reinterpret_cast<const float4 *>(ut) + ci[i]);
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (ci[i] >= 0) {
-                    a0 += v[i].x;
-                    a1 += v[i].y;
-                    a2 += v[i].z;
-                }
+            const float4 v0 = __ldg(reinterpret_cast<const float4 *>(ut) + c0);
+            const float4 v1 = __ldg(reinterpret_cast<const float4 *>(ut) + c1);
+            a0 += v0.x;
+            a1 += v0.y;
+            a2 += v0.z;
+            if (two) {
+                a0 += v1.x;
+                a1 += v1.y;
+                a2 += v1.z;
+            }
         } else {
-            double v[8][3];
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (ci[i] >= 0) {
-                    const double *q = ut + (size_t)ci[i] * 3;
-                    v[i][0] = q[0];
-                    v[i][1] = q[1];
-                    v[i][2] = q[2];
-                }
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (ci[i] >= 0) {
-                    a0 += v[i][0];
-                    a1 += v[i][1];
-                    a2 += v[i][2];
-                }
+            const double *q0 = ut + (size_t)c0 * 3, *q1 = ut + (size_t)c1 * 3;
+            const double x0 = q0[0], y0 = q0[1], z0 = q0[2], x1 = q1[0], y1 = q1[1], z1 = q1[2];
+            a0 += x0;
+            a1 += y0;
+            a2 += z0;
+            if (two) {
+                a0 += x1;
+                a1 += y1;
+                a2 += z1;
+            }
         }
     }
     const int m = fm[n];
@@ -236,32 +181,86 @@ __device__ __forceinline__ double scatter_node(int n, const int2 *__restrict__ n
     return loc;
 }
 
+// Scatter of the running meshes, with block partials of p.u; the last block
+// of a mesh forms its alpha (as a launch of its own, 4.6 us).
 template <typename UT>
 __global__ void __launch_bounds__(256)
 k_bt_scatter(const int *__restrict__ blk, const BSeg *__restrict__ segs, const int2 *__restrict__ nptr,
              const int *__restrict__ list, const UT *__restrict__ ut, const uint8_t *__restrict__ fm,
-             const double *__restrict__ p, double *__restrict__ u, double *__restrict__ part,
-             const PcgState *__restrict__ st)
+             const double *__restrict__ p, double *__restrict__ u, double *__restrict__ part, PcgState *st,
+             unsigned *__restrict__ count)
 {
     const int b = blockIdx.x;
     const BSeg &S = segs[blk[b]];
     if (st[S.sid].stop) return;   // no kernel writes the flag meanwhile: uniform per block
     const int n = S.node0 + (b - S.pbs) * kScatterNodes + threadIdx.x;
     double v[1] = {n < S.node0 + S.nn ? scatter_node<UT, 0>(n, nptr, list, ut, fm, p, u) : 0.0};
-    block_reduce<1>(v, 0u);
+    pdl_exit();
+    block_sum<1>(v);
     if (threadIdx.x == 0) part[b] = v[0];
+    if (!last_of(count + S.sid, S.nbs)) return;
+    sum_partials<1>(part + S.pbs, 0, S.nbs, v);
+    if (threadIdx.x == 0) st[S.sid].alpha = st[S.sid].up / v[0];
 }
 
-// residual rres = f - K x of one mesh; partials of rres.rres per local block
+// Residuals rres = f - K x of the paused meshes; the last block of a mesh
+// writes rr[sid] = rres.rres.
 __global__ void __launch_bounds__(256)
-k_bt_residual1(BSeg S, const int2 *__restrict__ nptr, const int *__restrict__ list,
-               const double *__restrict__ ut, const uint8_t *__restrict__ fm, const double *__restrict__ f,
-               double *__restrict__ rres, double *__restrict__ part)
+k_bt_residual(const int *__restrict__ blk, const BSeg *__restrict__ segs, const int2 *__restrict__ nptr,
+              const int *__restrict__ list, const double *__restrict__ ut, const uint8_t *__restrict__ fm,
+              const double *__restrict__ f, double *__restrict__ rres, double *__restrict__ part,
+              const PcgState *__restrict__ st, unsigned *__restrict__ count, double *__restrict__ rr)
 {
-    const int n = S.node0 + blockIdx.x * kScatterNodes + threadIdx.x;
+    const int b = blockIdx.x;
+    const BSeg &S = segs[blk[b]];
+    if (!st[S.sid].stop) return;
+    const int n = S.node0 + (b - S.pbs) * kScatterNodes + threadIdx.x;
     double v[1] = {n < S.node0 + S.nn ? scatter_node<double, 1>(n, nptr, list, ut, fm, f, rres) : 0.0};
-    block_reduce<1>(v, 0u);
-    if (threadIdx.x == 0) part[blockIdx.x] = v[0];
+    block_sum<1>(v);
+    if (threadIdx.x == 0) part[b] = v[0];
+    if (!last_of(count + S.sid, S.nbs)) return;
+    sum_partials<1>(part + S.pbs, 0, S.nbs, v);
+    if (threadIdx.x == 0) rr[S.sid] = v[0];
+}
+
+// Residual replacement of the meshes with a new threshold thr[sid] > 0:
+// r = rres, d = dinv*r; the last block of a mesh restarts its state.
+__global__ void __launch_bounds__(256)
+k_bt_replace(const int *__restrict__ blk, const BSeg *__restrict__ segs, const double *__restrict__ thr,
+             const double *__restrict__ rres, const double *__restrict__ dinv, double *__restrict__ r,
+             double *__restrict__ d, double *__restrict__ part, int cap, PcgState *__restrict__ st,
+             unsigned *__restrict__ count)
+{
+    const int b = blockIdx.x;
+    const BSeg &S = segs[blk[b]];
+    const double tol = thr[S.sid];
+    if (!(tol > 0.0)) return;
+    const size_t s0 = (size_t)3 * S.node0 + (size_t)(b - S.pbv) * kVectorSlots;
+    const size_t s1 = min(s0 + kVectorSlots, (size_t)3 * (S.node0 + S.nn));
+    double rd = 0.0, rr = 0.0;
+    for (size_t s = s0 + threadIdx.x; s < s1; s += blockDim.x) {
+        const double rv = rres[s], dv = dinv[s] * rv;
+        r[s] = rv;
+        d[s] = dv;
+        rd = fma(rv, dv, rd);
+        rr = fma(rv, rv, rr);
+    }
+    double v[2] = {rd, rr};
+    block_sum<2>(v);
+    if (threadIdx.x == 0) {
+        part[b] = v[0];
+        part[cap + b] = v[1];
+    }
+    if (!last_of(count + S.sid, S.nbv)) return;
+    sum_partials<2>(part + S.pbv, cap, S.nbv, v);
+    if (threadIdx.x == 0) {
+        PcgState &T = st[S.sid];
+        T.up = v[0];
+        T.rr = v[1];
+        T.tol = tol;
+        T.converged = 0;
+        T.stop = T.stop2 = v[1] == 0.0 ? 1 : 0;
+    }
 }
 
 // Jacobi diagonal of one mesh (ascending element order per node)
@@ -302,7 +301,7 @@ k_bt_init1(BSeg S, const double *__restrict__ f, const double *__restrict__ dinv
         rr = fma(rv, rv, rr);
     }
     double v[2] = {rd, rr};
-    block_reduce<2>(v, 0u);
+    block_sum<2>(v);
     if (threadIdx.x == 0) {
         part[blockIdx.x] = v[0];
         part[cap + blockIdx.x] = v[1];
@@ -311,9 +310,10 @@ k_bt_init1(BSeg S, const double *__restrict__ f, const double *__restrict__ dinv
 
 __global__ void k_bt_init2(BSeg S, const double *__restrict__ part, int cap, PcgState *__restrict__ st)
 {
-    const double rd = reduce_partials(part, S.nbv, false);
-    const double rr = reduce_partials(part + cap, S.nbv, false);
+    double v[2];
+    sum_partials<2>(part, cap, S.nbv, v);
     if (threadIdx.x == 0) {
+        const double rd = v[0], rr = v[1];
         PcgState &T = st[S.sid];
         T.up = rd;
         T.ff = rr;
@@ -321,38 +321,31 @@ __global__ void k_bt_init2(BSeg S, const double *__restrict__ part, int cap, Pcg
         T.metric = 1.0;
         T.iters = 0;
         T.converged = rr == 0.0 ? 1 : 0;
-        T.stop = rr == 0.0 ? 1 : 0;
+        T.stop = T.stop2 = rr == 0.0 ? 1 : 0;
         T.err = 0;
     }
 }
 
-// one block per active mesh: alpha = (r.d)/(p.u) from the scatter's partials,
-// formed once per mesh (not once per vector block: the FP64 reduction of a
-// large mesh's partials in every block costs more than the update itself)
+// x, r, d of the running meshes with partials of r.d and r.r.  Batched solves
+// stop on the relative residual, so checon_par's max|x| and max|dx| are not
+// formed.  The last block of a mesh does its bookkeeping (as a launch of its
+// own, 6.7 us): beta, the new r.d, the count and the stopping test.
 __global__ void __launch_bounds__(256)
-k_bt_alpha(const BSeg *__restrict__ segs, PcgState *__restrict__ st, const double *__restrict__ part_s)
+k_bt_update1(const int *__restrict__ blk, const BSeg *__restrict__ segs, PcgState *st, double *__restrict__ part_u,
+             int capv, double *__restrict__ x, double *__restrict__ r, double *__restrict__ d,
+             const double *__restrict__ p, const double *__restrict__ u, const double *__restrict__ dinv,
+             unsigned *__restrict__ count)
 {
-    const BSeg &S = segs[blockIdx.x];
-    if (st[S.sid].stop) return;
-    const double pu = reduce_partials(part_s + S.pbs, S.nbs, false);
-    if (threadIdx.x == 0) st[S.sid].alpha = st[S.sid].up / pu;
-}
-
-__global__ void __launch_bounds__(256)
-k_bt_update1(const int *__restrict__ blk, const BSeg *__restrict__ segs, const PcgState *__restrict__ st,
-             double *__restrict__ part_u, int capv, double *__restrict__ x, double *__restrict__ r,
-             double *__restrict__ d, const double *__restrict__ p, const double *__restrict__ u,
-             const double *__restrict__ dinv)
-{
+    pdl_enter();
     const int b = blockIdx.x;
     const BSeg &S = segs[blk[b]];
-    if (st[S.sid].stop) return;
+    if (st[S.sid].stop) {
+        if (b == S.pbv && threadIdx.x == 0) st[S.sid].stop2 = 1;   // read by update2 only
+        return;
+    }
     const double alpha = st[S.sid].alpha;
     const size_t s0 = (size_t)3 * S.node0 + (size_t)(b - S.pbv) * kVectorSlots;
     const size_t s1 = min(s0 + kVectorSlots, (size_t)3 * (S.node0 + S.nn));
-    // batched solves stop on the relative residual, so checon_par's max|x|
-    // and max|dx| (three FP64 operations per slot on GB300's slow FP64
-    // unit) are not formed
     double rd = 0.0, rr = 0.0;
     for (size_t s = s0 + threadIdx.x; s < s1; s += blockDim.x) {
         x[s] = fma(p[s], alpha, x[s]);
@@ -364,54 +357,43 @@ k_bt_update1(const int *__restrict__ blk, const BSeg *__restrict__ segs, const P
         rr = fma(rn, rn, rr);
     }
     double v[2] = {rd, rr};
-    block_reduce<2>(v, 0u);
+    pdl_exit();
+    block_sum<2>(v);
     if (threadIdx.x == 0) {
         part_u[0 * (size_t)capv + b] = v[0];
         part_u[1 * (size_t)capv + b] = v[1];
+    }
+    if (!last_of(count + S.sid, S.nbv)) return;
+    sum_partials<2>(part_u + S.pbv, capv, S.nbv, v);
+    if (threadIdx.x == 0) {
+        PcgState &T = st[S.sid];
+        const int k = T.iters + 1;
+        const double metric = sqrt(v[1]) / sqrt(T.ff);
+        const bool conv = metric <= T.tol;
+        T.beta = v[0] / T.up;
+        T.up = v[0];
+        T.iters = k;
+        T.rr = v[1];
+        T.metric = metric;
+        T.converged = conv ? 1 : 0;
+        if (!isfinite(v[0]) || !isfinite(v[1])) T.err = 1;
+        if (conv || k >= T.limit || T.err) T.stop = 1;
     }
 }
 
 __global__ void __launch_bounds__(256)
 k_bt_update2(const int *__restrict__ blk, const BSeg *__restrict__ segs, const PcgState *__restrict__ st,
-             const double *__restrict__ part_u, const double *__restrict__ d, double *__restrict__ p)
+             const double *__restrict__ d, double *__restrict__ p)
 {
+    pdl_enter();
     const int b = blockIdx.x;
     const BSeg &S = segs[blk[b]];
-    if (st[S.sid].stop) return;
-    const double rd = reduce_partials(part_u + S.pbv, S.nbv, false);
-    const double beta = rd / st[S.sid].up;
+    if (st[S.sid].stop2) return;
+    const double beta = st[S.sid].beta;
     const size_t s0 = (size_t)3 * S.node0 + (size_t)(b - S.pbv) * kVectorSlots;
     const size_t s1 = min(s0 + kVectorSlots, (size_t)3 * (S.node0 + S.nn));
     for (size_t s = s0 + threadIdx.x; s < s1; s += blockDim.x) p[s] = fma(p[s], beta, d[s]);
-}
-
-// one block per active mesh: the iteration's bookkeeping
-__global__ void __launch_bounds__(256)
-k_bt_finish(const BSeg *__restrict__ segs, PcgState *__restrict__ st, const double *__restrict__ part_u, int capv)
-{
-    const BSeg &S = segs[blockIdx.x];
-    if (st[S.sid].stop) return;
-    const double rd = reduce_partials(part_u + S.pbv, S.nbv, false);
-    const double rr = reduce_partials(part_u + capv + S.pbv, S.nbv, false);
-    if (threadIdx.x == 0) {
-        PcgState &T = st[S.sid];
-        const int k = T.iters + 1;
-        const double metric = sqrt(rr) / sqrt(T.ff);   // batched solves: relative residual
-        const bool conv = metric <= T.tol;
-        T.up = rd;
-        T.iters = k;
-        T.rr = rr;
-        T.metric = metric;
-        T.converged = conv ? 1 : 0;
-        if (!isfinite(rd) || !isfinite(rr)) T.err = 1;
-        if (conv || k >= T.limit || T.err) T.stop = 1;
-    }
-}
-
-__global__ void k_bt_sum(const double *__restrict__ part, int n, double *__restrict__ out)
-{
-    const double v = reduce_partials(part, n, false);
-    if (threadIdx.x == 0) *out = v;
+    pdl_exit();
 }
 
 // ---------------------------------------------------------------------------
@@ -480,7 +462,9 @@ struct Batch {
     uint8_t *fm = nullptr;
     double *f = nullptr, *x = nullptr, *r = nullptr, *d = nullptr, *p = nullptr, *u = nullptr, *dinv = nullptr,
            *rres = nullptr;
-    double *part_s = nullptr, *part_u = nullptr, *part_i = nullptr, *scr = nullptr, *gp = nullptr;
+    double *part_s = nullptr, *part_u = nullptr, *part_i = nullptr, *gp = nullptr;
+    double *rr = nullptr, *thr = nullptr, *h_scal = nullptr;   // [max_meshes] residual norms, new thresholds; pinned: both
+    unsigned *count = nullptr;       // [2 * max_meshes] arrivals of a mesh's scatter and vector blocks (last_of)
     PcgState *st = nullptr, *hst = nullptr;
     BSeg *d_segs = nullptr;
     int *d_blk_s = nullptr, *d_blk_v = nullptr;
@@ -547,11 +531,12 @@ Batch *get_batch(void **h)
 void free_batch(Batch &B)
 {
     void *ptrs[] = {B.km32p, B.km16p, B.kerr, B.emap, B.km64, B.coord, B.ediag, B.ut, B.mat_e, B.mat_v, B.conn, B.list, B.nptr, B.fm, B.f, B.x, B.r,
-                    B.d, B.p, B.u, B.dinv, B.rres, B.part_s, B.part_u, B.part_i, B.scr, B.gp, B.st, B.d_segs,
+                    B.d, B.p, B.u, B.dinv, B.rres, B.part_s, B.part_u, B.part_i, B.rr, B.thr, B.count, B.gp, B.st, B.d_segs,
                     B.d_blk_s, B.d_blk_v};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     if (B.hst) cudaFreeHost(B.hst);
+    if (B.h_scal) cudaFreeHost(B.h_scal);
     if (B.stage) cudaFreeHost(B.stage);
     if (B.stage_ev) cudaEventDestroy(B.stage_ev);
     if (B.g_exec) cudaGraphExecDestroy(B.g_exec);
@@ -626,53 +611,75 @@ BSeg seg_of(const Req &q)
     return S;
 }
 
-// A paused mesh: FP64 true residual; retire it (results to the host) or, in
-// the mixed mode while the true residual is above tol, replace its residual
-// and let it run on.
-int check_or_retire(Batch &B, int id)
+// The paused meshes `ids`: their FP64 true residuals in one launch per
+// kernel; then, in the mixed engines, those still above their tolerance get
+// their residual replaced and run on, and the others retire with their
+// results.  One wait for the norms and one for the results, whatever the
+// number of meshes (a residual, a wait and a replacement per mesh took a
+// sixth of the time of 24 small meshes).
+int settle(Batch &B, const std::vector<int> &ids)
 {
-    Req &q = B.active[id];
-    const BSeg S = seg_of(q);
-    const int ge = (q.nels + 7) / 8 < B.nsm * 8 ? (q.nels + 7) / 8 : B.nsm * 8;
-    k_bt_elem1<<<ge, 256, 0, B.stream>>>(S, B.km64, B.conn, B.x, B.ut);
-    if (launched(B, "k_bt_elem1")) return 1;
-    k_bt_residual1<<<q.nbs, 256, 0, B.stream>>>(S, B.nptr, B.list, B.ut, B.fm, B.f, B.rres, B.part_i);
-    if (launched(B, "k_bt_residual1")) return 1;
-    k_bt_sum<<<1, 256, 0, B.stream>>>(B.part_i, q.nbs, B.scr);
-    if (launched(B, "k_bt_sum")) return 1;
-    double rr = 0.0;
-    BCK(cudaMemcpyAsync(&rr, B.scr, sizeof(double), cudaMemcpyDeviceToHost, B.stream));
+    if (B.dirty && rebuild_tables(B)) return 1;   // a mesh was admitted or retired since the last launch
+    long long ge = (B.total_el + 7) / 8;
+    if (ge > (long long)B.nsm * 8) ge = (long long)B.nsm * 8;
+    k_bt_elem<<<(int)(ge < 1 ? 1 : ge), 256, 0, B.stream>>>(B.nseg, B.d_segs, B.total_el, B.km64, B.conn, B.x, B.ut, B.st,
+                                                            1);
+    if (launched(B, "k_bt_elem")) return 1;
+    k_bt_residual<<<B.nblk_s, 256, 0, B.stream>>>(B.d_blk_s, B.d_segs, B.nptr, B.list, B.ut, B.fm, B.f, B.rres, B.part_s,
+                                                  B.st, B.count, B.rr);
+    if (launched(B, "k_bt_residual")) return 1;
+    double *rr = B.h_scal, *thr = B.h_scal + B.max_meshes;
+    BCK(cudaMemcpyAsync(rr, B.rr, (size_t)B.max_meshes * sizeof(double), cudaMemcpyDeviceToHost, B.stream));
     BCK(cudaStreamSynchronize(B.stream));
-    const PcgState &T = B.hst[q.sid];
-    const double relt = T.ff > 0 ? std::sqrt(rr) / std::sqrt(T.ff) : 0.0;
-    if (B.prec != 64 && relt > q.tol && T.iters < q.limit && !T.err) {
-        const double thr = 0.1 * relt > q.tol ? 0.1 * relt : 0.5 * q.tol;
-        k_bt_replace1<<<q.nbv, 256, 0, B.stream>>>(S, B.rres, B.dinv, B.r, B.d, B.part_i, B.capb_v);
-        if (launched(B, "k_bt_replace1")) return 1;
-        k_bt_replace2<<<1, 256, 0, B.stream>>>(S, B.part_i, B.capb_v, thr, B.st);
-        if (launched(B, "k_bt_replace2")) return 1;
-        ++q.corrections;
-        return 0;
+    memset(thr, 0, (size_t)B.max_meshes * sizeof(double));
+    std::vector<int> retire;
+    std::vector<double> rel;
+    bool replace = false;
+    for (int id : ids) {
+        Req &q = B.active[id];
+        const PcgState &T = B.hst[q.sid];
+        const double relt = T.ff > 0 ? std::sqrt(rr[q.sid]) / std::sqrt(T.ff) : 0.0;
+        if (B.prec != 64 && relt > q.tol && T.iters < q.limit && !T.err) {
+            thr[q.sid] = 0.1 * relt > q.tol ? 0.1 * relt : 0.5 * q.tol;
+            ++q.corrections;
+            replace = true;
+        } else {
+            retire.push_back(id);
+            rel.push_back(T.err ? NAN : relt);
+        }
     }
-    const size_t ns = (size_t)3 * q.nn;
-    std::vector<double> xs(ns);
-    BCK(cudaMemcpyAsync(xs.data(), B.x + (size_t)3 * q.node0, ns * sizeof(double), cudaMemcpyDeviceToHost,
-                        B.stream));
+    if (replace) {
+        BCK(cudaMemcpyAsync(B.thr, thr, (size_t)B.max_meshes * sizeof(double), cudaMemcpyHostToDevice, B.stream));
+        k_bt_replace<<<B.nblk_v, 256, 0, B.stream>>>(B.d_blk_v, B.d_segs, B.thr, B.rres, B.dinv, B.r, B.d, B.part_i,
+                                                     B.capb_v, B.st, B.count + B.max_meshes);
+        if (launched(B, "k_bt_replace")) return 1;
+    }
+    std::vector<std::vector<double>> xs(retire.size());
+    for (size_t i = 0; i < retire.size(); ++i) {
+        const Req &q = B.active[retire[i]];
+        xs[i].resize((size_t)3 * q.nn);
+        BCK(cudaMemcpyAsync(xs[i].data(), B.x + (size_t)3 * q.node0, xs[i].size() * sizeof(double),
+                            cudaMemcpyDeviceToHost, B.stream));
+    }
+    if (retire.empty()) return 0;   // (h_scal is written again after the next sync's wait)
     BCK(cudaStreamSynchronize(B.stream));
-    Done dn;
-    dn.id = id;
-    dn.iters = T.iters;
-    dn.neq = q.neq;
-    dn.relres = T.err ? NAN : relt;
-    dn.x.resize(q.neq);
-    for (int e = 0; e < q.neq; ++e) dn.x[e] = xs[q.eq_slot[e]];
-    B.done.push_back(std::move(dn));
-    B.el_free.give(q.el0, q.nels);
-    B.node_free.give(q.node0, q.nn);
-    B.sid_free.push_back(q.sid);
-    B.order.erase(std::find(B.order.begin(), B.order.end(), id));
-    B.active.erase(id);
-    B.dirty = true;
+    for (size_t i = 0; i < retire.size(); ++i) {
+        Req &q = B.active[retire[i]];
+        Done dn;
+        dn.id = retire[i];
+        dn.iters = B.hst[q.sid].iters;
+        dn.neq = q.neq;
+        dn.relres = rel[i];
+        dn.x.resize(q.neq);
+        for (int e = 0; e < q.neq; ++e) dn.x[e] = xs[i][q.eq_slot[e]];
+        B.done.push_back(std::move(dn));
+        B.el_free.give(q.el0, q.nels);
+        B.node_free.give(q.node0, q.nn);
+        B.sid_free.push_back(q.sid);
+        B.order.erase(std::find(B.order.begin(), B.order.end(), retire[i]));
+        B.active.erase(retire[i]);
+        B.dirty = true;
+    }
     return 0;
 }
 
@@ -688,34 +695,28 @@ int batch_iterations(Batch &B, int n)
                                          B.kerr, B.emap))
                 return 1;
             B.launches++;
-            k_bt_scatter<float><<<B.nblk_s, 256, 0, B.stream>>>(B.d_blk_s, B.d_segs, B.nptr, B.list,
-                                                                (const float *)B.ut, B.fm, B.p, B.u, B.part_s,
-                                                                B.st);
         } else if (B.prec == 32) {
             if (launch_elem_sym32_mapped(B.stream, B.nsm, (int)B.total_el, B.km32p, B.conn, B.p, (float *)B.ut,
                                          B.kerr, B.emap))
                 return 1;
             B.launches++;
-            k_bt_scatter<float><<<B.nblk_s, 256, 0, B.stream>>>(B.d_blk_s, B.d_segs, B.nptr, B.list,
-                                                                (const float *)B.ut, B.fm, B.p, B.u, B.part_s,
-                                                                B.st);
         } else {
-            k_bt_elem<<<(int)ge, 256, 0, B.stream>>>(B.nseg, B.d_segs, B.total_el, B.km64, B.conn, B.p, B.ut,
-                                                     B.st);
+            k_bt_elem<<<(int)ge, 256, 0, B.stream>>>(B.nseg, B.d_segs, B.total_el, B.km64, B.conn, B.p, B.ut, B.st, 0);
             if (launched(B, "k_bt_elem")) return 1;
-            k_bt_scatter<double><<<B.nblk_s, 256, 0, B.stream>>>(B.d_blk_s, B.d_segs, B.nptr, B.list, B.ut, B.fm,
-                                                                 B.p, B.u, B.part_s, B.st);
         }
+        if (B.prec == 64)
+            k_bt_scatter<double><<<B.nblk_s, 256, 0, B.stream>>>(B.d_blk_s, B.d_segs, B.nptr, B.list, B.ut, B.fm, B.p,
+                                                                 B.u, B.part_s, B.st, B.count);
+        else
+            k_bt_scatter<float><<<B.nblk_s, 256, 0, B.stream>>>(B.d_blk_s, B.d_segs, B.nptr, B.list,
+                                                                (const float *)B.ut, B.fm, B.p, B.u, B.part_s, B.st,
+                                                                B.count);
         if (launched(B, "k_bt_scatter")) return 1;
-        k_bt_alpha<<<B.nseg, 256, 0, B.stream>>>(B.d_segs, B.st, B.part_s);
-        if (launched(B, "k_bt_alpha")) return 1;
-        k_bt_update1<<<B.nblk_v, 256, 0, B.stream>>>(B.d_blk_v, B.d_segs, B.st, B.part_u, B.capb_v, B.x, B.r, B.d,
-                                                      B.p, B.u, B.dinv);
+        launch_dependent(true, B.stream, B.nblk_v, 256, 0, k_bt_update1, B.d_blk_v, B.d_segs, B.st, B.part_u, B.capb_v,
+                         B.x, B.r, B.d, B.p, B.u, B.dinv, B.count + B.max_meshes);
         if (launched(B, "k_bt_update1")) return 1;
-        k_bt_update2<<<B.nblk_v, 256, 0, B.stream>>>(B.d_blk_v, B.d_segs, B.st, B.part_u, B.d, B.p);
+        launch_dependent(true, B.stream, B.nblk_v, 256, 0, k_bt_update2, B.d_blk_v, B.d_segs, B.st, B.d, B.p);
         if (launched(B, "k_bt_update2")) return 1;
-        k_bt_finish<<<B.nseg, 256, 0, B.stream>>>(B.d_segs, B.st, B.part_u, B.capb_v);
-        if (launched(B, "k_bt_finish")) return 1;
     }
     return 0;
 }
@@ -825,13 +826,16 @@ try {
     al((void **)&B->part_s, (size_t)B->capb_s * 8);
     al((void **)&B->part_u, (size_t)2 * B->capb_v * 8);   // r.d and r.r partials
     al((void **)&B->part_i, (size_t)2 * B->capb_v * 8);
-    al((void **)&B->scr, 64);
+    al((void **)&B->rr, (size_t)B->max_meshes * 8);
+    al((void **)&B->thr, (size_t)B->max_meshes * 8);
+    al((void **)&B->count, (size_t)2 * B->max_meshes * sizeof(unsigned));
     al((void **)&B->gp, 27 * 4 * 8);
     al((void **)&B->st, (size_t)B->max_meshes * sizeof(PcgState));
     al((void **)&B->d_segs, (size_t)B->max_meshes * sizeof(BSeg));
     al((void **)&B->d_blk_s, (size_t)B->capb_s * 4);
     al((void **)&B->d_blk_v, (size_t)B->capb_v * 4);
     if (ok && cudaMallocHost((void **)&B->hst, (size_t)B->max_meshes * sizeof(PcgState)) != cudaSuccess) ok = false;
+    if (ok && cudaMallocHost((void **)&B->h_scal, (size_t)2 * B->max_meshes * 8) != cudaSuccess) ok = false;
     if (ok && cudaEventCreateWithFlags(&B->stage_ev, cudaEventDisableTiming) != cudaSuccess) ok = false;
     if (!ok) {
         set_error("pf_batch_create: cannot allocate the arenas for a %lld-byte budget", *budget_bytes);
@@ -841,6 +845,7 @@ try {
     }
     cudaMemset(B->st, 0, (size_t)B->max_meshes * sizeof(PcgState));
     cudaMemset(B->kerr, 0, sizeof(int));
+    cudaMemset(B->count, 0, (size_t)2 * B->max_meshes * sizeof(unsigned));
     memset(B->hst, 0, (size_t)B->max_meshes * sizeof(PcgState));
     if ((B->prec == 32 && sym32_prepare()) || (B->prec == 16 && sym16_prepare())) {
         free_batch(*B);
@@ -1015,7 +1020,7 @@ try {
     T.tol = B.prec != 64 ? (0.1 > *tol ? 0.1 : *tol) : *tol;   // mixed: first replacement threshold
     T.limit = *limit;
     T.stop_mode = STOP_RELRES;
-    T.stop = 1;   // inactive until the init kernel runs
+    T.stop = T.stop2 = 1;   // inactive until the init kernel runs
     B.hst[sid] = T;
     BCK(cudaMemcpyAsync(B.st + sid, &B.hst[sid], sizeof(PcgState), cudaMemcpyHostToDevice, B.stream));
     BCK(cudaEventRecord(B.stage_ev, B.stream));
@@ -1105,8 +1110,7 @@ try {
     std::vector<int> fin;
     for (int id : B.order)
         if (B.hst[B.active[id].sid].stop) fin.push_back(id);
-    for (int id : fin)
-        if (check_or_retire(B, id)) return PF_FAILURE;
+    if (!fin.empty() && settle(B, fin)) return PF_FAILURE;
     if (n_active) *n_active = (int)(B.order.size() + B.pending.size());
     if (n_done) *n_done = (int)B.done.size();
     return PF_SUCCESS;

@@ -55,35 +55,6 @@ static __device__ __forceinline__ double warp_max(double v)
     return v;
 }
 
-// Reduces NV values over the block (kinds bit k set = max, else sum).  The
-// result is valid in every thread on return.  blockDim.x <= 1024.
-template <int NV>
-static __device__ __forceinline__ void block_reduce(double (&v)[NV], unsigned kinds)
-{
-    __shared__ double sh[NV][32];
-    __shared__ double res[NV];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) v[k] = ((kinds >> k) & 1) ? warp_max(v[k]) : warp_sum(v[k]);
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) sh[k][wid] = v[k];
-    }
-    __syncthreads();
-    if (wid == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            double t = (lane < nw) ? sh[k][lane] : 0.0;
-            t = ((kinds >> k) & 1) ? warp_max(t) : warp_sum(t);
-            if (lane == 0) res[k] = t;
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < NV; ++k) v[k] = res[k];
-    __syncthreads();
-}
-
 // The reductions of the PCG vector kernels (256 threads).  GB300 issues one
 // FP64 warp instruction per SM in 16 clocks, so a tree in every warp (eight
 // warps x five levels per value) costs more than the sums over a block's
@@ -162,21 +133,23 @@ static __device__ __forceinline__ void max_partials2(const double *part, size_t 
     mb = __longlong_as_double(b);
 }
 
-// True in the block that arrives last of the grid (in all its threads): the
-// others' writes before their arrival are visible to it.  The counter wraps
-// to zero by itself.  Thread 0 must have made the block's writes.
-static __device__ __forceinline__ bool last_block(unsigned *count)
+// True in the block that arrives last of the n that share a counter (in all
+// its threads): the others' writes before their arrival are visible to it.
+// The counter wraps to zero by itself.  Thread 0 must have made the block's
+// writes, or a barrier stand between them and this.
+static __device__ __forceinline__ bool last_of(unsigned *count, unsigned n)
 {
     __shared__ int s_last;
     if (threadIdx.x == 0) {
         __threadfence();
-        s_last = atomicInc(count, gridDim.x - 1) == gridDim.x - 1;
+        s_last = atomicInc(count, n - 1) == n - 1;
     }
     __syncthreads();
     const bool last = s_last != 0;
     if (last) __threadfence();
     return last;
 }
+static __device__ __forceinline__ bool last_block(unsigned *count) { return last_of(count, gridDim.x); }
 
 // The end of a PCG scatter: the block's share of p.u, and in the last block
 // the step length alpha = r.d / p.u.  One thread divides: the vector kernels
@@ -246,16 +219,6 @@ static __device__ __forceinline__ bool grid_barrier(unsigned long long *bar, int
     const bool ok = s_ok != 0;
     __syncthreads();
     return ok;
-}
-
-// Sums (or maxes) G block partials in a fixed order; same value in every block.
-static __device__ __forceinline__ double reduce_partials(const double *part, int G, bool is_max)
-{
-    double acc = 0.0;
-    for (int i = threadIdx.x; i < G; i += blockDim.x) acc = is_max ? fmax(acc, part[i]) : acc + part[i];
-    double v[1] = {acc};
-    block_reduce<1>(v, is_max ? 1u : 0u);
-    return v[0];
 }
 
 // SHAPE_DER for one node l of the 20-node brick (new_library.f90:865-896).

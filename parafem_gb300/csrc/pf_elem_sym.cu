@@ -307,9 +307,9 @@ int launch_elem_sym32_mapped(cudaStream_t stream, int nsm, int n, const float *k
 {
     if (n <= 0) return 0;
     constexpr int W = 14;
-    const int grid = n < nsm * W ? (n + W - 1) / W : nsm;
-    k_elem_sym32<W, 2, true><<<grid, W * 32, sym_smem_bytes<W, 2>(), stream>>>(n, kp, conn, p, ut, nullptr, err,
-                                                                                emap);
+    const int grid = n < nsm ? n : nsm;
+    launch_dependent(true, stream, grid, W * 32, sym_smem_bytes<W, 2>(), k_elem_sym32<W, 2, true>, n, kp, conn, p, ut,
+                     (const PcgState *)nullptr, err, emap);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_error("k_elem_sym32: launch failed: %s", cudaGetErrorString(e));
