@@ -138,6 +138,7 @@ static void free_mesh(Ctx &c)
 {
     drop_graph(c);
     multi_release(c);
+    rows_release(c);
     dfree(c.conn); dfree(c.node_ptr); dfree(c.node_list); dfree(c.slot_eq); dfree(c.eq_slot);
     dfree(c.freemask); dfree(c.coord); dfree(c.mat_e); dfree(c.mat_v); dfree(c.km64); dfree(c.km32);
     dfree(c.km32p); dfree(c.skm64); dfree(c.skm32); dfree(c.fstore); dfree(c.fscale); dfree(c.psplit);
@@ -533,7 +534,8 @@ static int setup_mesh(void **ctx, const int *nels_p, const int *nn_p, const int 
     if (g > (long long)c.nsm * kVecBlocks) g = (long long)c.nsm * kVecBlocks;
     c.G = (int)(g < 1 ? 1 : g);
     long long gs = ((long long)nn + 255) / 256;
-    if (gs > (long long)c.nsm * kScatterBlocks) gs = (long long)c.nsm * kScatterBlocks;
+    const int most = nod == 8 && nodof == 1 ? kRowBlocks : kScatterBlocks;
+    if (gs > (long long)c.nsm * most) gs = (long long)c.nsm * most;
     c.Gs = (int)(gs < 1 ? 1 : gs);
     const size_t ne = (size_t)nels;
     if (dalloc(&c.conn, ne * nod, "connectivity") || dalloc(&c.node_ptr, nn + 1, "node table") ||
@@ -614,6 +616,7 @@ try {
     drop_graph(c);
     TRY(launch_form_storkc(c, *nip, *kx, *ky, *kz));
     TRY(launch_assemble_diag(c));
+    TRY(rows_assemble(c));
     TRY(sync(c));
     c.have_km = true;
     return PF_SUCCESS;

@@ -58,6 +58,7 @@ enum { STOP_CHECON = 0, STOP_RELRES = 1 };
 // (4 to 8 measured alike for the vector kernels, 8 to 16 for the scatter;
 // 40 scatter blocks cost 20 % at 80^3).
 constexpr int kVecBlocks = 6, kScatterBlocks = 12;
+constexpr int kRowBlocks = 64;   // of the 8-node scalar product: rows are short, blocks are handed out as SMs free up
 // Most slots of a mesh whose iterations use programmatic dependent launches:
 // they save 1.5 to 3 us of an iteration (10^3 elements: 24.0 -> 22.0 us FP64,
 // 26.5 -> 23.6 mixed; 20^3: 47 -> 45, 34 -> 31), nothing measurable of the
@@ -118,6 +119,12 @@ struct Ctx {
     int kind = 0;               // KIND_SOLID20 (p121), KIND_SCALAR8 (p123) or KIND_SOLID8
     double *fstore = nullptr;   // [nslots] 8-node kinds: penalty store of fixed freedoms, 0 = free
     double *fscale = nullptr;   // [1] KIND_SOLID8: the PCG product at a fixed freedom is p * store * fscale
+    // KIND_SCALAR8: the assembled rows of storkc (pf_scalar8.cu), or null: the element products are used
+    long long *row_off = nullptr;   // [slices of 32 nodes + 1]
+    double *row_val = nullptr;
+    void *row_idx = nullptr;        // 16-bit offsets from row_base, or 32-bit columns (row_wide)
+    int *row_base = nullptr;
+    bool row_wide = false, row_keep = false;
     // one element matrix shared by every element (PCG_KM); per-element storkm unused
     bool shared = false;
     double *skm64 = nullptr;    // [3600] column-major
@@ -227,6 +234,8 @@ int launch_form_storkc(Ctx &c, int nip, double kx, double ky, double kz);
 int launch_elem8(Ctx &c, const double *p, const PcgState *st);
 int launch_scatter1(Ctx &c, int mode, const double *xin, const double *pf, double *out, PcgState *st);
 int launch_assemble_diag1(Ctx &c);
+int rows_assemble(Ctx &c);   // the assembled rows of the current storkc; waits for the stream
+void rows_release(Ctx &c);
 int launch_set_fixed(Ctx &c, int nfix, const int *slots_dev, double penalty);
 // pf_solid8.cu: 8-node elasticity bricks (24 freedoms per element), FP64
 int launch_elem24(Ctx &c, const double *p, const PcgState *st);

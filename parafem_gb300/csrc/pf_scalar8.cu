@@ -13,8 +13,20 @@
 //   k_scatter1        node-centric sum in ascending element order, with
 //                     p123's fixed freedoms: u = p * store at a node fixed by
 //                     the penalty method (p123.f90:127-131);
-//   k_assemble_diag1  the Jacobi diagonal (p123.f90:87-94).
+//   k_assemble_diag1  the Jacobi diagonal (p123.f90:87-94);
+//   k_rows*           the same sums with the element matrices added up by
+//                     node once, when storkc is formed: one row of the
+//                     assembled matrix per node, and
+//   k_row_product     the product, dot and fixed freedoms in one pass over
+//                     the rows.  A node of a brick mesh has 27 neighbours:
+//                     270 bytes and 27 FMA per node and product, where the
+//                     element products and the scatter move 710 bytes and
+//                     take 64 FMA and 8 additions per element.  The element
+//                     kernels serve meshes with a node of more than kRowMax
+//                     neighbours and contexts without memory for the rows.
 #include "pf_device.cuh"
+
+#include <vector>
 
 namespace pf {
 
@@ -113,6 +125,140 @@ k_scatter1(int nn, const int *__restrict__ ptr, const int *__restrict__ list, co
     scatter_tail(loc, part, MODE == 0 ? st : nullptr, count);
 }
 
+// ---------------------------------------------------------------------------
+// Assembled rows, in slices of 32 consecutive nodes: entry k of the rows of
+// slice s lies at off[s] + 32 k + lane, columns ascending, short rows padded
+// with zeros.  Column numbers are 16-bit offsets from the least column of
+// (slice, k) where every one fits (neighbouring nodes have neighbouring
+// columns), 32-bit numbers otherwise.
+constexpr int kRowMax = 64;   // entries of a row (a structured brick mesh has 27)
+
+// the ascending distinct columns of node n: their number, -1 when too many
+__device__ int row_columns(int n, const int *__restrict__ ptr, const int *__restrict__ list,
+                           const int *__restrict__ conn, int *cols)
+{
+    int cnt = 0;
+    for (int q = ptr[n]; q < ptr[n + 1]; ++q) {
+        const int *ce = conn + (size_t)(list[q] >> 3) * 8;
+        for (int j = 0; j < 8; ++j) {
+            const int c = ce[j];
+            int m = cnt;
+            while (m > 0 && cols[m - 1] > c) --m;
+            if (m > 0 && cols[m - 1] == c) continue;
+            if (cnt == kRowMax) return -1;
+            for (int i = cnt; i > m; --i) cols[i] = cols[i - 1];
+            cols[m] = c;
+            ++cnt;
+        }
+    }
+    return cnt;
+}
+
+__global__ void __launch_bounds__(128)
+k_rows_width(int nn, const int *__restrict__ ptr, const int *__restrict__ list, const int *__restrict__ conn,
+             int *__restrict__ width, int *__restrict__ bad)
+{
+    const int nslice = (nn + 31) / 32, lane = threadIdx.x & 31;
+    for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < nslice; s += (gridDim.x * blockDim.x) >> 5) {
+        int cols[kRowMax];
+        const int n = 32 * s + lane;
+        const int cnt = n < nn ? row_columns(n, ptr, list, conn, cols) : 0;
+        if (cnt < 0) atomicOr(bad, 1);
+        const int w = __reduce_max_sync(FULLMASK, cnt);
+        if (lane == 0) width[s] = w;
+    }
+}
+
+// Values summed in ascending element order; *bad: a 16-bit offset overflows.
+template <typename IT>
+__global__ void __launch_bounds__(128)
+k_rows_fill(int nn, const int *__restrict__ ptr, const int *__restrict__ list, const int *__restrict__ conn,
+            const double *__restrict__ kc, const long long *__restrict__ off, double *__restrict__ val,
+            IT *__restrict__ idx, int *__restrict__ base, int *__restrict__ bad)
+{
+    const int nslice = (nn + 31) / 32, lane = threadIdx.x & 31;
+    for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < nslice; s += (gridDim.x * blockDim.x) >> 5) {
+        int cols[kRowMax];
+        double v[kRowMax];
+        const int n = 32 * s + lane;
+        int cnt = 0;
+        if (n < nn) {
+            cnt = row_columns(n, ptr, list, conn, cols);
+            for (int k = 0; k < cnt; ++k) v[k] = 0.0;
+            for (int q = ptr[n]; q < ptr[n + 1]; ++q) {
+                const size_t e = (size_t)(list[q] >> 3);
+                const int a = list[q] & 7;
+                for (int j = 0; j < 8; ++j) {
+                    const int c = conn[e * 8 + j];
+                    int k = 0;
+                    while (cols[k] != c) ++k;
+                    v[k] += kc[e * 64 + a + 8 * j];
+                }
+            }
+        }
+        const long long o = off[s];
+        const int w = (int)((off[s + 1] - o) >> 5);
+        for (int k = 0; k < w; ++k) {
+            const int least = __reduce_min_sync(FULLMASK, k < cnt ? cols[k] : 0x7fffffff);
+            const int c = k < cnt ? cols[k] : least;
+            if (sizeof(IT) == 2 && c - least > 0xffff) atomicOr(bad, 1);
+            val[o + 32 * k + lane] = k < cnt ? v[k] : 0.0;
+            idx[o + 32 * k + lane] = (IT)(sizeof(IT) == 2 ? c - least : c);
+            if (lane == 0) base[(o >> 5) + k] = least;
+        }
+    }
+}
+
+// u = K x over the assembled rows, as k_elem8 and k_scatter1 form it:
+//   MODE 0: out = u, partial pf.u and alpha in a PCG run;  MODE 1: out = f - u, partial out.out
+// Bound by the FP64 pipe (30 operations per node, two per SM and clock: 56 us
+// at 100^3) and by HBM (294 B per node, 44 us): 90 us at 100^3, where k_elem8
+// and k_scatter1 take 180; 26 against 37 us at 50^3, 18 when the rows stay in
+// L2.  KEEP: the rows are read the ordinary way, so that those of a mesh that
+// fits stay in L2 from one product to the next; else they leave L2 first
+// (100^3: 98 us kept, 90 us not).
+constexpr size_t kRowKeepBytes = 64u << 20;
+template <int MODE, typename IT, bool KEEP>
+__global__ void __launch_bounds__(256)
+k_row_product(int nn, const long long *__restrict__ off, const double *__restrict__ val, const IT *__restrict__ idx,
+              const int *__restrict__ base, const uint8_t *__restrict__ fm, const double *__restrict__ fstore,
+              const double *__restrict__ xin, const double *__restrict__ pf, double *__restrict__ out,
+              double *__restrict__ part, PcgState *st, unsigned *__restrict__ count)
+{
+    pdl_enter();
+    if (st && st->stop) return;
+    double loc = 0.0;
+    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < nn; n += gridDim.x * blockDim.x) {
+        const int s = n >> 5, lane = n & 31;
+        const long long o = off[s];
+        const int w = (int)((off[s + 1] - o) >> 5);
+        const double *v = val + o + lane;
+        const IT *ix = idx + o + lane;
+        const int *b = base + (o >> 5);
+        double a = 0.0;
+#pragma unroll 9
+        for (int k = 0; k < w; ++k) {
+            const int i = (int)(KEEP ? __ldg(ix + 32 * k) : __ldcs(ix + 32 * k));
+            const int c = sizeof(IT) == 2 ? __ldg(b + k) + i : i;
+            a = fma(KEEP ? __ldg(v + 32 * k) : __ldcs(v + 32 * k), __ldg(xin + c), a);
+        }
+        const bool fr = fm[n] & 1;
+        const double fs = fstore[n];
+        if (abs_bits(fs)) a = xin[n] * fs;   // an integer test
+        if (MODE == 0) {
+            const double uv = fr ? a : 0.0;
+            out[n] = uv;
+            loc = fma(pf[n], uv, loc);
+        } else {
+            const double rv = fr ? pf[n] - a : 0.0;
+            out[n] = rv;
+            loc = fma(rv, rv, loc);
+        }
+    }
+    pdl_exit();
+    scatter_tail(loc, part, MODE == 0 ? st : nullptr, count);
+}
+
 __global__ void k_assemble_diag1(int nn, const int *__restrict__ ptr, const int *__restrict__ list,
                                  const double *__restrict__ ed, const uint8_t *__restrict__ fm,
                                  double *__restrict__ diag, double *__restrict__ dinv, double *__restrict__ fstore)
@@ -174,8 +320,98 @@ int launch_form_storkc(Ctx &c, int nip, double kx, double ky, double kz)
     return 0;
 }
 
+void rows_release(Ctx &c)
+{
+    void *p[] = {c.row_off, c.row_val, c.row_idx, c.row_base};
+    for (void *q : p)
+        if (q) cudaFree(q);
+    c.row_off = nullptr;
+    c.row_val = nullptr;
+    c.row_idx = nullptr;
+    c.row_base = nullptr;
+}
+
+// The assembled rows of the context's storkc; none (and success) where a row
+// is too long or the memory does not suffice.
+int rows_assemble(Ctx &c)
+{
+    rows_release(c);
+    const int nslice = (c.nn + 31) / 32, grid = grid8(c, c.nn, 128, 16);
+    int *d_width = nullptr, bad = 0;
+    std::vector<int> width(nslice);
+    std::vector<long long> off(nslice + 1, 0);
+    if (cudaMalloc((void **)&d_width, (size_t)nslice * sizeof(int)) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    cudaMemsetAsync(c.kerr + 1, 0, sizeof(int), c.stream);
+    k_rows_width<<<grid, 128, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, c.conn, d_width, c.kerr + 1);
+    int err = launched8(c, "k_rows_width");
+    cudaMemcpyAsync(width.data(), d_width, (size_t)nslice * sizeof(int), cudaMemcpyDeviceToHost, c.stream);
+    cudaMemcpyAsync(&bad, c.kerr + 1, sizeof(int), cudaMemcpyDeviceToHost, c.stream);
+    const cudaError_t e = cudaStreamSynchronize(c.stream);
+    cudaFree(d_width);
+    if (err) return 1;
+    if (e != cudaSuccess) {
+        set_error("k_rows_width: %s", cudaGetErrorString(e));
+        return 1;
+    }
+    if (bad) return 0;
+    for (int s = 0; s < nslice; ++s) off[s + 1] = off[s] + 32LL * width[s];
+    const size_t total = (size_t)off[nslice];
+    if (total == 0) return 0;
+    for (int bytes = 2; bytes <= 4; bytes += 2) {   // 16-bit columns first
+        if ((!c.row_off && cudaMalloc((void **)&c.row_off, (size_t)(nslice + 1) * sizeof(long long)) != cudaSuccess) ||
+            (!c.row_val && cudaMalloc((void **)&c.row_val, total * sizeof(double)) != cudaSuccess) ||
+            (!c.row_base && cudaMalloc((void **)&c.row_base, total / 32 * sizeof(int)) != cudaSuccess) ||
+            cudaMalloc(&c.row_idx, total * bytes) != cudaSuccess) {
+            cudaGetLastError();
+            rows_release(c);
+            return 0;
+        }
+        c.row_wide = bytes == 4;
+        c.row_keep = total * (8 + bytes) <= kRowKeepBytes;
+        cudaMemcpyAsync(c.row_off, off.data(), off.size() * sizeof(long long), cudaMemcpyHostToDevice, c.stream);
+        cudaMemsetAsync(c.kerr + 1, 0, sizeof(int), c.stream);
+        if (bytes == 2)
+            k_rows_fill<uint16_t><<<grid, 128, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, c.conn, c.km64, c.row_off,
+                                                              c.row_val, (uint16_t *)c.row_idx, c.row_base, c.kerr + 1);
+        else
+            k_rows_fill<int><<<grid, 128, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, c.conn, c.km64, c.row_off,
+                                                         c.row_val, (int *)c.row_idx, c.row_base, c.kerr + 1);
+        if (launched8(c, "k_rows_fill")) return 1;
+        cudaMemcpyAsync(&bad, c.kerr + 1, sizeof(int), cudaMemcpyDeviceToHost, c.stream);
+        const cudaError_t ef = cudaStreamSynchronize(c.stream);
+        if (ef != cudaSuccess) {
+            set_error("k_rows_fill: %s", cudaGetErrorString(ef));
+            return 1;
+        }
+        if (!bad) break;
+        cudaFree(c.row_idx);
+        c.row_idx = nullptr;
+    }
+    return 0;
+}
+
+static int launch_row_product(Ctx &c, int mode, const double *xin, const double *pf, double *out, PcgState *st)
+{
+    auto go = [&](auto *idx, auto kernel0, auto kernel1) {
+        launch_dependent(c.dependent && st, c.stream, c.Gs, 256, 0, mode ? kernel1 : kernel0, c.nn, c.row_off, c.row_val,
+                         idx, c.row_base, c.freemask, c.fstore, xin, pf, out, c.part_s, st, c.count);
+    };
+    const int *wide = (const int *)c.row_idx;
+    const uint16_t *narrow = (const uint16_t *)c.row_idx;
+    if (c.row_wide) go(wide, k_row_product<0, int, false>, k_row_product<1, int, false>);
+    else if (c.row_keep) go(narrow, k_row_product<0, uint16_t, true>, k_row_product<1, uint16_t, true>);
+    else go(narrow, k_row_product<0, uint16_t, false>, k_row_product<1, uint16_t, false>);
+    return launched8(c, "k_row_product");
+}
+
+// The element products; with assembled rows nothing: launch_scatter1 forms
+// the whole product.
 int launch_elem8(Ctx &c, const double *p, const PcgState *st)
 {
+    if (c.row_idx) return 0;
     launch_dependent(c.dependent && st, c.stream, grid8(c, (long long)c.nels * 8, 256, 8), 256, 0, k_elem8, c.nels, c.km64, c.conn, p,
                      (double *)c.utemp, st);
     return launched8(c, "k_elem8");
@@ -183,6 +419,7 @@ int launch_elem8(Ctx &c, const double *p, const PcgState *st)
 
 int launch_scatter1(Ctx &c, int mode, const double *xin, const double *pf, double *out, PcgState *st)
 {
+    if (c.row_idx) return launch_row_product(c, mode, xin, pf, out, st);
     if (mode == 0)
         k_scatter1<0><<<c.Gs, 256, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, (const double *)c.utemp, c.freemask,
                                                   c.fstore, xin, pf, out, c.part_s, st, c.count);
