@@ -187,7 +187,9 @@ int pf_set_graphs(void **ctx, const int *on);
  * per launch.  *on == 0, the default, launches the separate scatter, update
  * and finish kernels, replayed from CUDA graphs, which measure faster on
  * GB300.  Both give bitwise the same iterates.  Applies to 20-node
- * contexts; 8-node contexts always use the separate kernels. */
+ * contexts; 8-node contexts always use the separate kernels, and meshes of
+ * up to about 311,000 freedoms (other than mixed solves of one shared km)
+ * always run as one resident kernel (graphs and this switch make no difference to them). */
 int pf_set_persistent(void **ctx, const int *on);
 
 /* Self-check of the error path of the bulk-copy element kernels (no

@@ -21,10 +21,10 @@ EXE122 = os.path.join(OUT, "p122")
 PROGRAMS = [("p121_main.cpp", EXE), ("p123_main.cpp", EXE123), ("p122_main.cpp", EXE122)]
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-CUDA_SOURCES = ["pf_kernels.cu", "pf_elem_sym.cu", "pf_elem_h16.cu", "pf_fix.cu", "pf_shared.cu", "pf_scalar8.cu",
+CUDA_SOURCES = ["pf_kernels.cu", "pf_elem_sym.cu", "pf_elem_h16.cu", "pf_fix.cu", "pf_resident.cu", "pf_shared.cu", "pf_scalar8.cu",
                 "pf_solid8.cu", "pf_plastic.cu", "pf_batch.cu", "pf_multi.cu", "pf_abi.cu", "pf_noalloc.cu"]
 CXX_SOURCES = ["pf_host.cpp"]
-HEADERS = ["pf_internal.h", "pf_device.cuh", "pf_fix.cuh", "pf_tc.cuh"]
+HEADERS = ["pf_internal.h", "pf_device.cuh", "pf_fix.cuh", "pf_sym.cuh", "pf_tc.cuh"]
 
 _lock = threading.Lock()
 

@@ -180,7 +180,7 @@ static int check_kernel_error(Ctx &c)
         cudaMemsetAsync(c.kerr, 0, sizeof(int), c.stream);
         cudaStreamSynchronize(c.stream);
         if (err == 3)
-            set_error("persistent PCG kernel: a grid-wide barrier wait timed out (code 3)");
+            set_error("persistent PCG kernel: a grid-wide wait timed out (code 3)");
         else
             set_error("element kernel: a shared-memory bulk-copy wait timed out (code %d)", err);
         return 1;
@@ -239,6 +239,22 @@ static int run_pcg(Ctx &c, int prec, double *xsol, int limit)
 {
     int launched = 0;
     int chunk = 4;
+    if (resident_ok(c, prec)) {
+        // small meshes: the run in launches of up to 2000 iterations
+        while (launched < limit) {
+            const int todo = limit - launched < 2000 ? limit - launched : 2000;
+            TRY(launch_pcg_resident(c, prec, xsol, todo));
+            launched += todo;
+            TRY(pull_state(c));
+            if (c.hst->stop) break;
+        }
+        if (check_kernel_error(c)) return 1;
+        if (c.hst->err) {
+            set_error("PCG breakdown after %d iterations (non-finite r.d or |x|)", c.hst->iters);
+            return 1;
+        }
+        return 0;
+    }
     if (persist_fused64(c, prec)) {
         // whole FP64 iterations in persistent launches, one launch per chunk
         for (;;) {
@@ -441,6 +457,7 @@ try {
     if (c->st) cudaFree(c->st);
     if (c->kerr) cudaFree(c->kerr);
     if (c->count) cudaFree(c->count);
+    if (c->res_part) cudaFree(c->res_part);
     if (c->gbar) cudaFree(c->gbar);
     if (c->hst) cudaFreeHost(c->hst);
     if (c->stream) cudaStreamDestroy(c->stream);

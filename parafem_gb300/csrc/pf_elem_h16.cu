@@ -19,20 +19,18 @@
 // lane: forward distance d needs (D[d][l], D[d][l+30]) = word 30d + l, and
 // backward distance t = 30 - d needs D[t][l+d] and D[t][(l+d+30) mod 60],
 // the two halves of word 30t + (l+d) mod 30 (swapped when l+d >= 30).
-#include "pf_device.cuh"
-#include "pf_tc.cuh"
+#include "pf_sym.cuh"
 
 #include <cstdint>
-#include <cuda_fp16.h>
 
 namespace pf {
 
 using namespace tc;
 
 namespace {
-constexpr int kH16Words = 916;
-constexpr int kH16Bytes = kH16Words * 4;   // 3664
-constexpr int kPSlot = 120;                // floats of p per warp: 60 pairs (p[i], p[i+30 mod 60])
+constexpr int kH16Words = sym::kWords16;
+constexpr int kH16Bytes = sym::kBytes16;   // 3664
+constexpr int kPSlot = sym::kPSlot;
 constexpr unsigned kFull = 0xffffffffu;
 }  // namespace
 
@@ -82,7 +80,7 @@ k_elem_sym16(int nels, const uint32_t *__restrict__ kh, const int *__restrict__ 
     const int lane = threadIdx.x & 31;
     const int w = threadIdx.x >> 5;
     uint32_t *stage = reinterpret_cast<uint32_t *>(smem) + (size_t)w * kStages * kH16Words;
-    float2 *pp = reinterpret_cast<float2 *>(smem + (size_t)kWarps * kStages * kH16Bytes + (size_t)w * kPSlot * 4);
+    float *pp = reinterpret_cast<float *>(smem + (size_t)kWarps * kStages * kH16Bytes + (size_t)w * kPSlot * 4);
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem + (size_t)kWarps * kStages * kH16Bytes +
                                                  kWarps * kPSlot * 4) + w * kStages;
     static_assert((kWarps * kStages * kH16Bytes + kWarps * kPSlot * 4) % 8 == 0, "mbarrier alignment");
@@ -154,57 +152,16 @@ k_elem_sym16(int nels, const uint32_t *__restrict__ kh, const int *__restrict__ 
         int conn_next2 = 0;
         if (k + kAhead + 1 < nmine && lane < 20) conn_next2 = conn[(size_t)elem(k + kAhead + 1) * 20 + lane];
 
-        // p of element k less its mean translation (as the FP32 kernel)
-        {
-            float ha, la, hb, lb;
-            split_f64(pa, ha, la);
-            split_f64(pb, hb, lb);
-            const float t = 0.05f * sum_mod3(ha + hb, lane);
-            if (active) {   // pair i = (p[i], p[i+30 mod 60]): one 8-byte load per step of the walk
-                const float qa = (ha - t) + la, qb = (hb - t) + lb;
-                pp[lane] = make_float2(qa, qb);
-                pp[lane + 30] = make_float2(qb, qa);
-            }
-        }
+        sym::put_p<true>(lane, pa, pb, pp);
         const bool ok = __all_sync(kFull, mbar_wait(&bar[s], parity));
         if (!ok) {
             failed = true;
             break;
         }
         __syncwarp();
-        const uint32_t *Wd = stage + s * kH16Words;
-        float acc_a = 0.f, acc_b = 0.f;
-        if (active) {
-            const float2 *pl = pp + lane;
-            const float2 p00 = pl[0];   // (p[l], p[l+30])
-            const float2 w0 = __half22float2(*reinterpret_cast<const __half2 *>(Wd + lane));
-            float f0 = w0.x * p00.x, f1 = w0.y * p00.y, g0 = 0.f, g1 = 0.f;
-#pragma unroll
-            for (int d = 1; d < 30; ++d) {
-                const int t = 30 - d;
-                const float2 pd = pl[d];   // (p[l+d], p[l+d+30 mod 60])
-                const float p0 = pd.x, p1 = pd.y;
-                const float2 wf = __half22float2(*reinterpret_cast<const __half2 *>(Wd + 30 * d + lane));
-                f0 = fmaf(wf.x, p0, f0);                                      // K(l, l+d)
-                f1 = fmaf(wf.y, p1, f1);                                      // K(l+30, l+30+d)
-                const bool wrap = lane >= t;                                  // l + d >= 30
-                const float2 wb = __half22float2(
-                    *reinterpret_cast<const __half2 *>(Wd + 30 * t + (wrap ? lane - t : lane + d)));
-                g1 = fmaf(wrap ? wb.y : wb.x, p0, g1);                        // K(l+30, l+d)
-                g0 = fmaf(wrap ? wb.x : wb.y, p1, g0);                        // K(l, l+d+30)
-            }
-            const float d30 = __half2float(reinterpret_cast<const __half *>(Wd + 900)[lane]);   // K(l, l+30)
-            f0 = fmaf(d30, p00.y, f0);
-            f1 = fmaf(d30, p00.x, f1);
-            const float sc = __uint_as_float(Wd[915]);
-            acc_a = (f0 + g0) * sc;
-            acc_b = (f1 + g1) * sc;
-        }
-        {
-            const float t = 0.05f * sum_mod3(acc_a + acc_b, lane);
-            acc_a -= t;
-            acc_b -= t;
-        }
+        float acc_a, acc_b;
+        sym::walk16(lane, stage + s * kH16Words, pp, acc_a, acc_b);
+        sym::project_result(lane, acc_a, acc_b);
         if (active) {
             float *o = ut + (size_t)elem(k) * 80;   // node-padded: row i at (i/3)*4 + i%3
             st_global_hint(o + (lane / 3) * 4 + lane % 3, acc_a, pol);

@@ -29,8 +29,7 @@
 // Every wait on an mbarrier is bounded; a wait that runs out writes 2 to
 // the context's device error word and the warp drains its in-flight copies
 // (again with a bound) before it returns.
-#include "pf_device.cuh"
-#include "pf_tc.cuh"
+#include "pf_sym.cuh"
 
 #include <cstdint>
 
@@ -40,9 +39,9 @@ using namespace tc;
 
 namespace {
 
-constexpr int kPacked = 1832;                 // floats per element (1830 + 2 pad)
-constexpr int kPackedBytes = kPacked * 4;     // 7328
-constexpr int kPSlot = 120;                   // floats of p per warp (p_e twice)
+constexpr int kPacked = sym::kWords32;         // floats per element (1830 + 2 pad)
+constexpr int kPackedBytes = sym::kBytes32;    // 7328
+constexpr int kPSlot = sym::kPSlot;
 constexpr unsigned kFull = 0xffffffffu;
 
 }  // namespace
@@ -151,65 +150,16 @@ k_elem_sym32(int nels, const float *__restrict__ kp, const int *__restrict__ con
         int conn_next2 = 0;
         if (k + 2 < nmine && lane < 20) conn_next2 = conn[(size_t)elem(k + 2) * 20 + lane];
 
-        // p of element k, less its mean translation, into the warp's slot.
-        // K_e t = 0 for a rigid translation t, so the subtraction changes
-        // nothing in exact arithmetic; in FP32 it keeps the translation of
-        // a smooth p out of the rounding of p, of storkm's entries and of
-        // the sums (errors that grow with the square of the mesh size on
-        // the lowest modes).  The mean is formed from the FP32 high parts --
-        // any translation serves -- and (hi - t) + lo recovers p - t to FP32
-        // accuracy relative to p - t.
-        {
-            float ha, la, hb, lb;
-            split_f64(pa, ha, la);
-            split_f64(pb, hb, lb);
-            const float t = 0.05f * sum_mod3(ha + hb, lane);
-            if (active) {
-                const float qa = (ha - t) + la, qb = (hb - t) + lb;
-                pp[lane] = qa;
-                pp[lane + 60] = qa;
-                pp[lane + 30] = qb;
-                pp[lane + 90] = qb;
-            }
-        }
+        sym::put_p<false>(lane, pa, pb, pp);
         const bool ok = __all_sync(kFull, mbar_wait(&bar[s], parity));
         if (!ok) {
             failed = true;
             break;
         }
         __syncwarp();
-        // Row l and row l+30 as four running sums over the diagonals: step
-        // d pairs forward distance d (K(l, l+d), K(l+30, l+30+d)) with
-        // backward distance 30-d (K(l+30, l+d), K(l, l+30+d)), which use
-        // the same two p values.  Every address is the lane plus a constant.
-        const float *D = stage + s * kPacked;
-        float acc_a = 0.f, acc_b = 0.f;
-        if (active) {
-            const float *Dl = D + lane, *Dw = D + lane + 60;   // Dw: entries (l - t) mod 60 for t > l
-            const float *pl = pp + lane;
-            float f0 = Dl[0] * pl[0], f1 = Dl[30] * pl[30], g0 = 0.f, g1 = 0.f;
-#pragma unroll
-            for (int d = 1; d < 30; ++d) {
-                const int t = 30 - d;
-                const float p0 = pl[d], p1 = pl[30 + d];
-                f0 = fmaf(Dl[60 * d], p0, f0);                              // K(l, l+d)
-                f1 = fmaf(Dl[60 * d + 30], p1, f1);                         // K(l+30, l+30+d)
-                g1 = fmaf(Dl[60 * t + d], p0, g1);                          // K(l+30, l+d) = D[t][l+d]
-                g0 = fmaf((lane < t ? Dw : Dl)[59 * t], p1, g0);            // K(l, l-t) = D[t][(l-t) mod 60]
-            }
-            const float d30 = Dl[1800];                                     // K(l, l+30)
-            f0 = fmaf(d30, pl[30], f0);
-            f1 = fmaf(d30, pl[0], f1);
-            acc_a = f0 + g0;
-            acc_b = f1 + g1;
-        }
-        // the same projection on the result (t'K_e = 0 as well), so that
-        // the product stays symmetric: u_e = P K_e P p_e
-        {
-            const float t = 0.05f * sum_mod3(acc_a + acc_b, lane);
-            acc_a -= t;
-            acc_b -= t;
-        }
+        float acc_a, acc_b;
+        sym::walk32(lane, stage + s * kPacked, pp, acc_a, acc_b);
+        sym::project_result(lane, acc_a, acc_b);
         if (active) {
             float *o = ut + (size_t)elem(k) * 80;   // node-padded: row i at (i/3)*4 + i%3
             st_global_hint(o + (lane / 3) * 4 + lane % 3, acc_a, pol);

@@ -147,6 +147,7 @@ struct Ctx {
     // persistent PCG kernels (cooperative launches with grid-wide barriers)
     bool persistent = false;    // true: persistent cooperative kernels for the iteration (pf_set_persistent)
     unsigned long long *gbar = nullptr;   // [kPersistSlots] grid-barrier arrival counters, zeroed per run
+    double *res_part = nullptr;           // the resident PCG's arrival counter and shares, allocated on first use
     int pk_grid[kPersistSlots] = {};      // blocks of each persistent instantiation (0 = not sized)
 
     bool dependent = false;     // programmatic dependent launches in the iteration (small meshes)
@@ -203,6 +204,9 @@ int launch_pcg_iteration(Ctx &c, int prec, double *xsol);
 // iterations (element products included), up to niters per launch.
 int launch_pcg_tail(Ctx &c, int prec, double *xsol);
 int launch_pcg_fused64(Ctx &c, double *xsol, int niters);
+// pf_resident.cu: up to niters iterations of a small mesh in one launch
+bool resident_ok(const Ctx &c, int prec);
+int launch_pcg_resident(Ctx &c, int prec, double *xsol, int niters);
 bool persist_fused64(const Ctx &c, int prec);
 // One bounded mbarrier wait that nothing completes (the error path of the
 // bulk-copy kernels, without a fault): records code 2 in c.kerr.

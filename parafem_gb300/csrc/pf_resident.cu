@@ -1,0 +1,524 @@
+// pf_resident.cu -- whole PCG runs of small meshes in one cooperative launch.
+//
+// On a small mesh an iteration of four kernels is launch latency: 22 us on
+// 10^3 elements, of which the chip works perhaps three.  Here one CTA per SM
+// stays for the whole run.  A CTA owns a range of elements and a range of
+// slots; its elements' records stay in shared memory when they fit (14 FP64,
+// 28 FP32 or 48 FP16 records per SM: 12.8^3, 16^3, 19^3 elements on 152 SMs)
+// and stream through it otherwise.  An iteration (p121.f90:90-104 with
+// DOT_PRODUCT_P, maths.f90:168-215, and checon_par, maths.f90:1052-1062) is
+// three phases with one grid-wide exchange after each:
+//   elements  u_e = K_e p_e with p = d + beta p_old formed in the gather, so
+//             that p needs no phase of its own; results to utemp
+//   slots     u = sum over a node's elements; the owner keeps p; share of p.u
+//   update    x, r, d; shares of r.d and r.r (or checon_par's maxima)
+// An exchange is one counter that every CTA adds to (red.release) and one
+// thread of every CTA polls (ld.acquire): 1.2 us over 152 CTAs, where tagged
+// words that all CTAs poll took 2.1 us and words pushed into a mailbox per
+// CTA 3.8.  The CTAs' shares of a sum lie in memory beside it; every CTA adds
+// them in the same fixed order, so all decide alike and runs are bitwise
+// reproducible.  Every wait is bounded: one that runs out records code 3 and
+// stops the run.
+#include "pf_fix.cuh"
+#include "pf_sym.cuh"
+
+namespace pf {
+
+namespace {
+
+constexpr int kResThreads = 512;
+constexpr int kMaxBlocks = 256;   // shares a warp adds: eight per lane
+
+struct ResArgs {
+    int nels, ns, niters, per_slots;
+    const unsigned char *rec;
+    size_t stride;               // bytes from element to element: 0 for one matrix (FP64)
+    const int *conn;
+    void *ut;
+    const int *ptr, *list;
+    const uint8_t *fm;
+    double *x, *r, *d, *p;
+    const double *dinv;
+    PcgState *st;
+    unsigned long long *count;   // arrivals, zero at the launch
+    double *part;                // [4][kMaxBlocks] shares: p.u, r.d, r.r or max |x|, max |dx|
+    int *kerr;
+};
+
+// per precision: warps that form products, ring stages per warp, bytes of a
+// stage and of the warp's p words
+template <int PREC> struct Shape;
+template <> struct Shape<64> { static constexpr int W = 14, S = 1, stage = 3 * fx::kChunk0, pbytes = 960, rec = fx::kRecBytes; };
+template <> struct Shape<32> { static constexpr int W = 14, S = 2, stage = sym::kBytes32, pbytes = 480, rec = sym::kBytes32; };
+template <> struct Shape<16> { static constexpr int W = 16, S = 3, stage = sym::kBytes16, pbytes = 480, rec = sym::kBytes16; };
+// the p words double as the block sums' scratch (two doubles per thread)
+template <int PREC> constexpr int kScratch = Shape<PREC>::W * Shape<PREC>::pbytes > kResThreads * 16
+                                                 ? Shape<PREC>::W * Shape<PREC>::pbytes : kResThreads * 16;
+template <int PREC> constexpr size_t kResSmem =
+    (size_t)Shape<PREC>::W * Shape<PREC>::S * Shape<PREC>::stage + kScratch<PREC> + Shape<PREC>::W * 3 * 8;
+
+// One thread: its block's writes are out (with those of the threads it has
+// met at a barrier), and every block's are visible on return; false when the
+// wait ran out.
+__device__ __forceinline__ bool exchange(unsigned long long *count, unsigned long long target)
+{
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(count), "l"(1ULL) : "memory");
+    for (long long i = 0; i < kGridSpinLimit; ++i) {
+        unsigned long long v;
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(count) : "memory");
+        if (v >= target) return true;
+    }
+    return false;
+}
+
+// One warp: the blocks' shares added (or their greatest bits), in every lane
+__device__ __forceinline__ double add_shares(const double *p, int nblk, int lane)
+{
+    double v[kMaxBlocks / 32];
+#pragma unroll
+    for (int j = 0; j < kMaxBlocks / 32; ++j) v[j] = lane + 32 * j < nblk ? __ldcg(p + lane + 32 * j) : 0.0;
+    double s = v[0];
+#pragma unroll
+    for (int j = 1; j < kMaxBlocks / 32; ++j)
+        if (32 * j < nblk) s += v[j];
+    return warp_sum(s);
+}
+__device__ __forceinline__ long long max_shares(const double *p, int nblk, int lane)
+{
+    long long m = 0;
+#pragma unroll
+    for (int j = 0; j < kMaxBlocks / 32; ++j)
+        if (lane + 32 * j < nblk) m = max(m, __double_as_longlong(__ldcg(p + lane + 32 * j)));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(FULLMASK, m, o));
+    return m;
+}
+
+}  // namespace
+
+template <int PREC, bool CHECON, int NSL>
+__global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(ResArgs a)
+{
+    using Sh = Shape<PREC>;
+    using UT = typename std::conditional<PREC == 64, double, float>::type;
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ double s_val[4], s_part[2];
+    __shared__ int s_ok, s_stop;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5, nblk = gridDim.x, blk = blockIdx.x;
+    unsigned char *scratch = smem + (size_t)Sh::W * Sh::S * Sh::stage;
+    double *sh = reinterpret_cast<double *>(scratch);   // two rows of kResThreads
+    if (t == 0) {
+        s_stop = a.st->stop;
+        s_ok = 1;
+    }
+    __syncthreads();
+    if (s_stop) return;   // read once per block, before any block writes it
+    double up = a.st->up;
+    const double ff = a.st->ff, tol = a.st->tol;
+    int iters = a.st->iters;
+    const int limit = a.st->limit;
+    const double root_ff = CHECON ? 0.0 : sqrt(ff), bound = tol * root_ff, stop_rr = bound * bound;
+    unsigned long long target = 0;   // arrivals that complete the next exchange
+    double *p_pu = a.part, *p_rd = p_pu + kMaxBlocks, *p_2 = p_rd + kMaxBlocks, *p_3 = p_2 + kMaxBlocks;
+
+    // elements of this warp
+    const int per_el = (a.nels + nblk - 1) / nblk;
+    const int e1 = min(a.nels, (blk + 1) * per_el), first = blk * per_el + w;
+    const int nmine = w < Sh::W && first < e1 ? (e1 - first + Sh::W - 1) / Sh::W : 0;
+    const bool resident = nmine <= Sh::S || (PREC == 64 && a.stride == 0);
+    unsigned char *stage = smem + (size_t)(w < Sh::W ? w : 0) * Sh::S * Sh::stage;
+    unsigned char *pw = scratch + (size_t)(w < Sh::W ? w : 0) * Sh::pbytes;
+    uint64_t *bar = reinterpret_cast<uint64_t *>(scratch + kScratch<PREC>) + 3 * (w < Sh::W ? w : 0);
+    const uint64_t pol = tc::l2_evict_first_policy();
+    // ring slot c: chunk c of a record (FP64, one stage) or stage c
+    auto issue = [&](int c, int k) {
+        const size_t e = (size_t)first + (size_t)k * Sh::W;
+        if constexpr (PREC == 64) {
+            tc::mbar_expect_tx(&bar[c], fx::chunk_bytes(c));
+            tc::bulk_g2s_hint(stage + c * fx::kChunk0, a.rec + e * a.stride + fx::chunk_off(c), fx::chunk_bytes(c), &bar[c],
+                              pol);
+        } else {
+            tc::mbar_expect_tx(&bar[c], Sh::rec);
+            tc::bulk_g2s_hint(stage + c * Sh::stage, a.rec + e * a.stride, Sh::rec, &bar[c], pol);
+        }
+    };
+    if (nmine > 0) {
+        if (lane == 0) {
+            for (int c = 0; c < 3; ++c) tc::mbar_init(&bar[c], 1);
+            tc::mbar_fence_init();
+        }
+        __syncwarp();
+        if (lane == 0)
+            for (int c = 0; c < (PREC == 64 ? 3 : Sh::S); ++c)
+                if (PREC == 64 || c < nmine) issue(c, PREC == 64 ? 0 : c);
+    }
+    auto node = [&](int k) { return lane < 20 && nmine > 0 ? a.conn[((size_t)first + (size_t)(k % nmine) * Sh::W) * 20 + lane] : 0; };
+    const int nd0 = node(0), nd1 = node(1);
+    // this lane's two freedoms of an element: rows 2l, 2l+1 (FP64) or l, l+30
+    const int l30 = lane < 30 ? lane : 29;
+    const int ja = PREC == 64 ? 2 * l30 : l30, jb = PREC == 64 ? 2 * l30 + 1 : l30 + 30;
+    bool start = true;   // p is complete in memory; later p = d + beta p
+    double beta = 0.0;
+    auto gather = [&](int nd, double &va, double &vb) {
+        const int na = __shfl_sync(FULLMASK, nd, ja / 3), nb = __shfl_sync(FULLMASK, nd, jb / 3);
+        const size_t oa = (size_t)3 * na + ja % 3, ob = (size_t)3 * nb + jb % 3;
+        va = __ldcg(a.p + oa);
+        vb = __ldcg(a.p + ob);
+        if (!start) {
+            va = fma(va, beta, __ldcg(a.d + oa));
+            vb = fma(vb, beta, __ldcg(a.d + ob));
+        }
+    };
+
+    // slots of this thread
+    const int s0 = blk * a.per_slots, s1 = min(a.ns, s0 + a.per_slots);
+    const int nact = min(kResThreads, a.per_slots), nwact = (nact + 31) >> 5;   // threads and warps with slots
+    auto block_total = [&](int row) {   // by warp `row`, over the warps with slots
+        double s = sh[row * kResThreads + lane];
+        for (int j = 1; j < nwact; ++j) s += sh[row * kResThreads + lane + 32 * j];
+        return warp_sum(s);
+    };
+    auto meet = [&]() {   // by one thread, after all have raised target
+        if (exchange(a.count, target)) return;
+        s_ok = 0;
+        atomicExch(a.kerr, 3);
+        atomicExch(&a.st->stop, 1);
+    };
+
+    bool failed = false;
+    unsigned g = 0;   // elements this warp has multiplied (ring position)
+    double pc[NSL], uu[NSL];
+    int it = 0;
+    bool stop = false;
+    for (; it < a.niters && !stop; ++it) {
+        // ---- elements
+        if (nmine > 0) {
+            double pa, pb;
+            gather(nd0, pa, pb);
+            int nd = nd1;
+            for (int k = 0; k < nmine; ++k, ++g) {
+                double na = 0.0, nb = 0.0;
+                if (k + 1 < nmine) {
+                    gather(nd, na, nb);
+                    nd = node(k + 2);
+                }
+                const size_t e = (size_t)first + (size_t)k * Sh::W;
+                if constexpr (PREC == 64) {
+                    double u0, u1;
+                    const bool ok = fx::product(
+                        lane, pa, pb, reinterpret_cast<int4 *>(pw),
+                        [&](int c) -> const unsigned char * {
+                            const uint32_t par = resident ? 0u : (g & 1u);
+                            return __all_sync(FULLMASK, tc::mbar_wait(&bar[c], par)) ? stage + c * fx::kChunk0 : nullptr;
+                        },
+                        [&](int c) {
+                            __syncwarp();
+                            if (!resident && lane == 0) {
+                                tc::fence_proxy_async();
+                                issue(c, (k + 1) % nmine);
+                            }
+                        },
+                        u0, u1);
+                    if (!ok) {
+                        failed = true;
+                        break;
+                    }
+                    if (lane < 30)
+                        reinterpret_cast<double2 *>((double *)a.ut + e * 60)[lane] = make_double2(u0, u1);
+                } else {
+                    const int c = resident ? k : (int)(g % Sh::S);
+                    const uint32_t par = resident ? 0u : ((g / Sh::S) & 1u);
+                    float *pp = reinterpret_cast<float *>(pw);
+                    sym::put_p<PREC == 16>(lane, pa, pb, pp);
+                    if (!__all_sync(FULLMASK, tc::mbar_wait(&bar[c], par))) {
+                        failed = true;
+                        break;
+                    }
+                    __syncwarp();
+                    float ra, rb;
+                    if constexpr (PREC == 32)
+                        sym::walk32(lane, reinterpret_cast<const float *>(stage + c * Sh::stage), pp, ra, rb);
+                    else
+                        sym::walk16(lane, reinterpret_cast<const uint32_t *>(stage + c * Sh::stage), pp, ra, rb);
+                    sym::project_result(lane, ra, rb);
+                    if (lane < 30) {
+                        float *o = (float *)a.ut + e * 80;
+                        o[(lane / 3) * 4 + lane % 3] = ra;
+                        o[(lane / 3 + 10) * 4 + lane % 3] = rb;
+                    }
+                    __syncwarp();
+                    if (!resident && lane == 0) {
+                        tc::fence_proxy_async();
+                        issue(c, (k + Sh::S) % nmine);
+                    }
+                }
+                pa = na;
+                pb = nb;
+            }
+            if (failed && lane == 0) {
+                atomicExch(a.kerr, 2);
+                atomicExch(&a.st->stop, 1);
+                s_ok = 0;
+            }
+        }
+        __syncthreads();
+        if (!s_ok) break;
+        target += nblk;
+        if (t == kResThreads - 32) meet();   // a warp of its own: the others load meanwhile
+        // the owners' p, while the flags travel
+        int k0[NSL], k1[NSL];
+#pragma unroll
+        for (int i = 0; i < NSL; ++i) {
+            const int s = s0 + t + i * kResThreads;
+            pc[i] = 0.0;
+            k0[i] = k1[i] = 0;
+            if (s < s1) {
+                pc[i] = a.p[s];
+                if (!start) pc[i] = fma(pc[i], beta, a.d[s]);
+                k0[i] = __ldg(a.ptr + s / 3);
+                k1[i] = (__ldg(a.fm + s / 3) >> (s % 3)) & 1 ? __ldg(a.ptr + s / 3 + 1) : k0[i];   // restrained: u = 0
+            }
+        }
+        __syncthreads();
+        if (!s_ok) break;
+        // ---- slots
+        double pu = 0.0;
+#pragma unroll
+        for (int i = 0; i < NSL; ++i) {
+            const int s = s0 + t + i * kResThreads;
+            uu[i] = 0.0;
+            if (s < s1) {
+                const int dof = s % 3;
+                UT acc = 0;
+                for (int k = k0[i]; k < k1[i]; k += 4) {   // four contributions in flight, added in order
+                    UT v[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int ci = k + q < k1[i] ? __ldg(a.list + k + q) : -1;
+                        v[q] = ci < 0 ? (UT)0
+                               : PREC == 64 ? (UT)__ldcg((const double *)a.ut + (size_t)ci * 3 + dof)
+                                            : (UT)__ldcg((const float *)a.ut + (size_t)ci * 4 + dof);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (k + q < k1[i]) acc += v[q];
+                }
+                uu[i] = (double)acc;
+                a.p[s] = pc[i];   // every gather of the old p is behind the flags
+                pu = fma(pc[i], uu[i], pu);
+            }
+        }
+        sh[t] = pu;
+        double xo[NSL], ro[NSL], dv[NSL];   // in flight behind the sum
+#pragma unroll
+        for (int i = 0; i < NSL; ++i) {
+            const int s = s0 + t + i * kResThreads;
+            xo[i] = ro[i] = dv[i] = 0.0;
+            if (s < s1) {
+                xo[i] = a.x[s];
+                ro[i] = a.r[s];
+                dv[i] = __ldg(a.dinv + s);
+            }
+        }
+        target += nblk;
+        __syncthreads();
+        if (w == 0) {
+            const double mine = block_total(0);
+            if (lane == 0) {
+                p_pu[blk] = mine;
+                meet();
+            }
+            __syncwarp();
+            const double sum = add_shares(p_pu, nblk, lane);
+            if (lane == 0) s_val[0] = up / sum;
+        }
+        __syncthreads();
+        if (!s_ok) break;
+        // ---- update
+        const double alpha = s_val[0];
+        double rd = 0.0, rr = 0.0;
+        long long mx = 0, md = 0;
+#pragma unroll
+        for (int i = 0; i < NSL; ++i) {
+            const int s = s0 + t + i * kResThreads;
+            if (s < s1) {
+                const double xn = fma(pc[i], alpha, xo[i]);
+                a.x[s] = xn;
+                if (CHECON) {
+                    mx = max(mx, abs_bits(xn));
+                    md = max(md, abs_bits(xn - xo[i]));
+                }
+                const double rn = fma(-uu[i], alpha, ro[i]), dn = dv[i] * rn;
+                a.r[s] = rn;
+                a.d[s] = dn;
+                rd = fma(rn, dn, rd);
+                if (!CHECON) rr = fma(rn, rn, rr);
+            }
+        }
+        sh[t] = rd;
+        if (!CHECON) sh[kResThreads + t] = rr;
+        if (CHECON) block_max2(mx, md);   // (its barriers order sh too)
+        __syncthreads();
+        if (w == 0 || (w == 1 && !CHECON)) {
+            const double mine = block_total(w);
+            if (lane == 0) s_part[w] = mine;
+        }
+        target += nblk;
+        __syncthreads();
+        if (t == 0) {
+            p_rd[blk] = s_part[0];
+            p_2[blk] = CHECON ? __longlong_as_double(mx) : s_part[1];
+            if (CHECON) p_3[blk] = __longlong_as_double(md);
+            meet();
+        }
+        __syncthreads();
+        if (!s_ok) break;
+        if (w == 2) {   // beta and the stopping value side by side (warp 0, fresh from its wait, takes 0.8 us longer)
+            const double sum = add_shares(p_rd, nblk, lane);
+            if (lane == 0) {
+                s_val[1] = sum;
+                s_val[2] = sum / up;
+            }
+        } else if (w == 1 && CHECON) {
+            const long long m = max_shares(p_2, nblk, lane), q = max_shares(p_3, nblk, lane);
+            if (lane == 0) {
+                s_val[3] = __longlong_as_double(q) / __longlong_as_double(m);   // checon_par's measure
+                s_stop = isfinite(__longlong_as_double(m)) ? 0 : 1;
+            }
+        } else if (w == 1) {
+            const double sum = add_shares(p_2, nblk, lane);
+            if (lane == 0) {
+                s_val[3] = sum;
+                s_stop = 0;
+            }
+        }
+        __syncthreads();
+        const double rdn = s_val[1], measure = s_val[3];
+        beta = s_val[2];
+        ++iters;
+        // ||r|| / ||f|| <= tol as r.r <= (tol ||f||)^2: two roots and a
+        // division would be a tenth of the iteration
+        const bool conv = CHECON ? measure <= tol : measure <= stop_rr;
+        const bool bad = !isfinite(rdn) || s_stop != 0;
+        stop = conv || iters >= limit || bad;
+        if (blk == 0 && t == 0 && (stop || it + 1 == a.niters)) {
+            volatile PcgState *vs = a.st;
+            vs->up = rdn;
+            vs->beta = beta;
+            vs->iters = iters;
+            vs->rr = CHECON ? 0.0 : measure;
+            vs->metric = CHECON ? measure : sqrt(measure) / root_ff;
+            vs->converged = conv ? 1 : 0;
+            if (bad) vs->err = 1;
+            if (stop) vs->stop = vs->stop2 = 1;
+        }
+        up = rdn;
+        start = false;
+    }
+    // p of the next iteration, as update2 leaves it
+    if (s_ok && !start) {
+#pragma unroll
+        for (int i = 0; i < NSL; ++i) {
+            const int s = s0 + t + i * kResThreads;
+            if (s < s1) a.p[s] = fma(pc[i], beta, a.d[s]);
+        }
+    }
+    // wait (bounded) for the copies this warp still has in flight: the ring's
+    // next ones, or, when a wait ran out, whatever had been issued
+    if (nmine > 0 && (!resident || failed)) {
+        if constexpr (PREC == 64) {
+            for (int c = 0; c < 3; ++c) {
+                tc::mbar_wait(&bar[c], resident ? 0u : g & 1u);
+                if (failed && !resident) tc::mbar_wait(&bar[c], (g + 1) & 1u);
+            }
+        } else {
+            for (unsigned q = g; q < g + Sh::S; ++q)
+                if (!resident || (int)(q - g) < nmine) tc::mbar_wait(&bar[q % Sh::S], resident ? 0u : (q / Sh::S) & 1u);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Rule: 20-node meshes with records (one per element, or FP64 one for all)
+// whose slots fit the CTAs, four per thread (311,296 on 152 SMs: 28^3 elements).  Measured us per
+// iteration, this kernel / four kernels in a graph:
+//            6^3         10^3        16^3        20^3        24^3        28^3
+//   FP64     12.2/19.7   13.5/21.5   24.1/30.5   39.5/43.4   59.3/63.1   84.6/87.0
+//   FP32     13.6/23.4   13.7/22.7   18.3/28.8   27.1/33.0   37.7/43.8   49.1/56.8
+//   FP16     13.4/22.6   13.1/22.2   16.7/24.5   25.7/29.0   33.2/35.5   43.4/45.8
+// so that it takes every mesh that fits.  Of the 13.5 us at 10^3 the three
+// exchanges take 4, the products 3.5 and the sums and divisions 4.
+static int slots_per_block(const Ctx &c) { return (c.nslots + c.nsm - 1) / c.nsm; }
+
+bool resident_ok(const Ctx &c, int prec)
+{
+    if (c.kind != KIND_SOLID20 || c.nsm > kMaxBlocks) return false;
+    if (slots_per_block(c) > 4 * kResThreads) return false;
+    if (c.shared) return prec == PREC_FP64 && c.skmfix;
+    return prec == PREC_FP64 ? c.kmfix != nullptr : prec == PREC_FP32_SYM || prec == PREC_FP16_SYM;
+}
+
+template <int PREC, bool CHECON, int NSL>
+static int launch_resident_t(Ctx &c, double *xsol, int niters)
+{
+    constexpr size_t smem = kResSmem<PREC>;
+    static_assert(smem + 256 + 2 * 32 * 8 <= 227 * 1024, "shared memory per CTA");
+    const void *fn = (const void *)k_pcg_resident<PREC, CHECON, NSL>;
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    ResArgs a;
+    a.nels = c.nels;
+    a.ns = c.nslots;
+    a.niters = niters;
+    a.per_slots = slots_per_block(c);
+    a.stride = c.shared ? 0 : Shape<PREC>::rec;
+    a.rec = c.shared ? c.skmfix : PREC == 64 ? c.kmfix : PREC == 32 ? (const unsigned char *)c.km32p : (const unsigned char *)c.km16p;
+    a.conn = c.conn;
+    a.ut = c.utemp;
+    a.ptr = c.node_ptr;
+    a.list = c.node_list;
+    a.fm = c.freemask;
+    a.x = xsol;
+    a.r = c.r;
+    a.d = c.d;
+    a.p = c.p;
+    a.dinv = c.dinv;
+    a.st = c.st;
+    if (!c.res_part) {
+        const size_t bytes = 64 + 4 * kMaxBlocks * sizeof(double);
+        if (ctx_malloc(c, (void **)&c.res_part, bytes)) {
+            set_error("k_pcg_resident: cannot allocate %zu bytes of shares", bytes);
+            return 1;
+        }
+    }
+    a.count = reinterpret_cast<unsigned long long *>(c.res_part);
+    a.part = c.res_part + 8;
+    if (e == cudaSuccess) e = cudaMemsetAsync(a.count, 0, sizeof(unsigned long long), c.stream);
+    a.kerr = c.kerr;
+    void *args[] = {&a};
+    if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(fn, dim3(c.nsm), dim3(kResThreads), args, smem, c.stream);
+    c.launches++;
+    if (e != cudaSuccess) {
+        set_error("k_pcg_resident: cooperative launch of %d blocks failed: %s", c.nsm, cudaGetErrorString(e));
+        return 1;
+    }
+    return 0;
+}
+
+template <int PREC>
+static int launch_resident_p(Ctx &c, double *xsol, int niters)
+{
+    const bool ck = c.stop_mode == STOP_CHECON, one = slots_per_block(c) <= kResThreads;
+    if (PREC == 64 && ck)   // checon_par stops FP64 runs only
+        return one ? launch_resident_t<PREC, PREC == 64, 1>(c, xsol, niters)
+                   : launch_resident_t<PREC, PREC == 64, 4>(c, xsol, niters);
+    return one ? launch_resident_t<PREC, false, 1>(c, xsol, niters) : launch_resident_t<PREC, false, 4>(c, xsol, niters);
+}
+
+int launch_pcg_resident(Ctx &c, int prec, double *xsol, int niters)
+{
+    return prec == PREC_FP64 ? launch_resident_p<64>(c, xsol, niters)
+           : prec == PREC_FP32_SYM ? launch_resident_p<32>(c, xsol, niters)
+                                   : launch_resident_p<16>(c, xsol, niters);
+}
+
+}  // namespace pf
