@@ -168,6 +168,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(ResArgs a)
             va = fma(va, beta, __ldcg(a.d + oa));
             vb = fma(vb, beta, __ldcg(a.d + ob));
         }
+        if (PREC != 64 && lane >= 30) va = vb = 0.0;   // put_p's means are sums over all lanes
     };
 
     // slots of this thread

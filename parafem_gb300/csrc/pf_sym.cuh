@@ -17,7 +17,8 @@ constexpr int kPSlot = 120;                    // floats of p per warp
 constexpr int kWords32 = 1832, kWords16 = 916; // 4-byte words of a record
 constexpr int kBytes32 = kWords32 * 4, kBytes16 = kWords16 * 4;
 
-// p of an element, less its mean translation, into the warp's slot pp.
+// p of an element, less its mean translation, into the warp's slot pp.  Lanes 30
+// and 31 pass zeros.
 // K_e t = 0 for a rigid translation t, so the subtraction changes nothing in
 // exact arithmetic; in FP32 it keeps the translation of a smooth p out of
 // the rounding of p, of storkm's entries and of the sums (errors that grow
