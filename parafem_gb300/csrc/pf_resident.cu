@@ -7,11 +7,14 @@
 // 28 FP32 or 48 FP16 records per SM: 12.8^3, 16^3, 19^3 elements on 152 SMs)
 // and stream through it otherwise.  An iteration (p121.f90:90-104 with
 // DOT_PRODUCT_P, maths.f90:168-215, and checon_par, maths.f90:1052-1062) is
-// three phases with one grid-wide exchange after each:
+// two phases with one grid-wide exchange after each:
 //   elements  u_e = K_e p_e with p = d + beta p_old formed in the gather, so
-//             that p needs no phase of its own; results to utemp
-//   slots     u = sum over a node's elements; the owner keeps p; share of p.u
-//   update    x, r, d; shares of r.d and r.r (or checon_par's maxima)
+//             that p needs no phase of its own; results to utemp; share of
+//             p.u as the sum of p_e.u_e
+//   slots     u = sum over a node's elements; the owner keeps p; x, r, d;
+//             shares of r.d and r.r (or checon_par's maxima)
+// (With p.u formed from the summed u, a third exchange stands between u and
+// x: 13.5 us per iteration on 10^3 elements.)
 // An exchange is one counter that every CTA adds to (red.release) and one
 // thread of every CTA polls (ld.acquire): 1.2 us over 152 CTAs, where tagged
 // words that all CTAs poll took 2.1 us and words pushed into a mailbox per
@@ -193,6 +196,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(ResArgs a)
     bool stop = false;
     for (; it < a.niters && !stop; ++it) {
         // ---- elements
+        double pu = 0.0;
         if (nmine > 0) {
             double pa, pb;
             gather(nd0, pa, pb);
@@ -224,8 +228,11 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(ResArgs a)
                         failed = true;
                         break;
                     }
-                    if (lane < 30)
+                    if (lane < 30) {
                         reinterpret_cast<double2 *>((double *)a.ut + e * 60)[lane] = make_double2(u0, u1);
+                        pu = fma(pa, u0, pu);
+                        pu = fma(pb, u1, pu);
+                    }
                 } else {
                     const int c = resident ? k : (int)(g % Sh::S);
                     const uint32_t par = resident ? 0u : ((g / Sh::S) & 1u);
@@ -246,6 +253,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(ResArgs a)
                         float *o = (float *)a.ut + e * 80;
                         o[(lane / 3) * 4 + lane % 3] = ra;
                         o[(lane / 3 + 10) * 4 + lane % 3] = rb;
+                        pu = fma(pa, (double)ra, pu);
+                        pu = fma(pb, (double)rb, pu);
                     }
                     __syncwarp();
                     if (!resident && lane == 0) {
@@ -262,10 +271,21 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(ResArgs a)
                 s_ok = 0;
             }
         }
+        if (w < Sh::W) reinterpret_cast<double *>(pw)[lane] = pu;   // the warp's p words are free
+        target += nblk;
         __syncthreads();
         if (!s_ok) break;
-        target += nblk;
-        if (t == kResThreads - 32) meet();   // a warp of its own: the others load meanwhile
+        if (w == kResThreads / 32 - 1) {   // a warp of its own: the others load meanwhile
+            double mine = 0.0;
+#pragma unroll
+            for (int j = 0; j < Sh::W; ++j) mine += reinterpret_cast<const double *>(scratch + j * Sh::pbytes)[lane];
+            mine = warp_sum(mine);
+            if (lane == 0) {
+                p_pu[blk] = mine;
+                meet();
+            }
+            __syncwarp();
+        }
         // the owners' p, while the flags travel
         int k0[NSL], k1[NSL];
 #pragma unroll
@@ -282,14 +302,21 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(ResArgs a)
         }
         __syncthreads();
         if (!s_ok) break;
-        // ---- slots
-        double pu = 0.0;
+        // ---- slots; the step length meanwhile, by the warp that met
+        if (w == kResThreads / 32 - 1) {
+            const double sum = add_shares(p_pu, nblk, lane);
+            if (lane == 0) s_val[0] = up / sum;
+        }
+        double xo[NSL], ro[NSL], dv[NSL];
 #pragma unroll
         for (int i = 0; i < NSL; ++i) {
             const int s = s0 + t + i * kResThreads;
-            uu[i] = 0.0;
+            uu[i] = xo[i] = ro[i] = dv[i] = 0.0;
             if (s < s1) {
                 const int dof = s % 3;
+                xo[i] = a.x[s];
+                ro[i] = a.r[s];
+                dv[i] = __ldg(a.dinv + s);
                 UT acc = 0;
                 for (int k = k0[i]; k < k1[i]; k += 4) {   // four contributions in flight, added in order
                     UT v[4];
@@ -306,36 +333,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(ResArgs a)
                 }
                 uu[i] = (double)acc;
                 a.p[s] = pc[i];   // every gather of the old p is behind the flags
-                pu = fma(pc[i], uu[i], pu);
             }
-        }
-        sh[t] = pu;
-        double xo[NSL], ro[NSL], dv[NSL];   // in flight behind the sum
-#pragma unroll
-        for (int i = 0; i < NSL; ++i) {
-            const int s = s0 + t + i * kResThreads;
-            xo[i] = ro[i] = dv[i] = 0.0;
-            if (s < s1) {
-                xo[i] = a.x[s];
-                ro[i] = a.r[s];
-                dv[i] = __ldg(a.dinv + s);
-            }
-        }
-        target += nblk;
-        __syncthreads();
-        if (w == 0) {
-            const double mine = block_total(0);
-            if (lane == 0) {
-                p_pu[blk] = mine;
-                meet();
-            }
-            __syncwarp();
-            const double sum = add_shares(p_pu, nblk, lane);
-            if (lane == 0) s_val[0] = up / sum;
         }
         __syncthreads();
-        if (!s_ok) break;
-        // ---- update
         const double alpha = s_val[0];
         double rd = 0.0, rr = 0.0;
         long long mx = 0, md = 0;
@@ -443,12 +443,13 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(ResArgs a)
 // Rule: 20-node meshes with records (one per element, or FP64 one for all)
 // whose slots fit the CTAs, four per thread (311,296 on 152 SMs: 28^3 elements).  Measured us per
 // iteration, this kernel / four kernels in a graph:
-//            6^3         10^3        16^3        20^3        24^3        28^3
-//   FP64     12.2/19.7   13.5/21.5   24.1/30.5   39.5/43.4   59.3/63.1   84.6/87.0
-//   FP32     13.6/23.4   13.7/22.7   18.3/28.8   27.1/33.0   37.7/43.8   49.1/56.8
-//   FP16     13.4/22.6   13.1/22.2   16.7/24.5   25.7/29.0   33.2/35.5   43.4/45.8
-// so that it takes every mesh that fits.  Of the 13.5 us at 10^3 the three
-// exchanges take 4, the products 3.5 and the sums and divisions 4.
+//            10^3        16^3        20^3        24^3        28^3
+//   FP64     10.8/21.5   22.0/30.5   36.1/43.4   56.0/63.1   82.0/87.0
+//   FP32     11.4/22.7   15.7/28.8   24.3/33.0   34.3/43.8   46.1/56.8
+//   FP16     10.1/22.2   13.7/24.5   22.7/29.0   29.9/35.5   40.9/45.8
+// so that it takes every mesh that fits.  Of the 10.8 us at 10^3 (FP64)
+// the products take 3.8, the two exchanges 2.6 and the sums over the CTAs with
+// the two divisions 2.5.
 static int slots_per_block(const Ctx &c) { return (c.nslots + c.nsm - 1) / c.nsm; }
 
 bool resident_ok(const Ctx &c, int prec)
