@@ -181,15 +181,17 @@ int pf_set_graphs(void **ctx, const int *on);
 
 /* The PCG iteration's scatter, update passes and finish (p121.f90:90-104
  * with DOT_PRODUCT_P, maths.f90:168-215, and checon_par, maths.f90:999-1069)
- * run as one persistent cooperative kernel with grid-wide barriers when
- * *on != 0; FP64 solves (PF_MODE_P121, PF_MODE_FP64_RES) on per-element
- * storkm then run whole iterations, element products included, up to 32
- * per launch.  *on == 0, the default, launches the separate scatter, update
- * and finish kernels, replayed from CUDA graphs, which measure faster on
- * GB300.  Both give bitwise the same iterates.  Applies to 20-node
- * contexts; 8-node contexts always use the separate kernels, and meshes of
- * up to about 311,000 freedoms (other than mixed solves of one shared km)
- * always run as one resident kernel (graphs and this switch make no difference to them). */
+ * of meshes too large for the rule below run as one persistent cooperative
+ * kernel with grid-wide barriers when *on != 0; FP64 solves (PF_MODE_P121,
+ * PF_MODE_FP64_RES) on per-element storkm then run whole iterations, element
+ * products included, up to 32 per launch.  *on == 0, the default, launches
+ * the separate scatter, update and finish kernels, replayed from CUDA graphs,
+ * which measure faster on GB300.  Both give bitwise the same iterates.
+ * Applies to 20-node contexts; 8-node contexts always use the separate
+ * kernels.  20-node meshes of up to about 4,046,000 freedoms (on 152 SMs)
+ * always run one cooperative kernel behind the element products, and those
+ * of up to about 311,000 (other than mixed solves of one shared km) whole
+ * runs in one resident kernel: this switch makes no difference to them. */
 int pf_set_persistent(void **ctx, const int *on);
 
 /* Self-check of the error path of the bulk-copy element kernels (no

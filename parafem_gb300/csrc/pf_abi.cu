@@ -255,6 +255,7 @@ static int run_pcg(Ctx &c, int prec, double *xsol, int limit)
         }
         return 0;
     }
+    if (tail_ok(c) && prepare_tail(c)) return 1;
     if (persist_fused64(c, prec)) {
         // whole FP64 iterations in persistent launches, one launch per chunk
         for (;;) {

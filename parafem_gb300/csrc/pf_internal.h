@@ -65,6 +65,7 @@ constexpr int kRowBlocks = 64;   // of the 8-node scalar product: rows are short
 // 113 us at 40^3, and lose 0.5 % at 80^3.
 constexpr int kDependentSlots = 500000;
 constexpr int kPersistSlots = 8;   // persistent-kernel instantiations, one barrier counter and grid each
+constexpr int kTailBar = 6;         // the counter of the iteration tail (the persistent kernel's use 0 to 5)
 constexpr int kBarWords = 16;      // u64 words per counter (one 128-byte line each)
 // 20-node elasticity (p121), 8-node scalar (p123), 8-node elasticity (p122's demo)
 enum { KIND_SOLID20 = 0, KIND_SCALAR8 = 1, KIND_SOLID8 = 2 };
@@ -147,6 +148,7 @@ struct Ctx {
     // persistent PCG kernels (cooperative launches with grid-wide barriers)
     bool persistent = false;    // true: persistent cooperative kernels for the iteration (pf_set_persistent)
     unsigned long long *gbar = nullptr;   // [kPersistSlots] grid-barrier arrival counters, zeroed per run
+    bool tail_attr = false;               // shared-memory attribute of k_pcg_tail set
     double *res_part = nullptr;           // the resident PCG's arrival counter and shares, allocated on first use
     int pk_grid[kPersistSlots] = {};      // blocks of each persistent instantiation (0 = not sized)
 
@@ -207,6 +209,9 @@ int launch_pcg_fused64(Ctx &c, double *xsol, int niters);
 // pf_resident.cu: up to niters iterations of a small mesh in one launch
 bool resident_ok(const Ctx &c, int prec);
 int launch_pcg_resident(Ctx &c, int prec, double *xsol, int niters);
+int prepare_tail(Ctx &c);
+bool tail_ok(const Ctx &c);
+int launch_iteration_tail(Ctx &c, int prec, double *xsol);   // scatter, updates and finish of a PCG iteration
 bool persist_fused64(const Ctx &c, int prec);
 // One bounded mbarrier wait that nothing completes (the error path of the
 // bulk-copy kernels, without a fault): records code 2 in c.kerr.

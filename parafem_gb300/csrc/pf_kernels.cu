@@ -1089,7 +1089,7 @@ static int launch_persist_t(Ctx &c, double *xsol, int niters)
 
 bool persist_fused64(const Ctx &c, int prec)
 {
-    return c.persistent && prec == PREC_FP64 && !c.shared && c.kind == KIND_SOLID20;
+    return c.persistent && prec == PREC_FP64 && !c.shared && c.kind == KIND_SOLID20 && !tail_ok(c);
 }
 
 int launch_pcg_tail(Ctx &c, int prec, double *xsol)
@@ -1108,6 +1108,10 @@ int launch_pcg_fused64(Ctx &c, double *xsol, int niters)
 
 int launch_pcg_iteration(Ctx &c, int prec, double *xsol)
 {
+    if (tail_ok(c)) {
+        if (launch_elem(c, prec, c.p)) return 1;
+        return launch_iteration_tail(c, prec, xsol);
+    }
     if (c.persistent && c.kind == KIND_SOLID20) {
         if (persist_fused64(c, prec)) return launch_pcg_fused64(c, xsol, 1);
         if (launch_elem(c, prec, c.p)) return 1;

@@ -439,6 +439,18 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(ResArgs a)
     }
 }
 
+// The arrival counter and the CTAs' shares (outside any stream capture)
+static int ensure_shares(Ctx &c)
+{
+    if (c.res_part) return 0;
+    const size_t bytes = 64 + 4 * kMaxBlocks * sizeof(double);
+    if (ctx_malloc(c, (void **)&c.res_part, bytes)) {
+        set_error("PCG: cannot allocate %zu bytes of shares", bytes);
+        return 1;
+    }
+    return 0;
+}
+
 // ---------------------------------------------------------------------------
 // Rule: 20-node meshes with records (one per element, or FP64 one for all)
 // whose slots fit the CTAs, four per thread (311,296 on 152 SMs: 28^3 elements).  Measured us per
@@ -485,13 +497,7 @@ static int launch_resident_t(Ctx &c, double *xsol, int niters)
     a.p = c.p;
     a.dinv = c.dinv;
     a.st = c.st;
-    if (!c.res_part) {
-        const size_t bytes = 64 + 4 * kMaxBlocks * sizeof(double);
-        if (ctx_malloc(c, (void **)&c.res_part, bytes)) {
-            set_error("k_pcg_resident: cannot allocate %zu bytes of shares", bytes);
-            return 1;
-        }
-    }
+    if (ensure_shares(c)) return 1;
     a.count = reinterpret_cast<unsigned long long *>(c.res_part);
     a.part = c.res_part + 8;
     if (e == cudaSuccess) e = cudaMemsetAsync(a.count, 0, sizeof(unsigned long long), c.stream);
@@ -521,6 +527,341 @@ int launch_pcg_resident(Ctx &c, int prec, double *xsol, int niters)
     return prec == PREC_FP64 ? launch_resident_p<64>(c, xsol, niters)
            : prec == PREC_FP32_SYM ? launch_resident_p<32>(c, xsol, niters)
                                    : launch_resident_p<16>(c, xsol, niters);
+}
+
+// ---------------------------------------------------------------------------
+// The rest of an iteration behind the element products, in one cooperative
+// launch, for meshes that the resident kernel does not take: one CTA of 1024
+// threads per SM, which keeps u and then d of its slots in shared memory (7 of
+// the 13 vector streams of the separate kernels are left), and two exchanges
+// where they have launches.  Node sums go a thread per node (one 16-byte load
+// per FP32 contribution), everything else a thread per slot: sums per slot
+// took 162 instead of 152 us of a 64^3 iteration with one element matrix.
+// Bound by the chain of sums, exchange and division at 33^3 (8.8 of 19 us)
+// and by the FP64 pipe at 64^3 (eight operations per slot, two per SM and
+// clock: 45 us of 96).
+constexpr int kTailThreads = 1024;
+
+struct TailArgs {
+    int nn, per_nodes;
+    const void *ut;
+    const int *ptr, *list;
+    const uint8_t *fm;
+    double *x, *r, *p;
+    const double *dinv;
+    float2 *ps;                  // the FP32 parts of p (shared km), or null
+    PcgState *st;
+    unsigned long long *count;   // arrivals, zeroed by launch_pcg_init
+    double *part;
+    int *kerr;
+};
+
+// One warp: the sum over a block's threads, in four chains per lane
+__device__ __forceinline__ double tail_total(const double *sh, int lane)
+{
+    double v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        v[q] = sh[lane + 32 * q];
+#pragma unroll
+        for (int j = 1; j < kTailThreads / 128; ++j) v[q] += sh[lane + 32 * q + 128 * j];
+    }
+    return warp_sum((v[0] + v[1]) + (v[2] + v[3]));
+}
+
+template <typename UT, bool CHECON, bool FEW>
+__global__ void __launch_bounds__(kTailThreads, 1) k_pcg_tail(TailArgs a)
+{
+    extern __shared__ double su[];   // u, then d, of the block's slots
+    __shared__ double sh[2][kTailThreads];
+    __shared__ double s_val[4], s_part[2], s_bound;
+    __shared__ int s_ok, s_stop;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5, nblk = gridDim.x, blk = blockIdx.x;
+    if (t == 0) {
+        s_stop = a.st->stop;
+        s_ok = 1;
+    }
+    __syncthreads();
+    if (s_stop) return;   // read once per block, before any block writes it
+    const double up = a.st->up, tol = a.st->tol;
+    const int iters = a.st->iters;
+    unsigned long long target = (2ULL * iters + 1) * nblk;   // arrivals that complete the next exchange
+    double *p_pu = a.part, *p_rd = p_pu + kMaxBlocks, *p_2 = p_rd + kMaxBlocks, *p_3 = p_2 + kMaxBlocks;
+    auto meet = [&]() {
+        if (exchange(a.count, target)) return;
+        s_ok = 0;
+        atomicExch(a.kerr, 3);
+        atomicExch(&a.st->stop, 1);
+    };
+    // ---- node sums (ascending element order) and p.u
+    const int n0 = blk * a.per_nodes, n1 = min(a.nn, n0 + a.per_nodes), s0 = 3 * n0, s1 = 3 * n1;
+    double pu = 0.0;
+    int kn = 0, kn1 = 0;   // the next node's part of the list
+    if (n0 + t < n1) {
+        kn = __ldg(a.ptr + n0 + t);
+        kn1 = __ldg(a.ptr + n0 + t + 1);
+    }
+    for (int n = n0 + t; n < n1; n += kTailThreads) {
+        const int k0 = kn, k1 = kn1, m = __ldg(a.fm + n);
+        if (n + kTailThreads < n1) {
+            kn = __ldg(a.ptr + n + kTailThreads);
+            kn1 = __ldg(a.ptr + n + kTailThreads + 1);
+        }
+        const double *pn = a.p + (size_t)3 * n;
+        const double p0 = pn[0], p1 = pn[1], p2 = pn[2];
+        UT u0 = 0, u1 = 0, u2 = 0;
+        for (int k = k0; k < k1; k += 4) {   // four contributions in flight
+            int ci[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) ci[q] = __ldg(a.list + min(k + q, k1 - 1));
+            UT v[4][3];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if constexpr (sizeof(UT) == 4) {
+                    const float4 f = __ldg((const float4 *)a.ut + ci[q]);
+                    v[q][0] = f.x;
+                    v[q][1] = f.y;
+                    v[q][2] = f.z;
+                } else {
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) v[q][d] = __ldg((const double *)a.ut + (size_t)ci[q] * 3 + d);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (k + q < k1) {
+                    u0 += v[q][0];
+                    u1 += v[q][1];
+                    u2 += v[q][2];
+                }
+        }
+        const double e0 = m & 1 ? (double)u0 : 0.0, e1 = m & 2 ? (double)u1 : 0.0, e2 = m & 4 ? (double)u2 : 0.0;
+        double *o = su + 3 * (n - n0);
+        o[0] = e0;
+        o[1] = e1;
+        o[2] = e2;
+        pu = fma(p0, e0, pu);
+        pu = fma(p1, e1, pu);
+        pu = fma(p2, e2, pu);
+    }
+    sh[0][t] = pu;
+    // a block of at most two slots per thread has them in flight behind the sum
+    double xo[2], ro[2], dv[2], po[2];
+    if (FEW) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int s = s0 + t + i * kTailThreads;
+            if (s < s1) {
+                xo[i] = a.x[s];
+                ro[i] = a.r[s];
+                dv[i] = __ldg(a.dinv + s);
+                po[i] = a.p[s];
+            }
+        }
+    }
+    __syncthreads();
+    if (w == 0) {
+        const double mine = tail_total(sh[0], lane);
+        if (lane == 0) {
+            p_pu[blk] = mine;
+            meet();
+        }
+        __syncwarp();
+        const double sum = add_shares(p_pu, nblk, lane);
+        if (lane == 0) s_val[0] = up / sum;
+    } else if (w == 1 && !CHECON && lane == 0) {
+        s_bound = tol * sqrt(a.st->ff);
+    }
+    target += nblk;
+    __syncthreads();
+    if (!s_ok) return;
+    // ---- x, r, d
+    const double alpha = s_val[0];
+    double rd = 0.0, rr = 0.0;
+    long long mx = 0, md = 0;
+    auto move = [&](int s, double p, double x0) {
+        const double xn = fma(p, alpha, x0);
+        a.x[s] = xn;
+        if (CHECON) {
+            mx = max(mx, abs_bits(xn));
+            md = max(md, abs_bits(xn - x0));
+        }
+    };
+    auto residual = [&](int s, double r0, double di) {
+        const double rn = fma(-su[s - s0], alpha, r0), dn = di * rn;
+        a.r[s] = rn;
+        su[s - s0] = dn;
+        rd = fma(rn, dn, rd);
+        if (!CHECON) rr = fma(rn, rn, rr);
+    };
+    if (FEW) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int s = s0 + t + i * kTailThreads;
+            if (s < s1) {
+                move(s, po[i], xo[i]);
+                residual(s, ro[i], dv[i]);
+            }
+        }
+    } else {
+#pragma unroll 2
+        for (int s = s0 + t; s < s1; s += kTailThreads) {
+            move(s, a.p[s], a.x[s]);
+            residual(s, a.r[s], __ldg(a.dinv + s));
+        }
+    }
+    sh[0][t] = rd;
+    if (!CHECON) sh[1][t] = rr;
+    if (CHECON) block_max2(mx, md);
+    __syncthreads();
+    if (w == 0 || (w == 1 && !CHECON)) {
+        const double mine = tail_total(sh[w], lane);
+        if (lane == 0) s_part[w] = mine;
+    }
+    __syncthreads();
+    if (t == 0) {
+        p_rd[blk] = s_part[0];
+        p_2[blk] = CHECON ? __longlong_as_double(mx) : s_part[1];
+        if (CHECON) p_3[blk] = __longlong_as_double(md);
+        meet();
+    }
+    __syncthreads();
+    if (!s_ok) return;
+    if (w == 2) {
+        const double sum = add_shares(p_rd, nblk, lane);
+        if (lane == 0) {
+            s_val[1] = sum;
+            s_val[2] = sum / up;
+        }
+    } else if (w == 1 && blk == 0) {   // the stopping test is block 0's
+        if (CHECON) {
+            const long long m = max_shares(p_2, nblk, lane), q = max_shares(p_3, nblk, lane);
+            if (lane == 0) {
+                s_val[3] = __longlong_as_double(q) / __longlong_as_double(m);   // checon_par's measure
+                s_stop = isfinite(__longlong_as_double(m)) ? 0 : 1;
+            }
+        } else {
+            const double sum = add_shares(p_2, nblk, lane);
+            if (lane == 0) s_val[3] = sum;
+        }
+    }
+    __syncthreads();
+    // ---- p
+    const double beta = s_val[2];
+    auto direct = [&](int s, double p) {
+        const double pn = fma(p, beta, su[s - s0]);
+        a.p[s] = pn;
+        if (a.ps) {
+            float h, l;
+            tc::split_f64(pn, h, l);
+            a.ps[s] = make_float2(h, l);
+        }
+    };
+    if (FEW) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int s = s0 + t + i * kTailThreads;
+            if (s < s1) direct(s, po[i]);
+        }
+    } else {
+#pragma unroll 4
+        for (int s = s0 + t; s < s1; s += kTailThreads) direct(s, a.p[s]);
+    }
+    if (blk == 0 && t == 0) {
+        const double rdn = s_val[1], measure = s_val[3];
+        const bool conv = CHECON ? measure <= tol : measure <= s_bound * s_bound;
+        const bool bad = !isfinite(rdn) || s_stop != 0;
+        volatile PcgState *vs = a.st;
+        vs->up = rdn;
+        vs->beta = beta;
+        vs->iters = iters + 1;
+        vs->rr = CHECON ? 0.0 : measure;
+        vs->metric = CHECON ? measure : sqrt(measure) / sqrt(vs->ff);
+        vs->converged = conv ? 1 : 0;
+        if (bad) vs->err = 1;
+        if (conv || iters + 1 >= vs->limit || bad) vs->stop = vs->stop2 = 1;
+    }
+}
+
+constexpr int kTailMax = 26;   // slots per thread that fit in shared memory
+
+// Rule: 20-node meshes whose slots fit the CTAs' shared memory (4,046,848 on
+// 152 SMs).  us per iteration with this kernel / with scatter, update1 and
+// update2 in a graph:
+//                          33^3          45^3        55^3        64^3
+//   FP64                   120/125       278/288     497/502     778/782
+//   FP32                   67/74         147/162     254/263     402/409
+//   FP16                   52/59         103/117     173/182     271/273
+//   FP32, one matrix       36/43         61/74       95/103      153/153
+static int tail_nodes(const Ctx &c) { return (c.nn + c.nsm - 1) / c.nsm; }
+
+bool tail_ok(const Ctx &c)
+{
+    return c.kind == KIND_SOLID20 && c.nsm <= kMaxBlocks && 3 * tail_nodes(c) <= kTailMax * kTailThreads;
+}
+
+// The shared memory of the tail's largest form (outside any stream capture)
+int prepare_tail(Ctx &c)
+{
+    if (ensure_shares(c)) return 1;
+    if (c.tail_attr) return 0;
+    const void *fn[] = {(const void *)k_pcg_tail<double, true, false>, (const void *)k_pcg_tail<double, false, false>,
+                        (const void *)k_pcg_tail<float, true, false>, (const void *)k_pcg_tail<float, false, false>};
+    for (const void *f : fn) {
+        const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   kTailMax * kTailThreads * (int)sizeof(double));
+        if (e != cudaSuccess) {
+            set_error("k_pcg_tail: cannot reserve shared memory: %s", cudaGetErrorString(e));
+            return 1;
+        }
+    }
+    c.tail_attr = true;
+    return 0;
+}
+
+template <typename UT, bool CHECON, bool FEW>
+static int launch_tail_t(Ctx &c, double *xsol)
+{
+    TailArgs a;
+    a.nn = c.nn;
+    a.per_nodes = tail_nodes(c);
+    a.ut = c.utemp;
+    a.ptr = c.node_ptr;
+    a.list = c.node_list;
+    a.fm = c.freemask;
+    a.x = xsol;
+    a.r = c.r;
+    a.p = c.p;
+    a.dinv = c.dinv;
+    a.ps = c.shared ? c.psplit : nullptr;
+    a.st = c.st;
+    a.count = c.gbar + kTailBar * kBarWords;
+    a.part = c.res_part + 8;
+    a.kerr = c.kerr;
+    const size_t smem = (size_t)a.per_nodes * 3 * sizeof(double);
+    void *args[] = {&a};
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_pcg_tail<UT, CHECON, FEW>, dim3(c.nsm),
+                                                      dim3(kTailThreads), args, smem, c.stream);
+    c.launches++;
+    if (e != cudaSuccess) {
+        set_error("k_pcg_tail: cooperative launch of %d blocks failed: %s", c.nsm, cudaGetErrorString(e));
+        return 1;
+    }
+    return 0;
+}
+
+template <typename UT, bool CHECON>
+static int launch_tail_n(Ctx &c, double *xsol)
+{
+    return 3 * tail_nodes(c) <= 2 * kTailThreads ? launch_tail_t<UT, CHECON, true>(c, xsol)
+                                                 : launch_tail_t<UT, CHECON, false>(c, xsol);
+}
+
+int launch_iteration_tail(Ctx &c, int prec, double *xsol)
+{
+    const bool ck = c.stop_mode == STOP_CHECON;
+    if (prec == PREC_FP64) return ck ? launch_tail_n<double, true>(c, xsol) : launch_tail_n<double, false>(c, xsol);
+    return ck ? launch_tail_n<float, true>(c, xsol) : launch_tail_n<float, false>(c, xsol);
 }
 
 }  // namespace pf

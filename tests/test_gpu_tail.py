@@ -1,0 +1,82 @@
+"""The iteration tail (node sums, updates and finish in one launch) of meshes
+that the resident kernel does not take: against the C restatement of p121's
+PCG, at the sizes where its slots per thread and its range end."""
+import numpy as np
+import pytest
+
+import parafem_gb300 as P
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def solver(prob, shared=False):
+    s = P.Solver()
+    s.setup(prob["g_num"], prob["g_g"], prob["g_coord"], prob["nn"], prob["neq"])
+    s.set_material(100.0, 0.3)
+    if shared:
+        s.set_shared_km(s.form_km(1, 27))
+    else:
+        s.form_storkm(27)
+    return s
+
+
+@pytest.mark.parametrize("shape", [(30, 28, 29), (31, 30, 37)])
+@pytest.mark.parametrize("limit", [1, 3, 12])
+def test_early_iterates_match_the_oracle(shape, limit):
+    """The same operations in another summation order: a few hundred ulp after 12 iterations."""
+    prob = P.cube_problem(*shape)
+    km = O.form_storkm(prob["g_coord"], 27, 100.0, 0.3)
+    dg = O.diag(prob["g_g"], km, prob["neq"])
+    with solver(prob) as s:
+        for mode, test in ((P.MODE_P121, 0), (P.MODE_FP64_RES, 1)):
+            _, ref, _ = O.pcg(prob["g_g"], km, dg, prob["r"], 0.0, limit, test)
+            x, it, _ = s.solve(prob["r"], 0.0, limit, mode)
+            assert it == limit
+            assert np.abs(x - ref).max() <= 1e-12 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("shape", [(30, 28, 29), (33, 36, 31)])
+def test_modes_agree(shape):
+    prob = P.cube_problem(*shape)
+    with solver(prob) as s:
+        ref, it, rel = s.solve(prob["r"], 1e-12, 20000, P.MODE_FP64_RES)
+        assert rel <= 1e-11
+        assert np.linalg.norm(prob["r"] - s.ebe_matvec(ref, 64)) <= 2e-11 * np.linalg.norm(prob["r"])
+        y, jt, _ = s.solve(prob["r"], 1e-12, 20000, P.MODE_FP64_RES)
+        assert it == jt and np.array_equal(ref, y)          # bitwise reproducible
+        for mode in (P.MODE_MIXED, P.MODE_MIXED16, P.MODE_MIXED_RESTART):
+            x, _, rel = s.solve(prob["r"], 1e-9, 20000, mode)
+            assert rel <= 1e-9
+            assert np.linalg.norm(x - ref) <= 1e-7 * np.linalg.norm(ref)
+        x, _, _ = s.solve(prob["r"], 1e-11, 20000, P.MODE_P121)
+        assert np.linalg.norm(x - ref) <= 1e-7 * np.linalg.norm(ref)
+
+
+# 152 SMs: up to 311,296 freedoms are two per thread, 4,046,848 the most that the tail takes
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 3, 2), (12, 11, 10), (29, 29, 28), (30, 28, 29), (68, 68, 70), (70, 69, 70)])
+def test_one_element_matrix_for_all(shape):
+    prob = P.cube_problem(*shape)
+    with solver(prob, shared=True) as s:
+        x, it, rel = s.solve(prob["r"], 1e-9, 20000, P.MODE_MIXED)
+        assert rel <= 1e-9
+        assert np.linalg.norm(prob["r"] - s.ebe_matvec(x, 64)) <= 2e-9 * np.linalg.norm(prob["r"])
+        if shape[0] > 60:
+            ref, _, _ = s.solve(prob["r"], 1e-9, 20000, P.MODE_FP64_RES)
+            assert np.linalg.norm(prob["r"] - s.ebe_matvec(ref, 64)) <= 2e-9 * np.linalg.norm(prob["r"])
+
+
+@pytest.mark.parametrize("graphs", [True, False])
+def test_graphs_and_switches_make_no_difference(graphs):
+    prob = P.cube_problem(30, 29, 29)
+    out = []
+    for persistent in (True, False):
+        with solver(prob) as s:
+            s.set_graphs(graphs)
+            s.set_persistent(persistent)
+            out.append(s.solve(prob["r"], 0.0, 45, P.MODE_P121)[0])
+            out.append(s.solve(prob["r"], 0.0, 45, P.MODE_FP64_RES)[0])
+            assert s.solve(prob["r"], 1e-6, 20000, P.MODE_MIXED)[2] <= 1e-6
+    assert np.array_equal(out[0], out[2]) and np.array_equal(out[1], out[3])
+    # the two modes differ in their stopping test only
+    assert np.abs(out[0] - out[1]).max() <= 1e-12 * np.abs(out[0]).max()
