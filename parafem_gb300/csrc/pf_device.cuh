@@ -55,6 +55,27 @@ static __device__ __forceinline__ double warp_max(double v)
     return v;
 }
 
+// A CTA's share of a sum of one value per thread: each warp leaves its
+// values in its own `stride` bytes of shared memory (it is done with them),
+// the first adds the rows in order.  By all threads of W warps.
+template <int W>
+static __device__ __forceinline__ void cta_share(unsigned char *rows, int stride, double v, double *out)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __syncwarp();
+    reinterpret_cast<double *>(rows + (size_t)w * stride)[lane] = v;
+    __syncthreads();
+    if (w > 0) return;
+    double s0 = 0.0, s1 = 0.0;   // two chains
+#pragma unroll
+    for (int j = 0; j < W; j += 2) {
+        s0 += reinterpret_cast<const double *>(rows + (size_t)j * stride)[lane];
+        s1 += reinterpret_cast<const double *>(rows + (size_t)(j + 1) * stride)[lane];
+    }
+    s0 = warp_sum(s0 + s1);
+    if (lane == 0) *out = s0;
+}
+
 // The reductions of the PCG vector kernels (256 threads).  GB300 issues one
 // FP64 warp instruction per SM in 16 clocks, so a tree in every warp (eight
 // warps x five levels per value) costs more than the sums over a block's

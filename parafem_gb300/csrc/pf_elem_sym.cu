@@ -68,11 +68,11 @@ __global__ void k_pack_sym32(int nels, const double *__restrict__ km, float *__r
 // run time among the instantiations below).  kMapped kernels (serving
 // batches) read element numbers through emap; the solver's carry no
 // remapping.
-template <int kWarps, int kStages, bool kMapped>
+template <int kWarps, int kStages, bool kMapped, bool kShare>
 __global__ void __launch_bounds__(kWarps * 32, 1)
 k_elem_sym32(int nels, const float *__restrict__ kp, const int *__restrict__ conn,
              const double *__restrict__ p, float *__restrict__ ut, const PcgState *__restrict__ st,
-             int *__restrict__ err, const int *__restrict__ emap)
+             int *__restrict__ err, const int *__restrict__ emap, double *__restrict__ share)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     const int lane = threadIdx.x & 31;
@@ -96,8 +96,8 @@ k_elem_sym32(int nels, const float *__restrict__ kp, const int *__restrict__ con
     const int e0 = blockIdx.x * per_cta;
     const int e1 = min(nels, e0 + per_cta);
     const int first = e0 + w;
-    if (first >= e1) return;
-    const int nmine = (e1 - first + kWarps - 1) / kWarps;   // elements of this warp
+    if (!kShare && first >= e1) return;
+    const int nmine = first < e1 ? (e1 - first + kWarps - 1) / kWarps : 0;   // elements of this warp
     // the k-th element of this warp; emap (serving batches) maps the
     // position among the active elements to the arena element
     auto elem = [&](int k) {
@@ -134,12 +134,13 @@ k_elem_sym32(int nels, const float *__restrict__ kp, const int *__restrict__ con
     int conn_next = 0;
     double pa = 0.0, pb = 0.0;
     {
-        const int nd0 = lane < 20 ? conn[(size_t)elem(0) * 20 + lane] : 0;
+        const int nd0 = lane < 20 && (!kShare || nmine > 0) ? conn[(size_t)elem(0) * 20 + lane] : 0;
         gather(nd0, pa, pb);
         if (nmine > 1 && lane < 20) conn_next = conn[(size_t)elem(1) * 20 + lane];
     }
 
     bool failed = false;
+    double pu = 0.0;
     int k = 0;
     for (; k < nmine; ++k) {
         const int s = k % kStages;
@@ -169,6 +170,10 @@ k_elem_sym32(int nels, const float *__restrict__ kp, const int *__restrict__ con
             // read from DRAM once the results outgrow it)
             if (lane < 20) st_global_hint(o + lane * 4 + 3, 0.0f, pol);
         }
+        if constexpr (kShare) {
+            pu = fma(pa, (double)acc_a, pu);   // lanes 30 and 31: zeros
+            pu = fma(pb, (double)acc_b, pu);
+        }
         __syncwarp();   // every lane is done with stage s and the p slot
         if (lane == 0 && k + kStages < nmine) {
             fence_proxy_async();
@@ -186,6 +191,8 @@ k_elem_sym32(int nels, const float *__restrict__ kp, const int *__restrict__ con
         for (int kk = k; kk < nmine && kk < k + kStages; ++kk)
             mbar_wait(&bar[kk % kStages], (uint32_t)((kk / kStages) & 1));
     }
+    if constexpr (kShare)
+        cta_share<kWarps>(smem + (size_t)kWarps * kStages * kPackedBytes, kPSlot * 4, pu, share + blockIdx.x);
 }
 
 template <int W, int S>
@@ -194,17 +201,17 @@ constexpr size_t sym_smem_bytes()
     return (size_t)W * S * kPackedBytes + W * kPSlot * 4 + W * S * 8;
 }
 
-template <int W, int S>
-static int launch_sym_cfg(Ctx &c, const double *p, const PcgState *st)
+template <int W, int S, bool SHARE>
+static int launch_sym_cfg(Ctx &c, const double *p, const PcgState *st, double *share)
 {
     constexpr size_t smem = sym_smem_bytes<W, S>();
     static_assert(smem <= 227 * 1024, "shared memory per CTA");
     cudaError_t e;
     // the attribute is set once per context and configuration, before any
     // stream capture (the autotuner launches every configuration first)
-    const unsigned long long bit = 1ull << (W * 4 + S);   // W <= 15, S <= 3
+    const unsigned long long bit = 1ull << (W * 4 + S - (SHARE ? 1 : 0));   // W <= 15, S = 2 or 3
     if (!(c.sym_attr & bit)) {
-        e = cudaFuncSetAttribute(k_elem_sym32<W, S, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        e = cudaFuncSetAttribute(k_elem_sym32<W, S, false, SHARE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem);
         if (e != cudaSuccess) {
             set_error("k_elem_sym32: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
@@ -212,9 +219,8 @@ static int launch_sym_cfg(Ctx &c, const double *p, const PcgState *st)
         }
         c.sym_attr |= bit;
     }
-    const int grid = c.nels < c.nsm ? c.nels : c.nsm;   // a small mesh spreads its warps over the SMs
-    launch_dependent(c.dependent && st, c.stream, grid, W * 32, smem, k_elem_sym32<W, S, false>, c.nels, c.km32p, c.conn, p,
-                     (float *)c.utemp, st, c.kerr, nullptr);
+    launch_dependent(c.dependent && st, c.stream, element_ctas(c), W * 32, smem, k_elem_sym32<W, S, false, SHARE>, c.nels, c.km32p,
+                     c.conn, p, (float *)c.utemp, st, c.kerr, nullptr, share);
     c.launches++;
     e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -231,9 +237,9 @@ constexpr int kNumSymCfg = 3;
 static int launch_sym_index(Ctx &c, int idx, const double *p, const PcgState *st)
 {
     switch (idx) {
-    case 1: return launch_sym_cfg<12, 2>(c, p, st);
-    case 2: return launch_sym_cfg<8, 3>(c, p, st);
-    default: return launch_sym_cfg<14, 2>(c, p, st);
+    case 1: return launch_sym_cfg<12, 2, false>(c, p, st, nullptr);
+    case 2: return launch_sym_cfg<8, 3, false>(c, p, st, nullptr);
+    default: return launch_sym_cfg<14, 2, false>(c, p, st, nullptr);
     }
 }
 
@@ -243,7 +249,7 @@ static int launch_sym_index(Ctx &c, int idx, const double *p, const PcgState *st
 int sym32_prepare()
 {
     constexpr size_t smem = sym_smem_bytes<14, 2>();
-    const cudaError_t e = cudaFuncSetAttribute(k_elem_sym32<14, 2, true>,
+    const cudaError_t e = cudaFuncSetAttribute(k_elem_sym32<14, 2, true, false>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) {
         set_error("k_elem_sym32: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
@@ -258,8 +264,8 @@ int launch_elem_sym32_mapped(cudaStream_t stream, int nsm, int n, const float *k
     if (n <= 0) return 0;
     constexpr int W = 14;
     const int grid = n < nsm ? n : nsm;
-    launch_dependent(true, stream, grid, W * 32, sym_smem_bytes<W, 2>(), k_elem_sym32<W, 2, true>, n, kp, conn, p, ut,
-                     (const PcgState *)nullptr, err, emap);
+    launch_dependent(true, stream, grid, W * 32, sym_smem_bytes<W, 2>(), k_elem_sym32<W, 2, true, false>, n, kp, conn, p, ut,
+                     (const PcgState *)nullptr, err, emap, (double *)nullptr);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_error("k_elem_sym32: launch failed: %s", cudaGetErrorString(e));
@@ -279,9 +285,12 @@ int launch_pack_sym32_raw(cudaStream_t stream, int nsm, int nels, const double *
     return 0;
 }
 
-int launch_elem_sym32(Ctx &c, const double *p, const PcgState *st)
+// With shares of p.u: always 14 warps, so that their order -- and with it
+// the iterates -- does not hang on the autotuner's timing (14 warps are
+// within 1 % of its choice on every mesh measured, 10^3 to 80^3).
+int launch_elem_sym32(Ctx &c, const double *p, const PcgState *st, double *share)
 {
-    return launch_sym_index(c, c.sym_cfg, p, st);
+    return share ? launch_sym_cfg<14, 2, true>(c, p, st, share) : launch_sym_index(c, c.sym_cfg, p, st);
 }
 
 // Autotuner: times every configuration on this mesh (one warm-up and three
@@ -314,6 +323,7 @@ int autotune_sym32(Ctx &c, const double *p)
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     set_sym_config(c, best_i);
+    c.sym_forced = false;
     return 0;
 }
 

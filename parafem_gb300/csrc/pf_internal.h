@@ -141,6 +141,7 @@ struct Ctx {
     MultiBufs *multi = nullptr; // block-solve vectors, allocated on the first block solve or product
     bool mr_ok = false;         // multi->rec holds the tensor-core element records of the current storkm
     int sym_cfg = 0;            // autotuned configuration of the packed-symmetric kernel
+    bool sym_forced = false;    // chosen by pf_set_tuning
     int sym_warps = 14, sym_stages = 2;
     unsigned long long sym_attr = 0;   // configurations whose shared-memory attribute is set
     float tune_ms[4] = {0, 0, 0, 0};
@@ -166,6 +167,9 @@ struct Ctx {
     // last solve statistics
     double stats[8] = {0};
 };
+
+// CTAs of the bulk-copy element kernels: one per SM; a small mesh spreads its warps over the SMs
+inline int element_ctas(const Ctx &c) { return c.nels < c.nsm ? c.nels : c.nsm; }
 
 // Kernel launchers (pf_kernels.cu).  All run on ctx.stream and count launches.
 int launch_form_storkm(Ctx &c, int nip, bool exact_weights);
@@ -211,7 +215,9 @@ bool resident_ok(const Ctx &c, int prec);
 int launch_pcg_resident(Ctx &c, int prec, double *xsol, int niters);
 int prepare_tail(Ctx &c);
 bool tail_ok(const Ctx &c);
-int launch_iteration_tail(Ctx &c, int prec, double *xsol);   // scatter, updates and finish of a PCG iteration
+// the rest of an iteration, scatter to finish; npu shares of p.u lie in product_shares(c), or 0
+int launch_iteration_tail(Ctx &c, int prec, double *xsol, int npu);
+double *product_shares(Ctx &c);
 bool persist_fused64(const Ctx &c, int prec);
 // One bounded mbarrier wait that nothing completes (the error path of the
 // bulk-copy kernels, without a fault): records code 2 in c.kerr.
@@ -231,7 +237,7 @@ int launch_elem_sym16_mapped(cudaStream_t stream, int nsm, int n, const uint32_t
                              const double *p, float *ut, int *err, const int *emap);
 int launch_pack_sym16_raw(cudaStream_t stream, int nsm, int nels, const double *km, uint32_t *kh);
 void multi_release(Ctx &c);   // frees the context's block-solve buffers (pf_multi.cu)
-int launch_elem_sym32(Ctx &c, const double *p, const PcgState *st);
+int launch_elem_sym32(Ctx &c, const double *p, const PcgState *st, double *share = nullptr);
 int sym32_prepare();   // shared-memory attribute of the mapped launch (once per device, outside capture)
 int launch_elem_sym32_mapped(cudaStream_t stream, int nsm, int n, const float *kp, const int *conn, const double *p,
                              float *ut, int *err, const int *emap);

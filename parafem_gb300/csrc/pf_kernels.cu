@@ -935,12 +935,12 @@ int launch_slot_to_eq(Ctx &c, const double *slot, double *eq)
 // 20-node elements are formed in fixed point where the mesh has records
 // (c.kmfix), and by FP64 FMA where storkm is not symmetric or the records
 // found no memory.
-static int launch_products(Ctx &c, int prec, const double *p, const PcgState *st)
+static int launch_products(Ctx &c, int prec, const double *p, const PcgState *st, double *share = nullptr)
 {
     if (c.kind == KIND_SCALAR8) return launch_elem8(c, p, st);
     if (c.kind == KIND_SOLID8) return launch_elem24(c, p, st);
     if (c.shared) return launch_elem_shared(c, prec, p, st);
-    if (prec == PREC_FP32_SYM) return launch_elem_sym32(c, p, st);
+    if (prec == PREC_FP32_SYM) return launch_elem_sym32(c, p, st, share);
     if (prec == PREC_FP16_SYM) return launch_elem_sym16(c, p, st);
     if (prec == PREC_FP64 && c.kmfix) return launch_elem_fix(c, p, st);
     const int grid = grid_for(c, c.nels, 8, 8);
@@ -951,6 +951,16 @@ static int launch_products(Ctx &c, int prec, const double *p, const PcgState *st
         launch_dependent(c.dependent && st, c.stream, grid, 256, 0, k_elem<double, true>, c.nels, c.km64, c.conn, p,
                          (double *)c.utemp, st);
     return check_launch(c, "k_elem");
+}
+
+// Rule for shares of p.u from the products: the packed FP32 kernel, with the
+// warps that fix the shares' order.  us per iteration with them / without:
+// 33^3 65.0/68.4, 45^3 145/148, 64^3 392/401.  FP64 (121.7/121.6, 278/278,
+// 773/771) and FP16 (50.5/51.8, 103/104, 269/270; 55^3 175/172) gain nothing
+// that lasts: the products' FP64 operations cost what the exchange does.
+static bool leaves_shares(const Ctx &c, int prec)
+{
+    return c.kind == KIND_SOLID20 && !c.shared && prec == PREC_FP32_SYM && (!c.sym_forced || c.sym_cfg == 0);
 }
 
 int launch_elem(Ctx &c, int prec, const double *p) { return launch_products(c, prec, p, c.st); }
@@ -1109,8 +1119,9 @@ int launch_pcg_fused64(Ctx &c, double *xsol, int niters)
 int launch_pcg_iteration(Ctx &c, int prec, double *xsol)
 {
     if (tail_ok(c)) {
-        if (launch_elem(c, prec, c.p)) return 1;
-        return launch_iteration_tail(c, prec, xsol);
+        const int npu = leaves_shares(c, prec) ? element_ctas(c) : 0;
+        if (launch_products(c, prec, c.p, c.st, npu ? product_shares(c) : nullptr)) return 1;
+        return launch_iteration_tail(c, prec, xsol, npu);
     }
     if (c.persistent && c.kind == KIND_SOLID20) {
         if (persist_fused64(c, prec)) return launch_pcg_fused64(c, xsol, 1);

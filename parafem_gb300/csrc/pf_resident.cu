@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(ResArgs a)
 static int ensure_shares(Ctx &c)
 {
     if (c.res_part) return 0;
-    const size_t bytes = 64 + 4 * kMaxBlocks * sizeof(double);
+    const size_t bytes = 64 + 5 * kMaxBlocks * sizeof(double);
     if (ctx_malloc(c, (void **)&c.res_part, bytes)) {
         set_error("PCG: cannot allocate %zu bytes of shares", bytes);
         return 1;
@@ -537,9 +537,11 @@ int launch_pcg_resident(Ctx &c, int prec, double *xsol, int niters)
 // where they have launches.  Node sums go a thread per node (one 16-byte load
 // per FP32 contribution), everything else a thread per slot: sums per slot
 // took 162 instead of 152 us of a 64^3 iteration with one element matrix.
-// Bound by the chain of sums, exchange and division at 33^3 (8.8 of 19 us)
-// and by the FP64 pipe at 64^3 (eight operations per slot, two per SM and
-// clock: 45 us of 96).
+// Bound by the chain of sums, exchange and division at 33^3 (a third of it)
+// and by the FP64 pipe (eight operations per slot, two per SM and clock: 45
+// us at 64^3) and memory (270 MB, 40 us) together at 64^3, 80 us in all.
+// More loads in flight do not help: L2 prefetches of the next 32 nodes'
+// vectors and results took 394 and 405 instead of 392 us per iteration.
 constexpr int kTailThreads = 1024;
 
 struct TailArgs {
@@ -553,6 +555,8 @@ struct TailArgs {
     PcgState *st;
     unsigned long long *count;   // arrivals, zeroed by launch_pcg_init
     double *part;
+    const double *pu;            // [npu] the products' shares of p.u (DOT)
+    int npu;
     int *kerr;
 };
 
@@ -569,7 +573,12 @@ __device__ __forceinline__ double tail_total(const double *sh, int lane)
     return warp_sum((v[0] + v[1]) + (v[2] + v[3]));
 }
 
-template <typename UT, bool CHECON, bool FEW>
+// A warp goes through its nodes 32 at a time, sums by node and the rest by
+// slot: 96 slots, which change lanes through su.  DOT: the products' CTAs
+// have left their shares of p.u, so that alpha is known at once and the node
+// sums (latency) run together with x, r and d (the FP64 pipe).  Otherwise
+// p.u is formed here, behind an exchange.
+template <typename UT, bool CHECON, bool DOT>
 __global__ void __launch_bounds__(kTailThreads, 1) k_pcg_tail(TailArgs a)
 {
     extern __shared__ double su[];   // u, then d, of the block's slots
@@ -585,7 +594,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_pcg_tail(TailArgs a)
     if (s_stop) return;   // read once per block, before any block writes it
     const double up = a.st->up, tol = a.st->tol;
     const int iters = a.st->iters;
-    unsigned long long target = (2ULL * iters + 1) * nblk;   // arrivals that complete the next exchange
+    unsigned long long target = ((DOT ? 1ULL : 2ULL) * iters + 1) * nblk;   // arrivals that complete the next exchange
     double *p_pu = a.part, *p_rd = p_pu + kMaxBlocks, *p_2 = p_rd + kMaxBlocks, *p_3 = p_2 + kMaxBlocks;
     auto meet = [&]() {
         if (exchange(a.count, target)) return;
@@ -593,24 +602,13 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_pcg_tail(TailArgs a)
         atomicExch(a.kerr, 3);
         atomicExch(&a.st->stop, 1);
     };
-    // ---- node sums (ascending element order) and p.u
-    const int n0 = blk * a.per_nodes, n1 = min(a.nn, n0 + a.per_nodes), s0 = 3 * n0, s1 = 3 * n1;
-    double pu = 0.0;
-    int kn = 0, kn1 = 0;   // the next node's part of the list
-    if (n0 + t < n1) {
-        kn = __ldg(a.ptr + n0 + t);
-        kn1 = __ldg(a.ptr + n0 + t + 1);
-    }
-    for (int n = n0 + t; n < n1; n += kTailThreads) {
-        const int k0 = kn, k1 = kn1, m = __ldg(a.fm + n);
-        if (n + kTailThreads < n1) {
-            kn = __ldg(a.ptr + n + kTailThreads);
-            kn1 = __ldg(a.ptr + n + kTailThreads + 1);
-        }
-        const double *pn = a.p + (size_t)3 * n;
-        const double p0 = pn[0], p1 = pn[1], p2 = pn[2];
+    // this warp's nodes: 32 from node c on, then from c + kTailThreads on, ...
+    const int n0 = blk * a.per_nodes, n1 = min(a.nn, n0 + a.per_nodes), s0 = 3 * n0, s1 = 3 * n1, c0 = n0 + 32 * w;
+    // ---- sums over a node's elements (ascending) into su
+    auto node_sums = [&](int n) {
+        const int k1 = __ldg(a.ptr + n + 1), m = __ldg(a.fm + n);
         UT u0 = 0, u1 = 0, u2 = 0;
-        for (int k = k0; k < k1; k += 4) {   // four contributions in flight
+        for (int k = __ldg(a.ptr + n); k < k1; k += 4) {   // four contributions in flight
             int ci[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) ci[q] = __ldg(a.list + min(k + q, k1 - 1));
@@ -635,84 +633,113 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_pcg_tail(TailArgs a)
                     u2 += v[q][2];
                 }
         }
-        const double e0 = m & 1 ? (double)u0 : 0.0, e1 = m & 2 ? (double)u1 : 0.0, e2 = m & 4 ? (double)u2 : 0.0;
         double *o = su + 3 * (n - n0);
-        o[0] = e0;
-        o[1] = e1;
-        o[2] = e2;
-        pu = fma(p0, e0, pu);
-        pu = fma(p1, e1, pu);
-        pu = fma(p2, e2, pu);
-    }
-    sh[0][t] = pu;
-    // a block of at most two slots per thread has them in flight behind the sum
-    double xo[2], ro[2], dv[2], po[2];
-    if (FEW) {
+        o[0] = m & 1 ? (double)u0 : 0.0;   // restrained: u = 0
+        o[1] = m & 2 ? (double)u1 : 0.0;
+        o[2] = m & 4 ? (double)u2 : 0.0;
+    };
+    // ---- x, r, d of the 96 slots of 32 nodes
+    double alpha = 0.0, rd = 0.0, rr = 0.0;
+    long long mx = 0, md = 0;
+    double xo[3], ro[3], dv[3], po[3];
+    auto fetch = [&](int c) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int s = s0 + t + i * kTailThreads;
+        for (int j = 0; j < 3; ++j) {
+            const int s = 3 * c + lane + 32 * j;
             if (s < s1) {
-                xo[i] = a.x[s];
-                ro[i] = a.r[s];
-                dv[i] = __ldg(a.dinv + s);
-                po[i] = a.p[s];
+                po[j] = a.p[s];
+                xo[j] = a.x[s];
+                ro[j] = a.r[s];
+                dv[j] = __ldg(a.dinv + s);
             }
         }
-    }
-    __syncthreads();
-    if (w == 0) {
-        const double mine = tail_total(sh[0], lane);
-        if (lane == 0) {
-            p_pu[blk] = mine;
-            meet();
-        }
-        __syncwarp();
-        const double sum = add_shares(p_pu, nblk, lane);
-        if (lane == 0) s_val[0] = up / sum;
-    } else if (w == 1 && !CHECON && lane == 0) {
-        s_bound = tol * sqrt(a.st->ff);
-    }
-    target += nblk;
-    __syncthreads();
-    if (!s_ok) return;
-    // ---- x, r, d
-    const double alpha = s_val[0];
-    double rd = 0.0, rr = 0.0;
-    long long mx = 0, md = 0;
-    auto move = [&](int s, double p, double x0) {
-        const double xn = fma(p, alpha, x0);
-        a.x[s] = xn;
-        if (CHECON) {
-            mx = max(mx, abs_bits(xn));
-            md = max(md, abs_bits(xn - x0));
-        }
     };
-    auto residual = [&](int s, double r0, double di) {
-        const double rn = fma(-su[s - s0], alpha, r0), dn = di * rn;
-        a.r[s] = rn;
-        su[s - s0] = dn;
-        rd = fma(rn, dn, rd);
-        if (!CHECON) rr = fma(rn, rn, rr);
-    };
-    if (FEW) {
+    auto step = [&](int c) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int s = s0 + t + i * kTailThreads;
+        for (int j = 0; j < 3; ++j) {
+            const int s = 3 * c + lane + 32 * j;
             if (s < s1) {
-                move(s, po[i], xo[i]);
-                residual(s, ro[i], dv[i]);
+                const double xn = fma(po[j], alpha, xo[j]);
+                a.x[s] = xn;
+                if (CHECON) {
+                    mx = max(mx, abs_bits(xn));
+                    md = max(md, abs_bits(xn - xo[j]));
+                }
+                const double rn = fma(-su[s - s0], alpha, ro[j]), dn = dv[j] * rn;
+                a.r[s] = rn;
+                su[s - s0] = dn;
+                rd = fma(rn, dn, rd);
+                if (!CHECON) rr = fma(rn, rn, rr);
+            }
+        }
+    };
+    if (w == 1 && !CHECON && lane == 0) s_bound = tol * sqrt(a.st->ff);
+    if (DOT) {
+        if (c0 < n1) fetch(c0);
+        if (w == kTailThreads / 32 - 1) {   // it has its sums when the others have theirs
+            const double sum = add_shares(a.pu, a.npu, lane);
+            if (lane == 0) s_val[0] = up / sum;
+        }
+        if (c0 + lane < n1) node_sums(c0 + lane);
+        __syncthreads();
+        alpha = s_val[0];
+        for (int c = c0; c < n1;) {
+            step(c);
+            c += kTailThreads;
+            if (c < n1) {
+                fetch(c);
+                if (c + lane < n1) node_sums(c + lane);
+                __syncwarp();
             }
         }
     } else {
-#pragma unroll 2
-        for (int s = s0 + t; s < s1; s += kTailThreads) {
-            move(s, a.p[s], a.x[s]);
-            residual(s, a.r[s], __ldg(a.dinv + s));
+        double pu = 0.0;
+        for (int c = c0; c < n1; c += kTailThreads) {
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const int s = 3 * c + lane + 32 * j;
+                po[j] = s < s1 ? a.p[s] : 0.0;
+            }
+            if (c + lane < n1) node_sums(c + lane);
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const int s = 3 * c + lane + 32 * j;
+                if (s < s1) pu = fma(po[j], su[s - s0], pu);
+            }
+        }
+        sh[0][t] = pu;
+        if (c0 < n1) fetch(c0);
+        __syncthreads();
+        if (w == 0) {
+            const double mine = tail_total(sh[0], lane);
+            if (lane == 0) {
+                p_pu[blk] = mine;
+                meet();
+            }
+            __syncwarp();
+            const double sum = add_shares(p_pu, nblk, lane);
+            if (lane == 0) s_val[0] = up / sum;
+        }
+        target += nblk;
+        __syncthreads();
+        if (!s_ok) return;
+        alpha = s_val[0];
+        for (int c = c0; c < n1;) {
+            step(c);
+            c += kTailThreads;
+            if (c < n1) fetch(c);
         }
     }
     sh[0][t] = rd;
     if (!CHECON) sh[1][t] = rr;
     if (CHECON) block_max2(mx, md);
+    // p of the first slots, in flight beside the sums
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        const int s = 3 * c0 + lane + 32 * j;
+        po[j] = s < s1 ? a.p[s] : 0.0;
+    }
     __syncthreads();
     if (w == 0 || (w == 1 && !CHECON)) {
         const double mine = tail_total(sh[w], lane);
@@ -748,24 +775,26 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_pcg_tail(TailArgs a)
     __syncthreads();
     // ---- p
     const double beta = s_val[2];
-    auto direct = [&](int s, double p) {
-        const double pn = fma(p, beta, su[s - s0]);
-        a.p[s] = pn;
-        if (a.ps) {
-            float h, l;
-            tc::split_f64(pn, h, l);
-            a.ps[s] = make_float2(h, l);
-        }
-    };
-    if (FEW) {
+    for (int c = c0; c < n1;) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int s = s0 + t + i * kTailThreads;
-            if (s < s1) direct(s, po[i]);
+        for (int j = 0; j < 3; ++j) {
+            const int s = 3 * c + lane + 32 * j;
+            if (s < s1) {
+                const double pn = fma(po[j], beta, su[s - s0]);
+                a.p[s] = pn;
+                if (a.ps) {
+                    float h, l;
+                    tc::split_f64(pn, h, l);
+                    a.ps[s] = make_float2(h, l);
+                }
+            }
         }
-    } else {
-#pragma unroll 4
-        for (int s = s0 + t; s < s1; s += kTailThreads) direct(s, a.p[s]);
+        c += kTailThreads;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const int s = 3 * c + lane + 32 * j;
+            po[j] = s < s1 ? a.p[s] : 0.0;
+        }
     }
     if (blk == 0 && t == 0) {
         const double rdn = s_val[1], measure = s_val[3];
@@ -789,10 +818,10 @@ constexpr int kTailMax = 26;   // slots per thread that fit in shared memory
 // 152 SMs).  us per iteration with this kernel / with scatter, update1 and
 // update2 in a graph:
 //                          33^3          45^3        55^3        64^3
-//   FP64                   120/125       278/288     497/502     778/782
-//   FP32                   67/74         147/162     254/263     402/409
-//   FP16                   52/59         103/117     173/182     271/273
-//   FP32, one matrix       36/43         61/74       95/103      153/153
+//   FP64                   121/125       278/288     491/502     771/782
+//   FP32                   65/74         145/162     251/263     392/409
+//   FP16                   52/59         104/117     172/182     270/273
+//   FP32, one matrix       36/43         61/74       93/103      148/153
 static int tail_nodes(const Ctx &c) { return (c.nn + c.nsm - 1) / c.nsm; }
 
 bool tail_ok(const Ctx &c)
@@ -806,7 +835,7 @@ int prepare_tail(Ctx &c)
     if (ensure_shares(c)) return 1;
     if (c.tail_attr) return 0;
     const void *fn[] = {(const void *)k_pcg_tail<double, true, false>, (const void *)k_pcg_tail<double, false, false>,
-                        (const void *)k_pcg_tail<float, true, false>, (const void *)k_pcg_tail<float, false, false>};
+                        (const void *)k_pcg_tail<float, false, false>, (const void *)k_pcg_tail<float, false, true>};
     for (const void *f : fn) {
         const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    kTailMax * kTailThreads * (int)sizeof(double));
@@ -819,8 +848,8 @@ int prepare_tail(Ctx &c)
     return 0;
 }
 
-template <typename UT, bool CHECON, bool FEW>
-static int launch_tail_t(Ctx &c, double *xsol)
+template <typename UT, bool CHECON, bool DOT>
+static int launch_tail_t(Ctx &c, double *xsol, int npu)
 {
     TailArgs a;
     a.nn = c.nn;
@@ -837,10 +866,12 @@ static int launch_tail_t(Ctx &c, double *xsol)
     a.st = c.st;
     a.count = c.gbar + kTailBar * kBarWords;
     a.part = c.res_part + 8;
+    a.pu = c.res_part + 8 + 4 * kMaxBlocks;
+    a.npu = npu;
     a.kerr = c.kerr;
     const size_t smem = (size_t)a.per_nodes * 3 * sizeof(double);
     void *args[] = {&a};
-    const cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_pcg_tail<UT, CHECON, FEW>, dim3(c.nsm),
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_pcg_tail<UT, CHECON, DOT>, dim3(c.nsm),
                                                       dim3(kTailThreads), args, smem, c.stream);
     c.launches++;
     if (e != cudaSuccess) {
@@ -850,18 +881,14 @@ static int launch_tail_t(Ctx &c, double *xsol)
     return 0;
 }
 
-template <typename UT, bool CHECON>
-static int launch_tail_n(Ctx &c, double *xsol)
+int launch_iteration_tail(Ctx &c, int prec, double *xsol, int npu)
 {
-    return 3 * tail_nodes(c) <= 2 * kTailThreads ? launch_tail_t<UT, CHECON, true>(c, xsol)
-                                                 : launch_tail_t<UT, CHECON, false>(c, xsol);
+    const bool ck = c.stop_mode == STOP_CHECON;   // FP64 runs only
+    if (prec == PREC_FP64)
+        return ck ? launch_tail_t<double, true, false>(c, xsol, 0) : launch_tail_t<double, false, false>(c, xsol, 0);
+    return npu ? launch_tail_t<float, false, true>(c, xsol, npu) : launch_tail_t<float, false, false>(c, xsol, 0);
 }
 
-int launch_iteration_tail(Ctx &c, int prec, double *xsol)
-{
-    const bool ck = c.stop_mode == STOP_CHECON;
-    if (prec == PREC_FP64) return ck ? launch_tail_n<double, true>(c, xsol) : launch_tail_n<double, false>(c, xsol);
-    return ck ? launch_tail_n<float, true>(c, xsol) : launch_tail_n<float, false>(c, xsol);
-}
+double *product_shares(Ctx &c) { return c.res_part + 8 + 4 * kMaxBlocks; }
 
 }  // namespace pf

@@ -80,3 +80,17 @@ def test_graphs_and_switches_make_no_difference(graphs):
     assert np.array_equal(out[0], out[2]) and np.array_equal(out[1], out[3])
     # the two modes differ in their stopping test only
     assert np.abs(out[0] - out[1]).max() <= 1e-12 * np.abs(out[0]).max()
+
+
+def test_forced_products_change_the_iterates_by_rounding_only():
+    """14 warps leave shares of p.u for the tail, 12 do not; a solve in between changes nothing."""
+    prob = P.cube_problem(30, 29, 29)
+    with solver(prob) as s:
+        a = s.solve(prob["r"], 1e-9, 20000, P.MODE_MIXED)
+        s.set_tuning(1)
+        b = s.solve(prob["r"], 1e-9, 20000, P.MODE_MIXED)
+        s.set_tuning(0)
+        c = s.solve(prob["r"], 1e-9, 20000, P.MODE_MIXED)
+    assert b[2] <= 1e-9 and a[1] == c[1]
+    assert np.array_equal(a[0], c[0])
+    assert np.linalg.norm(a[0] - b[0]) <= 1e-7 * np.linalg.norm(a[0])
