@@ -1121,6 +1121,7 @@ int launch_pcg_iteration(Ctx &c, int prec, double *xsol)
     if (tail_ok(c)) {
         const int npu = leaves_shares(c, prec) ? element_ctas(c) : 0;
         if (launch_products(c, prec, c.p, c.st, npu ? product_shares(c) : nullptr)) return 1;
+        if (c.kind != KIND_SOLID20 && launch_scatter(c, prec, 0, c.p, c.u)) return 1;
         return launch_iteration_tail(c, prec, xsol, npu);
     }
     if (c.persistent && c.kind == KIND_SOLID20) {

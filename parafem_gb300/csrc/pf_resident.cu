@@ -545,12 +545,12 @@ int launch_pcg_resident(Ctx &c, int prec, double *xsol, int niters)
 constexpr int kTailThreads = 1024;
 
 struct TailArgs {
-    int nn, per_nodes;
+    int nn, per_nodes, ns;       // GIVEN: nodes of three slots each, in name only
     const void *ut;
     const int *ptr, *list;
     const uint8_t *fm;
     double *x, *r, *p;
-    const double *dinv;
+    const double *dinv, *u;
     float2 *ps;                  // the FP32 parts of p (shared km), or null
     PcgState *st;
     unsigned long long *count;   // arrivals, zeroed by launch_pcg_init
@@ -578,7 +578,9 @@ __device__ __forceinline__ double tail_total(const double *sh, int lane)
 // have left their shares of p.u, so that alpha is known at once and the node
 // sums (latency) run together with x, r and d (the FP64 pipe).  Otherwise
 // p.u is formed here, behind an exchange.
-template <typename UT, bool CHECON, bool DOT>
+// GIVEN (8-node meshes): the product kernel has left u and alpha.
+enum { TAIL_SUMS = 0, TAIL_DOT = 1, TAIL_GIVEN = 2 };
+template <typename UT, bool CHECON, int HOW>
 __global__ void __launch_bounds__(kTailThreads, 1) k_pcg_tail(TailArgs a)
 {
     extern __shared__ double su[];   // u, then d, of the block's slots
@@ -594,7 +596,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_pcg_tail(TailArgs a)
     if (s_stop) return;   // read once per block, before any block writes it
     const double up = a.st->up, tol = a.st->tol;
     const int iters = a.st->iters;
-    unsigned long long target = ((DOT ? 1ULL : 2ULL) * iters + 1) * nblk;   // arrivals that complete the next exchange
+    unsigned long long target = ((HOW == TAIL_SUMS ? 2ULL : 1ULL) * iters + 1) * nblk;   // arrivals that complete the next exchange
     double *p_pu = a.part, *p_rd = p_pu + kMaxBlocks, *p_2 = p_rd + kMaxBlocks, *p_3 = p_2 + kMaxBlocks;
     auto meet = [&]() {
         if (exchange(a.count, target)) return;
@@ -603,7 +605,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_pcg_tail(TailArgs a)
         atomicExch(&a.st->stop, 1);
     };
     // this warp's nodes: 32 from node c on, then from c + kTailThreads on, ...
-    const int n0 = blk * a.per_nodes, n1 = min(a.nn, n0 + a.per_nodes), s0 = 3 * n0, s1 = 3 * n1, c0 = n0 + 32 * w;
+    const int n0 = blk * a.per_nodes, n1 = min(a.nn, n0 + a.per_nodes), s0 = 3 * n0, s1 = min(a.ns, 3 * n1), c0 = n0 + 32 * w;
     // ---- sums over a node's elements (ascending) into su
     auto node_sums = [&](int n) {
         const int k1 = __ldg(a.ptr + n + 1), m = __ldg(a.fm + n);
@@ -651,6 +653,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_pcg_tail(TailArgs a)
                 xo[j] = a.x[s];
                 ro[j] = a.r[s];
                 dv[j] = __ldg(a.dinv + s);
+                if (HOW == TAIL_GIVEN) su[s - s0] = a.u[s];
             }
         }
     };
@@ -674,7 +677,13 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_pcg_tail(TailArgs a)
         }
     };
     if (w == 1 && !CHECON && lane == 0) s_bound = tol * sqrt(a.st->ff);
-    if (DOT) {
+    if (HOW == TAIL_GIVEN) {
+        alpha = a.st->alpha;
+        for (int c = c0; c < n1; c += kTailThreads) {
+            fetch(c);
+            step(c);
+        }
+    } else if (HOW == TAIL_DOT) {
         if (c0 < n1) fetch(c0);
         if (w == kTailThreads / 32 - 1) {   // it has its sums when the others have theirs
             const double sum = add_shares(a.pu, a.npu, lane);
@@ -814,19 +823,23 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_pcg_tail(TailArgs a)
 
 constexpr int kTailMax = 26;   // slots per thread that fit in shared memory
 
-// Rule: 20-node meshes whose slots fit the CTAs' shared memory (4,046,848 on
-// 152 SMs).  us per iteration with this kernel / with scatter, update1 and
+// Rule: meshes whose slots fit the CTAs' shared memory (4,046,848 on 152
+// SMs).  us per iteration with this kernel / with scatter, update1 and
 // update2 in a graph:
 //                          33^3          45^3        55^3        64^3
 //   FP64                   121/125       278/288     491/502     771/782
 //   FP32                   65/74         145/162     251/263     392/409
 //   FP16                   52/59         104/117     172/182     270/273
 //   FP32, one matrix       36/43         61/74       93/103      148/153
-static int tail_nodes(const Ctx &c) { return (c.nn + c.nsm - 1) / c.nsm; }
+// 8-node meshes (two updates before): p123 32^3 18.9/20.3, 50^3 26.8/30.4,
+// 100^3 92/95; below 30,000 slots (24^3: 19.4/17.4) two dependent launches
+// cost less than an exchange.
+static int tail_nodes(const Ctx &c) { return ((c.nslots + 2) / 3 + c.nsm - 1) / c.nsm; }
 
 bool tail_ok(const Ctx &c)
 {
-    return c.kind == KIND_SOLID20 && c.nsm <= kMaxBlocks && 3 * tail_nodes(c) <= kTailMax * kTailThreads;
+    if (c.kind != KIND_SOLID20 && c.nslots < 30000) return false;
+    return c.nsm <= kMaxBlocks && 3 * tail_nodes(c) <= kTailMax * kTailThreads;
 }
 
 // The shared memory of the tail's largest form (outside any stream capture)
@@ -834,8 +847,9 @@ int prepare_tail(Ctx &c)
 {
     if (ensure_shares(c)) return 1;
     if (c.tail_attr) return 0;
-    const void *fn[] = {(const void *)k_pcg_tail<double, true, false>, (const void *)k_pcg_tail<double, false, false>,
-                        (const void *)k_pcg_tail<float, false, false>, (const void *)k_pcg_tail<float, false, true>};
+    const void *fn[] = {(const void *)k_pcg_tail<double, true, TAIL_SUMS>, (const void *)k_pcg_tail<double, false, TAIL_SUMS>,
+                        (const void *)k_pcg_tail<float, false, TAIL_SUMS>, (const void *)k_pcg_tail<float, false, TAIL_DOT>,
+                        (const void *)k_pcg_tail<double, true, TAIL_GIVEN>, (const void *)k_pcg_tail<double, false, TAIL_GIVEN>};
     for (const void *f : fn) {
         const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    kTailMax * kTailThreads * (int)sizeof(double));
@@ -848,12 +862,14 @@ int prepare_tail(Ctx &c)
     return 0;
 }
 
-template <typename UT, bool CHECON, bool DOT>
+template <typename UT, bool CHECON, int HOW>
 static int launch_tail_t(Ctx &c, double *xsol, int npu)
 {
     TailArgs a;
-    a.nn = c.nn;
+    a.nn = (c.nslots + 2) / 3;
     a.per_nodes = tail_nodes(c);
+    a.ns = c.nslots;
+    a.u = c.u;
     a.ut = c.utemp;
     a.ptr = c.node_ptr;
     a.list = c.node_list;
@@ -871,7 +887,7 @@ static int launch_tail_t(Ctx &c, double *xsol, int npu)
     a.kerr = c.kerr;
     const size_t smem = (size_t)a.per_nodes * 3 * sizeof(double);
     void *args[] = {&a};
-    const cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_pcg_tail<UT, CHECON, DOT>, dim3(c.nsm),
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_pcg_tail<UT, CHECON, HOW>, dim3(c.nsm),
                                                       dim3(kTailThreads), args, smem, c.stream);
     c.launches++;
     if (e != cudaSuccess) {
@@ -884,9 +900,11 @@ static int launch_tail_t(Ctx &c, double *xsol, int npu)
 int launch_iteration_tail(Ctx &c, int prec, double *xsol, int npu)
 {
     const bool ck = c.stop_mode == STOP_CHECON;   // FP64 runs only
+    if (c.kind != KIND_SOLID20)
+        return ck ? launch_tail_t<double, true, TAIL_GIVEN>(c, xsol, 0) : launch_tail_t<double, false, TAIL_GIVEN>(c, xsol, 0);
     if (prec == PREC_FP64)
-        return ck ? launch_tail_t<double, true, false>(c, xsol, 0) : launch_tail_t<double, false, false>(c, xsol, 0);
-    return npu ? launch_tail_t<float, false, true>(c, xsol, npu) : launch_tail_t<float, false, false>(c, xsol, 0);
+        return ck ? launch_tail_t<double, true, TAIL_SUMS>(c, xsol, 0) : launch_tail_t<double, false, TAIL_SUMS>(c, xsol, 0);
+    return npu ? launch_tail_t<float, false, TAIL_DOT>(c, xsol, npu) : launch_tail_t<float, false, TAIL_SUMS>(c, xsol, 0);
 }
 
 double *product_shares(Ctx &c) { return c.res_part + 8 + 4 * kMaxBlocks; }

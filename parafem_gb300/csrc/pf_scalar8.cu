@@ -17,15 +17,17 @@
 //   k_rows*           the same sums with the element matrices added up by
 //                     node once, when storkc is formed: one row of the
 //                     assembled matrix per node, and
-//   k_row_product     the product, dot and fixed freedoms in one pass over
-//                     the rows.  A node of a brick mesh has 27 neighbours:
+//   k_row_ring, k_row_product   the product, dot and fixed freedoms in one
+//                     pass over the rows.  A node of a brick mesh has 27 neighbours:
 //                     270 bytes and 27 FMA per node and product, where the
 //                     element products and the scatter move 710 bytes and
 //                     take 64 FMA and 8 additions per element.  The element
 //                     kernels serve meshes with a node of more than kRowMax
 //                     neighbours and contexts without memory for the rows.
 #include "pf_device.cuh"
+#include "pf_tc.cuh"
 
+#include <algorithm>
 #include <vector>
 
 namespace pf {
@@ -211,12 +213,12 @@ k_rows_fill(int nn, const int *__restrict__ ptr, const int *__restrict__ list, c
 
 // u = K x over the assembled rows, as k_elem8 and k_scatter1 form it:
 //   MODE 0: out = u, partial pf.u and alpha in a PCG run;  MODE 1: out = f - u, partial out.out
-// Bound by the FP64 pipe (30 operations per node, two per SM and clock: 56 us
-// at 100^3) and by HBM (294 B per node, 44 us): 90 us at 100^3, where k_elem8
-// and k_scatter1 take 180; 26 against 37 us at 50^3, 18 when the rows stay in
-// L2.  KEEP: the rows are read the ordinary way, so that those of a mesh that
-// fits stay in L2 from one product to the next; else they leave L2 first
-// (100^3: 98 us kept, 90 us not).
+// For MODE 0 where k_row_ring does not take the rows.  Bound by the FP64 pipe
+// (30 operations per node, two per SM and clock: 56 us at 100^3) and by HBM
+// (294 B per node, 44 us), one after the other: 92 us at 100^3, where k_elem8
+// and k_scatter1 take 180.  KEEP: the rows are read the ordinary way, so that
+// those of a mesh that fits stay in L2 from one product to the next; else they
+// leave L2 first (100^3: 98 us kept, 90 us not).
 constexpr size_t kRowKeepBytes = 64u << 20;
 template <int MODE, typename IT, bool KEEP>
 __global__ void __launch_bounds__(256)
@@ -257,6 +259,113 @@ k_row_product(int nn, const long long *__restrict__ off, const double *__restric
     }
     pdl_exit();
     scatter_tail(loc, part, MODE == 0 ? st : nullptr, count);
+}
+
+// k_row_product<0> with the rows streamed through shared memory: one
+// persistent CTA of 20 warps per SM, one warp per slice of 32 rows; each warp
+// has the next slice's values and columns copied (cp.async.bulk) while the
+// other warps multiply, so that the memory and the FP64 pipe are busy
+// together.  The sums are k_row_product's, in its order.  Every wait on an
+// mbarrier is bounded, as in k_elem_sym32.  Bound by the FP64 pipe (50 us at
+// 100^3): 70 us, where k_row_product takes 92; 150^3 198 against 259, 32^3
+// 12.2 against 16.4 (fewer blocks to sum over), 50^3 to 64^3 alike.  8, 12, 16
+// and 24 warps: 92, 75, 71, 71 us at 100^3.
+// Rule: slices of at most 28 columns (27 in a mesh of bricks) with 16-bit
+// column offsets.
+constexpr int kRingWarps = 20, kRingWidth = 28;                  // widest slice that a stage holds
+constexpr int kRingIdx = kRingWidth * 32 * 8, kRingStage = kRingWidth * 32 * 10;
+constexpr int kRingSmem = kRingWarps * (kRingStage + 8);
+static_assert(kRingSmem + 64 <= 227 * 1024, "shared memory per CTA");
+__global__ void __launch_bounds__(kRingWarps * 32, 1)
+k_row_ring(int nn, const long long *__restrict__ off, const double *__restrict__ val, const uint16_t *__restrict__ idx,
+           const int *__restrict__ base, const uint8_t *__restrict__ fm, const double *__restrict__ fstore,
+           const double *__restrict__ xin, double *__restrict__ out, double *__restrict__ part, PcgState *st,
+           unsigned *__restrict__ count, int keep, int *__restrict__ err)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned char *stage = smem + (size_t)w * kRingStage;
+    const double *sv = reinterpret_cast<const double *>(stage) + lane;
+    const uint16_t *si = reinterpret_cast<const uint16_t *>(stage + kRingIdx) + lane;
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + (size_t)kRingWarps * kRingStage) + w;
+    // this CTA's contiguous range of slices, warps interleaved inside it
+    const int nslice = (nn + 31) / 32, per_cta = (nslice + gridDim.x - 1) / gridDim.x;
+    const int s1 = min(nslice, (int)(blockIdx.x + 1) * per_cta);
+    int s = blockIdx.x * per_cta + w;
+    const uint64_t pol = tc::l2_evict_first_policy();
+    auto issue = [&](long long o, int n) {   // n columns from entry o on (lane 0)
+        tc::mbar_expect_tx(bar, n * 320);
+        if (keep) {
+            tc::bulk_g2s(stage, val + o, n * 256, bar);
+            tc::bulk_g2s(stage + kRingIdx, idx + o, n * 64, bar);
+        } else {
+            tc::bulk_g2s_hint(stage, val + o, n * 256, bar, pol);
+            tc::bulk_g2s_hint(stage + kRingIdx, idx + o, n * 64, bar, pol);
+        }
+    };
+    long long o = 0;
+    int n = 0;
+    if (s < s1) {   // the rows are no kernel's of this iteration: before the wait for the one before
+        o = off[s];
+        n = (int)((off[s + 1] - o) >> 5);
+        if (lane == 0) {
+            tc::mbar_init(bar, 1);
+            tc::mbar_fence_init();
+            issue(o, n);
+        }
+    }
+    __syncwarp();
+    pdl_enter();
+    const bool stopped = st && st->stop;
+    double loc = 0.0;
+    bool ok = true;
+    for (uint32_t parity = 0; s < s1; s += kRingWarps, parity ^= 1) {
+        const int b = lane < n ? __ldg(base + (o >> 5) + lane) : 0;
+        const int row = 32 * s + lane;
+        const bool in = row < nn;
+        const int m = in ? fm[row] : 0;
+        const double fs = in ? fstore[row] : 0.0, p = in ? xin[row] : 0.0;
+        ok = __all_sync(FULLMASK, tc::mbar_wait(bar, parity));
+        if (!ok || stopped) break;
+        double a = 0.0;
+#pragma unroll 9
+        for (int k = 0; k < n; ++k) a = fma(sv[32 * k], __ldg(xin + __shfl_sync(FULLMASK, b, k) + si[32 * k]), a);
+        __syncwarp();   // every lane is done with the stage
+        if (s + kRingWarps < s1) {
+            o = off[s + kRingWarps];
+            n = (int)((off[s + kRingWarps + 1] - o) >> 5);
+            if (lane == 0) {
+                tc::fence_proxy_async();
+                issue(o, n);
+            }
+        }
+        if (in) {
+            if (abs_bits(fs)) a = p * fs;   // an integer test
+            const double uv = m & 1 ? a : 0.0;
+            out[row] = uv;
+            loc = fma(p, uv, loc);
+        }
+    }
+    if (stopped) return;
+    if (!ok && lane == 0) {
+        atomicExch(err, 2);
+        tc::mbar_wait(bar, 0);   // the one copy in flight, once more (bounded)
+        tc::mbar_wait(bar, 1);
+    }
+    pdl_exit();
+    cta_share<kRingWarps>(smem, kRingStage, loc, part + blockIdx.x);
+    if (!st || w > 0) return;
+    int last = 0;
+    if (lane == 0) {
+        __threadfence();
+        last = atomicInc(count, gridDim.x - 1) == gridDim.x - 1;
+    }
+    if (!__shfl_sync(FULLMASK, last, 0)) return;
+    __threadfence();
+    double v = 0.0;
+    for (int i = lane; i < (int)gridDim.x; i += 32) v += __ldcg(part + i);
+    v = warp_sum(v);
+    if (lane == 0) st->alpha = st->up / v;
 }
 
 __global__ void k_assemble_diag1(int nn, const int *__restrict__ ptr, const int *__restrict__ list,
@@ -358,6 +467,8 @@ int rows_assemble(Ctx &c)
     }
     if (bad) return 0;
     for (int s = 0; s < nslice; ++s) off[s + 1] = off[s] + 32LL * width[s];
+    const auto w = std::minmax_element(width.begin(), width.end());
+    c.row_ring = false;
     const size_t total = (size_t)off[nslice];
     if (total == 0) return 0;
     for (int bytes = 2; bytes <= 4; bytes += 2) {   // 16-bit columns first
@@ -386,7 +497,10 @@ int rows_assemble(Ctx &c)
             set_error("k_rows_fill: %s", cudaGetErrorString(ef));
             return 1;
         }
-        if (!bad) break;
+        if (!bad) {
+            c.row_ring = bytes == 2 && *w.first > 0 && *w.second <= kRingWidth;
+            break;
+        }
         cudaFree(c.row_idx);
         c.row_idx = nullptr;
     }
@@ -395,6 +509,21 @@ int rows_assemble(Ctx &c)
 
 static int launch_row_product(Ctx &c, int mode, const double *xin, const double *pf, double *out, PcgState *st)
 {
+    if (mode == 0 && c.row_ring) {
+        if (!c.row_attr) {   // by the first product, outside any stream capture
+            const cudaError_t e = cudaFuncSetAttribute(k_row_ring, cudaFuncAttributeMaxDynamicSharedMemorySize, kRingSmem);
+            if (e != cudaSuccess) {
+                set_error("k_row_ring: cannot reserve %d bytes of shared memory: %s", kRingSmem, cudaGetErrorString(e));
+                return 1;
+            }
+            c.row_attr = true;
+        }
+        const int grid = c.Gs < c.nsm ? c.Gs : c.nsm;   // c.part_s holds c.Gs shares
+        launch_dependent(c.dependent && st, c.stream, grid, kRingWarps * 32, kRingSmem, k_row_ring, c.nn, c.row_off, c.row_val,
+                         (const uint16_t *)c.row_idx, c.row_base, c.freemask, c.fstore, xin, out, c.part_s, st, c.count,
+                         c.row_keep ? 1 : 0, c.kerr);
+        return launched8(c, "k_row_ring");
+    }
     auto go = [&](auto *idx, auto kernel0, auto kernel1) {
         launch_dependent(c.dependent && st, c.stream, c.Gs, 256, 0, mode ? kernel1 : kernel0, c.nn, c.row_off, c.row_val,
                          idx, c.row_base, c.freemask, c.fstore, xin, pf, out, c.part_s, st, c.count);

@@ -86,3 +86,10 @@ def test_rows_with_32_bit_columns():
 @pytest.mark.parametrize("m", [5, 15, 16, 24])   # 22, 62, 66 and 98 neighbours: rows up to 64, element products beyond
 def test_fans_of_bricks(m):
     check(*fan(m))
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 2, 7), (3, 31, 30), (31, 31, 31), (33, 29, 40)])
+def test_rows_streamed_through_shared_memory(shape):
+    """One slice of 32 rows, a ragged last one, fewer and more slices than warps, and iterations above and below
+    30,000 slots."""
+    check(*box(*shape, False))
