@@ -557,6 +557,8 @@ struct TailArgs {
     double *part;
     const double *pu;            // [npu] the products' shares of p.u (DOT)
     int npu;
+    const unsigned char *rec;    // the next products' records, `ahead` of each of their CTAs to be fetched into L2
+    int rec_bytes, nels, per_el, ahead;
     int *kerr;
 };
 
@@ -743,6 +745,9 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_pcg_tail(TailArgs a)
     sh[0][t] = rd;
     if (!CHECON) sh[1][t] = rr;
     if (CHECON) block_max2(mx, md);
+    // the next products' first records on their way to L2
+    if (t < a.ahead && blk * a.per_el + t < min(a.nels, (blk + 1) * a.per_el))
+        tc::bulk_prefetch(a.rec + (size_t)(blk * a.per_el + t) * a.rec_bytes, a.rec_bytes);
     // p of the first slots, in flight beside the sums
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
@@ -814,12 +819,21 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_pcg_tail(TailArgs a)
         vs->beta = beta;
         vs->iters = iters + 1;
         vs->rr = CHECON ? 0.0 : measure;
-        vs->metric = CHECON ? measure : sqrt(measure) / sqrt(vs->ff);
         vs->converged = conv ? 1 : 0;
         if (bad) vs->err = 1;
-        if (conv || iters + 1 >= vs->limit || bad) vs->stop = vs->stop2 = 1;
+        if (conv || iters + 1 >= vs->limit || bad) {   // two roots and a division: only when they are read
+            vs->metric = CHECON ? measure : sqrt(measure) / sqrt(vs->ff);
+            vs->stop = vs->stop2 = 1;
+        }
     }
 }
+
+// Bytes of records per CTA fetched into L2 while the sums cross the chip:
+// the next products start from L2 instead of HBM.  us per iteration with
+// and without: 31^3 FP64 99.3/104.9, FP32 55.2/57.9, FP16 44.9/47.6; 36^3 146.3/147.3, 77.5/79.2, 59.8/61.0;
+// 45^3 and larger within 1 %.  More (120, 240 KB), or at the start of the
+// tail, is in the way of its own loads (31^3 120 MB: 108, 65.6, 51.2 us).
+constexpr int kAheadBytes = 60 << 10;
 
 constexpr int kTailMax = 26;   // slots per thread that fit in shared memory
 
@@ -862,10 +876,35 @@ int prepare_tail(Ctx &c)
     return 0;
 }
 
+// The records that the next products read first
+static void records_ahead(const Ctx &c, int prec, TailArgs &a)
+{
+    a.nels = c.nels;
+    a.per_el = (c.nels + element_ctas(c) - 1) / element_ctas(c);
+    a.ahead = 0;
+    a.rec = nullptr;
+    a.rec_bytes = 0;
+    if (c.kind != KIND_SOLID20 || c.shared) return;
+    if (prec == PREC_FP64 && c.kmfix) {
+        a.rec = c.kmfix;
+        a.rec_bytes = fx::kRecBytes;
+    } else if (prec == PREC_FP32_SYM) {
+        a.rec = (const unsigned char *)c.km32p;
+        a.rec_bytes = sym::kBytes32;
+    } else if (prec == PREC_FP16_SYM) {
+        a.rec = (const unsigned char *)c.km16p;
+        a.rec_bytes = sym::kBytes16;
+    } else {
+        return;
+    }
+    a.ahead = kAheadBytes / a.rec_bytes;
+}
+
 template <typename UT, bool CHECON, int HOW>
-static int launch_tail_t(Ctx &c, double *xsol, int npu)
+static int launch_tail_t(Ctx &c, int prec, double *xsol, int npu)
 {
     TailArgs a;
+    records_ahead(c, prec, a);
     a.nn = (c.nslots + 2) / 3;
     a.per_nodes = tail_nodes(c);
     a.ns = c.nslots;
@@ -901,10 +940,10 @@ int launch_iteration_tail(Ctx &c, int prec, double *xsol, int npu)
 {
     const bool ck = c.stop_mode == STOP_CHECON;   // FP64 runs only
     if (c.kind != KIND_SOLID20)
-        return ck ? launch_tail_t<double, true, TAIL_GIVEN>(c, xsol, 0) : launch_tail_t<double, false, TAIL_GIVEN>(c, xsol, 0);
+        return ck ? launch_tail_t<double, true, TAIL_GIVEN>(c, prec, xsol, 0) : launch_tail_t<double, false, TAIL_GIVEN>(c, prec, xsol, 0);
     if (prec == PREC_FP64)
-        return ck ? launch_tail_t<double, true, TAIL_SUMS>(c, xsol, 0) : launch_tail_t<double, false, TAIL_SUMS>(c, xsol, 0);
-    return npu ? launch_tail_t<float, false, TAIL_DOT>(c, xsol, npu) : launch_tail_t<float, false, TAIL_SUMS>(c, xsol, 0);
+        return ck ? launch_tail_t<double, true, TAIL_SUMS>(c, prec, xsol, 0) : launch_tail_t<double, false, TAIL_SUMS>(c, prec, xsol, 0);
+    return npu ? launch_tail_t<float, false, TAIL_DOT>(c, prec, xsol, npu) : launch_tail_t<float, false, TAIL_SUMS>(c, prec, xsol, 0);
 }
 
 double *product_shares(Ctx &c) { return c.res_part + 8 + 4 * kMaxBlocks; }

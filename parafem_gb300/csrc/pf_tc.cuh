@@ -94,6 +94,12 @@ __device__ __forceinline__ uint64_t l2_evict_first_policy()
     return pol;
 }
 
+// The bytes at src into L2 (both multiples of 16), with nobody waiting
+__device__ __forceinline__ void bulk_prefetch(const void *src, uint32_t bytes)
+{
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+
 // bulk_g2s with an L2 cache policy (l2_evict_first_policy)
 __device__ __forceinline__ void bulk_g2s_hint(void *dst, const void *src, uint32_t bytes, uint64_t *bar,
                                               uint64_t pol)
