@@ -417,7 +417,7 @@ def run_gb300(args, rank, world, local, dist):
             "peak_kind": f"{peak_kind} hbm_gbs", "bytes_per_launch": b_launch,
             "avg_launch_ms": avg_s * 1e3, "traffic": ncu_traffic("k_elem_sym32_cube100"),
             "scatter_avg_ms": ms_scat / args.steps}
-    extra["fp64_elem_hbm_frac"] = elem_bytes(nels, nslots, 28800, 8) / (ms64_elem / k2 / 1e3) / 1e9 / peak
+    extra["fp64_elem_hbm_frac"] = elem_bytes(nels, nslots, 14784, 8) / (ms64_elem / k2 / 1e3) / 1e9 / peak
     extra["fp32_full_elem_hbm_frac"] = elem_bytes(nels, nslots, 14400, 4) / (ms31_elem / k2 / 1e3) / 1e9 / peak
     extra["fp16_elem_hbm_frac"] = elem_bytes(nels, nslots, 3664, 4) / (ms16_elem / args.steps / 1e3) / 1e9 / peak
 
@@ -838,7 +838,7 @@ def run_p123(args, rank, world, local, dist):
             "solve": {"iters": it, "wall_s": t_solve, "device_s": st["solve_ms"] / 1e3,
                       "dof_iter_per_s": neq * it / t_solve, "potentials": [float(v) for v in x[nres - 1:nres + 3]],
                       "reference_book": {"iters": 180, "solver_s": 52.3833, "cores": 16}},
-            "roofline": {"kernel": "k_row_product (assembled FP64 storkc)", "bound": "hbm", "achieved": b_launch / avg_s / 1e9,
+            "roofline": {"kernel": "k_row_ring (assembled FP64 storkc)", "bound": "hbm", "achieved": b_launch / avg_s / 1e9,
                          "peak": peak, "unit": "GB/s", "frac": b_launch / avg_s / 1e9 / peak,
                          "peak_kind": f"{peak_kind} hbm_gbs", "bytes_per_launch": b_launch,
                          "avg_launch_ms": avg_s * 1e3, "traffic": None},

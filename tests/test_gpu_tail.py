@@ -94,3 +94,18 @@ def test_forced_products_change_the_iterates_by_rounding_only():
     assert b[2] <= 1e-9 and a[1] == c[1]
     assert np.array_equal(a[0], c[0])
     assert np.linalg.norm(a[0] - b[0]) <= 1e-7 * np.linalg.norm(a[0])
+
+
+@pytest.mark.parametrize("shared", [True, False])
+def test_beyond_the_tail_persistent_and_separate_kernels_agree(shared):
+    """4.3 million freedoms: more than the tail takes."""
+    prob = P.cube_problem(71, 70, 71)
+    out = []
+    with solver(prob, shared) as s:
+        for persistent in (True, False):
+            s.set_persistent(persistent)
+            out.append([s.solve(prob["r"], 0.0, 11, m)[0] for m in (P.MODE_P121, P.MODE_FP64_RES)])
+            if shared:
+                out[-1].append(s.solve(prob["r"], 0.1, 200, P.MODE_MIXED)[0])
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
