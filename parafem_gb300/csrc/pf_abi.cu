@@ -141,7 +141,7 @@ static void free_mesh(Ctx &c)
     rows_release(c);
     dfree(c.conn); dfree(c.node_ptr); dfree(c.node_list); dfree(c.slot_eq); dfree(c.eq_slot);
     dfree(c.freemask); dfree(c.coord); dfree(c.mat_e); dfree(c.mat_v); dfree(c.km64); dfree(c.km32);
-    dfree(c.km32p); dfree(c.skm64); dfree(c.skm32); dfree(c.fstore); dfree(c.fscale); dfree(c.psplit);
+    dfree(c.km32p); dfree(c.skm64); dfree(c.skm32); dfree(c.skma); dfree(c.fstore); dfree(c.fscale); dfree(c.psplit);
     dfree(c.km16p); dfree(c.kmfix); dfree(c.skmfix);
     c.km16_ok = false;
     c.km32_ok = false;
@@ -903,6 +903,7 @@ try {
         }
     CK(cudaMemcpyAsync(c.skm64, km, 3600 * sizeof(double), cudaMemcpyHostToDevice, c.stream));
     CK(cudaMemcpyAsync(c.skm32, k32.data(), (3600 + 192) * sizeof(float), cudaMemcpyHostToDevice, c.stream));
+    TRY(launch_shared_image(c));
     if (!c.skmfix && dalloc(&c.skmfix, fx::kRecBytes, "shared km")) return PF_FAILURE;
     CK(cudaMemsetAsync(c.kerr + 1, 0, sizeof(int), c.stream));
     TRY(launch_pack_storkm(c, 1, c.skm64, nullptr, c.skmfix, c.kerr + 1));

@@ -131,6 +131,7 @@ struct Ctx {
     bool shared = false;
     double *skm64 = nullptr;    // [3600] column-major
     float *skm32 = nullptr;     // [3600 + 192]: km, then the direction sums of its rows ([3][64])
+    unsigned char *skma = nullptr;   // km as the tensor-core product's A operand (k_shared_image)
     unsigned char *skmfix = nullptr;   // km's fixed-point record, or null (km not symmetric)
     bool shared_attr = false;   // shared-memory attribute of the tensor-core kernel set
     float2 *psplit = nullptr;   // [nslots] FP32 high and low parts of p (shared km): written with p
@@ -256,6 +257,7 @@ int launch_set_fixed(Ctx &c, int nfix, const int *slots_dev, double penalty);
 // pf_solid8.cu: 8-node elasticity bricks (24 freedoms per element), FP64
 int launch_elem24(Ctx &c, const double *p, const PcgState *st);
 int launch_scatter3_fixed(Ctx &c, const double *p, double *out, PcgState *st);
+int launch_shared_image(Ctx &c);
 int launch_shared_ediag(Ctx &c);
 void set_sym_config(Ctx &c, int idx);           // 0: 14 warps x 2 stages, 1: 12 x 2, 2: 8 x 3
 int launch_matvec_generic(int n_mat, int n_row, int n_col, const double *lhs,

@@ -8,8 +8,8 @@
 //   k_elem_shared64   FP64 on CUDA cores: km in shared memory, one warp per
 //                     element (bound by FP64 FMA throughput, as k_elem<double>).
 //   k_elem_shared_tc  FP32-class on the tensor cores: km split once into
-//                     three BF16 terms held in shared memory for the whole
-//                     kernel; tiles of 128 elements' gathered p values are
+//                     three BF16 terms (k_shared_image), copied into shared
+//                     memory for the whole kernel; tiles of 128 elements' gathered p values are
 //                     split the same way; the six products of order <= 2^-16
 //                     accumulate in FP32 in TMEM (M = 128: km's rows in four
 //                     blocks of five nodes, each block with the three
@@ -97,6 +97,38 @@ k_elem_shared64(int nels, const double *__restrict__ km, const int *__restrict__
     }
 }
 
+// km once, three BF16 terms.  A row 32w + i is K row 3(5w + i/3) + i%3
+// for i < 15 (nodes 5w..5w+4), the sum of K's 20 rows of direction
+// i - 15 for i = 15..17, zero otherwise.  The sums are zero in exact
+// arithmetic (K annihilates rigid translations); they carry the rounding
+// of the FP32 km and put each element's per-direction sum of results
+// beside its rows in the accumulator.  K(i,k) = km32[i + 60k]; the sums
+// follow km (km32[3600 + 64d + k]), so the prologue has no FP64 work.
+// Formed once with km, and copied whole into shared memory by every CTA:
+// splitting km there (2.2 us) and clearing the tiles that the gather warps
+// write in full anyway (0.7 us) were a fifth of a launch on small meshes (10^3
+// iteration 28.2 -> 25.9 us, 33^3 34.2 -> 31.4, 64^3 150 -> 146).
+__global__ void k_shared_image(const float *__restrict__ km32, unsigned char *__restrict__ img)
+{
+    for (int task = threadIdx.x; task < kSRowsA * 8; task += blockDim.x) {
+        const int row = task % kSRowsA, q = task / kSRowsA;
+        const int w = row >> 5, i = row & 31;
+        float xv[8];
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+            const int k = 8 * q + g;
+            float v = 0.f;
+            if (k < 60 && i < 15) {
+                v = km32[3 * (5 * w + i / 3) + i % 3 + 60 * k];
+            } else if (k < 60 && i < 18) {
+                v = km32[3600 + 64 * (i - 15) + k];   // formed on the host with km
+            }
+            xv[g] = v;
+        }
+        split3_store8(xv, img + kmajor_off(row, 8 * q), kSTermA);
+    }
+}
+
 // u_e = P km P p_e on the tensor cores for every element (FP32 results,
 // node-padded: row i of element e at e*80 + (i/3)*4 + i%3).
 // One persistent CTA of 22 warps per SM walks the tiles T = blockIdx.x +
@@ -114,7 +146,7 @@ k_elem_shared64(int nels, const double *__restrict__ km, const int *__restrict__
 // word, and the CTA waits (bounded) for the copies and MMAs it has in flight
 // before it frees its TMEM and returns.
 __global__ void __launch_bounds__(kSThreads, 1)
-k_elem_shared_tc(int nels, const float *__restrict__ km32, const int *__restrict__ conn,
+k_elem_shared_tc(int nels, const unsigned char *__restrict__ img, const int *__restrict__ conn,
                  const float2 *__restrict__ ps, float *__restrict__ ut, const PcgState *__restrict__ st,
                  int *__restrict__ err)
 {
@@ -128,46 +160,30 @@ k_elem_shared_tc(int nels, const float *__restrict__ km32, const int *__restrict
     uint64_t *b_empty = b_full + kSNB;
     uint64_t *a_full = b_empty + kSNB;
     uint64_t *a_empty = a_full + kSNA;
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(a_empty + kSNA);
+    uint64_t *i_full = a_empty + kSNA;   // km's operand has landed
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(i_full + 1);
     volatile int *s_fail = reinterpret_cast<volatile int *>(tslot + 1);
     int *s_count = reinterpret_cast<int *>(tslot + 2);   // [0] copies issued, [1] MMA groups committed
     int *s_stop = s_count + 2;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {   // km's operand is no kernel's of this iteration: before the wait for the one before
+        mbar_init(i_full, 1);
+        mbar_fence_init();
+        mbar_expect_tx(i_full, kSBufA);
+        bulk_g2s(A, img, kSBufA, i_full);
+    }
     pdl_enter();
     if (tid == 0) *s_stop = st ? st->stop : 0;
     __syncthreads();
-    if (*s_stop) return;   // uniform: read once per block
+    if (*s_stop) {   // uniform: read once per block
+        if (tid == 0) mbar_wait(i_full, 0);
+        return;
+    }
     const int ntiles = (nels + kNT - 1) / kNT;
     const int nmine = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
     auto tile = [&](int t) { return (int)blockIdx.x + t * (int)gridDim.x; };
     auto tile_n = [&](int t) { const int r = nels - tile(t) * kNT; return r < kNT ? r : kNT; };
 
-    // km once, three BF16 terms.  A row 32w + i is K row 3(5w + i/3) + i%3
-    // for i < 15 (nodes 5w..5w+4), the sum of K's 20 rows of direction
-    // i - 15 for i = 15..17, zero otherwise.  The sums are zero in exact
-    // arithmetic (K annihilates rigid translations); they carry the rounding
-    // of the FP32 km and put each element's per-direction sum of results
-    // beside its rows in the accumulator.  K(i,k) = km32[i + 60k]; the sums
-    // follow km (km32[3600 + 64d + k]), so the prologue has no FP64 work.
-    for (int i = tid; i < kSOffC / 16; i += kSThreads) reinterpret_cast<uint4 *>(sm)[i] = make_uint4(0, 0, 0, 0);
-    __syncthreads();
-    for (int task = tid; task < kSRowsA * 8; task += kSThreads) {
-        const int row = task % kSRowsA, q = task / kSRowsA;
-        const int w = row >> 5, i = row & 31;
-        float xv[8];
-#pragma unroll
-        for (int g = 0; g < 8; ++g) {
-            const int k = 8 * q + g;
-            float v = 0.f;
-            if (k < 60 && i < 15) {
-                v = km32[3 * (5 * w + i / 3) + i % 3 + 60 * k];
-            } else if (k < 60 && i < 18) {
-                v = km32[3600 + 64 * (i - 15) + k];   // formed on the host with km
-            }
-            xv[g] = v;
-        }
-        split3_store8(xv, A + kmajor_off(row, 8 * q), kSTermA);
-    }
     if (warp == 0) tmem_alloc(tslot, 512);
     if (tid == 0) {
         for (int i = 0; i < kSNC; ++i) {
@@ -281,7 +297,7 @@ k_elem_shared_tc(int nels, const float *__restrict__ km32, const int *__restrict
         }
     } else if (warp == kSMma) {
         int t = 0;
-        if (lane == 0) {
+        if (lane == 0 && wait(i_full, 0)) {
             for (; t < nmine; ++t) {
                 const int bb = t % kSNB, a = t % kSNA;
                 if (!wait(&b_full[bb], (uint32_t)((t / kSNB) & 1))) break;
@@ -347,6 +363,7 @@ k_elem_shared_tc(int nels, const float *__restrict__ km32, const int *__restrict
     if (*s_fail) {
         if (tid == 0) {
             atomicExch(err, 3);
+            mbar_wait(i_full, 0);
             for (int t = s_count[0] - kSNC; t < s_count[0]; ++t)
                 if (t >= 0) mbar_wait(&c_full[t % kSNC], (uint32_t)((t / kSNC) & 1));
             for (int t = s_count[1] - kSNA; t < s_count[1]; ++t)
@@ -364,6 +381,22 @@ __global__ void k_shared_ediag(int nels, const double *__restrict__ km, double *
     for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < (size_t)nels * 60;
          t += (size_t)gridDim.x * blockDim.x)
         ediag[t] = km[(t % 60) * 61];
+}
+
+int launch_shared_image(Ctx &c)
+{
+    if (!c.skma && ctx_malloc(c, (void **)&c.skma, kSBufA)) {
+        set_error("pf_set_shared_km: cannot allocate %d bytes", kSBufA);
+        return 1;
+    }
+    k_shared_image<<<1, 512, 0, c.stream>>>(c.skm32, c.skma);
+    c.launches++;
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+        set_error("k_shared_image: launch failed: %s", cudaGetErrorString(e));
+        return 1;
+    }
+    return 0;
 }
 
 int launch_shared_ediag(Ctx &c)
@@ -418,7 +451,7 @@ int launch_elem_shared(Ctx &c, int prec, const double *p, const PcgState *st)
         }
         const int ntiles = (c.nels + kNT - 1) / kNT;
         const int grid = ntiles < c.nsm ? ntiles : c.nsm;
-        launch_dependent(c.dependent && st, c.stream, grid, kSThreads, kSSmem, k_elem_shared_tc, c.nels, c.skm32, c.conn, c.psplit,
+        launch_dependent(c.dependent && st, c.stream, grid, kSThreads, kSSmem, k_elem_shared_tc, c.nels, c.skma, c.conn, c.psplit,
                          (float *)c.utemp, st, c.kerr);
     }
     c.launches++;
