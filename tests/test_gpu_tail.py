@@ -109,3 +109,30 @@ def test_beyond_the_tail_persistent_and_separate_kernels_agree(shared):
                 out[-1].append(s.solve(prob["r"], 0.1, 200, P.MODE_MIXED)[0])
     for x, y in zip(*out):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("n", [20, 22])
+def test_elasticity_on_8_node_bricks(n):
+    """27,783 freedoms (separate updates) and 36,501 (the tail behind the product of the 8-node bricks)."""
+    prob = P.box8_problem(n, n, n)
+    g_num, nn = prob["g_num"], prob["nn"]
+    z = np.zeros(nn)
+    for e in range(g_num.shape[0]):
+        z[g_num[e] - 1] = prob["g_coord"][e][2]
+    free = np.repeat((z > z.min() + 1e-9)[:, None], 3, axis=1)
+    eq = np.where(free, np.cumsum(free.ravel(), dtype=np.int32).reshape(nn, 3), 0).astype(np.int32)
+    neq = int(free.sum())
+    g_g = eq[g_num - 1].reshape(-1, 24)
+    r = np.zeros(neq)
+    top = np.flatnonzero(z > z.max() - 1e-9)
+    r[eq[top, 2] - 1] = -1.0 / top.size
+    r[eq[top, 0] - 1] = 0.3 / top.size
+    with P.Solver() as s:
+        s.setup_solid8(g_num, g_g, prob["g_coord"], nn, neq)
+        s.set_material(100.0, 0.3)
+        s.form_storkm(8)
+        x, _, rel = s.solve(r, 1e-11, 20000, P.MODE_FP64_RES)
+        assert rel <= 1e-10
+        assert np.linalg.norm(r - s.ebe_matvec(x, 64)) <= 1e-10 * np.linalg.norm(r)
+        y, _, _ = s.solve(r, 1e-11, 20000, P.MODE_P121)
+        assert np.linalg.norm(y - x) <= 1e-7 * np.linalg.norm(x)
