@@ -435,10 +435,11 @@ try {
         cudaMemset(c->count, 0, 2 * sizeof(unsigned)) != cudaSuccess ||
         cudaMalloc((void **)&c->gbar, sizeof(unsigned long long) * kPersistSlots * kBarWords) != cudaSuccess ||
         cudaMemset(c->gbar, 0, sizeof(unsigned long long) * kPersistSlots * kBarWords) != cudaSuccess ||
+        cudaMalloc((void **)&c->res_part, kShareBytes) != cudaSuccess ||
         cudaMallocHost((void **)&c->hst, sizeof(PcgState)) != cudaSuccess) {
         set_error("pf_ctx_create: cannot create stream/state");
+        dfree(c->st); dfree(c->kerr); dfree(c->count); dfree(c->gbar); dfree(c->res_part);
         if (c->stream) cudaStreamDestroy(c->stream);
-        if (c->st) cudaFree(c->st);
         delete c;
         return PF_FAILURE;
     }

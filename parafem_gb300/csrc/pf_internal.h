@@ -66,6 +66,8 @@ constexpr int kRowBlocks = 64;   // of the 8-node scalar product: rows are short
 constexpr int kDependentSlots = 500000;
 constexpr int kPersistSlots = 8;   // persistent-kernel instantiations, one barrier counter and grid each
 constexpr int kTailBar = 6;         // the counter of the iteration tail (the persistent kernel's use 0 to 5)
+constexpr int kShareBlocks = 256;   // most CTAs of the resident run and of the iteration tail
+constexpr size_t kShareBytes = 64 + 5 * kShareBlocks * sizeof(double);   // of Ctx::res_part
 constexpr int kBarWords = 16;      // u64 words per counter (one 128-byte line each)
 // 20-node elasticity (p121), 8-node scalar (p123), 8-node elasticity (p122's demo)
 enum { KIND_SOLID20 = 0, KIND_SCALAR8 = 1, KIND_SOLID8 = 2 };
@@ -152,7 +154,9 @@ struct Ctx {
     bool persistent = false;    // true: persistent cooperative kernels for the iteration (pf_set_persistent)
     unsigned long long *gbar = nullptr;   // [kPersistSlots] grid-barrier arrival counters, zeroed per run
     bool tail_attr = false;               // shared-memory attribute of k_pcg_tail set
-    double *res_part = nullptr;           // the resident PCG's arrival counter and shares, allocated on first use
+    double *res_part = nullptr;           // [kShareBytes] the resident PCG's arrival counter and the CTAs' shares.
+                                          //   Allocated with the context: an allocation between the choice of a
+                                          //   route and its launch could free the records it was chosen for (ctx_malloc)
     int pk_grid[kPersistSlots] = {};      // blocks of each persistent instantiation (0 = not sized)
 
     bool dependent = false;     // programmatic dependent launches in the iteration (small meshes)
@@ -182,7 +186,8 @@ int launch_form_storkm_raw(cudaStream_t stream, int nsm, int nels, int nip, cons
 int launch_cast_km32(Ctx &c);
 int launch_extract_ediag(Ctx &c);
 // cudaMalloc for a context; when it fails, the fixed-point records (which
-// the FP64 products can do without) are given back and it is tried again
+// the FP64 products can do without) are given back and it is tried again.
+// Called before a solve's route is chosen, never between that and a launch.
 int ctx_malloc(Ctx &c, void **p, size_t bytes);
 int ensure_km32(Ctx &c);   // the full FP32 storkm, if storkm changed; outside stream capture
 // pf_fix.cu: the packed forms of nels FP64 element matrices (kp or rec may be null), FP64 products from the records

@@ -30,7 +30,7 @@ namespace pf {
 namespace {
 
 constexpr int kResThreads = 512;
-constexpr int kMaxBlocks = 256;   // shares a warp adds: eight per lane
+constexpr int kMaxBlocks = kShareBlocks;   // shares a warp adds: eight per lane
 
 struct ResArgs {
     int nels, ns, niters, per_slots;
@@ -439,18 +439,6 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(ResArgs a)
     }
 }
 
-// The arrival counter and the CTAs' shares (outside any stream capture)
-static int ensure_shares(Ctx &c)
-{
-    if (c.res_part) return 0;
-    const size_t bytes = 64 + 5 * kMaxBlocks * sizeof(double);
-    if (ctx_malloc(c, (void **)&c.res_part, bytes)) {
-        set_error("PCG: cannot allocate %zu bytes of shares", bytes);
-        return 1;
-    }
-    return 0;
-}
-
 // ---------------------------------------------------------------------------
 // Rule: 20-node meshes with records (one per element, or FP64 one for all)
 // whose slots fit the CTAs, four per thread (311,296 on 152 SMs: 28^3 elements).  Measured us per
@@ -497,7 +485,6 @@ static int launch_resident_t(Ctx &c, double *xsol, int niters)
     a.p = c.p;
     a.dinv = c.dinv;
     a.st = c.st;
-    if (ensure_shares(c)) return 1;
     a.count = reinterpret_cast<unsigned long long *>(c.res_part);
     a.part = c.res_part + 8;
     if (e == cudaSuccess) e = cudaMemsetAsync(a.count, 0, sizeof(unsigned long long), c.stream);
@@ -859,7 +846,6 @@ bool tail_ok(const Ctx &c)
 // The shared memory of the tail's largest form (outside any stream capture)
 int prepare_tail(Ctx &c)
 {
-    if (ensure_shares(c)) return 1;
     if (c.tail_attr) return 0;
     const void *fn[] = {(const void *)k_pcg_tail<double, true, TAIL_SUMS>, (const void *)k_pcg_tail<double, false, TAIL_SUMS>,
                         (const void *)k_pcg_tail<float, false, TAIL_SUMS>, (const void *)k_pcg_tail<float, false, TAIL_DOT>,

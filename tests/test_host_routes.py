@@ -1,0 +1,72 @@
+"""The host code that chooses and prepares the kernels, without a GPU: the
+library's object files linked against a stand-in for the CUDA runtime
+(fake_cudart.cpp) that keeps a log of the launches and can refuse
+allocations and launches."""
+import ctypes
+import os
+import subprocess
+
+import pytest
+
+import parafem_gb300 as P
+from parafem_gb300 import _build, pfgpu
+
+
+@pytest.fixture(scope="session")
+def fake_lib(tmp_path_factory):
+    lib = _build.build()
+    objs = [os.path.join(_build.OUT, os.path.splitext(s)[0] + ".o") for s in _build.CUDA_SOURCES + _build.CXX_SOURCES]
+    if not all(os.path.exists(o) and os.path.getmtime(o) <= os.path.getmtime(lib) for o in objs):
+        _build.build(force=True)
+    out = str(tmp_path_factory.mktemp("fake"))
+    cuda = os.path.join(os.path.dirname(os.path.dirname(_build.nvcc())), "include")
+    so = os.path.join(out, "libpfgpu_fake.so")
+    subprocess.check_call(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I", cuda,
+                           os.path.join(os.path.dirname(__file__), "fake_cudart.cpp")] + objs + ["-o", so])
+    L = ctypes.CDLL(so)
+    for name, args in pfgpu._SIGS.items():
+        getattr(L, name).argtypes = args
+        getattr(L, name).restype = ctypes.c_int
+    L.fake_used.restype = ctypes.c_longlong
+    L.fake_limit.argtypes = [ctypes.c_longlong]
+    L.fake_log.restype = ctypes.c_char_p
+    return L
+
+
+@pytest.fixture
+def fake(fake_lib, monkeypatch):
+    fake_lib.fake_reset()
+    monkeypatch.setattr(pfgpu, "_lib", fake_lib)
+    yield fake_lib
+    fake_lib.fake_reset()
+
+
+def kernels(fake):
+    """(name, blocks) of the launches since the log was cleared."""
+    return [tuple(line.rsplit(" ", 1)) for line in fake.fake_log().decode().splitlines() if " " in line]
+
+
+def launched(fake, part):
+    return sum(part in name for name, _ in kernels(fake))
+
+
+def solver(n):
+    prob = P.cube_problem(n, n, n)
+    s = P.Solver()
+    s.setup(prob["g_num"], prob["g_g"], prob["g_coord"], prob["nn"], prob["neq"])
+    s.set_material(100.0, 0.3)
+    return s, prob["r"]
+
+
+@pytest.mark.parametrize("mode", [P.MODE_P121, P.MODE_FP64_RES])
+def test_a_full_device_leaves_no_launch_on_freed_records(fake, mode):
+    """A solve may give the fixed-point records back when an allocation fails.  No kernel may then be launched on
+    them: the run takes the records, or the products that do without."""
+    s, r = solver(3)
+    s.form_storkm(8)
+    fake.fake_limit(fake.fake_used())          # the device is full
+    fake.fake_clear_log()
+    s.solve(r, 1e-8, 3, mode)
+    assert fake.fake_stale() == 0
+    assert launched(fake, "k_pcg_resident") == 1
+    s.close()
