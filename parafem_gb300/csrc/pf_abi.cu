@@ -299,15 +299,17 @@ static int run_pcg(Ctx &c, int prec, double *xsol, int limit)
 
 int run_pcg_public(Ctx &c, int prec, double *xsol, int limit) { return run_pcg(c, prec, xsol, limit); }
 
-// ||f - K64 x||_2 / ||f||_2 on the device (fills c.rres).
-static int true_relres(Ctx &c, const double *x, double ff, double *out, double *dev2)
+// ||f - K64 x||_2 / ||f||_2 on the device (fills c.rres).  Fails when a wait
+// of its products ran out: the norm is then not one of this x.
+static int true_relres(Ctx &c, const double *x, double ff, double *out)
 {
     TRY(launch_residual(c, c.f, x, c.rres));
-    TRY(launch_sum_partials(c, 1, dev2));
-    double rr = 0.0;
-    CK(cudaMemcpyAsync(&rr, dev2, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    TRY(launch_sum_partials(c, 1, norms(c)));
+    struct { int err, bad; double rr; } h;
+    CK(cudaMemcpyAsync(&h, c.kerr, sizeof h, cudaMemcpyDeviceToHost, c.stream));
     CK(cudaStreamSynchronize(c.stream));
-    *out = ff > 0.0 ? std::sqrt(rr) / std::sqrt(ff) : 0.0;
+    if (h.err) return check_kernel_error(c);
+    *out = ff > 0.0 ? std::sqrt(h.rr) / std::sqrt(ff) : 0.0;
     return 0;
 }
 
@@ -429,8 +431,8 @@ try {
     if (c->nsm < 1) c->nsm = 1;
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaMalloc((void **)&c->st, sizeof(PcgState)) != cudaSuccess ||
-        cudaMalloc((void **)&c->kerr, 2 * sizeof(int)) != cudaSuccess ||
-        cudaMemset(c->kerr, 0, 2 * sizeof(int)) != cudaSuccess ||
+        cudaMalloc((void **)&c->kerr, kErrBytes) != cudaSuccess ||
+        cudaMemset(c->kerr, 0, kErrBytes) != cudaSuccess ||
         cudaMalloc((void **)&c->count, 2 * sizeof(unsigned)) != cudaSuccess ||
         cudaMemset(c->count, 0, 2 * sizeof(unsigned)) != cudaSuccess ||
         cudaMalloc((void **)&c->gbar, sizeof(unsigned long long) * kPersistSlots * kBarWords) != cudaSuccess ||
@@ -992,7 +994,7 @@ try {
 // K32 c = f - K64 x from c = 0 with FP32-storkm PCG, then x += c in FP64 and
 // the FP64 true residual is recomputed.  Every restart discards the Krylov
 // space, so the inner iterations add up to about twice the FP64 count.
-static int solve_mixed_restart(Ctx &c, double tol, int limit, double ff, double *dev2)
+static int solve_mixed_restart(Ctx &c, double tol, int limit, double ff)
 {
     const double eta_min = 1e-5;   // inner relative tolerance floor
     const int max_outer = 50;
@@ -1009,7 +1011,7 @@ static int solve_mixed_restart(Ctx &c, double tol, int limit, double ff, double 
         TRY(run_pcg(c, 32, c.c, limit - inner_total));
         inner_total += c.hst->iters;
         TRY(launch_axpy(c, c.x, c.c));
-        TRY(true_relres(c, c.x, ff, &rel, dev2));
+        TRY(true_relres(c, c.x, ff, &rel));
         ++mv64;
     }
     c.stats[0] = inner_total;
@@ -1027,7 +1029,7 @@ static int solve_mixed_restart(Ctx &c, double tol, int limit, double ff, double 
 // (defect correction) and the search direction is kept, so the Krylov space
 // built so far is not thrown away.  The solve ends when the TRUE relative
 // residual reaches tol.
-static int solve_mixed(Ctx &c, double tol, int limit, double ff, double *dev2, int inner_prec)
+static int solve_mixed(Ctx &c, double tol, int limit, double ff, int inner_prec)
 {
     const double drop = 0.1;
     const int max_corrections = 200;
@@ -1040,7 +1042,7 @@ static int solve_mixed(Ctx &c, double tol, int limit, double ff, double *dev2, i
         TRY(pull_state(c));
         const int done = c.hst->iters;
         if (!c.hst->stop) TRY(run_pcg(c, inner_prec, c.x, limit - done));
-        TRY(true_relres(c, c.x, ff, &rel, dev2));
+        TRY(true_relres(c, c.x, ff, &rel));
         ++mv64;
         if (rel <= tol || c.hst->iters >= limit || corrections >= max_corrections) break;
         anchor = rel;
@@ -1082,7 +1084,6 @@ try {
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
-    double *dev2 = c.scr;
     CK(cudaMemcpyAsync(c.eqbuf, r, (size_t)c.neq * sizeof(double), cudaMemcpyHostToDevice, c.stream));
     TRY(launch_eq_to_slot(c, c.eqbuf, c.f));
     CK(cudaEventRecord(e0, c.stream));
@@ -1095,9 +1096,9 @@ try {
         ff = c.hst->ff;
     }
     if (*mode == PF_MODE_MIXED || *mode == PF_MODE_MIXED16) {
-        rc = solve_mixed(c, *tol, *limit, ff, dev2, *mode == PF_MODE_MIXED16 ? PREC_FP16_SYM : PREC_FP32_SYM);
+        rc = solve_mixed(c, *tol, *limit, ff, *mode == PF_MODE_MIXED16 ? PREC_FP16_SYM : PREC_FP32_SYM);
     } else if (*mode == PF_MODE_MIXED_RESTART) {
-        rc = solve_mixed_restart(c, *tol, *limit, ff, dev2);
+        rc = solve_mixed_restart(c, *tol, *limit, ff);
     } else {
         rc = run_pcg(c, 64, c.x, *limit);
         c.stats[0] = c.hst->iters;
@@ -1109,7 +1110,7 @@ try {
     CK(cudaEventRecord(e1, c.stream));
     double rel = c.stats[3];
     if (*mode == PF_MODE_P121 || *mode == PF_MODE_FP64_RES)   // mixed modes end on a true residual
-        TRY(true_relres(c, c.x, ff, &rel, dev2));
+        TRY(true_relres(c, c.x, ff, &rel));
     float ms = 0.f;
     CK(cudaEventSynchronize(e1));
     CK(cudaEventElapsedTime(&ms, e0, e1));

@@ -67,6 +67,8 @@ constexpr int kDependentSlots = 500000;
 constexpr int kPersistSlots = 8;   // persistent-kernel instantiations, one barrier counter and grid each
 constexpr int kTailBar = 6;         // the counter of the iteration tail (the persistent kernel's use 0 to 5)
 constexpr int kShareBlocks = 256;   // most CTAs of the resident run and of the iteration tail
+constexpr int kNorms = 128;           // most true residuals formed at once (load cases of a block solve)
+constexpr size_t kErrBytes = 2 * sizeof(int) + kNorms * sizeof(double);   // of Ctx::kerr
 constexpr size_t kShareBytes = 64 + 5 * kShareBlocks * sizeof(double);   // of Ctx::res_part
 constexpr int kBarWords = 16;      // u64 words per counter (one 128-byte line each)
 // 20-node elasticity (p121), 8-node scalar (p123), 8-node elasticity (p122's demo)
@@ -96,8 +98,10 @@ struct Ctx {
     unsigned char *kmfix = nullptr;   // [nels] fixed-point records (pf_fix.cuh) for the FP64 products, or null:
                                       //   storkm not symmetric, or no device memory for them
     float *km32p = nullptr;     // [nels*1832] packed symmetric storkm (packed_off), FP32
-    int *kerr = nullptr;        // device error word: 2 = a bulk-copy wait timed out, 3 = a grid barrier did;
-                                //   kerr[1]: set by k_pack_storkm when a matrix does not fit its record
+    int *kerr = nullptr;        // [kErrBytes] device error word: 2 = a bulk-copy wait timed out, 3 = a grid barrier did;
+                                //   kerr[1]: set by k_pack_storkm when a matrix does not fit its record;
+                                //   behind them the squared norms of true residuals (norms), so that
+                                //   one copy brings a residual and whether its products ended in order
     unsigned *count = nullptr;  // [2] arrivals of the blocks of the scatter and of update1 (last_block)
     bool fix_attr = false;      // shared-memory attribute of the fixed-point kernel set
     bool have_km = false;
@@ -173,6 +177,9 @@ struct Ctx {
     // last solve statistics
     double stats[8] = {0};
 };
+
+// The squared norms behind the error word
+inline double *norms(const Ctx &c) { return reinterpret_cast<double *>(c.kerr + 2); }
 
 // CTAs of the bulk-copy element kernels: one per SM; a small mesh spreads its warps over the SMs
 inline int element_ctas(const Ctx &c) { return c.nels < c.nsm ? c.nels : c.nsm; }

@@ -39,7 +39,7 @@ using namespace tc;
 
 namespace {
 
-constexpr int kMaxK = 128;           // load cases of one block solve
+constexpr int kMaxK = kNorms;        // load cases of one block solve
 constexpr int kMaxKB = 64;           // cases of one tensor-core pass (the MMA's N)
 constexpr unsigned kFullMask = 0xffffffffu;
 
@@ -1019,7 +1019,7 @@ struct MultiBufs {
     float *ut32 = nullptr;
     float2 *Ps = nullptr;           // [ns*k] FP32 high and low parts of P (the tensor-core product's input)
     unsigned char *rec = nullptr;   // [nels][kRecBytes] tensor-core element records
-    double *ut64 = nullptr, *part = nullptr, *sums = nullptr;
+    double *ut64 = nullptr, *part = nullptr;
     MState *st = nullptr;
     MState *hst = nullptr;
     unsigned *count = nullptr;      // [2] arrivals of the blocks of the scatter and of update1 (last_block)
@@ -1039,11 +1039,11 @@ struct MultiBufs {
 namespace {
 void mb_free_vectors(MultiBufs &m)
 {
-    void *p[] = {m.F, m.X, m.R, m.D, m.P, m.U, m.RR, m.eq, m.ut32, m.Ps, m.ut64, m.part, m.sums, m.st, m.count};
+    void *p[] = {m.F, m.X, m.R, m.D, m.P, m.U, m.RR, m.eq, m.ut32, m.Ps, m.ut64, m.part, m.st, m.count};
     for (void *q : p)
         if (q) cudaFree(q);
     if (m.hst) cudaFreeHost(m.hst);
-    m.F = m.X = m.R = m.D = m.P = m.U = m.RR = m.eq = m.ut64 = m.part = m.sums = nullptr;
+    m.F = m.X = m.R = m.D = m.P = m.U = m.RR = m.eq = m.ut64 = m.part = nullptr;
     m.ut32 = nullptr;
     m.Ps = nullptr;
     m.st = nullptr;
@@ -1271,7 +1271,6 @@ static int mr_alloc(Ctx &c, int k)
     if (ctx_malloc(c, (void **)&m.Ps, n * 8)) goto fail;
     if (ctx_malloc(c, (void **)&m.ut64, (size_t)c.nels * 60 * k * 8)) goto fail;
     if (ctx_malloc(c, (void **)&m.part, parts * 8)) goto fail;
-    if (ctx_malloc(c, (void **)&m.sums, kMaxK * 8)) goto fail;
     if (ctx_malloc(c, (void **)&m.st, sizeof(MState))) goto fail;
     if (ctx_malloc(c, (void **)&m.count, 2 * sizeof(unsigned))) goto fail;
     if (cudaMemset(m.count, 0, 2 * sizeof(unsigned)) != cudaSuccess) goto fail;
@@ -1336,16 +1335,32 @@ static int mr_prepare_tc(Ctx &c)
     return 0;
 }
 
-// FP64 true residuals of all cases; returns per-case ||f - K x||^2 in rr_out
-static int mr_true_residual(Ctx &c, double *rr_out)
+static int mr_kernel_error(Ctx &c, const char *who)
+{
+    int kerr = 0;
+    MCK(cudaMemcpy(&kerr, c.kerr, sizeof(int), cudaMemcpyDeviceToHost));
+    if (kerr) {
+        cudaMemset(c.kerr, 0, sizeof(int));
+        set_error("%s: element product wait timed out", who);
+        return 1;
+    }
+    return 0;
+}
+
+// FP64 true residuals of all cases; returns per-case ||f - K x||^2 in rr_out.
+// Fails when a wait of the products ran out: the norms are then not those of X.
+static int mr_true_residual(Ctx &c, const char *who, double *rr_out)
 {
     MultiBufs &m = *c.multi;
     if (mr_elem(c, 64, m.X, nullptr)) return 1;
     if (mr_scatter(c, 64, 1, m.F, m.RR, nullptr)) return 1;
-    k_mr_sums<<<1, case_threads(m.k), 0, c.stream>>>(m.part, m.Gs, m.k, m.sums);
+    k_mr_sums<<<1, case_threads(m.k), 0, c.stream>>>(m.part, m.Gs, m.k, norms(c));
     if (mr_launched(c, "k_mr_sums")) return 1;
-    MCK(cudaMemcpyAsync(rr_out, m.sums, m.k * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    struct { int err, bad; double rr[kMaxK]; } h;
+    MCK(cudaMemcpyAsync(&h, c.kerr, 2 * sizeof(int) + m.k * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
     MCK(cudaStreamSynchronize(c.stream));
+    if (h.err) return mr_kernel_error(c, who);
+    for (int j = 0; j < m.k; ++j) rr_out[j] = h.rr[j];
     return 0;
 }
 
@@ -1353,18 +1368,6 @@ static int mr_check_k(const char *who, int k)
 {
     if (k < 8 || k > kMaxK || k % 8) {
         set_error("%s: k must be a multiple of 8 in 8..%d (got %d)", who, kMaxK, k);
-        return 1;
-    }
-    return 0;
-}
-
-static int mr_kernel_error(Ctx &c, const char *who)
-{
-    int kerr = 0;
-    MCK(cudaMemcpy(&kerr, c.kerr, sizeof(int), cudaMemcpyDeviceToHost));
-    if (kerr) {
-        cudaMemset(c.kerr, 0, sizeof(int));
-        set_error("%s: tensor-core product wait timed out", who);
         return 1;
     }
     return 0;
@@ -1454,7 +1457,7 @@ try {
         }
         if (!m.hst->any_flag) continue;
         // some active case reached its threshold (or the limit): FP64 true residuals
-        if (mr_true_residual(c, rr.data())) return PF_FAILURE;
+        if (mr_true_residual(c, "pf_solve_multi", rr.data())) return PF_FAILURE;
         int n_active = 0;
         for (int j = 0; j < k; ++j) {
             rel[j] = m.hst->ff[j] > 0 ? std::sqrt(rr[j]) / std::sqrt(m.hst->ff[j]) : 0.0;

@@ -21,7 +21,7 @@ bool g_capture = false;
 std::string g_log;
 struct Rule {
     std::string kernel;
-    int error, arg, value;
+    int error, arg, offset, value;
 };
 std::vector<Rule> g_rules;
 cudaError_t g_last = cudaSuccess;
@@ -52,7 +52,7 @@ cudaError_t launch(const void *fn, dim3 grid, void **args, bool cooperative)
             if (it != g_freed.begin() && q < std::prev(it)->first + std::prev(it)->second) ++g_stale;
         }
     for (const Rule &r : g_rules)
-        if (!r.error && name.find(r.kernel) != std::string::npos) **(int **)args[r.arg] = r.value;
+        if (!r.error && name.find(r.kernel) != std::string::npos) memcpy(*(char **)args[r.arg] + r.offset, &r.value, sizeof(int));
     g_log += (g_capture ? "captured " : "") + name + " " + std::to_string(grid.x) + "\n";
     return cudaSuccess;
 }
@@ -97,8 +97,9 @@ long long fake_used() { return g_used; }
 void fake_limit(long long bytes) { g_limit = bytes; }
 int fake_stale() { return g_stale; }
 void fake_coop_error(int e) { g_coop_error = e; }
-void fake_fail(const char *kernel, int e) { g_rules.push_back({kernel, e, 0, 0}); }
-void fake_poke(const char *kernel, int arg, int value) { g_rules.push_back({kernel, 0, arg, value}); }
+void fake_fail(const char *kernel, int e) { g_rules.push_back({kernel, e, 0, 0, 0}); }
+void fake_poke(const char *kernel, int arg, int offset, int value) { g_rules.push_back({kernel, 0, arg, offset, value}); }
+void fake_clear_rules() { g_rules.clear(); }
 
 // the runtime
 void **__cudaRegisterFatBinary(void *)

@@ -6,6 +6,7 @@ import ctypes
 import os
 import subprocess
 
+import numpy as np
 import pytest
 
 import parafem_gb300 as P
@@ -69,4 +70,33 @@ def test_a_full_device_leaves_no_launch_on_freed_records(fake, mode):
     s.solve(r, 1e-8, 3, mode)
     assert fake.fake_stale() == 0
     assert launched(fake, "k_pcg_resident") == 1
+    s.close()
+
+
+@pytest.mark.parametrize("mode", [P.MODE_P121, P.MODE_FP64_RES, P.MODE_MIXED, P.MODE_MIXED_RESTART, P.MODE_MIXED16])
+def test_a_wait_that_runs_out_in_the_final_residual_fails_that_solve(fake, mode):
+    """The products of the true residual wait for bulk copies; when one runs out they leave old results behind.  (Ten
+    iterations, all in the resident kernel: the only k_elem_fix of the call is the residual's.)"""
+    s, r = solver(3)
+    s.form_storkm(8)
+    fake.fake_poke(b"k_elem_fix", 6, 0, 2)
+    with pytest.raises(P.PfError, match="wait timed out"):
+        s.solve(r, 1e-8, 10, mode)
+    fake.fake_clear_rules()
+    s.solve(r, 1e-8, 10, mode)                 # reported once, not against a later call
+    s.close()
+
+
+def test_a_wait_that_runs_out_in_a_block_residual_fails_that_solve(fake):
+    s, r = solver(3)
+    s.form_storkm(8)
+    rk = np.repeat(r[:, None], 8, axis=1)
+    any_flag = 6 * 128 * 8 + 3 * 128 * 4       # of MState: every case wants a residual after the first update
+    fake.fake_poke(b"k_mr_update1", 2, any_flag, 1)
+    fake.fake_poke(b"k_mr_elem_fix", 6, 0, 2)
+    with pytest.raises(P.PfError, match="wait timed out"):
+        s.solve_multi(rk, 1e-8, 10, 32)
+    fake.fake_clear_rules()
+    fake.fake_poke(b"k_mr_update1", 2, any_flag, 1)
+    s.solve_multi(rk, 1e-8, 10, 32)
     s.close()
