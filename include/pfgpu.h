@@ -123,7 +123,10 @@ int pf_get_storkm(void **ctx, const int *first, const int *count, double *storkm
 int pf_get_diag(void **ctx, double *diag);
 
 /* One element-by-element product u = K p in equation order (GATHER,
- * element MATMUL, SCATTER of p121.f90:92-97).  prec 64: FP64 storkm;
+ * element MATMUL, SCATTER of p121.f90:92-97).  prec 64: FP64 storkm, every
+ * row to the accuracy of a sum of FP64 FMA (the solves' own FP64 products,
+ * in fixed point, keep it in the 2-norm of D^(-1/2) u, D the diagonal: an
+ * element's part of row i to 2^-47 sqrt(K_ii) max_j sqrt(K_jj) |p_j|);
  * 32: packed-symmetric FP32 storkm (used by PF_MODE_MIXED); 31: full FP32
  * storkm; 16: packed-symmetric FP16 storkm scaled per element (used by
  * PF_MODE_MIXED16).  The packed products are P K_e P p_e, P removing each

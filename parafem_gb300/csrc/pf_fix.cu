@@ -109,15 +109,18 @@ k_pack_storkm(int nels, const double *__restrict__ km, float *__restrict__ kp, u
 // 80^3 cube, 0.89 of the measured copy bandwidth; the FP64 FMA product of
 // the same mesh, k_elem<double>, is bound by the FP64 pipe and takes 3.35 ms
 // (40^3: 0.167 against 0.431 ms).  Error against extended precision on
-// distorted heterogeneous meshes: 0.2-0.4 of k_elem<double>'s for dense p,
-// the same (one rounding) where p has single entries.  Loading the blocks
+// distorted heterogeneous meshes, 2-norm: 0.2-0.4 of k_elem<double>'s for
+// dense p, the same where p has single entries; single rows can be worse
+// (pf_fix.cuh, weak_rows).  Loading the blocks
 // straight into registers instead of through shared memory took 1.41 ms.
+// ROWS: with the rows that FMA holds better formed so from km (weak_rows).
 constexpr int kFixWarps = 14;
 constexpr size_t kFixSmem = (size_t)kFixWarps * (3 * fx::kChunk0 + 960 + 3 * 8);
 static_assert(kFixSmem <= 227 * 1024, "shared memory per CTA");
+template <bool ROWS>
 __global__ void __launch_bounds__(kFixWarps * 32, 1)
 k_elem_fix(int nels, const unsigned char *__restrict__ rec, const int *__restrict__ conn, const double *__restrict__ p,
-           double *__restrict__ ut, const PcgState *__restrict__ st, int *__restrict__ err)
+           double *__restrict__ ut, const PcgState *__restrict__ st, int *__restrict__ err, const double *__restrict__ km)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -155,9 +158,10 @@ k_elem_fix(int nels, const unsigned char *__restrict__ rec, const int *__restric
     bool ok = true;
     for (; k < nmine; ++k) {
         double na, nb, u0, u1;
+        bool weak0, weak1;
         fx::gather2<true>(nd, lane, p, na, nb);   // of the next element (of node 0 behind the last)
         nd = node(k + 2);
-        ok = fx::product(
+        ok = fx::product<ROWS>(
             lane, pa, pb, pq,
             [&](int c) -> const unsigned char * {
                 chunk = c;
@@ -170,8 +174,9 @@ k_elem_fix(int nels, const unsigned char *__restrict__ rec, const int *__restric
                     issue(c, k + 1);
                 }
             },
-            u0, u1);
+            u0, u1, weak0, weak1);
         if (!ok) break;
+        if (ROWS) fx::weak_rows(lane, pa, pb, km + (size_t)(first + k * kFixWarps) * 3600, weak0, weak1, u0, u1);
         if (lane < 30) reinterpret_cast<double2 *>(ut + (size_t)(first + k * kFixWarps) * 60)[lane] = make_double2(u0, u1);
         pa = na;
         pb = nb;
@@ -189,9 +194,10 @@ k_elem_fix(int nels, const unsigned char *__restrict__ rec, const int *__restric
 // that a record is read once for all of them and the products are bitwise
 // those of the single-case kernel.  Bound by instruction issue (1.8 ns per
 // element and case over the chip, against 6.3 ns by FP64 FMA).
+template <bool ROWS>
 __global__ void __launch_bounds__(kFixWarps * 32, 1)
 k_mr_elem_fix(int nels, int nk, const unsigned char *__restrict__ rec, const int *__restrict__ conn,
-              const double *__restrict__ P, double *__restrict__ ut, int *__restrict__ err)
+              const double *__restrict__ P, double *__restrict__ ut, int *__restrict__ err, const double *__restrict__ km)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -228,7 +234,8 @@ k_mr_elem_fix(int nels, int nk, const unsigned char *__restrict__ rec, const int
             const int jn = j + 1 < nk ? j + 1 : j;
             const double na = qa[jn], nb = qb[jn];   // of the next case
             double u0, u1;
-            ok = fx::product(
+            bool weak0, weak1;
+            ok = fx::product<ROWS>(
                 lane, pa, pb, pq,
                 [&](int c) -> const unsigned char * {
                     if (j > 0) return stage + c * fx::kChunk0;
@@ -243,8 +250,9 @@ k_mr_elem_fix(int nels, int nk, const unsigned char *__restrict__ rec, const int
                         issue(c, e + kFixWarps);
                     }
                 },
-                u0, u1);
+                u0, u1, weak0, weak1);
             if (!ok) break;
+            if (ROWS) fx::weak_rows(lane, pa, pb, km + (size_t)e * 3600, weak0, weak1, u0, u1);
             if (lane < 30) {
                 o[j] = u0;
                 o[nk + j] = u1;
@@ -264,9 +272,11 @@ k_mr_elem_fix(int nels, int nk, const unsigned char *__restrict__ rec, const int
 // memory; bitwise the products of k_elem_fix on copies of it.  Bound by
 // instruction issue: 0.93 ms on an 80^3 cube, k_elem_shared64 3.29 ms.
 constexpr int kSharedFixWarps = 8;
+template <bool ROWS>
 __global__ void __launch_bounds__(kSharedFixWarps * 32, 2)
 k_elem_shared_fix(int nels, const unsigned char *__restrict__ rec, const int *__restrict__ conn,
-                  const double *__restrict__ p, double *__restrict__ ut, const PcgState *__restrict__ st)
+                  const double *__restrict__ p, double *__restrict__ ut, const PcgState *__restrict__ st,
+                  const double *__restrict__ km)
 {
     __shared__ int4 pq[kSharedFixWarps][60];
     __shared__ __align__(16) unsigned char r[fx::kRecBytes];
@@ -284,10 +294,13 @@ k_elem_shared_fix(int nels, const unsigned char *__restrict__ rec, const int *__
     nd = node(e + stride);
     for (; e < nels; e += stride) {
         double na, nb, u0, u1;
+        bool weak0, weak1;
         fx::gather2<true>(nd, lane, p, na, nb);
         nd = node(e + 2 * stride);
-        fx::product(
-            lane, pa, pb, pq[w], [&](int c) -> const unsigned char * { return r + fx::chunk_off(c); }, [](int) {}, u0, u1);
+        fx::product<ROWS>(
+            lane, pa, pb, pq[w], [&](int c) -> const unsigned char * { return r + fx::chunk_off(c); }, [](int) {}, u0, u1,
+            weak0, weak1);
+        if (ROWS) fx::weak_rows(lane, pa, pb, km, weak0, weak1, u0, u1);
         if (lane < 30) reinterpret_cast<double2 *>(ut + (size_t)e * 60)[lane] = make_double2(u0, u1);
         pa = na;
         pb = nb;
@@ -317,9 +330,11 @@ int launch_pack_storkm(Ctx &c, int nels, const double *km, float *kp, unsigned c
 static int fix_attributes(Ctx &c)
 {
     if (c.fix_attr) return 0;
-    cudaError_t e = cudaFuncSetAttribute(k_elem_fix, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFixSmem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_mr_elem_fix, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFixSmem);
+    const void *fn[] = {(const void *)k_elem_fix<false>, (const void *)k_elem_fix<true>, (const void *)k_mr_elem_fix<false>,
+                        (const void *)k_mr_elem_fix<true>};
+    cudaError_t e = cudaSuccess;
+    for (const void *f : fn)
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFixSmem);
     if (e != cudaSuccess) {
         set_error("fixed-point products: cannot reserve %zu bytes of shared memory: %s", kFixSmem, cudaGetErrorString(e));
         return 1;
@@ -328,30 +343,33 @@ static int fix_attributes(Ctx &c)
     return 0;
 }
 
-int launch_elem_fix(Ctx &c, const double *p, const PcgState *st)
+int launch_elem_fix(Ctx &c, const double *p, const PcgState *st, bool rows)
 {
     if (fix_attributes(c)) return 1;
     // one CTA per SM, and on small meshes as few warps per SM as the mesh has
     const int grid = c.nels < c.nsm ? c.nels : c.nsm;
-    launch_dependent(c.dependent && st, c.stream, grid, kFixWarps * 32, kFixSmem, k_elem_fix, c.nels, c.kmfix, c.conn, p,
-                     (double *)c.utemp, st, c.kerr);
+    launch_dependent(c.dependent && st, c.stream, grid, kFixWarps * 32, kFixSmem,
+                     rows ? k_elem_fix<true> : k_elem_fix<false>, c.nels, c.kmfix, c.conn, p, (double *)c.utemp, st, c.kerr,
+                     c.km64);
     return fix_launched(c, "k_elem_fix");
 }
 
-int launch_mr_elem_fix(Ctx &c, int k, const double *P, double *ut)
+int launch_mr_elem_fix(Ctx &c, int k, const double *P, double *ut, bool rows)
 {
     if (fix_attributes(c)) return 1;
     const int grid = c.nels < c.nsm ? c.nels : c.nsm;
-    k_mr_elem_fix<<<grid, kFixWarps * 32, kFixSmem, c.stream>>>(c.nels, k, c.kmfix, c.conn, P, ut, c.kerr);
+    auto kernel = rows ? k_mr_elem_fix<true> : k_mr_elem_fix<false>;
+    kernel<<<grid, kFixWarps * 32, kFixSmem, c.stream>>>(c.nels, k, c.kmfix, c.conn, P, ut, c.kerr, c.km64);
     return fix_launched(c, "k_mr_elem_fix");
 }
 
-int launch_elem_shared_fix(Ctx &c, const double *p, const PcgState *st)
+int launch_elem_shared_fix(Ctx &c, const double *p, const PcgState *st, bool rows)
 {
     const int nb = (c.nels + kSharedFixWarps - 1) / kSharedFixWarps;
     const int grid = nb < c.nsm * 2 ? nb : c.nsm * 2;
-    launch_dependent(c.dependent && st, c.stream, grid, kSharedFixWarps * 32, 0, k_elem_shared_fix, c.nels, c.skmfix, c.conn, p,
-                     (double *)c.utemp, st);
+    launch_dependent(c.dependent && st, c.stream, grid, kSharedFixWarps * 32, 0,
+                     rows ? k_elem_shared_fix<true> : k_elem_shared_fix<false>, c.nels, c.skmfix, c.conn, p, (double *)c.utemp, st,
+                     c.skm64);
     return fix_launched(c, "k_elem_shared_fix");
 }
 

@@ -10,11 +10,20 @@
 // split into a high word and a signed 29-bit low word; three of the four
 // cross products are summed EXACTLY (no carry can leave 63 bits:
 // 60 x 2^28 x 2^28 and 60 x 2 x 2^56), so a result does not depend on the
-// order of its terms and is rounded once, when it becomes FP64 again.  The
-// parts dropped -- bits of K' and p' below 2^-57 and the product of the two
-// low words -- are about 2^-56 of the row's largest term, where a sum of 60
-// FP64 FMA loses about 2^-53.  The exponents s_i per row keep that true for
-// thin and distorted elements, whose rows differ in size.
+// order of its terms and is rounded once, when it becomes FP64 again.
+//
+// Dropped are bits of K' and p' below 2^-57 and the product of the two low
+// words: per row at most 60 x 3 x 2^-58 in the scaled units, that is
+//     |error of u_i| <= 2^-47 sqrt(K_ii) max_j sqrt(K_jj) |p_j|,
+// a bound by the element's largest scaled value, not by the row's own terms.
+// In the 2-norm of D^(-1/2) u (D the diagonal) the error is a fifth to two
+// fifths of that of 60 FP64 FMA, also in thin and distorted elements, whose
+// rows differ in size; that is the norm in which a Jacobi-scaled PCG sees
+// it, so the solves and their true residuals take this product.  A row
+// whose terms K_ij p_j are all small beside the element's largest scaled
+// value has fewer correct bits than by FMA, none at 2^-57 of it; the
+// products that a caller asks for (pf_ebe_matvec) form such rows again by
+// FMA (weak_rows).
 #pragma once
 #include "pf_device.cuh"
 
@@ -104,7 +113,7 @@ __host__ __device__ __forceinline__ int fix_scale(long long kbits)
     return -((e + 4096 + 1) / 2 - 2048);   // -ceil(e / 2)
 }
 
-// one instruction (from C the compiler forms the product and adds it: three)
+// (long long)a * b + c (written so in C: 1.61 instead of 1.41 ms of an 80^3 product)
 __device__ __forceinline__ long long madw(int a, int b, long long c)
 {
     long long d;
@@ -137,6 +146,23 @@ __device__ __forceinline__ void block_bwd(Sums &s, const int4 a, const int4 b, c
 {
     block_fwd(s, make_int4(a.x, a.y, b.x, b.y), make_int4(a.z, a.w, b.z, b.w), q);
 }
+
+// The largest |K'(i,j) p'(j)| of two rows in 28 + extra fractional bits, from
+// the high words, for weak_rows
+struct Largest {
+    unsigned a = 0, b = 0;
+};
+__device__ __forceinline__ void larger_fwd(Largest &s, const int4 a, const int4 b, const int4 q)
+{
+    const unsigned q0 = (unsigned)abs(q.x) << 3, q1 = (unsigned)abs(q.z) << 3;
+    s.a = max(s.a, max(__umulhi((unsigned)abs(a.x) << 1, q0), __umulhi((unsigned)abs(a.z) << 1, q1)));
+    s.b = max(s.b, max(__umulhi((unsigned)abs(b.x) << 1, q0), __umulhi((unsigned)abs(b.z) << 1, q1)));
+}
+__device__ __forceinline__ void larger_bwd(Largest &s, const int4 a, const int4 b, const int4 q)
+{
+    larger_fwd(s, make_int4(a.x, a.y, b.x, b.y), make_int4(a.z, a.w, b.z, b.w), q);
+}
+constexpr int kWeakBits = 5;   // a row whose terms are all below 2^-5 of the scaled units is a weak one
 
 __device__ __forceinline__ Sums shift_from(const Sums &s, int src)
 {
@@ -188,9 +214,10 @@ __device__ __forceinline__ double fix_result(long long h, long long m, int kmax,
 // shared memory per warp, the words of p twice over so that l + s needs no
 // wrap.  Chunk c of the record is read between enter(c), which returns its
 // address or null to give up (product() then returns false), and leave(c).
-template <typename Enter, typename Leave>
+// ROWS: weak0 and weak1 say which of the two rows weak_rows has to form.
+template <bool ROWS, typename Enter, typename Leave>
 __device__ __forceinline__ bool product(int lane, double pa, double pb, int4 *__restrict__ pq, Enter enter, Leave leave,
-                                        double &u0, double &u1)
+                                        double &u0, double &u1, bool &weak0, bool &weak1)
 {
     const int l = lane < 30 ? lane : 29, prev = lane == 0 ? 29 : l - 1;
     const unsigned char *r = enter(0);
@@ -209,10 +236,12 @@ __device__ __forceinline__ bool product(int lane, double pa, double pb, int4 *__
     }
     __syncwarp();
     Sums f, t;
+    Largest lf, lt;
     {
         const int4 k0 = *reinterpret_cast<const int4 *>(r + kOff0 + 16 * l);
         const int2 k11 = *reinterpret_cast<const int2 *>(r + kOff11 + 8 * l);
         block_fwd(f, k0, make_int4(k0.z, k0.w, k11.x, k11.y), own);
+        if constexpr (ROWS) larger_fwd(lf, k0, make_int4(k0.z, k0.w, k11.x, k11.y), own);
     }
     {
         const int l15 = l < 15 ? l : 14;
@@ -221,6 +250,10 @@ __device__ __forceinline__ bool product(int lane, double pa, double pb, int4 *__
         if (l >= 15) a = b = make_int4(0, 0, 0, 0);
         block_fwd(f, a, b, pq[l + 15]);
         block_bwd(t, a, b, own);
+        if constexpr (ROWS) {
+            larger_fwd(lf, a, b, pq[l + 15]);
+            larger_bwd(lt, a, b, own);
+        }
     }
     const int4 *pl = pq + l;
     auto diagonal = [&](const unsigned char *rl, int s) {   // rl: the chunk, at this lane's 16 bytes
@@ -229,6 +262,12 @@ __device__ __forceinline__ bool product(int lane, double pa, double pb, int4 *__
         t = shift_from(t, prev);
         block_fwd(f, a, b, pl[s]);
         block_bwd(t, a, b, own);
+        if constexpr (ROWS) {
+            lt.a = __shfl_sync(FULLMASK, lt.a, prev);
+            lt.b = __shfl_sync(FULLMASK, lt.b, prev);
+            larger_fwd(lf, a, b, pl[s]);
+            larger_bwd(lt, a, b, own);
+        }
     };
     r += 16 * l;
 #pragma unroll
@@ -249,7 +288,47 @@ __device__ __forceinline__ bool product(int lane, double pa, double pb, int4 *__
     u0 = fix_result(f.h0 + t.h0, f.m0 + t.m0, kmax - extra, ex.x);
     u1 = fix_result(f.h1 + t.h1, f.m1 + t.m1, kmax - extra, ex.y);
     if (!finite) u0 = u1 = __longlong_as_double(0x7ff8000000000000LL);
+    if constexpr (ROWS) {
+        const unsigned bound = 1u << (28 + extra - kWeakBits);
+        const bool any = kmax != kNoKey;   // p_e = 0: so is the product
+        weak0 = !finite || (max(lf.a, __shfl_sync(FULLMASK, lt.a, prev)) < bound && any);
+        weak1 = !finite || (max(lf.b, __shfl_sync(FULLMASK, lt.b, prev)) < bound && any);
+    }
     return true;
+}
+template <typename Enter, typename Leave>
+__device__ __forceinline__ bool product(int lane, double pa, double pb, int4 *__restrict__ pq, Enter enter, Leave leave,
+                                        double &u0, double &u1)
+{
+    bool weak0, weak1;
+    return product<false>(lane, pa, pb, pq, enter, leave, u0, u1, weak0, weak1);
+}
+
+// The weak rows of an element by FMA, in k_elem's order, from its matrix ke.
+// Largest error of a row over the sum of its |K_ij p_j|, and the 2-norm of
+// all errors over 2^-53 that of the sums, 40 bricks of 100 x 1 x 0.02:
+//                             fixed point      FMA            with this
+//   normal p                  2^-52.6  0.27    2^-51.3  0.59  2^-52.6  0.27
+//   one p = 1, rest 1e-9      2^-34.7  0.53    2^-50.1  1.94  2^-50.1  0.44
+//   p over 20 decades         2^-43.3  0.46    2^-50.5  0.84  2^-50.5  0.45
+__device__ __forceinline__ void weak_rows(int lane, double pa, double pb, const double *__restrict__ ke, bool weak0, bool weak1,
+                                          double &u0, double &u1)
+{
+    if (!__any_sync(FULLMASK, weak0 || weak1)) return;
+    const double *kr = ke + 2 * (lane < 30 ? lane : 29);
+    double a0 = 0.0, a1 = 0.0;
+#pragma unroll 6
+    for (int j = 0; j < 60; j += 2) {
+        const double p0 = __shfl_sync(FULLMASK, pa, j >> 1), p1 = __shfl_sync(FULLMASK, pb, j >> 1);
+        const double2 k0 = __ldg(reinterpret_cast<const double2 *>(kr + 60 * j));
+        const double2 k1 = __ldg(reinterpret_cast<const double2 *>(kr + 60 * j + 60));
+        a0 = fma(k0.x, p0, a0);
+        a1 = fma(k0.y, p0, a1);
+        a0 = fma(k1.x, p1, a0);
+        a1 = fma(k1.y, p1, a1);
+    }
+    if (weak0) u0 = a0;
+    if (weak1) u1 = a1;
 }
 
 // Lane l's part of the connectivity is node l; p at its two freedoms.  NC: p

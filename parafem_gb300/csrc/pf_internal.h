@@ -199,9 +199,10 @@ int ctx_malloc(Ctx &c, void **p, size_t bytes);
 int ensure_km32(Ctx &c);   // the full FP32 storkm, if storkm changed; outside stream capture
 // pf_fix.cu: the packed forms of nels FP64 element matrices (kp or rec may be null), FP64 products from the records
 int launch_pack_storkm(Ctx &c, int nels, const double *km, float *kp, unsigned char *rec, int *bad);
-int launch_elem_fix(Ctx &c, const double *p, const PcgState *st);
-int launch_elem_shared_fix(Ctx &c, const double *p, const PcgState *st);
-int launch_mr_elem_fix(Ctx &c, int k, const double *P, double *ut);   // k cases, P[slot * k + j] -> ut[(60 e + i) * k + j]
+// (rows: with every row to the accuracy of FMA)
+int launch_elem_fix(Ctx &c, const double *p, const PcgState *st, bool rows);
+int launch_elem_shared_fix(Ctx &c, const double *p, const PcgState *st, bool rows);
+int launch_mr_elem_fix(Ctx &c, int k, const double *P, double *ut, bool rows);   // k cases, P[slot * k + j] -> ut[(60 e + i) * k + j]
 int launch_assemble_diag(Ctx &c);
 int launch_eq_to_slot(Ctx &c, const double *eq, double *slot);
 int launch_slot_to_eq(Ctx &c, const double *slot, double *eq);
@@ -257,7 +258,7 @@ int launch_elem_sym32_mapped(cudaStream_t stream, int nsm, int n, const float *k
                              float *ut, int *err, const int *emap);
 int launch_pack_sym32_raw(cudaStream_t stream, int nsm, int nels, const double *km, float *kp);
 int autotune_sym32(Ctx &c, const double *p);   // picks c.sym_cfg by timing on this mesh
-int launch_elem_shared(Ctx &c, int prec, const double *p, const PcgState *st);   // shared km
+int launch_elem_shared(Ctx &c, int prec, const double *p, const PcgState *st, bool rows = false);   // shared km
 // 8-node scalar (p123) kernels; km64 holds storkc(8,8,e) in such a context
 int launch_form_storkc(Ctx &c, int nip, double kx, double ky, double kz);
 int launch_elem8(Ctx &c, const double *p, const PcgState *st);

@@ -935,14 +935,14 @@ int launch_slot_to_eq(Ctx &c, const double *slot, double *eq)
 // 20-node elements are formed in fixed point where the mesh has records
 // (c.kmfix), and by FP64 FMA where storkm is not symmetric or the records
 // found no memory.
-static int launch_products(Ctx &c, int prec, const double *p, const PcgState *st, double *share = nullptr)
+static int launch_products(Ctx &c, int prec, const double *p, const PcgState *st, double *share = nullptr, bool rows = false)
 {
     if (c.kind == KIND_SCALAR8) return launch_elem8(c, p, st);
     if (c.kind == KIND_SOLID8) return launch_elem24(c, p, st);
-    if (c.shared) return launch_elem_shared(c, prec, p, st);
+    if (c.shared) return launch_elem_shared(c, prec, p, st, rows);
     if (prec == PREC_FP32_SYM) return launch_elem_sym32(c, p, st, share);
     if (prec == PREC_FP16_SYM) return launch_elem_sym16(c, p, st);
-    if (prec == PREC_FP64 && c.kmfix) return launch_elem_fix(c, p, st);
+    if (prec == PREC_FP64 && c.kmfix) return launch_elem_fix(c, p, st, rows);
     const int grid = grid_for(c, c.nels, 8, 8);
     if (prec == PREC_FP32_FULL)
         launch_dependent(c.dependent && st, c.stream, grid, 256, 0, k_elem<float, true>, c.nels, c.km32, c.conn, p, (float *)c.utemp,
@@ -988,10 +988,11 @@ int launch_scatter(Ctx &c, int prec, int mode, const double *pf, double *out)
     return check_launch(c, "k_scatter");
 }
 
-// u = K p outside a PCG run (state-independent).
+// u = K p outside a PCG run (state-independent), for the caller: every FP64
+// row is as accurate as by FMA.
 int launch_matvec(Ctx &c, int prec, const double *p, double *u)
 {
-    if (launch_products(c, prec, p, nullptr)) return 1;
+    if (launch_products(c, prec, p, nullptr, nullptr, true)) return 1;
     if (c.kind == KIND_SCALAR8) return launch_scatter1(c, 0, p, p, u, nullptr);
     if (c.kind == KIND_SOLID8) return launch_scatter3_fixed(c, p, u, nullptr);
     if (prec != PREC_FP64)

@@ -1202,8 +1202,9 @@ static int mr_tc_product(Ctx &c, int w, const int *skip)
 
 // U = K P for the block (prec 16: tensor cores, on P's split copy m.Ps, which
 // must hold P; 32: CUDA-core FP32, 64: FP64 into ut64).  skip: device flag
-// that turns the launch into a no-op.
-static int mr_elem(Ctx &c, int prec, const double *P, const int *skip)
+// that turns the launch into a no-op.  rows: every FP64 row to the accuracy
+// of FMA, for the caller's products.
+static int mr_elem(Ctx &c, int prec, const double *P, const int *skip, bool rows = false)
 {
     MultiBufs &m = *c.multi;
     if (prec == 16) return mr_tc_product(c, m.kb, skip);
@@ -1212,7 +1213,7 @@ static int mr_elem(Ctx &c, int prec, const double *P, const int *skip)
         k_mr_elem_cc<float, float><<<grid, 256, 0, c.stream>>>(c.nels, m.k, c.km32, c.conn, P, m.ut32, skip);
         return mr_launched(c, "k_mr_elem_cc<float>");
     }
-    if (c.kmfix) return launch_mr_elem_fix(c, m.k, P, m.ut64);   // outside the iterations: no flag
+    if (c.kmfix) return launch_mr_elem_fix(c, m.k, P, m.ut64, rows);   // outside the iterations: no flag
     k_mr_elem_cc<double, double><<<grid, 256, 0, c.stream>>>(c.nels, m.k, c.km64, c.conn, P, m.ut64, skip);
     return mr_launched(c, "k_mr_elem_cc<double>");
 }
@@ -1533,7 +1534,7 @@ try {
         if (mr_launched(c, "k_mr_psplit")) return PF_FAILURE;
         if (mr_prepare_tc(c)) return PF_FAILURE;
     }
-    if (mr_elem(c, *prec, m.P, nullptr)) return PF_FAILURE;
+    if (mr_elem(c, *prec, m.P, nullptr, true)) return PF_FAILURE;
     if (mr_scatter(c, *prec, 0, m.P, m.U, nullptr)) return PF_FAILURE;
     k_mr_slot_to_eq<<<c.nsm * 8, 256, 0, c.stream>>>(c.neq, k, c.eq_slot, m.U, m.eq);
     if (mr_launched(c, "k_mr_slot_to_eq")) return PF_FAILURE;

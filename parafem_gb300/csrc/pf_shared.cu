@@ -424,10 +424,10 @@ __global__ void k_split_p(int ns, const double *__restrict__ p, float2 *__restri
     }
 }
 
-int launch_elem_shared(Ctx &c, int prec, const double *p, const PcgState *st)
+int launch_elem_shared(Ctx &c, int prec, const double *p, const PcgState *st, bool rows)
 {
     cudaError_t e;
-    if (prec == PREC_FP64 && c.skmfix) return launch_elem_shared_fix(c, p, st);
+    if (prec == PREC_FP64 && c.skmfix) return launch_elem_shared_fix(c, p, st, rows);
     if (prec == PREC_FP64) {   // km not symmetric
         long long g = ((long long)c.nels + 7) / 8;
         if (g > (long long)c.nsm * 8) g = (long long)c.nsm * 8;

@@ -183,3 +183,65 @@ def test_non_finite_values_stay_non_finite():
             u = s.ebe_matvec(p, 64)
             assert not np.isfinite(u[neq // 2])
         assert not s.ebe_matvec(np.zeros(neq), 64).any()
+
+
+def wide_fields(neq, rng):
+    """Values of very different size inside an element: most rows' terms are small beside the element's largest."""
+    one = np.zeros(neq)
+    one[neq // 2] = 1.0
+    return {"one": one, "one over noise": np.where(one > 0, 1.0, 1e-9 * rng.standard_normal(neq)),
+            "few": np.where(rng.random(neq) < 0.03, rng.standard_normal(neq), 0.0),
+            "20 decades": rng.standard_normal(neq) * 10.0 ** (-20.0 * rng.random(neq))}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,amp,size", SHAPES)
+@pytest.mark.parametrize("how", ["storkm", "one matrix", "cases"])
+def test_every_row_is_as_accurate_as_by_fma(shape, amp, size, how):
+    """In fixed point a row is off by 180 x 2^-58 of the scaled units (test_products_against_extended_precision), and
+    only rows with a term of 2^-5 or more are left so: 2^-45.5 of the sum of their |K_ij p_j|, or twice that, since
+    terms are compared by their high words.  The others are off by what 60 FP64 FMA leave, 2^-47, and the sums over
+    the elements by 2^-49 of it: below 2^-43."""
+    g_num, g_coord, nn, g_g, neq = mesh(*shape, 0.0 if how == "one matrix" else amp, size)
+    nels = g_num.shape[0]
+    fields = wide_fields(neq, np.random.default_rng(12))
+    with P.Solver() as s:
+        s.setup(g_num, g_g, g_coord, nn, neq)
+        if how == "one matrix":
+            s.set_material(100.0, 0.3)
+            one = s.form_km(1, 27)
+            s.set_shared_km(one)
+            km = np.repeat(np.asarray(one).reshape(1, 60, 60), nels, axis=0)
+        else:
+            s.set_material(*P.random_material(nels, 3, 1.0, 1000.0, 0.2, 0.35))
+            s.form_storkm(27)
+            km = s.get_storkm()
+        if how == "cases":
+            u = s.ebe_matvec_multi(np.stack(2 * list(fields.values()), axis=1), 64)
+            us = [u[:, j] for j in range(len(fields))]
+        else:
+            us = [s.ebe_matvec(p, 64) for p in fields.values()]
+    for p, u in zip(fields.values(), us):
+        ref, mag, _ = reference(km, g_g, p)
+        assert np.all(np.abs(u - ref) <= 2.0 ** -43 * mag)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+def test_infinities_and_nan_reach_the_rows_that_they_reach_by_fma(bad):
+    g_num, g_coord, nn, g_g, neq = mesh(3, 2, 3, 0.08)
+    rng = np.random.default_rng(3)
+    p = rng.standard_normal(neq)
+    p[neq // 2] = bad
+    with P.Solver() as s:
+        s.setup(g_num, g_g, g_coord, nn, neq)
+        s.set_material(100.0, 0.3)
+        s.form_storkm(27)
+        km = s.get_storkm()
+        u = s.ebe_matvec(p, 64)
+        uk = s.ebe_matvec_multi(np.repeat(p[:, None], 8, axis=1), 64)[:, 5]
+    with np.errstate(invalid="ignore"):
+        ref = reference(km, g_g, p)[0]
+    for got in (u, uk):
+        assert np.array_equal(np.isnan(got), np.isnan(ref)) and np.array_equal(np.isfinite(got), np.isfinite(ref))
+        assert np.array_equal(np.sign(got[np.isinf(ref)]), np.sign(ref[np.isinf(ref)]))
