@@ -132,6 +132,7 @@ struct Ctx {
     void *row_idx = nullptr;        // 16-bit offsets from row_base, or 32-bit columns (row_wide)
     int *row_base = nullptr;
     bool row_wide = false, row_keep = false;
+    bool row_skip = false;          // some rows are padded with -0.0, to be stepped over
     bool row_ring = false, row_attr = false;   // the rows fit k_row_ring's stages; its shared-memory attribute is set
     // one element matrix shared by every element (PCG_KM); per-element storkm unused
     bool shared = false;

@@ -129,10 +129,15 @@ k_scatter1(int nn, const int *__restrict__ ptr, const int *__restrict__ list, co
 
 // ---------------------------------------------------------------------------
 // Assembled rows, in slices of 32 consecutive nodes: entry k of the rows of
-// slice s lies at off[s] + 32 k + lane, columns ascending, short rows padded
-// with zeros.  Column numbers are 16-bit offsets from the least column of
-// (slice, k) where every one fits (neighbouring nodes have neighbouring
-// columns), 32-bit numbers otherwise.
+// slice s lies at off[s] + 32 k + lane, columns ascending.  Column numbers are
+// 16-bit offsets from the least column of (slice, k) where every one fits
+// (neighbouring nodes have neighbouring columns), 32-bit numbers otherwise.
+// Short rows are padded with 0 at a column of their own: at another node's,
+// 0 x Inf or 0 x NaN would carry that node's value into a row that is not its
+// neighbour.  Where no column of its own lies within 16 bits (the last layer
+// of a mesh with more than 65,535 nodes per layer) the row is padded with
+// -0.0, which no sum that starts from 0 is, and the products step over it
+// (SKIP; in all meshes that test would cost 1.5 % of an iteration).
 constexpr int kRowMax = 64;   // entries of a row (a structured brick mesh has 27)
 
 // the ascending distinct columns of node n: their number, -1 when too many
@@ -171,7 +176,14 @@ k_rows_width(int nn, const int *__restrict__ ptr, const int *__restrict__ list, 
     }
 }
 
-// Values summed in ascending element order; *bad: a 16-bit offset overflows.
+template <bool SKIP>
+__device__ __forceinline__ double row_step(double k, double x, double a)
+{
+    return SKIP && __double_as_longlong(k) == (long long)0x8000000000000000ULL ? a : fma(k, x, a);
+}
+
+// Values summed in ascending element order; *bad, bit 0: a 16-bit offset
+// overflows, bit 1: rows padded with -0.0.
 template <typename IT>
 __global__ void __launch_bounds__(128)
 k_rows_fill(int nn, const int *__restrict__ ptr, const int *__restrict__ list, const int *__restrict__ conn,
@@ -201,10 +213,21 @@ k_rows_fill(int nn, const int *__restrict__ ptr, const int *__restrict__ list, c
         const long long o = off[s];
         const int w = (int)((off[s + 1] - o) >> 5);
         for (int k = 0; k < w; ++k) {
-            const int least = __reduce_min_sync(FULLMASK, k < cnt ? cols[k] : 0x7fffffff);
-            const int c = k < cnt ? cols[k] : least;
-            if (sizeof(IT) == 2 && c - least > 0xffff) atomicOr(bad, 1);
-            val[o + 32 * k + lane] = k < cnt ? v[k] : 0.0;
+            const int first = __reduce_min_sync(FULLMASK, k < cnt ? cols[k] : 0x7fffffff);
+            int c = k < cnt ? cols[k] : first;   // (a row without columns is no freedom's)
+            if (k >= cnt && cnt > 0)             // its least column from `first` on, or its last
+                for (int m = cnt - 1; m >= 0 && (m == cnt - 1 || cols[m] >= first); --m) c = cols[m];
+            int least = __reduce_min_sync(FULLMASK, c);
+            double pad = 0.0;
+            if (sizeof(IT) == 2 && __any_sync(FULLMASK, c - least > 0xffff)) {
+                least = first;
+                if (k >= cnt) {
+                    c = first;
+                    pad = -0.0;
+                }
+                atomicOr(bad, c - least > 0xffff ? 1 : 2);
+            }
+            val[o + 32 * k + lane] = k < cnt ? v[k] : pad;
             idx[o + 32 * k + lane] = (IT)(sizeof(IT) == 2 ? c - least : c);
             if (lane == 0) base[(o >> 5) + k] = least;
         }
@@ -220,7 +243,7 @@ k_rows_fill(int nn, const int *__restrict__ ptr, const int *__restrict__ list, c
 // those of a mesh that fits stay in L2 from one product to the next; else they
 // leave L2 first (100^3: 98 us kept, 90 us not).
 constexpr size_t kRowKeepBytes = 64u << 20;
-template <int MODE, typename IT, bool KEEP>
+template <int MODE, typename IT, bool KEEP, bool SKIP>
 __global__ void __launch_bounds__(256)
 k_row_product(int nn, const long long *__restrict__ off, const double *__restrict__ val, const IT *__restrict__ idx,
               const int *__restrict__ base, const uint8_t *__restrict__ fm, const double *__restrict__ fstore,
@@ -242,7 +265,7 @@ k_row_product(int nn, const long long *__restrict__ off, const double *__restric
         for (int k = 0; k < w; ++k) {
             const int i = (int)(KEEP ? __ldg(ix + 32 * k) : __ldcs(ix + 32 * k));
             const int c = sizeof(IT) == 2 ? __ldg(b + k) + i : i;
-            a = fma(KEEP ? __ldg(v + 32 * k) : __ldcs(v + 32 * k), __ldg(xin + c), a);
+            a = row_step<SKIP>(KEEP ? __ldg(v + 32 * k) : __ldcs(v + 32 * k), __ldg(xin + c), a);
         }
         const bool fr = fm[n] & 1;
         const double fs = fstore[n];
@@ -276,6 +299,7 @@ constexpr int kRingWarps = 20, kRingWidth = 28;                  // widest slice
 constexpr int kRingIdx = kRingWidth * 32 * 8, kRingStage = kRingWidth * 32 * 10;
 constexpr int kRingSmem = kRingWarps * (kRingStage + 8);
 static_assert(kRingSmem + 64 <= 227 * 1024, "shared memory per CTA");
+template <bool SKIP>
 __global__ void __launch_bounds__(kRingWarps * 32, 1)
 k_row_ring(int nn, const long long *__restrict__ off, const double *__restrict__ val, const uint16_t *__restrict__ idx,
            const int *__restrict__ base, const uint8_t *__restrict__ fm, const double *__restrict__ fstore,
@@ -329,7 +353,7 @@ k_row_ring(int nn, const long long *__restrict__ off, const double *__restrict__
         if (!ok || stopped) break;
         double a = 0.0;
 #pragma unroll 9
-        for (int k = 0; k < n; ++k) a = fma(sv[32 * k], __ldg(xin + __shfl_sync(FULLMASK, b, k) + si[32 * k]), a);
+        for (int k = 0; k < n; ++k) a = row_step<SKIP>(sv[32 * k], __ldg(xin + __shfl_sync(FULLMASK, b, k) + si[32 * k]), a);
         __syncwarp();   // every lane is done with the stage
         if (s + kRingWarps < s1) {
             o = off[s + kRingWarps];
@@ -497,7 +521,8 @@ int rows_assemble(Ctx &c)
             set_error("k_rows_fill: %s", cudaGetErrorString(ef));
             return 1;
         }
-        if (!bad) {
+        if (!(bad & 1)) {
+            c.row_skip = bad != 0;
             c.row_ring = bytes == 2 && *w.first > 0 && *w.second <= kRingWidth;
             break;
         }
@@ -511,7 +536,9 @@ static int launch_row_product(Ctx &c, int mode, const double *xin, const double 
 {
     if (mode == 0 && c.row_ring) {
         if (!c.row_attr) {   // by the first product, outside any stream capture
-            const cudaError_t e = cudaFuncSetAttribute(k_row_ring, cudaFuncAttributeMaxDynamicSharedMemorySize, kRingSmem);
+            cudaError_t e = cudaFuncSetAttribute(k_row_ring<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRingSmem);
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(k_row_ring<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRingSmem);
             if (e != cudaSuccess) {
                 set_error("k_row_ring: cannot reserve %d bytes of shared memory: %s", kRingSmem, cudaGetErrorString(e));
                 return 1;
@@ -519,8 +546,9 @@ static int launch_row_product(Ctx &c, int mode, const double *xin, const double 
             c.row_attr = true;
         }
         const int grid = c.Gs < c.nsm ? c.Gs : c.nsm;   // c.part_s holds c.Gs shares
-        launch_dependent(c.dependent && st, c.stream, grid, kRingWarps * 32, kRingSmem, k_row_ring, c.nn, c.row_off, c.row_val,
-                         (const uint16_t *)c.row_idx, c.row_base, c.freemask, c.fstore, xin, out, c.part_s, st, c.count,
+        launch_dependent(c.dependent && st, c.stream, grid, kRingWarps * 32, kRingSmem,
+                         c.row_skip ? k_row_ring<true> : k_row_ring<false>, c.nn, c.row_off, c.row_val, (const uint16_t *)c.row_idx,
+                         c.row_base, c.freemask, c.fstore, xin, out, c.part_s, st, c.count,
                          c.row_keep ? 1 : 0, c.kerr);
         return launched8(c, "k_row_ring");
     }
@@ -530,9 +558,10 @@ static int launch_row_product(Ctx &c, int mode, const double *xin, const double 
     };
     const int *wide = (const int *)c.row_idx;
     const uint16_t *narrow = (const uint16_t *)c.row_idx;
-    if (c.row_wide) go(wide, k_row_product<0, int, false>, k_row_product<1, int, false>);
-    else if (c.row_keep) go(narrow, k_row_product<0, uint16_t, true>, k_row_product<1, uint16_t, true>);
-    else go(narrow, k_row_product<0, uint16_t, false>, k_row_product<1, uint16_t, false>);
+    if (c.row_wide) go(wide, k_row_product<0, int, false, false>, k_row_product<1, int, false, false>);
+    else if (c.row_skip) go(narrow, k_row_product<0, uint16_t, false, true>, k_row_product<1, uint16_t, false, true>);
+    else if (c.row_keep) go(narrow, k_row_product<0, uint16_t, true, false>, k_row_product<1, uint16_t, true, false>);
+    else go(narrow, k_row_product<0, uint16_t, false, false>, k_row_product<1, uint16_t, false, false>);
     return launched8(c, "k_row_product");
 }
 

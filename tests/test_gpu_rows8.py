@@ -93,3 +93,28 @@ def test_rows_streamed_through_shared_memory(shape):
     """One slice of 32 rows, a ragged last one, fewer and more slices than warps, and iterations above and below
     30,000 slots."""
     check(*box(*shape, False))
+
+
+@pytest.mark.parametrize("shape,shuffle", [((5, 4, 3), False), ((11, 7, 9), True), ((33, 29, 40), False), ((41, 41, 41), True),
+                                           ((260, 256, 2), False), ((256, 2, 260), False), ((2, 260, 256), False)])
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_a_value_that_is_not_finite_reaches_its_neighbours_only(shape, shuffle, bad):
+    """Boundary rows are shorter than their slice, and padded.  In a layer of 67,077 nodes the last layer's rows have
+    no column within 16 bits of those of the layer before, with which they share a slice."""
+    g_num, coords = box(*shape, shuffle)
+    nn = coords.shape[0]
+    g_g, neq = P.number_equations1(g_num, np.ones(nn, np.int32))
+    g_coord = np.ascontiguousarray(coords[g_num - 1].transpose(0, 2, 1))
+    x = np.random.default_rng(6).standard_normal(neq)
+    with P.Solver() as s:
+        s.setup_scalar8(g_num, g_g, g_coord, nn, neq)
+        s.form_storkc(8, 2.0, 1.0, 3.0)
+        u = s.ebe_matvec(x, 64)
+        row = int(np.diff(np.unique(g_num[0]))[1]) + 1      # nodes from row to row: the last layer's slice-mates reach these
+        for q in [0, neq // 2] + [max(neq - 1 - i, 1) for i in list(range(9)) + list(range(max(row - 4, 0), row + 9))]:
+            xb = x.copy()
+            xb[q] = bad
+            ub = s.ebe_matvec(xb, 64)
+            near = np.unique(g_g[(g_g == q + 1).any(axis=1)]) - 1
+            far = np.setdiff1d(np.arange(neq), near)
+            assert not np.isfinite(ub[near]).any() and np.array_equal(ub[far], u[far])
