@@ -74,6 +74,13 @@ __device__ __forceinline__ bool exchange(unsigned long long *count, unsigned lon
     return false;
 }
 
+// ||r|| <= tol ||f|| as a bound for r.r: a negative tolerance is never met
+__device__ __forceinline__ double stop_square(double tol, double root_ff)
+{
+    const double b = tol * root_ff;
+    return tol >= 0.0 ? b * b : -1.0;
+}
+
 // One warp: the blocks' shares added (or their greatest bits), in every lane
 __device__ __forceinline__ double add_shares(const double *p, int nblk, int lane)
 {
@@ -120,7 +127,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(ResArgs a)
     const double ff = a.st->ff, tol = a.st->tol;
     int iters = a.st->iters;
     const int limit = a.st->limit;
-    const double root_ff = CHECON ? 0.0 : sqrt(ff), bound = tol * root_ff, stop_rr = bound * bound;
+    const double root_ff = CHECON ? 0.0 : sqrt(ff), stop_rr = stop_square(tol, root_ff);
     unsigned long long target = 0;   // arrivals that complete the next exchange
     double *p_pu = a.part, *p_rd = p_pu + kMaxBlocks, *p_2 = p_rd + kMaxBlocks, *p_3 = p_2 + kMaxBlocks;
 
@@ -665,7 +672,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_pcg_tail(TailArgs a)
             }
         }
     };
-    if (w == 1 && !CHECON && lane == 0) s_bound = tol * sqrt(a.st->ff);
+    if (w == 1 && !CHECON && lane == 0) s_bound = stop_square(tol, sqrt(a.st->ff));
     if (HOW == TAIL_GIVEN) {
         alpha = a.st->alpha;
         for (int c = c0; c < n1; c += kTailThreads) {
@@ -799,7 +806,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_pcg_tail(TailArgs a)
     }
     if (blk == 0 && t == 0) {
         const double rdn = s_val[1], measure = s_val[3];
-        const bool conv = CHECON ? measure <= tol : measure <= s_bound * s_bound;
+        const bool conv = CHECON ? measure <= tol : measure <= s_bound;
         const bool bad = !isfinite(rdn) || s_stop != 0;
         volatile PcgState *vs = a.st;
         vs->up = rdn;

@@ -86,3 +86,17 @@ def test_breakdown_is_reported():
                 s.solve(r, 1e-8, 100, mode)
         x, it, rel = s.solve(prob["r"], 1e-10, 5000, P.MODE_FP64_RES)
         assert rel <= 1e-9
+
+
+@pytest.mark.parametrize("mode", [P.MODE_P121, P.MODE_FP64_RES])
+def test_a_negative_tolerance_is_never_met(mode):
+    """The run ends at its limit, in the resident kernel, behind the products of 20- and of 8-node bricks."""
+    for shape in ((3, 3, 3), (30, 29, 28)):
+        prob = P.cube_problem(*shape)
+        with solver(prob) as s:
+            assert s.solve(prob["r"], -1.0, 9, mode)[1] == 9
+    prob = P.box8_problem(32, 32, 32)
+    with P.Solver() as s:
+        s.setup_scalar8(prob["g_num"], prob["g_g"], prob["g_coord"], prob["nn"], prob["neq"])
+        s.form_storkc(8, 1.0, 1.0, 1.0)
+        assert s.solve(np.ones(prob["neq"]), -1.0, 9, mode)[1] == 9
