@@ -194,7 +194,7 @@ constexpr int kGraphIters = 8;   // PCG iterations per graph replay
 // stopping test and element-kernel configuration, captured on first use.
 static int iteration_graph(Ctx &c, int prec, double *xsol, cudaGraphExec_t *out)
 {
-    const int tuning = c.sym_cfg + (c.sym_forced ? 16 : 0);
+    const int tuning = c.sym_cfg + (c.sym_forced ? 16 : 0) + (c.no_coop ? 32 : 0);
     if (c.it_graph && c.it_prec == prec && c.it_xsol == xsol && c.it_stop_mode == c.stop_mode &&
         c.it_sym_cfg == tuning) {
         *out = c.it_graph;
@@ -244,17 +244,22 @@ static int run_pcg(Ctx &c, int prec, double *xsol, int limit)
         // small meshes: the run in launches of up to 2000 iterations
         while (launched < limit) {
             const int todo = limit - launched < 2000 ? limit - launched : 2000;
-            TRY(launch_pcg_resident(c, prec, xsol, todo));
+            const int rc = launch_pcg_resident(c, prec, xsol, todo);
+            if (rc == kRefused) break;
+            TRY(rc);
             launched += todo;
             TRY(pull_state(c));
             if (c.hst->stop) break;
         }
-        if (check_kernel_error(c)) return 1;
-        if (c.hst->err) {
-            set_error("PCG breakdown after %d iterations (non-finite r.d or |x|)", c.hst->iters);
-            return 1;
+        if (!c.no_coop) {
+            if (check_kernel_error(c)) return 1;
+            if (c.hst->err) {
+                set_error("PCG breakdown after %d iterations (non-finite r.d or |x|)", c.hst->iters);
+                return 1;
+            }
+            return 0;
         }
-        return 0;
+        // refused: the state is that of an iteration's end, and the separate kernels go on from it
     }
     if (tail_ok(c) && prepare_tail(c)) return 1;
     if (persist_fused64(c, prec)) {

@@ -158,6 +158,7 @@ struct Ctx {
     // persistent PCG kernels (cooperative launches with grid-wide barriers)
     bool persistent = false;    // true: persistent cooperative kernels for the iteration (pf_set_persistent)
     unsigned long long *gbar = nullptr;   // [kPersistSlots] grid-barrier arrival counters, zeroed per run
+    bool no_coop = false;                 // a launch of one CTA per SM was refused: the separate kernels instead
     bool tail_attr = false;               // shared-memory attribute of k_pcg_tail set
     double *res_part = nullptr;           // [kShareBytes] the resident PCG's arrival counter and the CTAs' shares.
                                           //   Allocated with the context: an allocation between the choice of a
@@ -226,7 +227,11 @@ int launch_pcg_iteration(Ctx &c, int prec, double *xsol);
 // iterations (element products included), up to niters per launch.
 int launch_pcg_tail(Ctx &c, int prec, double *xsol);
 int launch_pcg_fused64(Ctx &c, double *xsol, int niters);
-// pf_resident.cu: up to niters iterations of a small mesh in one launch
+// pf_resident.cu: up to niters iterations of a small mesh in one launch.
+// This and launch_iteration_tail need every SM at once; where the device
+// refuses that (a part of it, taken by another program, say) they return
+// kRefused, nothing has run, and resident_ok and tail_ok are false from then on.
+constexpr int kRefused = 2;
 bool resident_ok(const Ctx &c, int prec);
 int launch_pcg_resident(Ctx &c, int prec, double *xsol, int niters);
 int prepare_tail(Ctx &c);

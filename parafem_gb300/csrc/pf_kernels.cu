@@ -1123,7 +1123,11 @@ int launch_pcg_iteration(Ctx &c, int prec, double *xsol)
         const int npu = leaves_shares(c, prec) ? element_ctas(c) : 0;
         if (launch_products(c, prec, c.p, c.st, npu ? product_shares(c) : nullptr)) return 1;
         if (c.kind != KIND_SOLID20 && launch_scatter(c, prec, 0, c.p, c.u)) return 1;
-        return launch_iteration_tail(c, prec, xsol, npu);
+        const int rc = launch_iteration_tail(c, prec, xsol, npu);
+        if (rc != kRefused) return rc;
+        if (c.kind == KIND_SOLID20 && launch_scatter(c, prec, 0, c.p, c.u)) return 1;
+        if (launch_update1(c, xsol)) return 1;
+        return launch_update2(c);
     }
     if (c.persistent && c.kind == KIND_SOLID20) {
         if (persist_fused64(c, prec)) return launch_pcg_fused64(c, xsol, 1);

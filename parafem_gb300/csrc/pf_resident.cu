@@ -461,10 +461,22 @@ static int slots_per_block(const Ctx &c) { return (c.nslots + c.nsm - 1) / c.nsm
 
 bool resident_ok(const Ctx &c, int prec)
 {
-    if (c.kind != KIND_SOLID20 || c.nsm > kMaxBlocks) return false;
+    if (c.kind != KIND_SOLID20 || c.nsm > kMaxBlocks || c.no_coop) return false;
     if (slots_per_block(c) > 4 * kResThreads) return false;
     if (c.shared) return prec == PREC_FP64 && c.skmfix;
     return prec == PREC_FP64 ? c.kmfix != nullptr : prec == PREC_FP32_SYM || prec == PREC_FP16_SYM;
+}
+
+// The result of a cooperative launch that failed with e
+static int coop_failed(Ctx &c, const char *name, cudaError_t e)
+{
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported) {
+        cudaGetLastError();
+        c.no_coop = true;
+        return kRefused;
+    }
+    set_error("%s: cooperative launch of %d blocks failed: %s", name, c.nsm, cudaGetErrorString(e));
+    return 1;
 }
 
 template <int PREC, bool CHECON, int NSL>
@@ -498,11 +510,8 @@ static int launch_resident_t(Ctx &c, double *xsol, int niters)
     a.kerr = c.kerr;
     void *args[] = {&a};
     if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(fn, dim3(c.nsm), dim3(kResThreads), args, smem, c.stream);
+    if (e != cudaSuccess) return coop_failed(c, "k_pcg_resident", e);
     c.launches++;
-    if (e != cudaSuccess) {
-        set_error("k_pcg_resident: cooperative launch of %d blocks failed: %s", c.nsm, cudaGetErrorString(e));
-        return 1;
-    }
     return 0;
 }
 
@@ -846,6 +855,7 @@ static int tail_nodes(const Ctx &c) { return ((c.nslots + 2) / 3 + c.nsm - 1) / 
 
 bool tail_ok(const Ctx &c)
 {
+    if (c.no_coop) return false;
     if (c.kind != KIND_SOLID20 && c.nslots < 30000) return false;
     return c.nsm <= kMaxBlocks && 3 * tail_nodes(c) <= kTailMax * kTailThreads;
 }
@@ -921,11 +931,8 @@ static int launch_tail_t(Ctx &c, int prec, double *xsol, int npu)
     void *args[] = {&a};
     const cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_pcg_tail<UT, CHECON, HOW>, dim3(c.nsm),
                                                       dim3(kTailThreads), args, smem, c.stream);
+    if (e != cudaSuccess) return coop_failed(c, "k_pcg_tail", e);
     c.launches++;
-    if (e != cudaSuccess) {
-        set_error("k_pcg_tail: cooperative launch of %d blocks failed: %s", c.nsm, cudaGetErrorString(e));
-        return 1;
-    }
     return 0;
 }
 

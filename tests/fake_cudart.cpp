@@ -89,6 +89,8 @@ void fake_reset()
     g_stale = g_coop_error = 0;
     g_rules.clear();
     g_log.clear();
+    for (auto &f : g_freed) free(f.first);
+    g_freed.clear();
     g_last = cudaSuccess;
 }
 void fake_clear_log() { g_log.clear(); }

@@ -100,3 +100,48 @@ def test_a_wait_that_runs_out_in_a_block_residual_fails_that_solve(fake):
     fake.fake_poke(b"k_mr_update1", 2, any_flag, 1)
     s.solve_multi(rk, 1e-8, 10, 32)
     s.close()
+
+
+COOPERATIVE_LAUNCH_TOO_LARGE, LAUNCH_OUT_OF_RESOURCES, NOT_SUPPORTED = 720, 701, 801
+
+
+@pytest.mark.parametrize("error", [COOPERATIVE_LAUNCH_TOO_LARGE, LAUNCH_OUT_OF_RESOURCES, NOT_SUPPORTED])
+@pytest.mark.parametrize("n,mode", [(3, P.MODE_P121), (3, P.MODE_MIXED), (29, P.MODE_FP64_RES), (29, P.MODE_MIXED)])
+def test_where_all_sms_are_refused_the_separate_kernels_run(fake, error, n, mode):
+    """3^3 elements would take the resident kernel, 29^3 the iteration tail."""
+    s, r = solver(n)
+    s.form_storkm(8)
+    fake.fake_coop_error(error)
+    fake.fake_clear_log()
+    s.solve(r, 1e-8, 7, mode)
+    names = [k for k, _ in kernels(fake)]
+    assert not any("k_pcg_resident" in k or "k_pcg_tail" in k for k in names)
+    # FP64: and one product for the residual; mixed: its one residual too
+    assert launched(fake, "k_elem") == 8 and launched(fake, "k_scatter") == 8
+    assert launched(fake, "k_pcg_update1") == 7 and launched(fake, "k_pcg_update2") == 7
+    fake.fake_clear_log()
+    s.solve(r, 1e-8, 20, mode)                 # and in graphs, from the fifth iteration on
+    assert launched(fake, "captured") > 0 and launched(fake, "k_pcg_tail") == 0
+    s.close()
+
+
+def test_where_all_sms_are_refused_8_node_meshes_run_on(fake):
+    prob = P.box8_problem(31, 31, 31)          # 32,768 slots: the iteration tail
+    s = P.Solver()
+    s.setup_scalar8(prob["g_num"], prob["g_g"], prob["g_coord"], prob["nn"], prob["neq"])
+    s.form_storkc(8, 1.0, 1.0, 1.0)
+    for error, tails in ((0, 7), (COOPERATIVE_LAUNCH_TOO_LARGE, 0)):
+        fake.fake_coop_error(error)
+        fake.fake_clear_log()
+        s.solve(np.ones(prob["neq"]), 1e-8, 7, P.MODE_P121)
+        assert launched(fake, "k_pcg_tail") == tails and launched(fake, "k_pcg_update2") == 7 - tails
+    s.close()
+
+
+def test_other_errors_of_a_cooperative_launch_are_reported(fake):
+    s, r = solver(3)
+    s.form_storkm(8)
+    fake.fake_coop_error(719)                  # a launch failure
+    with pytest.raises(P.PfError, match="cooperative launch"):
+        s.solve(r, 1e-8, 7, P.MODE_P121)
+    s.close()
