@@ -912,11 +912,16 @@ try {
     CK(cudaMemcpyAsync(c.skm64, km, 3600 * sizeof(double), cudaMemcpyHostToDevice, c.stream));
     CK(cudaMemcpyAsync(c.skm32, k32.data(), (3600 + 192) * sizeof(float), cudaMemcpyHostToDevice, c.stream));
     TRY(launch_shared_image(c));
-    if (!c.skmfix && dalloc(&c.skmfix, fx::kRecBytes, "shared km")) return PF_FAILURE;
-    CK(cudaMemsetAsync(c.kerr + 1, 0, sizeof(int), c.stream));
-    TRY(launch_pack_storkm(c, 1, c.skm64, nullptr, c.skmfix, c.kerr + 1));
+    if (!c.skmfix && cudaMalloc((void **)&c.skmfix, fx::kRecBytes) != cudaSuccess) {
+        cudaGetLastError();   // FP64 products by FP64 FMA instead
+        c.skmfix = nullptr;
+    }
     int bad = 0;
-    CK(cudaMemcpyAsync(&bad, c.kerr + 1, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    if (c.skmfix) {
+        CK(cudaMemsetAsync(c.kerr + 1, 0, sizeof(int), c.stream));
+        TRY(launch_pack_storkm(c, 1, c.skm64, nullptr, c.skmfix, c.kerr + 1));
+        CK(cudaMemcpyAsync(&bad, c.kerr + 1, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    }
     TRY(sync(c));
     drop_graph(c);
     if (bad) dfree(c.skmfix);

@@ -15,7 +15,7 @@
 namespace {
 std::map<const void *, std::string> g_kernels;
 std::map<char *, size_t> g_live, g_freed;
-long long g_limit = -1, g_used = 0;
+long long g_limit = -1, g_used = 0, g_refused_size = -1;
 int g_stale = 0, g_coop_error = 0;
 bool g_capture = false;
 std::string g_log;
@@ -60,7 +60,7 @@ cudaError_t launch(const void *fn, dim3 grid, void **args, bool cooperative)
 cudaError_t allocate(void **p, size_t bytes)
 {
     *p = nullptr;
-    if (g_limit >= 0 && g_used + (long long)bytes > g_limit) return result(cudaErrorMemoryAllocation);
+    if ((g_limit >= 0 && g_used + (long long)bytes > g_limit) || (long long)bytes == g_refused_size) return result(cudaErrorMemoryAllocation);
     char *q = (char *)calloc(bytes ? bytes : 1, 1);
     g_live[q] = bytes;
     g_used += (long long)bytes;
@@ -85,7 +85,7 @@ extern "C" {
 // the tests' controls
 void fake_reset()
 {
-    g_limit = -1;
+    g_limit = g_refused_size = -1;
     g_stale = g_coop_error = 0;
     g_rules.clear();
     g_log.clear();
@@ -97,6 +97,7 @@ void fake_clear_log() { g_log.clear(); }
 const char *fake_log() { return g_log.c_str(); }
 long long fake_used() { return g_used; }
 void fake_limit(long long bytes) { g_limit = bytes; }
+void fake_refuse_size(long long bytes) { g_refused_size = bytes; }
 int fake_stale() { return g_stale; }
 void fake_coop_error(int e) { g_coop_error = e; }
 void fake_fail(const char *kernel, int e) { g_rules.push_back({kernel, e, 0, 0, 0}); }

@@ -29,7 +29,7 @@ def fake_lib(tmp_path_factory):
         getattr(L, name).argtypes = args
         getattr(L, name).restype = ctypes.c_int
     L.fake_used.restype = ctypes.c_longlong
-    L.fake_limit.argtypes = [ctypes.c_longlong]
+    L.fake_limit.argtypes = L.fake_refuse_size.argtypes = [ctypes.c_longlong]
     L.fake_log.restype = ctypes.c_char_p
     return L
 
@@ -144,4 +144,24 @@ def test_other_errors_of_a_cooperative_launch_are_reported(fake):
     fake.fake_coop_error(719)                  # a launch failure
     with pytest.raises(P.PfError, match="cooperative launch"):
         s.solve(r, 1e-8, 7, P.MODE_P121)
+    s.close()
+
+
+RECORD = 14784                                 # bytes of one matrix's fixed-point record
+
+
+@pytest.mark.parametrize("n", [3, 29])
+def test_one_matrix_without_memory_for_its_record_takes_the_fma_products(fake, n):
+    s, r = solver(n)
+    fake.fake_refuse_size(RECORD)
+    s.set_shared_km(np.eye(60))
+    fake.fake_clear_log()
+    s.solve(r, 1e-8, 3, P.MODE_FP64_RES)
+    s.ebe_matvec(r, 64)
+    assert launched(fake, "k_elem_shared64") == 5 and launched(fake, "_fix") == 0
+    fake.fake_refuse_size(-1)
+    s.set_shared_km(np.eye(60))
+    fake.fake_clear_log()
+    s.ebe_matvec(r, 64)
+    assert launched(fake, "k_elem_shared_fix") == 1
     s.close()
