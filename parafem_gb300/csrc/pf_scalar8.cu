@@ -462,29 +462,37 @@ void rows_release(Ctx &c)
     c.row_val = nullptr;
     c.row_idx = nullptr;
     c.row_base = nullptr;
+    c.row_wide = c.row_keep = c.row_skip = c.row_ring = false;
 }
 
-// The assembled rows of the context's storkc; none (and success) where a row
-// is too long or the memory does not suffice.
-int rows_assemble(Ctx &c)
+// A kernel of the assembly was launched: 0, 1 (failed), or -1 where it found
+// no memory (its rows are assembled in local memory)
+static int rows_launched(Ctx &c, const char *name)
 {
-    rows_release(c);
+    const cudaError_t e = cudaPeekAtLastError();
+    if (e == cudaErrorMemoryAllocation || e == cudaErrorLaunchOutOfResources) {
+        cudaGetLastError();
+        return -1;
+    }
+    return launched8(c, name);
+}
+
+// The result of rows_assemble, -1 where the memory does not suffice
+static int rows_build(Ctx &c)
+{
     const int nslice = (c.nn + 31) / 32, grid = grid8(c, c.nn, 128, 16);
     int *d_width = nullptr, bad = 0;
     std::vector<int> width(nslice);
     std::vector<long long> off(nslice + 1, 0);
-    if (cudaMalloc((void **)&d_width, (size_t)nslice * sizeof(int)) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
+    if (cudaMalloc((void **)&d_width, (size_t)nslice * sizeof(int)) != cudaSuccess) return -1;
     cudaMemsetAsync(c.kerr + 1, 0, sizeof(int), c.stream);
     k_rows_width<<<grid, 128, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, c.conn, d_width, c.kerr + 1);
-    int err = launched8(c, "k_rows_width");
+    const int err = rows_launched(c, "k_rows_width");
     cudaMemcpyAsync(width.data(), d_width, (size_t)nslice * sizeof(int), cudaMemcpyDeviceToHost, c.stream);
     cudaMemcpyAsync(&bad, c.kerr + 1, sizeof(int), cudaMemcpyDeviceToHost, c.stream);
     const cudaError_t e = cudaStreamSynchronize(c.stream);
     cudaFree(d_width);
-    if (err) return 1;
+    if (err) return err;
     if (e != cudaSuccess) {
         set_error("k_rows_width: %s", cudaGetErrorString(e));
         return 1;
@@ -492,21 +500,15 @@ int rows_assemble(Ctx &c)
     if (bad) return 0;
     for (int s = 0; s < nslice; ++s) off[s + 1] = off[s] + 32LL * width[s];
     const auto w = std::minmax_element(width.begin(), width.end());
-    c.row_ring = false;
     const size_t total = (size_t)off[nslice];
     if (total == 0) return 0;
+    if (cudaMalloc((void **)&c.row_off, (size_t)(nslice + 1) * sizeof(long long)) != cudaSuccess ||
+        cudaMalloc((void **)&c.row_val, total * sizeof(double)) != cudaSuccess ||
+        cudaMalloc((void **)&c.row_base, total / 32 * sizeof(int)) != cudaSuccess)
+        return -1;
+    cudaMemcpyAsync(c.row_off, off.data(), off.size() * sizeof(long long), cudaMemcpyHostToDevice, c.stream);
     for (int bytes = 2; bytes <= 4; bytes += 2) {   // 16-bit columns first
-        if ((!c.row_off && cudaMalloc((void **)&c.row_off, (size_t)(nslice + 1) * sizeof(long long)) != cudaSuccess) ||
-            (!c.row_val && cudaMalloc((void **)&c.row_val, total * sizeof(double)) != cudaSuccess) ||
-            (!c.row_base && cudaMalloc((void **)&c.row_base, total / 32 * sizeof(int)) != cudaSuccess) ||
-            cudaMalloc(&c.row_idx, total * bytes) != cudaSuccess) {
-            cudaGetLastError();
-            rows_release(c);
-            return 0;
-        }
-        c.row_wide = bytes == 4;
-        c.row_keep = total * (8 + bytes) <= kRowKeepBytes;
-        cudaMemcpyAsync(c.row_off, off.data(), off.size() * sizeof(long long), cudaMemcpyHostToDevice, c.stream);
+        if (cudaMalloc(&c.row_idx, total * bytes) != cudaSuccess) return -1;
         cudaMemsetAsync(c.kerr + 1, 0, sizeof(int), c.stream);
         if (bytes == 2)
             k_rows_fill<uint16_t><<<grid, 128, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, c.conn, c.km64, c.row_off,
@@ -514,14 +516,17 @@ int rows_assemble(Ctx &c)
         else
             k_rows_fill<int><<<grid, 128, 0, c.stream>>>(c.nn, c.node_ptr, c.node_list, c.conn, c.km64, c.row_off,
                                                          c.row_val, (int *)c.row_idx, c.row_base, c.kerr + 1);
-        if (launched8(c, "k_rows_fill")) return 1;
+        const int ef = rows_launched(c, "k_rows_fill");
+        if (ef) return ef;
         cudaMemcpyAsync(&bad, c.kerr + 1, sizeof(int), cudaMemcpyDeviceToHost, c.stream);
-        const cudaError_t ef = cudaStreamSynchronize(c.stream);
-        if (ef != cudaSuccess) {
-            set_error("k_rows_fill: %s", cudaGetErrorString(ef));
+        const cudaError_t es = cudaStreamSynchronize(c.stream);
+        if (es != cudaSuccess) {
+            set_error("k_rows_fill: %s", cudaGetErrorString(es));
             return 1;
         }
         if (!(bad & 1)) {
+            c.row_wide = bytes == 4;
+            c.row_keep = total * (8 + bytes) <= kRowKeepBytes;
             c.row_skip = bad != 0;
             c.row_ring = bytes == 2 && *w.first > 0 && *w.second <= kRingWidth;
             break;
@@ -530,6 +535,19 @@ int rows_assemble(Ctx &c)
         c.row_idx = nullptr;
     }
     return 0;
+}
+
+// The assembled rows of the context's storkc; none (and success) where a row
+// is too long or the memory does not suffice, none either after an error:
+// rows that are there are whole.
+int rows_assemble(Ctx &c)
+{
+    rows_release(c);
+    const int rc = rows_build(c);
+    if (rc == 0) return 0;
+    cudaGetLastError();
+    rows_release(c);
+    return rc > 0;
 }
 
 static int launch_row_product(Ctx &c, int mode, const double *xin, const double *pf, double *out, PcgState *st)

@@ -200,6 +200,7 @@ cudaError_t cudaGetLastError()
     g_last = cudaSuccess;
     return e;
 }
+cudaError_t cudaPeekAtLastError() { return g_last; }
 const char *cudaGetErrorString(cudaError_t) { return "an error of the stand-in runtime"; }
 cudaError_t cudaMalloc(void **p, size_t bytes) { return allocate(p, bytes); }
 cudaError_t cudaMallocAsync(void **p, size_t bytes, cudaStream_t) { return allocate(p, bytes); }

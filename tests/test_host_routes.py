@@ -165,3 +165,38 @@ def test_one_matrix_without_memory_for_its_record_takes_the_fma_products(fake, n
     s.ebe_matvec(r, 64)
     assert launched(fake, "k_elem_shared_fix") == 1
     s.close()
+
+
+def scalar8(fake, n=9):
+    """p123's bricks; the stand-in's first slice of rows is 27 wide, so that rows are assembled."""
+    prob = P.box8_problem(n, n, n)
+    s = P.Solver()
+    s.setup_scalar8(prob["g_num"], prob["g_g"], prob["g_coord"], prob["nn"], prob["neq"])
+    fake.fake_poke(b"k_rows_width", 4, 0, 27)
+    return s, np.ones(prob["neq"])
+
+
+MEMORY_ALLOCATION, LAUNCH_FAILURE = 2, 719
+
+
+@pytest.mark.parametrize("kernel", [b"k_rows_width", b"k_rows_fill"])
+def test_rows_that_could_not_be_assembled_are_not_used(fake, kernel):
+    s, r = scalar8(fake)
+    s.form_storkc(8, 1.0, 1.0, 1.0)
+    fake.fake_clear_log()
+    s.ebe_matvec(r, 64)
+    assert launched(fake, "k_row_") == 1 and launched(fake, "k_elem8") == 0
+    fake.fake_fail(kernel, MEMORY_ALLOCATION)      # the element products instead
+    s.form_storkc(8, 1.0, 1.0, 1.0)
+    fake.fake_clear_log()
+    s.ebe_matvec(r, 64)
+    assert launched(fake, "k_row_") == 0 and launched(fake, "k_elem8") == 1
+    fake.fake_reset()
+    fake.fake_poke(b"k_rows_width", 4, 0, 27)
+    fake.fake_fail(kernel, LAUNCH_FAILURE)         # an error, and no half-filled rows for later calls
+    with pytest.raises(P.PfError):
+        s.form_storkc(8, 1.0, 1.0, 1.0)
+    fake.fake_clear_log()
+    s.ebe_matvec(r, 64)
+    assert launched(fake, "k_row_") == 0
+    s.close()
