@@ -108,16 +108,26 @@ int ctx_malloc(Ctx &c, void **p, size_t bytes)
 {
     *p = nullptr;
     cudaError_t e = cudaMalloc(p, bytes);
-    if (e != cudaSuccess && c.kmfix) {
+    if (e != cudaSuccess && (c.kmfix || c.row_idx)) {
         cudaGetLastError();
         drop_graph(c);
         cudaStreamSynchronize(c.stream);
         dfree(c.kmfix);
+        rows_release(c);
         e = cudaMalloc(p, bytes);
     }
     if (e == cudaSuccess) return 0;
     cudaGetLastError();
     *p = nullptr;
+    return 1;
+}
+
+// dalloc for a context that may hold what ctx_malloc gives back
+template <typename T>
+static int dalloc(Ctx &c, T **ptr, size_t count, const char *what)
+{
+    if (ctx_malloc(c, (void **)ptr, (count ? count : 1) * sizeof(T)) == 0) return 0;
+    set_error("cannot allocate %s (%zu bytes)", what, count * sizeof(T));
     return 1;
 }
 
@@ -696,7 +706,7 @@ try {
         slots[i] = eq_slot[eqs[i]];
     }
     int *d_slots = nullptr;
-    if (dalloc(&d_slots, (size_t)*nfix, "fixed freedoms")) return PF_FAILURE;
+    if (dalloc(c, &d_slots, (size_t)*nfix, "fixed freedoms")) return PF_FAILURE;
     cudaError_t e = cudaMemcpyAsync(d_slots, slots.data(), (size_t)*nfix * sizeof(int), cudaMemcpyHostToDevice,
                                     c.stream);
     int bad = e != cudaSuccess;
@@ -726,7 +736,7 @@ try {
         }
     dfree(c.mat_e);
     dfree(c.mat_v);
-    if (dalloc(&c.mat_e, *n, "material") || dalloc(&c.mat_v, *n, "material")) return PF_FAILURE;
+    if (dalloc(c, &c.mat_e, *n, "material") || dalloc(c, &c.mat_v, *n, "material")) return PF_FAILURE;
     c.nmat = *n;
     CK(cudaMemcpyAsync(c.mat_e, e, *n * sizeof(double), cudaMemcpyHostToDevice, c.stream));
     CK(cudaMemcpyAsync(c.mat_v, v, *n * sizeof(double), cudaMemcpyHostToDevice, c.stream));
@@ -856,7 +866,7 @@ try {
     }
     const size_t e = (size_t)*iel - 1;
     double *buf = nullptr;   // Gauss table (108) + km (3600) + element diagonal (60)
-    if (dalloc(&buf, 108 + 3600 + 60, "element matrix")) return PF_FAILURE;
+    if (dalloc(c, &buf, 108 + 3600 + 60, "element matrix")) return PF_FAILURE;
     const int m = c.nmat == 1 ? 0 : (int)e;
     int bad = launch_sample(c.stream, *nip, (*flags & PF_FORM_EXACT_WEIGHTS) != 0, buf);
     if (!bad)
@@ -895,9 +905,9 @@ try {
             set_error("pf_set_shared_km: km(%d,%d) = %g is not a positive stiffness", i + 1, i + 1, km[61 * i]);
             return PF_FAILURE;
         }
-    if (!c.skm64 && dalloc(&c.skm64, 3600, "shared km")) return PF_FAILURE;
-    if (!c.skm32 && dalloc(&c.skm32, 3600 + 192, "shared km")) return PF_FAILURE;
-    if (!c.psplit && dalloc(&c.psplit, (size_t)c.nslots, "split search direction")) return PF_FAILURE;
+    if (!c.skm64 && dalloc(c, &c.skm64, 3600, "shared km")) return PF_FAILURE;
+    if (!c.skm32 && dalloc(c, &c.skm32, 3600 + 192, "shared km")) return PF_FAILURE;
+    if (!c.psplit && dalloc(c, &c.psplit, (size_t)c.nslots, "split search direction")) return PF_FAILURE;
     // FP32 km, then the direction sums of its rows, sum over a of K(3a + d, k)
     // at 3600 + 64d + k (summed in FP64, zero for k = 60..63): the tensor-core
     // product's A operand carries them to remove the results' mean translation

@@ -194,8 +194,9 @@ int launch_form_storkm_raw(cudaStream_t stream, int nsm, int nels, int nip, cons
                            double *ediag);
 int launch_cast_km32(Ctx &c);
 int launch_extract_ediag(Ctx &c);
-// cudaMalloc for a context; when it fails, the fixed-point records (which
-// the FP64 products can do without) are given back and it is tried again.
+// cudaMalloc for a context; when it fails, the fixed-point records and the
+// assembled rows (which the products can do without) are given back and it is
+// tried again: they take no memory from what a caller asks for later.
 // Called before a solve's route is chosen, never between that and a launch.
 int ctx_malloc(Ctx &c, void **p, size_t bytes);
 int ensure_km32(Ctx &c);   // the full FP32 storkm, if storkm changed; outside stream capture

@@ -200,3 +200,26 @@ def test_rows_that_could_not_be_assembled_are_not_used(fake, kernel):
     s.ebe_matvec(r, 64)
     assert launched(fake, "k_row_") == 0
     s.close()
+
+
+def test_records_and_rows_give_way_to_later_allocations(fake):
+    """On a device that the records or rows have filled, what a context allocates later finds their memory."""
+    s, r = solver(3)
+    for later in (lambda: s.set_material(np.full(27, 100.0), np.full(27, 0.3)), lambda: s.form_km(1, 8),
+                  lambda: s.set_shared_km(np.eye(60))):
+        s.form_storkm(8)
+        fake.fake_clear_log()
+        s.ebe_matvec(r, 64)
+        assert launched(fake, "k_elem_fix") == 1
+        fake.fake_limit(fake.fake_used())
+        later()
+        fake.fake_limit(-1)
+    s.close()
+    s, r = scalar8(fake)
+    s.form_storkc(8, 1.0, 1.0, 1.0)
+    fake.fake_limit(fake.fake_used())
+    s.set_fixed([1, 2], 1e20)
+    fake.fake_clear_log()
+    s.ebe_matvec(r, 64)
+    assert launched(fake, "k_row_") == 0 and launched(fake, "k_elem8") == 1
+    s.close()
