@@ -145,10 +145,12 @@ int pf_solve(void **ctx, const double *r, const double *tol, const int *limit,
  *  [6] true relative residual */
 int pf_solve_stats(void **ctx, double *stats, const int *n);
 
-/* Times `steps` PCG iterations on the resident state (prec 64, 32, 31 or 16) with
- * CUDA events on the library stream.  ms_total: all steps; ms_elem: summed
- * duration of the element-product kernel launches; ms_scatter: summed
- * duration of the node-scatter kernel launches. */
+/* Times `steps` PCG iterations on the resident load vector (prec 64, 32, 31 or 16)
+ * with CUDA events on the library stream.  ms_total: all steps, by the
+ * kernels that a solve of this context takes and launched as it launches
+ * them; ms_elem: summed duration of the element-product launches,
+ * ms_scatter: of the node-scatter launches, in as many iterations of
+ * separate kernels before those. */
 int pf_bench_iterations(void **ctx, const int *prec, const int *steps,
                         double *ms_total, double *ms_elem, double *ms_scatter);
 

@@ -244,8 +244,8 @@ static int iteration_graph(Ctx &c, int prec, double *xsol, cudaGraphExec_t *out)
 // Runs PCG iterations until the device state says stop.  The state is read
 // back every `chunk` iterations; iterations launched after the stop return
 // at once (every kernel checks the flag).  Whole groups of kGraphIters
-// iterations are replayed from a CUDA graph (one launch instead of five
-// per iteration); the remainder below the limit is launched directly.
+// iterations are replayed from a CUDA graph (one launch instead of two to
+// four per iteration); the remainder below the limit is launched directly.
 static int run_pcg(Ctx &c, int prec, double *xsol, int limit)
 {
     int launched = 0;
@@ -309,6 +309,34 @@ static int run_pcg(Ctx &c, int prec, double *xsol, int limit)
         set_error("PCG breakdown after %d iterations (non-finite r.d or |x|)", c.hst->iters);
         return 1;
     }
+    return 0;
+}
+
+// n iterations by run_pcg's choice of kernels, without its reads of the
+// state, between two events
+static int solver_iterations(Ctx &c, int prec, double *xsol, int n, cudaEvent_t from, cudaEvent_t to)
+{
+    if (resident_ok(c, prec)) {
+        CK(cudaEventRecord(from, c.stream));
+        const int rc = launch_pcg_resident(c, prec, xsol, n);
+        if (rc != kRefused) {
+            TRY(rc);
+            CK(cudaEventRecord(to, c.stream));
+            return 0;
+        }
+    }
+    if (tail_ok(c) && prepare_tail(c)) return 1;
+    cudaGraphExec_t ge = nullptr;
+    const bool fused = persist_fused64(c, prec);
+    if (!fused && c.use_graphs && n >= kGraphIters) TRY(iteration_graph(c, prec, xsol, &ge));
+    CK(cudaEventRecord(from, c.stream));
+    for (; fused && n > 0; n -= 32) TRY(launch_pcg_fused64(c, xsol, n < 32 ? n : 32));
+    for (; ge && n >= kGraphIters; n -= kGraphIters) {
+        CK(cudaGraphLaunch(ge, c.stream));
+        c.launches += c.it_launches;
+    }
+    for (; n > 0; --n) TRY(launch_pcg_iteration(c, prec, xsol));
+    CK(cudaEventRecord(to, c.stream));
     return 0;
 }
 
@@ -1174,6 +1202,8 @@ try {
     if (*prec == 16) TRY(ensure_km16(c));
     if (*prec == 31 && !c.shared) TRY(ensure_km32(c));
     const int n = *steps;
+    // first by kernel: products, scatter and updates launched one by one
+    const long long l0 = c.launches;
     // never-converging run on the resident load vector (tol 0, no limit hit)
     TRY(launch_pcg_init(c, c.f, c.c, STOP_RELRES, 0.0, n + 1));
     TRY(pull_state(c));
@@ -1184,19 +1214,13 @@ try {
     std::vector<cudaEvent_t> ev(3 * (size_t)n + 1);
     for (auto &e : ev) CK(cudaEventCreate(&e));
     CK(cudaEventRecord(ev[0], c.stream));
-    const bool tail = c.persistent && c.kind == KIND_SOLID20;
     for (int i = 0; i < n; ++i) {
         TRY(launch_elem(c, *prec, c.p));
         CK(cudaEventRecord(ev[3 * i + 1], c.stream));
-        if (tail) {   // scatter, updates and finish in one persistent launch
-            TRY(launch_pcg_tail(c, *prec, c.c));
-            CK(cudaEventRecord(ev[3 * i + 2], c.stream));
-        } else {
-            TRY(launch_scatter(c, *prec, 0, c.p, c.u));
-            CK(cudaEventRecord(ev[3 * i + 2], c.stream));
-            TRY(launch_update1(c, c.c));
-            TRY(launch_update2(c));
-        }
+        TRY(launch_scatter(c, *prec, 0, c.p, c.u));
+        CK(cudaEventRecord(ev[3 * i + 2], c.stream));
+        TRY(launch_update1(c, c.c));
+        TRY(launch_update2(c));
         CK(cudaEventRecord(ev[3 * i + 3], c.stream));
     }
     CK(cudaStreamSynchronize(c.stream));
@@ -1209,8 +1233,14 @@ try {
         te += a;
         ts += b;
     }
+    // then the iterations as a solve runs them
     float tot = 0;
-    CK(cudaEventElapsedTime(&tot, ev[0], ev[3 * (size_t)n]));
+    c.launches = l0;
+    TRY(launch_pcg_init(c, c.f, c.c, STOP_RELRES, 0.0, n + 1));
+    TRY(solver_iterations(c, *prec, c.c, n, ev[0], ev[1]));
+    CK(cudaStreamSynchronize(c.stream));
+    TRY(check_kernel_error(c));
+    CK(cudaEventElapsedTime(&tot, ev[0], ev[1]));
     for (auto &e : ev) cudaEventDestroy(e);
     if (ms_total) *ms_total = tot;
     if (ms_elem) *ms_elem = te;

@@ -223,3 +223,24 @@ def test_records_and_rows_give_way_to_later_allocations(fake):
     s.ebe_matvec(r, 64)
     assert launched(fake, "k_row_") == 0 and launched(fake, "k_elem8") == 1
     s.close()
+
+
+def names(fake):
+    return {k.replace("captured ", "") for k, _ in kernels(fake)}
+
+
+@pytest.mark.parametrize("n,prec,mode", [(3, 64, P.MODE_FP64_RES), (29, 64, P.MODE_FP64_RES), (29, 32, P.MODE_MIXED)])
+def test_iterations_are_timed_with_the_kernels_of_a_solve(fake, n, prec, mode):
+    s, r = solver(n)
+    s.form_storkm(8)
+    fake.fake_clear_log()
+    s.solve(r, 1e-8, 20, mode)
+    solve = {k for k in names(fake) if "k_pcg_resident" in k or "k_pcg_tail" in k or "k_elem" in k}
+    before = s.launches()
+    fake.fake_clear_log()
+    s.bench_iterations(prec, 20)
+    assert any("k_pcg_resident" in k or "k_pcg_tail" in k for k in solve)
+    assert {k for k in solve if "k_pcg" in k} <= names(fake)
+    # the launches of the timed iterations alone are counted: the initialisation's and theirs
+    assert s.launches() - before == (2 + 1 if n == 3 else 2 + 2 * 20)
+    s.close()
