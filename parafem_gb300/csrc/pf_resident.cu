@@ -2,8 +2,8 @@
 //
 // On a small mesh an iteration of four kernels is launch latency: 22 us on
 // 10^3 elements, of which the chip works perhaps three.  Here one CTA per SM
-// stays for the whole run.  A CTA owns a range of elements and a range of
-// slots; its elements' records stay in shared memory when they fit (14 FP64,
+// (of half the SMs on the smallest meshes) stays for the whole run.  A CTA
+// owns a range of elements and a range of slots; its elements' records stay in shared memory when they fit (14 FP64,
 // 28 FP32 or 48 FP16 records per SM: 12.8^3, 16^3, 19^3 elements on 152 SMs)
 // and stream through it otherwise.  An iteration (p121.f90:90-104 with
 // DOT_PRODUCT_P, maths.f90:168-215, and checon_par, maths.f90:1052-1062) is
@@ -457,12 +457,29 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(ResArgs a)
 // so that it takes every mesh that fits.  Of the 10.8 us at 10^3 (FP64)
 // the products take 3.8, the two exchanges 2.6 and the sums over the CTAs with
 // the two divisions 2.5.
-static int slots_per_block(const Ctx &c) { return (c.nslots + c.nsm - 1) / c.nsm; }
+//
+// The kernel holds its SMs for the whole run, so that runs of other contexts
+// wait for it.  Meshes whose products lose nothing by it take half the SMs,
+// and two such runs go side by side: those of at most so many elements per
+// CTA, in FP64 three (they share the SM's integer pipe), in FP32 one per
+// product warp, in FP16 seven.  Solves per second of one context / of eight in
+// threads, all SMs, half of them, and the separate kernels (no resident runs):
+//            6^3 FP64   8^3 FP64   6^3 FP32   10^3 FP32  12^3 FP32  8^3 FP16   10^3 FP16
+//   all      700/716    555/565    455/612    296/356    240/288    396/510    337/407
+//   half     706/1432   513/1044   467/1250   295/681    211/481    399/996    324/766
+//   separate 244/1333   195/789    170/876    136/508    120/365    157/785    114/494
+// (the number of CTAs must not depend on what else runs: it orders the sums).
+static int resident_ctas(const Ctx &c, int prec)
+{
+    const int half = c.nsm / 2, per = prec == PREC_FP64 ? 3 : prec == PREC_FP32_SYM ? Shape<32>::W : 7;
+    return half > 0 && c.nels <= per * half ? half : c.nsm;
+}
+static int slots_per_block(const Ctx &c, int ctas) { return (c.nslots + ctas - 1) / ctas; }
 
 bool resident_ok(const Ctx &c, int prec)
 {
     if (c.kind != KIND_SOLID20 || c.nsm > kMaxBlocks || c.no_coop) return false;
-    if (slots_per_block(c) > 4 * kResThreads) return false;
+    if (slots_per_block(c, resident_ctas(c, prec)) > 4 * kResThreads) return false;
     if (c.shared) return prec == PREC_FP64 && c.skmfix;
     return prec == PREC_FP64 ? c.kmfix != nullptr : prec == PREC_FP32_SYM || prec == PREC_FP16_SYM;
 }
@@ -480,7 +497,7 @@ static int coop_failed(Ctx &c, const char *name, cudaError_t e)
 }
 
 template <int PREC, bool CHECON, int NSL>
-static int launch_resident_t(Ctx &c, double *xsol, int niters)
+static int launch_resident_t(Ctx &c, double *xsol, int niters, int ctas)
 {
     constexpr size_t smem = kResSmem<PREC>;
     static_assert(smem + 256 + 2 * 32 * 8 <= 227 * 1024, "shared memory per CTA");
@@ -490,7 +507,7 @@ static int launch_resident_t(Ctx &c, double *xsol, int niters)
     a.nels = c.nels;
     a.ns = c.nslots;
     a.niters = niters;
-    a.per_slots = slots_per_block(c);
+    a.per_slots = slots_per_block(c, ctas);
     a.stride = c.shared ? 0 : Shape<PREC>::rec;
     a.rec = c.shared ? c.skmfix : PREC == 64 ? c.kmfix : PREC == 32 ? (const unsigned char *)c.km32p : (const unsigned char *)c.km16p;
     a.conn = c.conn;
@@ -509,7 +526,7 @@ static int launch_resident_t(Ctx &c, double *xsol, int niters)
     if (e == cudaSuccess) e = cudaMemsetAsync(a.count, 0, sizeof(unsigned long long), c.stream);
     a.kerr = c.kerr;
     void *args[] = {&a};
-    if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(fn, dim3(c.nsm), dim3(kResThreads), args, smem, c.stream);
+    if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(fn, dim3(ctas), dim3(kResThreads), args, smem, c.stream);
     if (e != cudaSuccess) return coop_failed(c, "k_pcg_resident", e);
     c.launches++;
     return 0;
@@ -518,11 +535,12 @@ static int launch_resident_t(Ctx &c, double *xsol, int niters)
 template <int PREC>
 static int launch_resident_p(Ctx &c, double *xsol, int niters)
 {
-    const bool ck = c.stop_mode == STOP_CHECON, one = slots_per_block(c) <= kResThreads;
+    const int n = resident_ctas(c, PREC);
+    const bool ck = c.stop_mode == STOP_CHECON, one = slots_per_block(c, n) <= kResThreads;
     if (PREC == 64 && ck)   // checon_par stops FP64 runs only
-        return one ? launch_resident_t<PREC, PREC == 64, 1>(c, xsol, niters)
-                   : launch_resident_t<PREC, PREC == 64, 4>(c, xsol, niters);
-    return one ? launch_resident_t<PREC, false, 1>(c, xsol, niters) : launch_resident_t<PREC, false, 4>(c, xsol, niters);
+        return one ? launch_resident_t<PREC, PREC == 64, 1>(c, xsol, niters, n)
+                   : launch_resident_t<PREC, PREC == 64, 4>(c, xsol, niters, n);
+    return one ? launch_resident_t<PREC, false, 1>(c, xsol, niters, n) : launch_resident_t<PREC, false, 4>(c, xsol, niters, n);
 }
 
 int launch_pcg_resident(Ctx &c, int prec, double *xsol, int niters)

@@ -1,6 +1,8 @@
 """Small meshes, whose PCG runs as one resident kernel: against the C
 restatement of p121's PCG, at the sizes where its element ring, its slots per
 thread and its launches of 2000 iterations change."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -100,3 +102,29 @@ def test_a_negative_tolerance_is_never_met(mode):
         s.setup_scalar8(prob["g_num"], prob["g_g"], prob["g_coord"], prob["nn"], prob["neq"])
         s.form_storkc(8, 1.0, 1.0, 1.0)
         assert s.solve(np.ones(prob["neq"]), -1.0, 9, mode)[1] == 9
+
+
+def test_contexts_in_threads_leave_each_other_alone():
+    """Resident runs of half the SMs side by side, of all of them one after the other, and iterations with the tail
+    and products in between: every solve bitwise as alone."""
+    jobs = [((3, 3, 3), P.MODE_P121), ((6, 6, 6), P.MODE_P121), ((6, 6, 6), P.MODE_MIXED), ((10, 10, 10), P.MODE_MIXED16),
+            ((12, 11, 10), P.MODE_P121), ((30, 28, 29), P.MODE_MIXED)]
+    probs = [P.cube_problem(*shape) for shape, _ in jobs]
+    solvers = [solver(prob) for prob in probs]
+    alone = [s.solve(q["r"], 1e-8, 20000, m) for s, q, (_, m) in zip(solvers, probs, jobs)]
+    bad = []
+
+    def run(i):
+        for _ in range(8):
+            x, it, _ = solvers[i].solve(probs[i]["r"], 1e-8, 20000, jobs[i][1])
+            if it != alone[i][1] or not np.array_equal(x, alone[i][0]):
+                bad.append(i)
+
+    threads = [threading.Thread(target=run, args=(i,)) for i in range(len(jobs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for s in solvers:
+        s.close()
+    assert not bad

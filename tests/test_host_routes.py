@@ -244,3 +244,15 @@ def test_iterations_are_timed_with_the_kernels_of_a_solve(fake, n, prec, mode):
     # the launches of the timed iterations alone are counted: the initialisation's and theirs
     assert s.launches() - before == (2 + 1 if n == 3 else 2 + 2 * 20)
     s.close()
+
+
+@pytest.mark.parametrize("n,mode,blocks", [(6, P.MODE_P121, 76), (7, P.MODE_P121, 152), (10, P.MODE_MIXED, 76), (11, P.MODE_MIXED, 152),
+                                           (8, P.MODE_MIXED16, 76), (9, P.MODE_MIXED16, 152)])
+def test_the_smallest_runs_take_half_the_sms(fake, n, mode, blocks):
+    """Two of them go side by side (the stand-in has 152 SMs)."""
+    s, r = solver(n)
+    s.form_storkm(8)
+    fake.fake_clear_log()
+    s.solve(r, 1e-8, 3, mode)
+    assert {int(b) for k, b in kernels(fake) if "k_pcg_resident" in k} == {blocks}
+    s.close()
