@@ -202,12 +202,13 @@ int pf_set_persistent(void **ctx, const int *on);
 /* Self-check of the error path of the bulk-copy element kernels (no
  * reference counterpart).  Every mbarrier wait in those kernels is bounded;
  * one that runs out records an error word that the next synchronising call
- * reports as PF_FAILURE.  This runs one such wait, limited to *polls polls,
- * on a barrier that no copy completes (no copy is ever in flight), and
- * reports it the same way: it returns PF_FAILURE with the message "element
+ * reports as PF_FAILURE.  So do the grid-wide waits of the kernels that run
+ * on every SM.  This runs one wait of each kind, limited to *polls polls: a
+ * grid-wide one that nothing completes, then one on a barrier that no copy
+ * completes (no copy is ever in flight).  It reports the second the same way: it returns PF_FAILURE with the message "element
  * kernel: a shared-memory bulk-copy wait timed out (code 2)" and clears the
  * word, so the context's next call runs normally.  It returns PF_SUCCESS
- * only if the wait completed, which would mean the check itself is broken. */
+ * only if one of them completed, which would mean the check itself is broken. */
 int pf_check_wait_timeout(void **ctx, const int *polls);
 
 /* ---- p123: 3-D Laplace with 8-node bricks (src/programs/5th_ed/p123/p123.f90) ----

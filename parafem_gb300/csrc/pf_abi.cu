@@ -1360,6 +1360,11 @@ try {
         set_error("pf_check_wait_timeout: *polls must be at least 1");
         return PF_FAILURE;
     }
+    TRY(launch_exchange_probe(*cp, *polls));
+    if (!check_kernel_error(*cp)) {
+        set_error("pf_check_wait_timeout: the grid-wide wait completed, so its timeout path did not run");
+        return PF_SUCCESS;
+    }
     TRY(launch_wait_probe(*cp, *polls));
     if (check_kernel_error(*cp)) return PF_FAILURE;   // the timeout, reported as the kernels report it
     set_error("pf_check_wait_timeout: the wait completed, so the timeout path did not run");

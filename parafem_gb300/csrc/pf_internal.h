@@ -244,6 +244,8 @@ bool persist_fused64(const Ctx &c, int prec);
 // One bounded mbarrier wait that nothing completes (the error path of the
 // bulk-copy kernels, without a fault): records code 2 in c.kerr.
 int launch_wait_probe(Ctx &c, long long polls);
+// The same of the resident run's and the iteration tail's exchange: code 3.
+int launch_exchange_probe(Ctx &c, long long polls);
 int launch_axpy(Ctx &c, double *y, const double *xv);          // y += x
 int launch_replace(Ctx &c, double tol);   // r = rres, d = diag*r, up = r.d; p kept
 int launch_sum_partials(Ctx &c, int nvals, double *out_dev);   // out[0] = sum of part_s

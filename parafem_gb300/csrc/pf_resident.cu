@@ -63,10 +63,11 @@ template <int PREC> constexpr size_t kResSmem =
 // One thread: its block's writes are out (with those of the threads it has
 // met at a barrier), and every block's are visible on return; false when the
 // wait ran out.
-__device__ __forceinline__ bool exchange(unsigned long long *count, unsigned long long target)
+__device__ __forceinline__ bool exchange(unsigned long long *count, unsigned long long target,
+                                         long long polls = kGridSpinLimit)
 {
     asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(count), "l"(1ULL) : "memory");
-    for (long long i = 0; i < kGridSpinLimit; ++i) {
+    for (long long i = 0; i < polls; ++i) {
         unsigned long long v;
         asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(count) : "memory");
         if (v >= target) return true;
@@ -105,6 +106,12 @@ __device__ __forceinline__ long long max_shares(const double *p, int nblk, int l
 }
 
 }  // namespace
+
+// One exchange that nothing completes, as pf_check_wait_timeout runs it
+__global__ void k_exchange_probe(unsigned long long *count, long long polls, int *kerr)
+{
+    if (threadIdx.x == 0 && !exchange(count, ~0ULL, polls)) atomicExch(kerr, 3);
+}
 
 template <int PREC, bool CHECON, int NSL>
 __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(ResArgs a)
@@ -962,6 +969,19 @@ int launch_iteration_tail(Ctx &c, int prec, double *xsol, int npu)
     if (prec == PREC_FP64)
         return ck ? launch_tail_t<double, true, TAIL_SUMS>(c, prec, xsol, 0) : launch_tail_t<double, false, TAIL_SUMS>(c, prec, xsol, 0);
     return npu ? launch_tail_t<float, false, TAIL_DOT>(c, prec, xsol, npu) : launch_tail_t<float, false, TAIL_SUMS>(c, prec, xsol, 0);
+}
+
+// (the resident run zeroes the counter before every launch)
+int launch_exchange_probe(Ctx &c, long long polls)
+{
+    k_exchange_probe<<<1, 32, 0, c.stream>>>(reinterpret_cast<unsigned long long *>(c.res_part), polls, c.kerr);
+    c.launches++;
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+        set_error("k_exchange_probe: launch failed: %s", cudaGetErrorString(e));
+        return 1;
+    }
+    return 0;
 }
 
 double *product_shares(Ctx &c) { return c.res_part + 8 + 4 * kMaxBlocks; }

@@ -128,3 +128,15 @@ def test_contexts_in_threads_leave_each_other_alone():
     for s in solvers:
         s.close()
     assert not bad
+
+
+def test_an_exchange_that_nothing_completes_runs_out():
+    """The check runs the exchange and the bulk-copy wait, both to their limit; the context goes on."""
+    prob = P.cube_problem(3, 3, 3)
+    with solver(prob) as s:
+        x, it, _ = s.solve(prob["r"], 1e-10, 5000, P.MODE_FP64_RES)
+        before = s.launches()
+        rc, msg = s.check_wait_timeout(64)
+        assert rc != 0 and "code 2" in msg and s.launches() - before == 2
+        y, jt, _ = s.solve(prob["r"], 1e-10, 5000, P.MODE_FP64_RES)
+        assert it == jt and np.array_equal(x, y)

@@ -256,3 +256,14 @@ def test_the_smallest_runs_take_half_the_sms(fake, n, mode, blocks):
     s.solve(r, 1e-8, 3, mode)
     assert {int(b) for k, b in kernels(fake) if "k_pcg_resident" in k} == {blocks}
     s.close()
+
+
+def test_a_grid_wide_wait_that_runs_out_fails_that_solve(fake):
+    s, r = solver(29)
+    s.form_storkm(8)
+    fake.fake_poke(b"k_elem_fix", 6, 0, 3)     # the error word as k_pcg_tail leaves it
+    with pytest.raises(P.PfError, match=r"grid-wide wait timed out \(code 3\)"):
+        s.solve(r, 1e-8, 3, P.MODE_FP64_RES)
+    fake.fake_clear_rules()
+    s.solve(r, 1e-8, 3, P.MODE_FP64_RES)
+    s.close()
