@@ -136,3 +136,63 @@ def test_elasticity_on_8_node_bricks(n):
         assert np.linalg.norm(r - s.ebe_matvec(x, 64)) <= 1e-10 * np.linalg.norm(r)
         y, _, _ = s.solve(r, 1e-11, 20000, P.MODE_P121)
         assert np.linalg.norm(y - x) <= 1e-7 * np.linalg.norm(x)
+
+
+@pytest.fixture(scope="module")
+def beyond():
+    """4.3 million freedoms, one storkm per element: the separate kernels, as the largest workloads run."""
+    prob = P.cube_problem(71, 70, 71)
+    with solver(prob) as s:
+        yield prob, s
+
+
+@pytest.mark.parametrize("mode", [P.MODE_MIXED, P.MODE_MIXED16])
+def test_beyond_the_tail_mixed_solves_converge(beyond, mode):
+    prob, s = beyond
+    x, it, rel = s.solve(prob["r"], 1e-6, 20000, mode)
+    assert it > 100 and rel <= 1e-6
+    assert np.linalg.norm(prob["r"] - s.ebe_matvec(x, 64)) <= 1.01e-6 * np.linalg.norm(prob["r"])
+    y, jt, _ = s.solve(prob["r"], 1e-6, 20000, mode)
+    assert it == jt and np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("mode", [P.MODE_P121, P.MODE_FP64_RES])
+def test_beyond_the_tail_graphs_and_persistent_kernels_give_the_same_iterates(beyond, mode):
+    """45 iterations: 4, 8, 16 and 17 to a read of the state, 40 of them replayed from graphs where those are on."""
+    prob, s = beyond
+    out = []
+    for graphs, persistent in ((True, False), (False, False), (True, True)):
+        s.set_graphs(graphs)
+        s.set_persistent(persistent)
+        x, it, rel = s.solve(prob["r"], 0.0, 45, mode)
+        assert it == 45
+        true = np.linalg.norm(prob["r"] - s.ebe_matvec(x, 64)) / np.linalg.norm(prob["r"])
+        assert abs(rel - true) <= 1e-9 * true
+        out.append(x)
+    s.set_graphs(True)
+    s.set_persistent(False)
+    assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+
+
+def test_beyond_the_tail_persistent_kernels_run_mixed_solves(beyond):
+    prob, s = beyond
+    ref = s.solve(prob["r"], 0.01, 20000, P.MODE_MIXED)
+    s.set_persistent(True)
+    x, it, rel = s.solve(prob["r"], 0.01, 20000, P.MODE_MIXED)
+    s.set_persistent(False)
+    assert it == ref[1] and rel == ref[2] and np.array_equal(x, ref[0])
+
+
+def test_beyond_the_tail_8_node_bricks():
+    """160^3 bricks of p123: 4,173,281 freedoms."""
+    prob = P.box8_problem(160, 160, 160)
+    r = np.random.default_rng(8).standard_normal(prob["neq"])
+    with P.Solver() as s:
+        s.setup_scalar8(prob["g_num"], prob["g_g"], prob["g_coord"], prob["nn"], prob["neq"])
+        s.form_storkc(8, 1.0, 1.0, 1.0)
+        x, it, rel = s.solve(r, 1e-8, 20000, P.MODE_FP64_RES)
+        assert it > 30 and rel <= 2e-8
+        assert np.linalg.norm(r - s.ebe_matvec(x, 64)) <= 2e-8 * np.linalg.norm(r)
+        s.set_graphs(False)
+        y, jt, _ = s.solve(r, 1e-8, 20000, P.MODE_FP64_RES)
+        assert it == jt and np.array_equal(x, y)
