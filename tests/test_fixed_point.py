@@ -1,9 +1,15 @@
 """FP64 element products in 64-bit fixed point: the record layout and walk on
 the CPU, and the GPU products against extended precision."""
+import ctypes
+import os
+import subprocess
+from fractions import Fraction
+
 import numpy as np
 import pytest
 
 import parafem_gb300 as P
+from parafem_gb300 import _build
 
 
 # ---------------------------------------------------------------------------
@@ -245,3 +251,96 @@ def test_infinities_and_nan_reach_the_rows_that_they_reach_by_fma(bad):
     for got in (u, uk):
         assert np.array_equal(np.isnan(got), np.isnan(ref)) and np.array_equal(np.isfinite(got), np.isfinite(ref))
         assert np.array_equal(np.sign(got[np.isinf(ref)]), np.sign(ref[np.isinf(ref)]))
+
+
+# ---------------------------------------------------------------------------
+# the library's own helpers, on the host
+@pytest.fixture(scope="module")
+def helpers(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("fix") / "fix_host.so")
+    subprocess.check_call([_build.nvcc()] + _build.ARCH + ["-O1", "-std=c++17", "-shared", "-Xcompiler", "-fPIC", "-I", _build.INCLUDE,
+                           "-I", _build.SRC, os.path.join(os.path.dirname(__file__), "fix_host.cu"), "-o", so])
+    L = ctypes.CDLL(so)
+    L.fix_scale.argtypes = [ctypes.c_double]
+    L.fix_size.argtypes = [ctypes.c_double, ctypes.c_int, ctypes.c_int]
+    L.fix_entry.argtypes = [ctypes.c_double] + 3 * [ctypes.c_int] + 2 * [ctypes.POINTER(ctypes.c_int)]
+    return L
+
+
+def words(L, k, si, sk, extra):
+    h, l = ctypes.c_int(), ctypes.c_int()
+    ok = L.fix_entry(k, si, sk, extra, ctypes.byref(h), ctypes.byref(l))
+    return ok, h.value, l.value
+
+
+def test_offsets_are_the_restated_ones(helpers):
+    assert helpers.record_bytes() == RECORD
+    assert all(helpers.row_off(s, h) == row_off(s, h) for s in range(1, 16) for h in (0, 1))
+
+
+@pytest.mark.parametrize("k", [1.0, 0.25, 0.2500001, 0.9999999, 2.0, 3.999, 4.0, 1e-300, 1e300, 5e-308, 1.7e308, 123.456])
+def test_scaled_diagonal_lies_between_a_quarter_and_one(helpers, k):
+    s = helpers.fix_scale(k)
+    assert 0.25 <= Fraction(k) * Fraction(4) ** s < 1
+
+
+@pytest.mark.parametrize("extra", [0, 2])
+def test_words_hold_the_rounded_entry(helpers, extra):
+    """K' in 57 + extra bits to half a unit, the high word within 2^(28 + extra), the low one within 2^28."""
+    rng = np.random.default_rng(9)
+    vals = np.concatenate([rng.uniform(-1, 1, 200) * 2.0 ** rng.integers(-80, 1, 200), [1 - 2.0 ** -53, -1 + 2.0 ** -53, 0.0, 2.0 ** -59, 2.0 ** -60]])
+    for k in vals:
+        for si, sk in ((0, 0), (300, -290), (-512, 512)):
+            ks = float(np.ldexp(k, -si - sk))
+            ok, h, l = words(helpers, ks, si, sk, extra)
+            exact = Fraction(ks) * Fraction(2) ** (si + sk + 57 + extra)
+            assert ok and abs(h) <= 1 << (28 + extra) and -(1 << 28) <= l < 1 << 28
+            assert abs((h << 29) + l - exact) <= Fraction(1, 2)
+    for k in (1.0, -1.5, np.inf, -np.inf, np.nan):
+        assert not words(helpers, k, 0, 0, extra)[0]
+
+
+@pytest.mark.parametrize("top", [3.9749, 3.9751])
+def test_row_sums_leave_63_bits_on_both_sides_of_the_rule_for_two_more_bits(helpers, top):
+    """k_pack_storkm adds fix_size over 15 entries per quarter row and gives an element two more bits when every
+    quarter stays below 15.9 / 4.  Then the sums of |h| |h'| and of the two mixed products over 60 entries, h' up to
+    2^28 and low words up to 2^28, stay below 2^63."""
+    k = top / 15
+    quarter = 15 * helpers.fix_size(k, 0, 0)
+    wide = quarter >= int(15.9 / 4 * (1 << 20))
+    assert wide == (top > 3.975)
+    # the least quarter row that may still have the two bits, in real entries: each fix_size is an entry rounded up
+    extra = 0 if wide else 2
+    _, h, l = words(helpers, k, 0, 0, extra)
+    full = 60 if not wide else 60 * (1 / k)             # up to |K'| = 1 everywhere
+    assert full * abs(h) * (1 << 28) < 1 << 63
+    assert full * abs(h) * (1 << 28) + 60 * (1 << 28) * (1 << 28) < 1 << 63
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("c", [0.2649, 0.2651, 0.999])
+@pytest.mark.parametrize("how", ["storkm", "one matrix", "cases"])
+def test_products_at_the_largest_sums(c, how):
+    """|K'_ij| = c everywhere and p_j at full scale with the signs of the row: 0.2649 has row sums of 15.894, the most
+    that two more bits are given for, 0.2651 is just beyond, 0.999 the most without.  A sum beyond 63 bits would be
+    off by 2^64 units.  Bound as in test_products_against_extended_precision; sqrt(K_ii) max sqrt(K_jj) |p_j| is c."""
+    rng = np.random.default_rng(17)
+    sign = rng.choice([-1.0, 1.0], 60)
+    f = 1.0 - 1e-7 * rng.random((60, 60))
+    km = c * sign[:, None] * sign[None, :] * np.minimum(f, f.T)
+    g_num, g_coord, nn = P.mesh_cube(1, 1, 1)
+    g_g = np.zeros((1, 60), np.int32)
+    for a in range(20):
+        g_g[0, 3 * a:3 * a + 3] = 3 * (g_num[0, a] - 1) + np.arange(1, 4)
+    p = np.zeros(60)
+    p[g_g[0] - 1] = sign * (1.0 - 1e-9 * rng.random(60))
+    with P.Solver() as s:
+        s.setup(g_num, g_g, g_coord, nn, 60)
+        if how == "one matrix":
+            s.set_shared_km(km)
+        else:
+            s.set_storkm(km[None])
+        u = s.ebe_matvec_multi(np.repeat(p[:, None], 8, axis=1), 64)[:, 3] if how == "cases" else s.ebe_matvec(p, 64)
+    ref, mag, big = reference(km[None], g_g, p)
+    assert np.abs(ref).min() > 59.9 * c
+    assert np.all(np.abs(u - ref) <= 2.0 ** -47 * big + 2.0 ** -49 * mag)
