@@ -166,7 +166,10 @@ int pf_element_stresses(void **ctx, const double *xnew, const int *first, const 
 /* The autotuner's choice for the packed-symmetric FP32 element kernel, made
  * at pf_form_storkm / pf_set_storkm by timing every configuration on this
  * mesh: warps per CTA, shared-memory stages per warp, and the measured
- * milliseconds per launch of the configurations (14,2), (12,2), (8,3). */
+ * milliseconds per launch of the configurations (14,2), (12,2), (8,3).
+ * pf_ebe_matvec and solves of more than about 4,046,000 freedoms use it.
+ * Resident runs have a form of their own, and solves in between run (14,2)
+ * unless pf_set_tuning forces another. */
 int pf_tuning(void **ctx, int *warps, int *stages, float *ms);
 
 /* The same for the packed FP16 element kernel (PF_MODE_MIXED16, pf_ebe_matvec
@@ -192,11 +195,14 @@ int pf_set_graphs(void **ctx, const int *on);
  * products included, up to 32 per launch.  *on == 0, the default, launches
  * the separate scatter, update and finish kernels, replayed from CUDA graphs,
  * which measure faster on GB300.  Both give bitwise the same iterates.
- * Applies to 20-node contexts; 8-node contexts always use the separate
- * kernels.  20-node meshes of up to about 4,046,000 freedoms (on 152 SMs)
- * always run one cooperative kernel behind the element products, and those
- * of up to about 311,000 (other than mixed solves of one shared km) whole
- * runs in one resident kernel: this switch makes no difference to them. */
+ * Applies to 20-node contexts.  Meshes of up to about 4,046,000 freedoms (on
+ * 152 SMs; 8-node ones of 30,000 and more) run one cooperative kernel behind
+ * the products, and 20-node ones of up to about 311,000 (other than mixed
+ * solves of one shared km) whole runs in one resident kernel: this switch
+ * makes no difference to them.  Where the device refuses a launch on all of
+ * its SMs, they take the separate kernels.  A resident run holds its SMs (half
+ * of them on the smallest meshes) until it ends: other work on the device,
+ * solves of other contexts included, waits. */
 int pf_set_persistent(void **ctx, const int *on);
 
 /* Self-check of the error path of the bulk-copy element kernels (no

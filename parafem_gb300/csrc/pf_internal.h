@@ -59,10 +59,13 @@ enum { STOP_CHECON = 0, STOP_RELRES = 1 };
 // 40 scatter blocks cost 20 % at 80^3).
 constexpr int kVecBlocks = 6, kScatterBlocks = 12;
 constexpr int kRowBlocks = 64;   // of the 8-node scalar product: rows are short, blocks are handed out as SMs free up
-// Most slots of a mesh whose iterations use programmatic dependent launches:
-// they save 1.5 to 3 us of an iteration (10^3 elements: 24.0 -> 22.0 us FP64,
-// 26.5 -> 23.6 mixed; 20^3: 47 -> 45, 34 -> 31), nothing measurable of the
-// 113 us at 40^3, and lose 0.5 % at 80^3.
+// Most slots of a mesh whose iterations use programmatic dependent launches.
+// What is left of them are the kernels of 8-node meshes (us per iteration with
+// / without: p123 8^3 16.3/17.7, 15^3 16.5/18.3, 29^3 18.5/19.5; elasticity
+// 10^3 22.7/24.2, 20^3 32.5/33.8), the product before the tail with one
+// element matrix (6^3 28.8/29.4, 28^3 28.8/29.1).  From 311,296 slots on, where
+// other products stand before the tail, nothing is measurable (31^3 with one
+// matrix 31.2/31.3, FP64 100.4/100.5): the line is not a sharp one.
 constexpr int kDependentSlots = 500000;
 constexpr int kPersistSlots = 8;   // persistent-kernel instantiations, one barrier counter and grid each
 constexpr int kTailBar = 6;         // the counter of the iteration tail (the persistent kernel's use 0 to 5)
