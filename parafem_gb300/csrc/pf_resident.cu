@@ -468,17 +468,21 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(ResArgs a)
 // The kernel holds its SMs for the whole run, so that runs of other contexts
 // wait for it.  Meshes whose products lose nothing by it take half the SMs,
 // and two such runs go side by side: those of at most so many elements per
-// CTA, in FP64 three (they share the SM's integer pipe), in FP32 one per
-// product warp, in FP16 seven.  Solves per second of one context / of eight in
-// threads, all SMs, half of them, and the separate kernels (no resident runs):
-//            6^3 FP64   8^3 FP64   6^3 FP32   10^3 FP32  12^3 FP32  8^3 FP16   10^3 FP16
-//   all      700/716    555/565    455/612    296/356    240/288    396/510    337/407
-//   half     706/1432   513/1044   467/1250   295/681    211/481    399/996    324/766
-//   separate 244/1333   195/789    170/876    136/508    120/365    157/785    114/494
-// (the number of CTAs must not depend on what else runs: it orders the sums).
+// CTA, in FP64 three (they share the SM's integer pipe), in FP32 ten, in FP16
+// seven.  us per iteration on all SMs / on half (one context's spread by where
+// its counter lies is 4 %, but these are of the same contexts):
+//            6^3          4 x 8 x 7    7^3          8^3          9^3          10^3
+//   FP64     11.1/10.5    11.0/10.4    11.5/11.5    10.6/11.6    11.3/12.4    11.5/13.6
+//   FP32     13.0/12.5    12.5/11.6    12.6/12.9    12.7/12.4    12.5/12.5    12.9/13.1
+//   FP16     12.7/12.2    12.2/11.4    12.5/12.2    11.7/11.7    11.5/11.7    11.6/12.1
+// and solves per second of eight contexts in threads, all / half / the separate
+// kernels that have no such runs: 6^3 FP64 716/1432/1333, FP32 612/1250/876,
+// 9^3 FP32 413/798/669, 8^3 FP16 510/996/785; where all SMs are kept, 8^3 FP64
+// 565/1044/789, 10^3 FP32 356/681/508, FP16 407/766/494.
+// (The number of CTAs must not depend on what else runs: it orders the sums.)
 static int resident_ctas(const Ctx &c, int prec)
 {
-    const int half = c.nsm / 2, per = prec == PREC_FP64 ? 3 : prec == PREC_FP32_SYM ? Shape<32>::W : 7;
+    const int half = c.nsm / 2, per = prec == PREC_FP64 ? 3 : prec == PREC_FP32_SYM ? 10 : 7;
     return half > 0 && c.nels <= per * half ? half : c.nsm;
 }
 static int slots_per_block(const Ctx &c, int ctas) { return (c.nslots + ctas - 1) / ctas; }

@@ -107,7 +107,7 @@ def test_a_negative_tolerance_is_never_met(mode):
 def test_contexts_in_threads_leave_each_other_alone():
     """Resident runs of half the SMs side by side, of all of them one after the other, and iterations with the tail
     and products in between: every solve bitwise as alone."""
-    jobs = [((3, 3, 3), P.MODE_P121), ((6, 6, 6), P.MODE_P121), ((6, 6, 6), P.MODE_MIXED), ((10, 10, 10), P.MODE_MIXED16),
+    jobs = [((3, 3, 3), P.MODE_P121), ((6, 6, 6), P.MODE_P121), ((6, 6, 6), P.MODE_MIXED), ((8, 8, 8), P.MODE_MIXED16),
             ((12, 11, 10), P.MODE_P121), ((30, 28, 29), P.MODE_MIXED)]
     probs = [P.cube_problem(*shape) for shape, _ in jobs]
     solvers = [solver(prob) for prob in probs]

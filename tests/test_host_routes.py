@@ -246,7 +246,7 @@ def test_iterations_are_timed_with_the_kernels_of_a_solve(fake, n, prec, mode):
     s.close()
 
 
-@pytest.mark.parametrize("n,mode,blocks", [(6, P.MODE_P121, 76), (7, P.MODE_P121, 152), (10, P.MODE_MIXED, 76), (11, P.MODE_MIXED, 152),
+@pytest.mark.parametrize("n,mode,blocks", [(6, P.MODE_P121, 76), (7, P.MODE_P121, 152), (9, P.MODE_MIXED, 76), (10, P.MODE_MIXED, 152),
                                            (8, P.MODE_MIXED16, 76), (9, P.MODE_MIXED16, 152)])
 def test_the_smallest_runs_take_half_the_sms(fake, n, mode, blocks):
     """Two of them go side by side (the stand-in has 152 SMs)."""
